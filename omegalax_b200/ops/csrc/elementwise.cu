@@ -591,10 +591,11 @@ __global__ void ce_fwd_bwd_kernel(bf16* __restrict__ logits, long long ld, int V
 // logit per row): one warp per row.  lse_out feeds the gradient pass over the bf16 logits.
 __global__ void ce_finish_kernel(const float2* __restrict__ stats, int n_tiles, const float* __restrict__ tgt_logit,
                                  const float* __restrict__ mask, float* __restrict__ loss_sum,
-                                 float* __restrict__ lse_out, long long R) {
+                                 float* __restrict__ lse_out, long long R, const int* __restrict__ rows_dev,
+                                 int rows_off) {
   const long long row = (blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
-  if (row >= R) return;
+  if (row >= R || (rows_dev && row >= __ldg(rows_dev) - rows_off)) return;
   const float2* sp = stats + row * n_tiles;
   float mx = -INFINITY, sm = 0.f;
   for (int i = lane; i < n_tiles; i += 32) {
@@ -682,6 +683,112 @@ __global__ void ce_vp_grad_kernel(bf16* __restrict__ logits, long long ld, int V
     }
     o.x = ou[0]; o.y = ou[1]; o.z = ou[2]; o.w = ou[3];
     ov[i] = o;
+  }
+}
+
+// Supervised rows only.  A conversation's prompt and padding carry no loss, and a row without loss needs
+// none of the head's three products, so the rows with a mask other than zero are numbered here, in order,
+// and gathered.  One CTA: the scan is serial over tiles of 1024 rows (1.5 us each), next to products of
+// milliseconds.  rows[c] is the row of number c (-1 past the count), place[row] its number or -1.
+__global__ void __launch_bounds__(1024) ce_count_kernel(const float* __restrict__ mask, const int* __restrict__ targets,
+                                                        long long M, int* __restrict__ rows, int* __restrict__ place,
+                                                        int* __restrict__ tgt_out, float* __restrict__ mask_out,
+                                                        int* __restrict__ count) {
+  __shared__ int part[32];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  int base = 0;
+  for (long long r0 = 0; r0 < M; r0 += 1024) {
+    const long long r = r0 + threadIdx.x;
+    const float mk = r < M ? mask[r] : 0.f;
+    const bool on = mk != 0.f;
+    const unsigned votes = __ballot_sync(0xffffffffu, on);
+    if (lane == 0) part[warp] = __popc(votes);
+    __syncthreads();
+    int before = base, total = 0;
+    for (int w = 0; w < 32; ++w) {
+      if (w < warp) before += part[w];
+      total += part[w];
+    }
+    const int c = before + __popc(votes & ((1u << lane) - 1));
+    if (r < M) place[r] = on ? c : -1;
+    if (on) {
+      rows[c] = (int)r;
+      tgt_out[c] = targets[r];
+      mask_out[c] = mk;
+    }
+    base += total;
+    __syncthreads();
+  }
+  if (threadIdx.x == 0) *count = base;
+  for (long long c = base + threadIdx.x; c < M; c += 1024) {
+    rows[c] = -1;
+    tgt_out[c] = -1;
+    mask_out[c] = 0.f;
+  }
+}
+
+// Hidden rows in that order; the reduction of the weight gradient runs in blocks of 64 rows, so the rows
+// after the last one are zeroed that far.
+__global__ void ce_gather_kernel(const bf16* __restrict__ h, const int* __restrict__ rows, const int* __restrict__ count,
+                                 bf16* __restrict__ out, long long M, int D) {
+  const int dv = D >> 3;
+  const long long n = *count, end = min((n + 63) / 64 * 64, M);
+  for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < end * dv; t += (long long)gridDim.x * blockDim.x) {
+    const long long c = t / dv;
+    const int i = (int)(t - c * dv);
+    reinterpret_cast<uint4*>(out + c * D)[i] =
+        c < n ? reinterpret_cast<const uint4*>(h + (long long)rows[c] * D)[i] : make_uint4(0, 0, 0, 0);
+  }
+}
+
+// Gradient rows back in their places, times the upstream gradient; zero where there was no loss.
+__global__ void ce_scatter_kernel(const float* __restrict__ dh, const int* __restrict__ place, const float* __restrict__ g,
+                                  bf16* __restrict__ out, long long M, int D) {
+  const int dv = D >> 3;
+  const float gs = *g;
+  for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < M * dv; t += (long long)gridDim.x * blockDim.x) {
+    const long long r = t / dv;
+    const int i = (int)(t - r * dv);
+    const int c = place[r];
+    uint4 o = make_uint4(0, 0, 0, 0);
+    if (c >= 0) {
+      const float4* s = reinterpret_cast<const float4*>(dh + (long long)c * D) + 2 * i;
+      const float4 a = s[0], b = s[1];
+      o.x = pack_bf16(a.x * gs, a.y * gs); o.y = pack_bf16(a.z * gs, a.w * gs);
+      o.z = pack_bf16(b.x * gs, b.y * gs); o.w = pack_bf16(b.z * gs, b.w * gs);
+    }
+    reinterpret_cast<uint4*>(out + r * D)[i] = o;
+  }
+}
+
+// ce_vp_grad_kernel over counted rows: logits -> dlogits in place, zeros up to the next multiple of 64 rows.
+__global__ void ce_counted_grad_kernel(bf16* __restrict__ logits, long long ld, int V, const int* __restrict__ targets,
+                                       const float* __restrict__ lse_in, const float* __restrict__ mask,
+                                       const float* __restrict__ grad_scale, const int* __restrict__ rows_dev, int rows_off) {
+  const int row = blockIdx.x, n = __ldg(rows_dev) - rows_off;
+  if (row >= (n + 63) / 64 * 64 || n <= 0) return;
+  uint4* ov = reinterpret_cast<uint4*>(logits + (long long)row * ld);
+  const int nv = V >> 3;
+  if (row >= n) {
+    for (int i = threadIdx.x; i < nv; i += blockDim.x) ov[i] = make_uint4(0, 0, 0, 0);
+    return;
+  }
+  const int tgt = targets[row];
+  const float lse = lse_in[row];
+  const float gs = mask[row] * *grad_scale;
+  for (int i = threadIdx.x; i < nv; i += blockDim.x) {
+    const uint4 q = ov[i];
+    const uint32_t u[4] = {q.x, q.y, q.z, q.w};
+    uint32_t o[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const float2 t = unpack_bf16(u[j]);
+      const int c0 = i * 8 + 2 * j;
+      const float p0 = __expf(t.x - lse) - (c0 == tgt ? 1.f : 0.f);
+      const float p1 = __expf(t.y - lse) - (c0 + 1 == tgt ? 1.f : 0.f);
+      o[j] = pack_bf16(p0 * gs, p1 * gs);
+    }
+    ov[i] = make_uint4(o[0], o[1], o[2], o[3]);
   }
 }
 
@@ -1016,10 +1123,42 @@ int ob_sigmoid_gate_bwd(const void* o, const void* gate, const void* dout, void*
 }
 
 int ob_ce_finish(const void* stats, int n_tiles, const float* tgt_logit, const float* mask, float* loss_sum,
-                 float* lse_out, long long R, cudaStream_t s) {
+                 float* lse_out, long long R, const int* rows_dev, int rows_off, cudaStream_t s) {
   if (R <= 0) return 0;
   ce_finish_kernel<<<grid_for(R * 32, 256), 256, 0, s>>>((const float2*)stats, n_tiles, tgt_logit, mask, loss_sum,
-                                                         lse_out, R);
+                                                         lse_out, R, rows_dev, rows_off);
+  OB_CHECK_LAUNCH();
+  return 0;
+}
+
+int ob_ce_count(const float* mask, const int* targets, long long M, int* rows, int* place, int* tgt_out, float* mask_out,
+                int* count, cudaStream_t s) {
+  ce_count_kernel<<<1, 1024, 0, s>>>(mask, targets, M, rows, place, tgt_out, mask_out, count);
+  OB_CHECK_LAUNCH();
+  return 0;
+}
+
+int ob_ce_gather(const void* h, const int* rows, const int* count, void* out, long long M, int D, cudaStream_t s) {
+  if (D % 8) return 6001;
+  if (M <= 0) return 0;
+  ce_gather_kernel<<<grid_for(M * (D / 8), 256), 256, 0, s>>>((const bf16*)h, rows, count, (bf16*)out, M, D);
+  OB_CHECK_LAUNCH();
+  return 0;
+}
+
+int ob_ce_scatter(const float* dh, const int* place, const float* g, void* out, long long M, int D, cudaStream_t s) {
+  if (D % 8) return 6001;
+  if (M <= 0) return 0;
+  ce_scatter_kernel<<<grid_for(M * (D / 8), 256), 256, 0, s>>>(dh, place, g, (bf16*)out, M, D);
+  OB_CHECK_LAUNCH();
+  return 0;
+}
+
+int ob_ce_counted_grad(void* logits, long long R, int V, long long ld, const int* targets, const float* lse, const float* mask,
+                       const float* grad_scale, const int* rows_dev, int rows_off, cudaStream_t s) {
+  if (V % 8 || ld % 8) return 6001;
+  if (R <= 0) return 0;
+  ce_counted_grad_kernel<<<(unsigned)R, 512, 0, s>>>((bf16*)logits, ld, V, targets, lse, mask, grad_scale, rows_dev, rows_off);
   OB_CHECK_LAUNCH();
   return 0;
 }

@@ -58,6 +58,10 @@ struct GemmArgs {
   // slices of k_per_split elements; every (tile, slice) is one unit of work and its partial result
   // is added to C with vector reductions.
   int raster_gm, k_splits, k_per_split;
+  // 512 x 256 tile kernel: with rows_dev, only the first *rows_dev - rows_off rows hold anything.  They are
+  // rows of C (rows_in_k 0) or the reduction (rows_in_k 1); the reduction is then cut on the device.
+  const int* rows_dev;
+  int rows_off, rows_in_k;
   int* status;
 };
 

@@ -507,6 +507,28 @@ int ob_gemm_bf16_pair(const void* A, const void* B, void* C, const void* residua
   return launch_pair<true, false>(A, B, g, a_rows, a_cols, lda, b_rows, b_cols, ldb, stream);
 }
 
+// The three products of the fused linear + cross-entropy over rows that the device counted: the first
+// n = *rows_dev - rows_off of the `rows` rows given here hold anything.
+//   kind 0  C bf16 [rows, N] = A [rows, K] B [N, K]^T, with the softmax statistics of ob_gemm_bf16_pair
+//   kind 1  C fp32 [rows, N] += A [rows, K] B [K, N]          (rows at and after n receive unspecified values)
+//   kind 2  C fp32 [M, N] += A [rows, M]^T B [rows, N]        (rows n .. next multiple of 64 hold zeros)
+// Here M / N / K are those of C and of the reduction; `rows` is M (kinds 0, 1) or K (kind 2).
+int ob_gemm_counted_rows(int kind, const void* A, const void* B, void* C, int M, int N, int K, long long lda,
+                         long long ldb, long long ldc, const int* rows_dev, int rows_off, const int* ce_targets,
+                         void* ce_stats, float* ce_tgt, int* status, cudaStream_t stream) {
+  if (M <= 0 || N <= 0 || K <= 0) return 0;
+  if ((lda & 7) || (ldb & 7)) return 6001;
+  if ((((uintptr_t)A) & 15) || (((uintptr_t)B) & 15)) return 6002;
+  if (kind < 0 || kind > 2 || rows_dev == nullptr || (kind == 0) != (ce_stats != nullptr)) return 6005;
+  GemmArgs g = {};
+  g.M = M; g.N = N; g.K = K; g.mode = 0;
+  g.C = C; g.ldc = ldc; g.out_mode = kind == 0 ? 0 : 2;
+  g.ce_targets = ce_targets; g.ce_stats = (float2*)ce_stats; g.ce_tgt = ce_tgt;
+  g.rows_dev = rows_dev; g.rows_off = rows_off; g.rows_in_k = kind == 2;
+  g.status = status;
+  return launch_pair_wide(A, B, g, lda, ldb, kind == 2, kind != 0, pick_gm(2 * K), 0, stream);
+}
+
 // Same contract as ob_gemm_bf16_peer_reduce (fp32 result rows added into the owning GPUs' buffers
 // with vector reductions over NVLink), computed by CTA pairs.
 // bf16_out: 0 fp32 reduction, 1 bf16 reduction, 2 + s = bf16 store into slab s of the owner's staging

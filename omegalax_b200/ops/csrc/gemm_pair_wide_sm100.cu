@@ -49,12 +49,44 @@ struct WideTile {
   int cols_valid;
 };
 
-__device__ __forceinline__ WideTile wide_tile(const GemmArgs& p, int t, int rank) {
+// What a launch works on: everything, or the rows that the device counted.
+struct WideWork {
+  int K, num_m_blocks, total_tiles, k_splits, k_per_split;
+};
+
+__device__ __forceinline__ WideWork wide_work(const GemmArgs& p, int pairs) {
+  WideWork w = {p.K, p.num_m_blocks, p.total_tiles, p.k_splits, p.k_per_split};
+  if (p.rows_dev == nullptr) return w;
+  const int n = min(max(__ldg(p.rows_dev) - p.rows_off, 0), p.rows_in_k ? p.K : p.M);
+  if (p.rows_in_k) w.K = n;
+  else w.num_m_blocks = (n + 511) / 512;
+  w.total_tiles = n > 0 ? w.num_m_blocks * p.num_n_blocks : 0;
+  const int kb = (w.K + BK - 1) / BK;
+  w.k_splits = 1;
+  w.k_per_split = kb * BK;
+  if (p.out_mode != 2) return w;
+  // Slices of the reduction: fewest k-blocks on the longest path, where emptying a tile costs as much as
+  // about eight k-blocks (512 x 256 fp32 through the TMA unit: 4 us) and a slice has at least sixteen.
+  int best = 0x7fffffff;
+  for (int s = 1; s <= 32; ++s) {
+    const int per = (kb + s - 1) / s;
+    if (s > 1 && per < 16) break;
+    const int cost = ((w.total_tiles * ((kb + per - 1) / per) + pairs - 1) / pairs) * (per + 8);
+    if (cost < best) {
+      best = cost;
+      w.k_per_split = per * BK;
+      w.k_splits = (kb + per - 1) / per;
+    }
+  }
+  return w;
+}
+
+__device__ __forceinline__ WideTile wide_tile(const GemmArgs& p, int num_m_blocks, int t, int rank) {
   const int GM = p.raster_gm;
   const int per_group = GM * p.num_n_blocks;
   const int g = t / per_group;
   const int first_m = g * GM;
-  const int gm = min(GM, p.num_m_blocks - first_m);
+  const int gm = min(GM, num_m_blocks - first_m);
   const int r = t - g * per_group;
   const int mb = first_m + (r % gm);
   const int nb = r / gm;
@@ -90,7 +122,8 @@ gemm_bf16_pair_wide_kernel(const __grid_constant__ CUtensorMap tmA, const __grid
   const bool leader = rank == 0;
   const int pair0 = (int)(blockIdx.x >> 1);
   const int pair_step = (int)(gridDim.x >> 1);
-  const int total_units = p.total_tiles * p.k_splits;
+  const WideWork wk = wide_work(p, pair_step);
+  const int total_units = wk.total_tiles * wk.k_splits;
 
   if (threadIdx.x == 0) {
     for (int i = 0; i < kWideStages; ++i) {
@@ -121,11 +154,11 @@ gemm_bf16_pair_wide_kernel(const __grid_constant__ CUtensorMap tmA, const __grid
       uint32_t phase = 0;
       bool ok = true;
       for (int u = pair0; u < total_units && ok; u += pair_step) {
-        const int ks = u / p.total_tiles;        // slice-major: a wave of units shares operand panels
-        const int t = u - ks * p.total_tiles;
-        const int k_begin = ks * p.k_per_split;
-        const int k_end = min(p.K, k_begin + p.k_per_split);
-        const WideTile ti = wide_tile(p, t, rank);
+        const int ks = u / wk.total_tiles;        // slice-major: a wave of units shares operand panels
+        const int t = u - ks * wk.total_tiles;
+        const int k_begin = ks * wk.k_per_split;
+        const int k_end = min(wk.K, k_begin + wk.k_per_split);
+        const WideTile ti = wide_tile(p, wk.num_m_blocks, t, rank);
         for (int k0 = k_begin; k0 < k_end; k0 += BK) {
           ok = mbar_wait(&empty_bar[stage], phase ^ 1, abort_flag, p.status, OB_ERR_WAIT_EMPTY);
           if (!ok) break;
@@ -162,9 +195,9 @@ gemm_bf16_pair_wide_kernel(const __grid_constant__ CUtensorMap tmA, const __grid
       uint32_t tile_phase = 0;
       bool ok = true;
       for (int u = pair0; u < total_units && ok; u += pair_step) {
-        const int ks = u / p.total_tiles;
-        const int k_begin = ks * p.k_per_split;
-        const int k_end = min(p.K, k_begin + p.k_per_split);
+        const int ks = u / wk.total_tiles;
+        const int k_begin = ks * wk.k_per_split;
+        const int k_end = min(wk.K, k_begin + wk.k_per_split);
         uint32_t accumulate = 0;
         for (int k0 = k_begin; k0 < k_end && ok; k0 += BK) {
           ok = mbar_wait(&full_bar[stage], phase, abort_flag, p.status, OB_ERR_WAIT_FULL);
@@ -218,10 +251,10 @@ gemm_bf16_pair_wide_kernel(const __grid_constant__ CUtensorMap tmA, const __grid
     uint32_t tile_phase = 0;
     bool ok = true;
     for (int u = pair0; u < total_units && ok; u += pair_step) {
-      const int ks = u / p.total_tiles;
-      const int t = u - ks * p.total_tiles;
-      const bool empty_k = min(p.K, ks * p.k_per_split + p.k_per_split) <= ks * p.k_per_split;
-      const WideTile ti = wide_tile(p, t, rank);
+      const int ks = u / wk.total_tiles;
+      const int t = u - ks * wk.total_tiles;
+      const bool empty_k = min(wk.K, ks * wk.k_per_split + wk.k_per_split) <= ks * wk.k_per_split;
+      const WideTile ti = wide_tile(p, wk.num_m_blocks, t, rank);
       ok = mbar_wait(&tfull_bar[0], tile_phase, abort_flag, p.status, OB_ERR_WAIT_TMEM_FULL);
       if (!ok) break;
       tc_fence_after();
@@ -447,7 +480,9 @@ static int launch_wide(const void* A, const void* B, GemmArgs args, long long a_
   // reduction slices (reducing output modes only): fewest that fill the last wave to 95 %
   args.k_splits = 1;
   args.k_per_split = args.K > 0 ? ((args.K + BK - 1) / BK) * BK : BK;
-  if (args.out_mode >= 2 && args.out_mode <= 4 && args.K >= 2048 && forced_splits != 0) {
+  if (args.rows_dev != nullptr) {
+    args.k_splits = 2;   // the device decides; stores that bypass the TMA unit have to be reductions
+  } else if (args.out_mode >= 2 && args.out_mode <= 4 && args.K >= 2048 && forced_splits != 0) {
     const int kblocks = (args.K + BK - 1) / BK;
     int best = 1;
     double best_eff = 0.0;
@@ -465,8 +500,8 @@ static int launch_wide(const void* A, const void* B, GemmArgs args, long long a_
     args.k_per_split = per * BK;
     args.k_splits = (kblocks + per - 1) / per;
   }
-  if (pairs > args.total_tiles * args.k_splits) pairs = args.total_tiles * args.k_splits;
-  if (pairs <= 0) return 0;
+  if (args.rows_dev == nullptr && pairs > args.total_tiles * args.k_splits) pairs = args.total_tiles * args.k_splits;
+  if (pairs <= 0 || args.total_tiles <= 0) return 0;
   if (args.ce_stats != nullptr && !(tma_out && args.out_mode == 0)) return 6008;   // statistics live in the TMA bf16 epilogue
   kern<<<2 * pairs, kGemmThreads, WideSmem::kTotal, stream>>>(tmA, tmB, tmC, args, tma_out);
   OB_CHECK_LAUNCH();

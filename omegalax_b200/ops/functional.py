@@ -632,7 +632,8 @@ class _LinearCEFn(torch.autograd.Function):
     of exponentials per 256-column tile, the target's logit) in its epilogue, so the loss and the
     log-sum-exp are those of fp32 logits, as in the reference (omegalax/trainers/loss.py:24-35); the
     bf16 copy of the chunk's logits that it also writes is turned into dlogits in place and feeds
-    the dH and dW GEMMs of the same sweep.  No [B,T,V] tensor exists and the backward only
+    the dH and dW GEMMs of the same sweep.  Only rows with a nonzero mask take part: they are numbered
+    on the device, and the products read the count there.  No [B,T,V] tensor exists and the backward only
     rescales; dW goes straight into ``w.main_grad`` when it exists.  (Keeping dlogits out of
     memory altogether would need the [chunk, D] dH accumulator in TMEM, 4096 columns against the
     512 there are, or a third pass of the logits GEMM, which costs more than the traffic saved.)
@@ -647,7 +648,6 @@ class _LinearCEFn(torch.autograd.Function):
         need_grad = h.requires_grad or w.requires_grad
         mg = getattr(w, "main_grad", None)
         pg = getattr(w, "peer_grad", None)
-        dh = torch.empty_like(h) if need_grad else None
         dw = None
         if need_grad and w.requires_grad and pg is None:
             dw = mg if mg is not None else torch.zeros(V, D, dtype=torch.float32, device=dev)
@@ -659,6 +659,29 @@ class _LinearCEFn(torch.autograd.Function):
         tgt_logit = torch.zeros(min(chunk, M), dtype=torch.float32, device=dev)
         lse = torch.empty(min(chunk, M), dtype=torch.float32, device=dev)
         fp32_stats = os.environ.get("OMEGALAX_B200_CE_STATS", "1") == "1" and h.shape[1] % 8 == 0
+        if fp32_stats and pg is None and M > 0:
+            # Rows without loss (prompts, padding) take no part in the head: the others are gathered and counted
+            # on the device.  Chunks past the count return at once, so the chunk bounds need no host copy of it.
+            # (With gradients that leave over NVLink the whole rows go on: that GEMM takes no count.)
+            w = K._row_major_2d(w)
+            count, rows, place, t32, mk = K.ce_supervised(mk, t32)
+            h = K.ce_gather(h, rows, count)
+            dh = torch.zeros(M, D, dtype=torch.float32, device=dev) if need_grad else None
+            for r0 in range(0, M, chunk):
+                r1 = min(M, r0 + chunk)
+                n, at = r1 - r0, (count, r0)
+                K.gemm_counted(0, h[r0:r1], w, logits[:n], at, ce=(t32[r0:r1], stats[:n], tgt_logit[:n]))
+                K.ce_finish(stats[:n], tgt_logit[:n], mk[r0:r1], loss_sum, lse[:n], at)
+                if need_grad:
+                    K.ce_counted_grad_(logits[:n], t32[r0:r1], lse[:n], mk[r0:r1], scale_t, at)
+                    K.gemm_counted(1, logits[:n], w, dh[r0:r1], at)
+                    if dw is not None:
+                        K.gemm_counted(2, logits[:n], h[r0:r1], dw, at)
+            ctx.save_for_backward(dh, place)
+            ctx.counted, ctx.dw, ctx.w_dtype = True, None if mg is not None else dw, w.dtype
+            return (loss_sum * scale_t).squeeze(0)
+        ctx.counted = False
+        dh = torch.empty_like(h) if need_grad else None
         for r0 in range(0, M, chunk):
             r1 = min(M, r0 + chunk)
             lg = logits[: r1 - r0]
@@ -685,9 +708,13 @@ class _LinearCEFn(torch.autograd.Function):
 
     @staticmethod
     def backward(ctx, g):
-        (dh,) = ctx.saved_tensors
-        dw = ctx.dw
-        gh = None if dh is None else (dh * g.to(dh.dtype))
+        dh, dw = ctx.saved_tensors[0], ctx.dw
+        if dh is None:
+            gh = None
+        elif ctx.counted:
+            gh = K.ce_scatter(dh, ctx.saved_tensors[1], g.to(torch.float32).contiguous())
+        else:
+            gh = dh * g.to(dh.dtype)
         gw = None if dw is None else (dw * g).to(ctx.w_dtype)
         return gh, gw, None, None, None, None
 

@@ -374,11 +374,64 @@ def sigmoid_gate_bwd(o, gate, dout):
     return d_o, d_gate
 
 
-def ce_finish(stats, tgt_logit, mask, loss_sum, lse_out):
-    """Row log-sum-exp and masked loss from the statistics the logits GEMM wrote (``gemm(..., ce=)``)."""
+def ce_finish(stats, tgt_logit, mask, loss_sum, lse_out, counted=(None, 0)):
+    """Row log-sum-exp and masked loss from the statistics the logits GEMM wrote (``gemm(..., ce=)``).
+    ``counted`` as in ``gemm_counted``."""
     R, n_tiles = stats.shape[0], stats.shape[1]
     _call("ob_ce_finish", stats.data_ptr(), n_tiles, tgt_logit.data_ptr(), lib.ptr(mask), loss_sum.data_ptr(),
-          lse_out.data_ptr(), R, lib.stream_ptr())
+          lse_out.data_ptr(), R, lib.ptr(counted[0]), counted[1], lib.stream_ptr())
+
+
+def ce_supervised(mask, targets):
+    """Rows with a nonzero mask, in order: (count int32 [1], rows [M] of every number, place [M] of every
+    row or -1, their targets, their mask)."""
+    M, dev = mask.numel(), mask.device
+    rows, place, tgt = torch.empty(3, M, dtype=torch.int32, device=dev).unbind(0)
+    mk = torch.empty(M, dtype=torch.float32, device=dev)
+    count = torch.empty(1, dtype=torch.int32, device=dev)
+    _call("ob_ce_count", mask.data_ptr(), targets.data_ptr(), M, rows.data_ptr(), place.data_ptr(), tgt.data_ptr(), mk.data_ptr(),
+          count.data_ptr(), lib.stream_ptr())
+    return count, rows, place, tgt, mk
+
+
+def ce_gather(h, rows, count):
+    """The counted rows of h [M, D] first; what follows their next multiple of 64 stays unwritten."""
+    out = torch.empty_like(h)
+    _call("ob_ce_gather", h.data_ptr(), rows.data_ptr(), count.data_ptr(), out.data_ptr(), h.shape[0], h.shape[1],
+          lib.stream_ptr())
+    return out
+
+
+def ce_scatter(dh, place, g):
+    """bf16 rows: g times row ``place`` of fp32 ``dh``, or zero."""
+    out = torch.empty(dh.shape, dtype=bf16, device=dh.device)
+    _call("ob_ce_scatter", dh.data_ptr(), place.data_ptr(), g.data_ptr(), out.data_ptr(), dh.shape[0], dh.shape[1],
+          lib.stream_ptr())
+    return out
+
+
+def ce_counted_grad_(logits, targets, lse, mask, grad_scale, counted):
+    """Logits -> dlogits in place for the counted rows, zeros up to their next multiple of 64."""
+    R, V = logits.shape
+    _call("ob_ce_counted_grad", logits.data_ptr(), R, V, logits.stride(0), targets.data_ptr(), lse.data_ptr(), mask.data_ptr(),
+          grad_scale.data_ptr(), counted[0].data_ptr(), counted[1], lib.stream_ptr())
+
+
+def gemm_counted(kind: int, a, b, out, counted, ce=None):
+    """The head's products when only the first ``counted[0]`` (int32 [1] on the device) - ``counted[1]`` rows
+    of ``a`` hold anything.  kind 0: out bf16 = a b^T with the statistics ``ce``; kind 1: out fp32 += a b;
+    kind 2: out fp32 += a^T b."""
+    (M, K) = (a.shape[1], a.shape[0]) if kind == 2 else a.shape
+    N = b.shape[1] if kind else b.shape[0]
+    ce_ptrs = (None, None, None) if ce is None else (ce[0].data_ptr(), ce[1].data_ptr(), ce[2].data_ptr())
+    if b.shape[0 if kind else 1] != K or out.shape != (M, N) or out.dtype != (torch.float32 if kind else bf16):
+        raise ValueError("operands or output do not fit")
+    for t in (a, b, out):
+        if t.stride(1) != 1:
+            raise ValueError("row-major operands expected")
+    _call("ob_gemm_counted_rows", kind, a.data_ptr(), b.data_ptr(), out.data_ptr(), M, N, K, a.stride(0), b.stride(0), out.stride(0),
+          counted[0].data_ptr(), counted[1], *ce_ptrs, lib.status_tensor(a.device).data_ptr(), lib.stream_ptr())
+    return out
 
 
 def embedding_fwd(ids, table):

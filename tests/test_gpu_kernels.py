@@ -480,6 +480,40 @@ def test_linear_cross_entropy():
     assert _rel_err(w.grad, wr.grad) < 3e-2
 
 
+@pytest.mark.parametrize("M,n,chunk", [(1, 1, 64), (70, 0, 64), (700, 1, 256), (700, 63, 256), (700, 64, 256), (700, 257, 256),
+                                       (1100, 1100, 512), (1100, 513, 4096)])
+@pytest.mark.parametrize("main_grad", [False, True])
+def test_linear_cross_entropy_supervised_rows(M, n, chunk, main_grad):
+    """Counts around the 64-row blocks of the weight gradient, the 512-row tiles and the chunks; V and D leave ragged tiles.
+    Tolerances of ``test_linear_cross_entropy``: gradients come from bf16 dlogits."""
+    from omegalax_b200.ops import functional as Fn, lib
+    torch.manual_seed(31)
+    D, V = 264, 2056
+    h = torch.randn(M, D, device=_dev()).to(bf16).requires_grad_(True)
+    w = (torch.randn(V, D, device=_dev()) * 0.1).to(bf16).requires_grad_(True)
+    y = torch.randint(0, V, (M,), device=_dev(), dtype=torch.int32)
+    mask = torch.zeros(M, device=_dev())
+    mask[torch.randperm(M, device=_dev())[:n]] = torch.rand(n, device=_dev()) + 0.5
+    before = torch.randn(V, D, device=_dev()) * 1e-3
+    if main_grad:
+        w.main_grad = before.clone()
+    loss = Fn.linear_cross_entropy(h, w, y, mask, 1.0 / max(n, 1), chunk=chunk)
+    loss.backward()
+    _check(lib)
+    hr, wr = h.detach().double().requires_grad_(True), w.detach().double().requires_grad_(True)
+    nll = torch.nn.functional.cross_entropy(hr @ wr.t(), y.long(), reduction="none")
+    ref = (nll * mask).sum() / max(n, 1)
+    ref.backward()
+    assert abs(float(loss) - float(ref)) <= 1e-5 * abs(float(ref)) + 1e-6
+    assert not h.grad[mask == 0].any() and torch.isfinite(h.grad).all()
+    dw = w.main_grad - before if main_grad else w.grad
+    if n:
+        assert _rel_err(h.grad, hr.grad) < 3e-2
+        assert _rel_err(dw, wr.grad) < 3e-2
+    else:
+        assert not dw.any()
+
+
 def test_embedding_and_optimizer_kernels():
     from omegalax_b200.ops import kernels as Kn, lib
     torch.manual_seed(9)
