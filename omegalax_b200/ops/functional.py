@@ -659,10 +659,11 @@ class _LinearCEFn(torch.autograd.Function):
         tgt_logit = torch.zeros(min(chunk, M), dtype=torch.float32, device=dev)
         lse = torch.empty(min(chunk, M), dtype=torch.float32, device=dev)
         fp32_stats = os.environ.get("OMEGALAX_B200_CE_STATS", "1") == "1" and h.shape[1] % 8 == 0
-        if fp32_stats and pg is None and M > 0:
+        if fp32_stats and pg is None and M >= 2048:
             # Rows without loss (prompts, padding) take no part in the head: the others are gathered and counted
             # on the device.  Chunks past the count return at once, so the chunk bounds need no host copy of it.
-            # (With gradients that leave over NVLink the whole rows go on: that GEMM takes no count.)
+            # (With gradients that leave over NVLink the whole rows go on: that GEMM takes no count.  So do fewer than
+            # 2048 rows: such a step is bound by its launches, and 3 rows of 333 took 6.87 ms, counted 7.12.)
             w = K._row_major_2d(w)
             count, rows, place, t32, mk = K.ce_supervised(mk, t32)
             h = K.ce_gather(h, rows, count)

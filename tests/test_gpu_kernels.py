@@ -480,8 +480,8 @@ def test_linear_cross_entropy():
     assert _rel_err(w.grad, wr.grad) < 3e-2
 
 
-@pytest.mark.parametrize("M,n,chunk", [(1, 1, 64), (70, 0, 64), (700, 1, 256), (700, 63, 256), (700, 64, 256), (700, 257, 256),
-                                       (1100, 1100, 512), (1100, 513, 4096)])
+@pytest.mark.parametrize("M,n,chunk", [(2048, 0, 1024), (2050, 1, 1024), (2050, 63, 1024), (2050, 64, 1024), (2050, 1025, 1024),
+                                       (2112, 2112, 4096), (2500, 1537, 512)])
 @pytest.mark.parametrize("main_grad", [False, True])
 def test_linear_cross_entropy_supervised_rows(M, n, chunk, main_grad):
     """Counts around the 64-row blocks of the weight gradient, the 512-row tiles and the chunks; V and D leave ragged tiles.
