@@ -128,6 +128,13 @@ def _acc_main_grad(w, fn_into, fn_new):
 
 
 # ----------------------------------------------------------------------------- linear
+def _few(w):
+    """Products of few rows are chosen by size when serving.  Weights of a training engine keep the tile kernels: a
+    step that small is bound by its launches (0.6B width, 3 rows of 333: 7.0 ms on the host, 5.5 on the
+    device), and first forward, re-run and other row counts share one order of sums."""
+    return False if hasattr(w, "main_grad") else None
+
+
 class _LinearFn(torch.autograd.Function):
     @staticmethod
     def forward(ctx, x, w, residual, y_pre=None, bias=None):
@@ -138,7 +145,7 @@ class _LinearFn(torch.autograd.Function):
         if y is None and ag is not None and bias is None:   # sharded weight gathered inside this GEMM's launch
             y = ag.run(x2.contiguous(), w, residual)
         if y is None:
-            y = K.gemm(x2, w, residual=residual, bias=bias)   # bias and residual are added in the GEMM epilogue
+            y = K.gemm(x2, w, residual=residual, bias=bias, few=_few(w))   # bias and residual are added in the GEMM epilogue
         ctx.save_for_backward(x2, w)
         ctx.shp = shp
         ctx.has_res = residual is not None
@@ -394,7 +401,7 @@ class _SwiGLULinearFn(torch.autograd.Function):
         g2 = gu.reshape(-1, shp[-1])
         y = y_pre
         if y is None:
-            y = K.gemm(K.swiglu_fwd(g2), w, residual=residual)
+            y = K.gemm(K.swiglu_fwd(g2), w, residual=residual, few=_few(w))
         ctx.save_for_backward(g2, w)
         ctx.shp = shp
         ctx.has_res = residual is not None

@@ -67,9 +67,18 @@ def _use_pair(M: int, N: int, K: int, wgrad: bool = False) -> bool:
     return big and not wgrad and N <= 8192 and K <= 8192
 
 
+def _use_few(M: int, N: int, K: int) -> bool:
+    """The kernel for few rows, where streaming the weights or filling the SMs is the bound.  Up to 128 rows it
+    reads every weight once (N 4096, K 12288: 22 us for one row, 81 on 128 x 128 tiles; N 151936, K 4096: 191,
+    516); above, while its 128 x 128 panels fit the SMs in one wave of two (M 500, N 6144, K 4096: 33 us against
+    51; M 1000, N 6144: 64 against 55, beyond the wave).  Short reductions leave nothing to share out
+    (M 128, N 8192, K 512: 9.9 against 9.5)."""
+    return K > 0 and (M <= 64 or (K >= 768 and (M <= 128 or -(-M // 128) * -(-N // 128) <= 296)))
+
+
 def gemm(a, b, *, a_mn: bool = False, b_mn: bool = False, out=None, out_dtype=bf16,
          accumulate: bool = False, residual=None, bn: int = 0, pair: bool | None = None, bias=None,
-         ce=None):
+         ce=None, few: bool | None = None, splits: int = 0):
     """C = op(A) op(B)^T on the tcgen05 kernel.
 
     a: [M,K] (a_mn False) or [K,M] (a_mn True); b: [N,K] (b_mn False) or [K,N] (b_mn True).
@@ -77,6 +86,8 @@ def gemm(a, b, *, a_mn: bool = False, b_mn: bool = False, out=None, out_dtype=bf
     ``bias`` (bf16 [N]) and ``residual`` (bf16 [M,N]) are added in the epilogue.  ``ce`` =
     (targets int32 [M], stats fp32 [M, ceil(N/256), 2], target_logit fp32 [M]) asks the 512 x 256
     tile kernel for the cross-entropy statistics of the fp32 accumulator (bf16 output only).
+    ``few`` (K-major operands) overrides the choice of the kernel for few rows, ``splits`` its CTAs per
+    column panel.
     """
     a = _row_major_2d(a)
     b = _row_major_2d(b)
@@ -105,6 +116,12 @@ def gemm(a, b, *, a_mn: bool = False, b_mn: bool = False, out=None, out_dtype=bf
     st = lib.status_tensor(a.device)
     if bias is not None and (bias.dtype != bf16 or bias.numel() != N or not bias.is_contiguous()):
         raise ValueError("bias must be a contiguous bf16 vector of N elements")
+    if few is None:
+        few = bn == 0 and pair is None and ce is None and not (a_mn or b_mn) and _use_few(M, N, K)
+    if few:
+        _call("ob_gemm_few", a.data_ptr(), b.data_ptr(), out.data_ptr(), res_ptr, M, N, K, a.stride(0), b.stride(0), out.stride(0),
+              ldr, mode, lib.ptr(bias), splits, st.data_ptr(), lib.stream_ptr())
+        return out
     if pair is None:
         pair = bn == 0 and _use_pair(M, N, K, wgrad=a_mn and b_mn)
     if ce is not None:

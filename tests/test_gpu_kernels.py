@@ -288,6 +288,31 @@ def test_gemm_epilogues(bn):
     assert _rel_err(o32, ref) < 1e-2
 
 
+@pytest.mark.parametrize("M", [1, 16, 17, 33, 65, 128, 300])
+@pytest.mark.parametrize("N,K,splits", [(8, 8, 0), (136, 264, 1), (136, 1032, 2), (1000, 2056, 8), (264, 2048, 4)])
+def test_gemm_few_rows(M, N, K, splits):
+    """Edges of the row tiles, ragged panels and slices, outputs that take no vector stores: per element against fp32 as the
+    other products."""
+    from omegalax_b200.ops import kernels as Kn, lib
+    torch.manual_seed(34)
+    x = torch.randn(M, K, device=_dev()).to(bf16)
+    w = torch.randn(N, K, device=_dev()).to(bf16)
+    ref = x.float() @ w.float().t()
+    bias, res = torch.randn(N, device=_dev()).to(bf16), torch.randn(M, N, device=_dev()).to(bf16)
+    kw = dict(few=True, splits=splits)
+    _assert_gemm_close(Kn.gemm(x, w, bias=bias, residual=res, **kw), ref + bias.float() + res.float(), K)
+    acc = torch.randn(M, N, device=_dev())
+    before = acc.clone()
+    _assert_gemm_close(Kn.gemm(x, w, out=acc, accumulate=True, **kw), ref + before, K)
+    odd = torch.zeros(M, N + 3, device=_dev(), dtype=bf16)
+    Kn.gemm(x, w, out=odd[:, 1:N + 1], **kw)
+    _check(lib)
+    _assert_gemm_close(odd[:, 1:N + 1], ref, K)
+    assert not odd[:, 0].any() and not odd[:, N + 1:].any()
+    if M == 300:      # the kernel that the sizes choose agrees
+        _assert_gemm_close(Kn.gemm(x, w), ref, K)
+
+
 @pytest.mark.parametrize("pair", [False, True])
 def test_gemm_grouped_and_wgrad(pair):
     """Grouped expert GEMMs (forward, input gradient, weight gradient) on the single-CTA kernel
