@@ -603,6 +603,31 @@ def test_attention_backward(causal, T, B):
     assert _rel_err(dv, vr.grad.reshape(N, G, HD)) < 3e-2
 
 
+@pytest.mark.parametrize("F,D,out", [(384, 264, torch.float32), (336, 256, torch.float32), (384, 264, bf16)])
+def test_grouped_pair_outputs_by_slab(F, D, out):
+    """Outputs of the CTA pairs through the TMA unit (F a multiple of 32, ragged last columns) and past it (F is not), with
+    an expert that gets no rows; per expert against fp32 with ``_assert_gemm_close``."""
+    from omegalax_b200.ops import kernels as Kn, lib
+    torch.manual_seed(33)
+    offs = [0, 256, 256, 1024]
+    offsets = torch.tensor(offs, device=_dev(), dtype=torch.int32)
+    x, dy = torch.randn(1024, D, device=_dev()).to(bf16), torch.randn(1024, F, device=_dev()).to(bf16)
+    if out == bf16:
+        w = (torch.randn(3, F, D, device=_dev()) * 0.05).to(bf16)
+        y = Kn.gemm_grouped(x, w, offsets, pair=True)
+        _check(lib)
+        for e in range(3):
+            _assert_gemm_close(y[offs[e]:offs[e + 1]], x[offs[e]:offs[e + 1]].float() @ w[e].float().t(), D)
+        return
+    for accumulate in (True, False):
+        dw = torch.full((3, F, D), 0.25, device=_dev())
+        Kn.gemm_grouped_wgrad(dy, x, offsets, dw, accumulate=accumulate, pair=True)
+        _check(lib)
+        for e in range(3):
+            rows = slice(offs[e], offs[e + 1])
+            _assert_gemm_close(dw[e], dy[rows].float().t() @ x[rows].float() + 0.25 * accumulate, max(offs[e + 1] - offs[e], 1))
+
+
 def test_paged_decode_matches_full_forward():
     """Prefill a left-padded batch into the paged cache, then decode 6 steps with the paged
     kernels; every step's logits must agree with a full forward over the grown sequence."""
