@@ -20,8 +20,15 @@
 // its own (one per quadrant, 64 columns), so draining dQ^T of step i-1 overlaps E of step i and
 // the S^T buffer is handed back to the tensor core without waiting for the softmax warps.
 //
+// Few kv heads leave few CTAs (one sequence of 3001 with 2 kv heads: 48 of 148 SMs, and a causal walk is up to
+// 24 times as long for the first tile as for the last).  Then `hsplit` CTAs share the query heads of a
+// (key tile, kv head); each stores fp32 partial sums and a second kernel adds them in order.  The grid is
+// flat with the tile index slowest, so the longest walks start first.  In us, before and after: 32 heads of 256 on 2,
+// one row of 3001: 6785, 1228; 32 heads of 128 on 4, one row of 4096: 1000, 531 (two shares); on 8, two rows of
+// 4096: 1324, 983 (one share: the order alone).
+//
 // Heads of 256 (template HD = 256): dK and dV of a 128-key tile would need all 512 TMEM columns, so
-// the kernel runs twice, once per 128-wide half `dh` of the head dimension.  Each pass computes
+// the grid holds every CTA twice, once per 128-wide half `dh` of the head dimension.  Each pass computes
 // S^T and dP^T over all 256 dimensions (they need the full dot products) and the three gradient
 // products for its half only (dV[:, half], dK[:, half], dQ[:, half]).  The K and V tiles take
 // 128 KB of shared memory there, which leaves room for a single Q/dO stage and no dQ staging tile:
@@ -50,7 +57,8 @@ struct AttnBwdArgs {
   long long total_rows;
   int H, G;
   int causal;
-  int dh;                // which 128-wide half of the head dimension this pass differentiates (HD 256)
+  int batch, hsplit;     // sequences; CTAs that share the query heads of one (key tile, kv head)
+  float* dkv_part;       // hsplit > 1: fp32 [hsplit][2][rows][G * HD] partial dK and dV
   float scale, scale_log2;
   int* status;
 };
@@ -95,12 +103,17 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
 
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
-  const int b = blockIdx.z;
-  const int g = blockIdx.y;
-  const int R = p.H / p.G;
+  int bx = (int)blockIdx.x;
+  const int hs = bx % p.hsplit; bx /= p.hsplit;
+  const int g = bx % p.G; bx /= p.G;
+  const int dh = HD == 128 ? 0 : (bx & 1);      // half of the head dimension that this CTA differentiates
+  if (HD != 128) bx >>= 1;
+  const int b = bx % p.batch, tile = bx / p.batch;
+  const int R = p.H / p.G / p.hsplit;           // query heads of this CTA
+  const int h0 = (g * p.hsplit + hs) * R;       // first of them
   const int seq_start = __ldg(p.cu_seqlens + b);
   const int seqlen = __ldg(p.cu_seqlens + b + 1) - seq_start;
-  const int k0 = blockIdx.x * 128;
+  const int k0 = tile * 128;
   if (k0 >= seqlen) return;
   const int nq_total = (seqlen + kQT - 1) / kQT;
   const int i_first = p.causal ? (k0 / kQT) : 0;
@@ -160,7 +173,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
       if (lane == 0) ok = mbar_wait(&qdo_empty[s], ph, abort_flag, p.status, OB_ERR_WAIT_EMPTY);
       ok = __shfl_sync(0xffffffffu, (int)ok, 0) != 0;
       if (!ok) break;
-      const int h = g * R + it / nqt;
+      const int h = h0 + it / nqt;
       const int q0 = (i_first + it % nqt) * kQT;
       if (lane == 0) {
         mbar_expect_tx(&qdo_full[s], 2 * L::kQTile);
@@ -245,9 +258,9 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
         tc_fence_after();
         const int s = it % kQStages;
         // the 128-wide head-dim slice of this pass: two 64-column blocks of every tile
-        const uint32_t qa = smem_u32(smem + L::kQOff + s * L::kQTile) + p.dh * 16384;
-        const uint32_t da = smem_u32(smem + L::kDOOff + s * L::kQTile) + p.dh * 16384;
-        const uint32_t kah = ka + p.dh * 32768;
+        const uint32_t qa = smem_u32(smem + L::kQOff + s * L::kQTile) + dh * 16384;
+        const uint32_t da = smem_u32(smem + L::kDOOff + s * L::kQTile) + dh * 16384;
+        const uint32_t kah = ka + dh * 32768;
         const uint32_t dsa = smem_u32(smem + L::kDSOff + bb * 16384);
         // dV += P^T dO ; dK += dS^T Q : reduce over the 64 queries (4 steps of 16)
 #pragma unroll
@@ -296,10 +309,10 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
       if constexpr (HD != 128) {
         // no staging tile: thread r adds head-dim element r of every query row (a warp covers 128
         // consecutive bytes of one row per instruction)
-        const int h = g * R + it / nqt;
+        const int h = h0 + it / nqt;
         const int q0 = (i_first + it % nqt) * kQT;
         const int qvalid = min(kQT, seqlen - q0);
-        float* dst = p.dq_acc + ((long long)(seq_start + q0) * p.H + h) * HD + p.dh * kHD + r;
+        float* dst = p.dq_acc + ((long long)(seq_start + q0) * p.H + h) * HD + dh * kHD + r;
         const long long rs = (long long)p.H * HD;
 #pragma unroll
         for (int i = 0; i < 32; ++i) {
@@ -326,7 +339,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
       if (issuer) {
         ok = mbar_wait(dqs_full, it & 1, abort_flag, p.status, OB_ERR_WAIT_MISC);
         if (ok) {
-          const int h = g * R + it / nqt;
+          const int h = h0 + it / nqt;
           const int q0 = (i_first + it % nqt) * kQT;
           tma_reduce_add_2d(&tmDQ, dq_s, h * kHD, seq_start + q0);
           tma_store_commit();
@@ -406,8 +419,10 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
       tc_fence_after();
       // every lane runs the aligned TMEM loads; only the stores are predicated
       const long long grow = (long long)seq_start + (key_ok ? kpos : 0);
-      bf16* dkp = p.dk + grow * p.dk_row_stride + (long long)g * HD + p.dh * kHD;
-      bf16* dvp = p.dv + grow * p.dv_row_stride + (long long)g * HD + p.dh * kHD;
+      bf16* dkp = p.dk + grow * p.dk_row_stride + (long long)g * HD + dh * kHD;
+      bf16* dvp = p.dv + grow * p.dv_row_stride + (long long)g * HD + dh * kHD;
+      const long long gw = (long long)p.G * HD;
+      float* part = p.dkv_part + ((long long)hs * 2 * p.total_rows + grow) * gw + (long long)g * HD + dh * kHD;
 #pragma unroll 1
       for (int cc = 0; cc < 2; ++cc) {
         const int c = half * 2 + cc;
@@ -415,7 +430,14 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
         tmem_ld32(T_DK + lane_addr + c * 32, a);
         tmem_ld32(T_DV + lane_addr + c * 32, bq);
         tmem_ld_wait();
-        if (key_ok) {
+        if (key_ok && p.hsplit > 1) {
+#pragma unroll
+          for (int i = 0; i < 8; ++i) {
+            *reinterpret_cast<uint4*>(part + c * 32 + i * 4) = make_uint4(a[i * 4], a[i * 4 + 1], a[i * 4 + 2], a[i * 4 + 3]);
+            *reinterpret_cast<uint4*>(part + p.total_rows * gw + c * 32 + i * 4) =
+                make_uint4(bq[i * 4], bq[i * 4 + 1], bq[i * 4 + 2], bq[i * 4 + 3]);
+          }
+        } else if (key_ok) {
 #pragma unroll
           for (int i = 0; i < 4; ++i) {
             uint4 x, y;
@@ -446,6 +468,26 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
     tc_fence_after();
     tmem_dealloc(tmem_base, 512);
   }
+}
+
+// dK and dV = sums of the partial ones, in order.  One thread per four channels; blockIdx.y: 0 dK, 1 dV.
+__global__ void attn_bwd_parts_kernel(const float* __restrict__ part, bf16* __restrict__ dk, bf16* __restrict__ dv, long long rows,
+                                      int width, int parts, long long dk_stride, long long dv_stride,
+                                      const int* __restrict__ cu_seqlens, int batch) {
+  const int wv = width >> 2;
+  const long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+  if (t >= rows * wv) return;
+  const long long row = t / wv;
+  if (row < __ldg(cu_seqlens) || row >= __ldg(cu_seqlens + batch)) return;   // no sequence: left as it was
+  const int c = (int)(t - row * wv) * 4;
+  const float* src = part + ((long long)blockIdx.y * rows + row) * width + c;
+  float4 s = *reinterpret_cast<const float4*>(src);
+  for (int i = 1; i < parts; ++i) {
+    const float4 x = *reinterpret_cast<const float4*>(src + (long long)i * 2 * rows * width);
+    s.x += x.x; s.y += x.y; s.z += x.z; s.w += x.w;
+  }
+  bf16* dst = blockIdx.y == 0 ? dk + row * dk_stride + c : dv + row * dv_stride + c;
+  *reinterpret_cast<uint2*>(dst) = make_uint2(pack_bf16(s.x, s.y), pack_bf16(s.z, s.w));
 }
 
 // delta[h, row] = sum_d dO[row,h,d] * O[row,h,d]; one warp per (row, head).
@@ -480,17 +522,19 @@ extern "C" {
 //   lse: [H, rows] from the forward;  delta: scratch [H, rows] fp32
 //   dq_acc: scratch [rows, H, 128] fp32 (this call zeroes it);  dq: [rows, H, 128] bf16 out
 //   dk, dv: [rows, G, 128] bf16 out with their own row strides
+//   hsplit (divides H / G), dkv_part: with more than one part, scratch fp32 [hsplit, 2, rows, G * 128]
 int ob_attn_bwd(const void* q, const void* k, const void* v, const void* out, const void* dout,
                 const float* lse, float* delta, float* dq_acc, void* dq, void* dk, void* dv,
                 const int* cu_seqlens, int B, int max_seqlen, long long total_rows, int H, int G,
                 int HD, long long q_row_stride, long long k_row_stride, long long v_row_stride,
                 long long o_row_stride, long long do_row_stride, long long dk_row_stride,
-                long long dv_row_stride, float scale, int causal, int* status,
+                long long dv_row_stride, float scale, int causal, int hsplit, float* dkv_part, int* status,
                 cudaStream_t stream) {
   if (B <= 0 || total_rows <= 0) return 0;
   if (HD != 128 && HD != 256) return 6005;
   if ((q_row_stride | k_row_stride | v_row_stride | do_row_stride | dk_row_stride | dv_row_stride) & 7)
     return 6001;
+  if (hsplit < 1 || H % G || (H / G) % hsplit || (hsplit > 1 && dkv_part == nullptr)) return 6005;
   {
     long long warps = total_rows * H;
     int threads = 256;
@@ -523,18 +567,24 @@ int ob_attn_bwd(const void* q, const void* k, const void* v, const void* out, co
   a.total_rows = total_rows; a.H = H; a.G = G; a.causal = causal;
   a.scale = scale; a.scale_log2 = scale * 1.4426950408889634f;
   a.status = status;
-  dim3 grid((max_seqlen + 127) / 128, G, B);
+  a.batch = B; a.hsplit = hsplit; a.dkv_part = dkv_part;
+  const long long ctas = (long long)((max_seqlen + 127) / 128) * B * G * hsplit * (HD / 128);
+  if (ctas > 0x7fffffff) return 6005;
+  const unsigned grid = (unsigned)ctas;
   if (HD == 128) {
     OB_ENSURE_DYN_SMEM(attn_bwd_kernel<128>, AttnBwdSmem<128>::kTotal);
     attn_bwd_kernel<128><<<grid, kBwdThreads, AttnBwdSmem<128>::kTotal, stream>>>(tmQ, tmK, tmV, tmDO, tmDQ, a);
     OB_CHECK_LAUNCH();
   } else {
     OB_ENSURE_DYN_SMEM(attn_bwd_kernel<256>, AttnBwdSmem<256>::kTotal);
-    for (int dh = 0; dh < 2; ++dh) {   // one pass per 128-wide half of the head dimension
-      a.dh = dh;
-      attn_bwd_kernel<256><<<grid, kBwdThreads, AttnBwdSmem<256>::kTotal, stream>>>(tmQ, tmK, tmV, tmDO, tmDQ, a);
-      OB_CHECK_LAUNCH();
-    }
+    attn_bwd_kernel<256><<<grid, kBwdThreads, AttnBwdSmem<256>::kTotal, stream>>>(tmQ, tmK, tmV, tmDO, tmDQ, a);
+    OB_CHECK_LAUNCH();
+  }
+  if (hsplit > 1) {
+    const long long threads = total_rows * (G * HD / 4);
+    attn_bwd_parts_kernel<<<dim3((unsigned)((threads + 255) / 256), 2), 256, 0, stream>>>(
+        dkv_part, (bf16*)dk, (bf16*)dv, total_rows, G * HD, hsplit, dk_row_stride, dv_row_stride, cu_seqlens, B);
+    OB_CHECK_LAUNCH();
   }
   // fp32 accumulation buffer -> bf16 dq
   extern int ob_cast_f32_bf16(const float*, void*, long long, cudaStream_t);
@@ -594,5 +644,5 @@ extern "C" int ob_attn_bwd_noalloc(const void* q, const void* k, const void* v, 
   // ob_attn_bwd zeroes dq_acc itself (cudaMemsetAsync on `stream`) and overwrites delta fully.
   return ob_attn_bwd(q, k, v, out, dout, lse, delta, dq_acc, dq, dk, dv, cu_seqlens, B, max_seqlen, total_rows, H,
                      G, HD, q_row_stride, k_row_stride, v_row_stride, o_row_stride, do_row_stride, dk_row_stride,
-                     dv_row_stride, scale, causal, status, stream);
+                     dv_row_stride, scale, causal, 1, nullptr, status, stream);
 }

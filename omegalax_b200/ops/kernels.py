@@ -341,7 +341,17 @@ def attn_fwd(q, k, v, cu_seqlens, max_seqlen, scale, causal, want_lse=True):
 _attn_scratch: dict = {}
 
 
-def attn_bwd(q, k, v, o, lse, do, cu_seqlens, max_seqlen, scale, causal, dk_out=None, dv_out=None):
+def attn_bwd_splits(tiles: int, H: int, G: int, steps: int) -> int:
+    """CTAs that share the query heads of a key tile: doubled while (tile, kv head) pairs leave SMs without a CTA, and
+    a CTA keeps sixteen steps of 64 queries.  32 heads on 4, one row of 4096 (128 pairs): 1062 us, with two CTAs
+    580, with four 576; on 8, two rows of 4096 (512 pairs): 1076, 1147, 1289 (partial sums to store and add)."""
+    n, R = 1, H // G
+    while tiles * G * n < 200 and R % (2 * n) == 0 and R // (2 * n) * steps >= 16:
+        n *= 2
+    return n
+
+
+def attn_bwd(q, k, v, o, lse, do, cu_seqlens, max_seqlen, scale, causal, dk_out=None, dv_out=None, splits: int | None = None):
     """Gradients of ``attn_fwd`` (head_dim 128).  Returns dq [N,H,K], dk, dv [N,G,K].
     ``dk_out`` / ``dv_out`` may be row-strided views (e.g. slices of a fused dqkv buffer).
     The fp32 dq accumulation buffer and the delta vector are cached per shape and reused."""
@@ -358,12 +368,15 @@ def attn_bwd(q, k, v, o, lse, do, cu_seqlens, max_seqlen, scale, causal, dk_out=
                    lib.scratch("attn_bwd delta", H * N, torch.float32, q.device))
         _attn_scratch[key] = scratch
     dq_acc, delta = scratch
+    if splits is None:
+        splits = attn_bwd_splits(-(-int(max_seqlen) // 128) * (cu_seqlens.numel() - 1) * (Kd // 128), H, G, -(-int(max_seqlen) // 64))
+    part = torch.empty(splits, 2, N, G * Kd, dtype=torch.float32, device=q.device) if splits > 1 else None
     st = lib.status_tensor(q.device)
     _call("ob_attn_bwd", q.data_ptr(), k.data_ptr(), v.data_ptr(), o.data_ptr(), do.data_ptr(),
           lse.data_ptr(), delta.data_ptr(), dq_acc.data_ptr(), dq.data_ptr(), dk.data_ptr(),
           dv.data_ptr(), cu_seqlens.data_ptr(), cu_seqlens.numel() - 1, int(max_seqlen), N, H, G, Kd,
           q.stride(0), k.stride(0), v.stride(0), o.stride(0), do.stride(0), dk.stride(0), dv.stride(0),
-          float(scale), int(causal), st.data_ptr(), lib.stream_ptr())
+          float(scale), int(causal), splits, lib.ptr(part), st.data_ptr(), lib.stream_ptr())
     return dq, dk, dv
 
 

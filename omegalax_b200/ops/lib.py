@@ -42,7 +42,7 @@ _SIGS = {
     "ob_gemm_bf16_pair_grouped": [P, P, P, P, I, I, I, I, L, L, I, I, P, P],
     "ob_gemm_bf16_pair_grouped_wgrad": [P, P, P, P, I, I, I, I, L, L, I, P, P],
     "ob_attn_fwd": [P, P, P, P, P, P, I, I, L, I, I, I, L, L, L, L, F, I, P, P],
-    "ob_attn_bwd": [P, P, P, P, P, P, P, P, P, P, P, P, I, I, L, I, I, I, L, L, L, L, L, L, L, F, I, P, P],
+    "ob_attn_bwd": [P, P, P, P, P, P, P, P, P, P, P, P, I, I, L, I, I, I, L, L, L, L, L, L, L, F, I, I, P, P, P],
     "ob_attn_fwd_two_part": [P, P, P, P, P, P, I, I, L, I, I, I, I, L, L, L, L, F, P, P],
     "ob_embed_rows": [P, P, P, I, I, I, I, P, P],
     "ob_ln_rows": [P, P, P, P, I, I, F, I, P],

@@ -628,6 +628,32 @@ def test_grouped_pair_outputs_by_slab(F, D, out):
             _assert_gemm_close(dw[e], dy[rows].float().t() @ x[rows].float() + 0.25 * accumulate, max(offs[e + 1] - offs[e], 1))
 
 
+@pytest.mark.parametrize("HD,H,G,lens,splits", [(128, 8, 1, [700], None), (128, 8, 2, [130, 1, 64], 2), (128, 4, 1, [129, 300], 4),
+                                                (256, 16, 1, [400], None), (256, 4, 2, [65, 191], 2)])
+def test_attention_backward_shared_query_heads(HD, H, G, lens, splits):
+    """Several CTAs share the query heads of a key tile: against fp32 with the tolerances of the tests above, and rows of no
+    sequence stay as they were."""
+    from omegalax_b200.ops import kernels as Kn, reference as R, lib
+    torch.manual_seed(32)
+    lead, N = 5, sum(lens) + 5 + 9
+    q, do = (torch.randn(N, H, HD, device=_dev()).to(bf16) for _ in range(2))
+    k, v = (torch.randn(N, G, HD, device=_dev()).to(bf16) for _ in range(2))
+    cu = torch.tensor([lead] + list(torch.tensor(lens).cumsum(0) + lead), device=_dev(), dtype=torch.int32)
+    inner = slice(lead, lead + sum(lens))
+    o, lse = Kn.attn_fwd(q, k, v, cu, max(lens), HD ** -0.5, True)
+    o[:lead], o[inner.stop:] = 0, 0
+    dkv = torch.full((N, 2 * G * HD), 3.0, dtype=bf16, device=_dev())
+    dk, dv = (t.view(N, G, HD) for t in dkv.split(G * HD, -1))
+    assert splits or Kn.attn_bwd_splits(-(-max(lens) // 128) * len(lens) * (HD // 128), H, G, -(-max(lens) // 64)) > 1
+    dq, _, _ = Kn.attn_bwd(q, k, v, o, lse, do, cu, max(lens), HD ** -0.5, True, dk_out=dk, dv_out=dv, splits=splits)
+    _check(lib)
+    qr, kr, vr = (t[inner].float().requires_grad_(True) for t in (q, k, v))
+    ref = R.attention_varlen(qr, kr, vr, cu - lead, causal=True, scale=HD ** -0.5)
+    ref.backward(do[inner].float())
+    assert _rel_err(dq[inner], qr.grad) < 3e-2 and _rel_err(dk[inner], kr.grad) < 3e-2 and _rel_err(dv[inner], vr.grad) < 3e-2
+    assert (dkv[:lead] == 3).all() and (dkv[inner.stop:] == 3).all()
+
+
 def test_paged_decode_matches_full_forward():
     """Prefill a left-padded batch into the paged cache, then decode 6 steps with the paged
     kernels; every step's logits must agree with a full forward over the grown sequence."""
