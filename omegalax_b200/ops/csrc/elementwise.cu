@@ -842,51 +842,63 @@ __global__ void sumsq_kernel(const float* __restrict__ g, long long n, float* __
 // already-reduced squared gradient norm so the host never synchronises:
 //   g' = g * grad_mul * min(1, max_norm / (sqrt(norm_sq) * grad_mul + 1e-6))
 // Writes the fp32 master, both moments, the bf16 compute copy, and zeroes the gradient.
-__global__ void adamw_kernel(float* __restrict__ p, float* __restrict__ m, float* __restrict__ v,
-                             float* __restrict__ g, bf16* __restrict__ p16, long long n, float lr,
-                             float b1, float b2, float eps, float wd, float bc1, float bc2,
-                             float grad_mul, const float* __restrict__ norm_sq, float max_norm,
-                             int zero_grad) {
+// Bound by HBM (34 bytes a parameter: 1.63 G parameters 9.34 ms, 5.9 TB/s; 10.09 before).  ibc1 / ibc2 are the
+// reciprocals of the bias corrections, rounded once from double precision on the host: one division per
+// parameter is left instead of three.
+struct AdamArgs {
+  float lr, b1, b2, eps, wd, ibc1, ibc2;
+};
+
+__device__ __forceinline__ void adam_one(const AdamArgs& a, float mul, float& p, float& m, float& v, float g) {
+  const float gr = g * mul;
+  m = a.b1 * m + (1.f - a.b1) * gr;
+  v = a.b2 * v + (1.f - a.b2) * gr * gr;
+  p = p - a.lr * ((m * a.ibc1) / (sqrtf(v * a.ibc2) + a.eps) + a.wd * p);
+}
+
+// A thread has two groups of four parameters in flight, 128 bytes of loads before any arithmetic.
+__global__ void __launch_bounds__(256) adamw_kernel(float* __restrict__ p, float* __restrict__ m, float* __restrict__ v,
+                                                    float* __restrict__ g, bf16* __restrict__ p16, long long n, AdamArgs a,
+                                                    float grad_mul, const float* __restrict__ norm_sq, float max_norm,
+                                                    int zero_grad) {
   float mul = grad_mul;
   if (norm_sq && max_norm > 0.f) {
     float nrm = sqrtf(*norm_sq) * grad_mul;
     mul *= fminf(1.f, max_norm / (nrm + 1e-6f));
   }
-  const long long n4 = n >> 2;
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n4;
-       i += (long long)gridDim.x * blockDim.x) {
-    float4 pp = reinterpret_cast<float4*>(p)[i], mm = reinterpret_cast<float4*>(m)[i],
-           vv = reinterpret_cast<float4*>(v)[i], gg = reinterpret_cast<float4*>(g)[i];
-    float pa[4] = {pp.x, pp.y, pp.z, pp.w}, ma[4] = {mm.x, mm.y, mm.z, mm.w},
-          va[4] = {vv.x, vv.y, vv.z, vv.w}, ga[4] = {gg.x, gg.y, gg.z, gg.w};
+  constexpr int U = 2;
+  const long long n4 = n >> 2, step = (long long)gridDim.x * (256 * U);
+  float4 *p4 = reinterpret_cast<float4*>(p), *m4 = reinterpret_cast<float4*>(m), *v4 = reinterpret_cast<float4*>(v),
+         *g4 = reinterpret_cast<float4*>(g);
+  for (long long i0 = blockIdx.x * (long long)(256 * U) + threadIdx.x; i0 < n4; i0 += step) {
+    float4 pp[U], mm[U], vv[U], gg[U];
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      float gr = ga[j] * mul;
-      ma[j] = b1 * ma[j] + (1.f - b1) * gr;
-      va[j] = b2 * va[j] + (1.f - b2) * gr * gr;
-      float mh = ma[j] / bc1, vh = va[j] / bc2;
-      pa[j] = pa[j] - lr * (mh / (sqrtf(vh) + eps) + wd * pa[j]);
+    for (int u = 0; u < U; ++u) {
+      const long long i = i0 + 256 * u;
+      if (i < n4) {
+        pp[u] = __ldcs(p4 + i); mm[u] = __ldcs(m4 + i); vv[u] = __ldcs(v4 + i); gg[u] = __ldcs(g4 + i);
+      }
     }
-    reinterpret_cast<float4*>(p)[i] = make_float4(pa[0], pa[1], pa[2], pa[3]);
-    reinterpret_cast<float4*>(m)[i] = make_float4(ma[0], ma[1], ma[2], ma[3]);
-    reinterpret_cast<float4*>(v)[i] = make_float4(va[0], va[1], va[2], va[3]);
-    if (zero_grad) reinterpret_cast<float4*>(g)[i] = make_float4(0.f, 0.f, 0.f, 0.f);
-    if (p16) {
-      uint2 o;
-      o.x = pack_bf16(pa[0], pa[1]);
-      o.y = pack_bf16(pa[2], pa[3]);
-      reinterpret_cast<uint2*>(p16)[i] = o;
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const long long i = i0 + 256 * u;
+      if (i >= n4) break;
+      adam_one(a, mul, pp[u].x, mm[u].x, vv[u].x, gg[u].x);
+      adam_one(a, mul, pp[u].y, mm[u].y, vv[u].y, gg[u].y);
+      adam_one(a, mul, pp[u].z, mm[u].z, vv[u].z, gg[u].z);
+      adam_one(a, mul, pp[u].w, mm[u].w, vv[u].w, gg[u].w);
+      __stcs(p4 + i, pp[u]);
+      __stcs(m4 + i, mm[u]);
+      __stcs(v4 + i, vv[u]);
+      if (zero_grad) __stcs(g4 + i, make_float4(0.f, 0.f, 0.f, 0.f));
+      if (p16) __stcs(reinterpret_cast<uint2*>(p16) + i, make_uint2(pack_bf16(pp[u].x, pp[u].y), pack_bf16(pp[u].z, pp[u].w)));
     }
   }
   if (blockIdx.x == 0) {
     for (long long i = (n4 << 2) + threadIdx.x; i < n; i += blockDim.x) {
-      float gr = g[i] * mul;
-      float mi = b1 * m[i] + (1.f - b1) * gr;
-      float vi = b2 * v[i] + (1.f - b2) * gr * gr;
-      float pi = p[i] - lr * ((mi / bc1) / (sqrtf(vi / bc2) + eps) + wd * p[i]);
-      p[i] = pi; m[i] = mi; v[i] = vi;
+      adam_one(a, mul, p[i], m[i], v[i], g[i]);
       if (zero_grad) g[i] = 0.f;
-      if (p16) p16[i] = __float2bfloat16(pi);
+      if (p16) p16[i] = __float2bfloat16(p[i]);
     }
   }
 }
@@ -1222,14 +1234,13 @@ int ob_sumsq(const float* g, long long n, float* out, cudaStream_t s) {
 }
 
 int ob_adamw(float* p, float* m, float* v, float* g, void* p16, long long n, float lr, float b1,
-             float b2, float eps, float wd, float bc1, float bc2, float grad_mul,
+             float b2, float eps, float wd, double bc1, double bc2, float grad_mul,
              const float* norm_sq, float max_norm, int zero_grad, cudaStream_t s) {
   if (n <= 0) return 0;
   if ((((uintptr_t)p) | ((uintptr_t)m) | ((uintptr_t)v) | ((uintptr_t)g)) & 15) return 6002;
   if (p16 && (((uintptr_t)p16) & 7)) return 6002;
-  adamw_kernel<<<grid_for(n / 4 + 1, 256), 256, 0, s>>>(p, m, v, g, (bf16*)p16, n, lr, b1, b2, eps,
-                                                        wd, bc1, bc2, grad_mul, norm_sq, max_norm,
-                                                        zero_grad);
+  const AdamArgs a = {lr, b1, b2, eps, wd, (float)(1.0 / bc1), (float)(1.0 / bc2)};
+  adamw_kernel<<<grid_for(n / 8 + 1, 256), 256, 0, s>>>(p, m, v, g, (bf16*)p16, n, a, grad_mul, norm_sq, max_norm, zero_grad);
   OB_CHECK_LAUNCH();
   return 0;
 }
