@@ -58,6 +58,18 @@ __device__ __forceinline__ uint32_t bits_between(int lo, int hi) {
   return upto & from;
 }
 
+template <bool V>
+struct AttnFlag { static constexpr bool value = V; };
+
+// two single-precision multiply-adds in one instruction
+__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
+  float2 d;
+  asm("{\n.reg .b64 x, y, z;\nmov.b64 x, {%2, %3};\nmov.b64 y, {%4, %5};\nmov.b64 z, {%6, %7};\n"
+      "fma.rn.f32x2 x, x, y, z;\nmov.b64 {%0, %1}, x;\n}"
+      : "=f"(d.x), "=f"(d.y) : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y), "f"(c.x), "f"(c.y));
+  return d;
+}
+
 template <int QB, int VB, int KST, int VST>
 struct AttnFwdSmem {
   static constexpr int kQTile = 128 * QB * 64 * 2;    // one 128-row query / key tile
@@ -274,26 +286,32 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
       const bool need_mask = (kbase + 128 > seqlen) || (p.causal && kbase + 127 > q0 + w * 128) ||
                              (kWindow && p.window > 0 && kbase <= q0 + w * 128 + 127 - p.window);
       const int klimit = p.causal ? min(seqlen - 1, qpos) : seqlen - 1;  // last visible key
-      // pass 1: row maximum
-      float mx = -INFINITY;
-#pragma unroll 1
-      for (int c = 0; c < 4; ++c) {
-        uint32_t v[32];
-        tmem_ld32(s_addr + c * 32, v);
-        tmem_ld_wait();
-        if (kWindow && need_mask) {
-          const uint32_t seen = bits_between(kfirst - kbase - c * 32, klimit - kbase - c * 32);
+      // The whole row of scores stays in registers between maximum and exponentials: four loads in flight and one wait,
+      // where two passes of four loads waited eight times (32 heads on 8, two rows of 4096: 404 us, now 360).
+      uint32_t v[128];
 #pragma unroll
-          for (int i = 0; i < 32; ++i) mx = fmaxf(mx, (seen >> i) & 1 ? __uint_as_float(v[i]) : -INFINITY);
-        } else if (need_mask) {
+      for (int c = 0; c < 4; ++c) tmem_ld32(s_addr + c * 32, v + c * 32);
+      tmem_ld_wait();
+      const int lim = klimit - kbase;      // last visible column
+      float mx4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
+      if (kWindow && need_mask) {          // hidden scores become -inf, their exponentials 0
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+          const uint32_t seen = bits_between(kfirst - kbase - c * 32, lim - c * 32);
 #pragma unroll
           for (int i = 0; i < 32; ++i)
-            if (kbase + c * 32 + i <= klimit) mx = fmaxf(mx, __uint_as_float(v[i]));
-        } else {
-#pragma unroll
-          for (int i = 0; i < 32; ++i) mx = fmaxf(mx, __uint_as_float(v[i]));
+            if (!((seen >> i) & 1)) v[c * 32 + i] = 0xff800000u;
         }
       }
+      if (!kWindow && need_mask) {
+#pragma unroll
+        for (int i = 0; i < 128; ++i)
+          if (i <= lim) mx4[i & 3] = fmaxf(mx4[i & 3], __uint_as_float(v[i]));
+      } else {
+#pragma unroll
+        for (int i = 0; i < 128; ++i) mx4[i & 3] = fmaxf(mx4[i & 3], __uint_as_float(v[i]));
+      }
+      const float mx = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3]));
       m_run = fmaxf(m_run, mx * p.scale_log2);
       // move the reference (and rescale O) only when some row of this warp needs it; the TMEM
       // accesses below are warp-wide, so the decision is too
@@ -321,33 +339,29 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
       }
       const float m_safe = (m_ref == -INFINITY) ? 0.f : m_ref;
       float lsum = 0.f;
-      // pass 2: probabilities, packed bf16 into the first 64 columns of S
-#pragma unroll 1
-      for (int c = 0; c < 4; ++c) {
-        uint32_t v[32];
-        tmem_ld32(s_addr + c * 32, v);
-        tmem_ld_wait();
-        uint32_t pk[16];
-        uint32_t seen = 0xffffffffu;
-        if (kWindow && need_mask) seen = bits_between(kfirst - kbase - c * 32, klimit - kbase - c * 32);
-        if (kWindow && seen != 0xffffffffu) {      // hidden scores become -inf, their exponentials 0
+      const float2 sc = make_float2(p.scale_log2, p.scale_log2), off = make_float2(-m_safe, -m_safe);
+      // probabilities, packed bf16 into the first 64 columns of S
+      auto probabilities = [&](auto masked) {
 #pragma unroll
-          for (int i = 0; i < 32; ++i)
-            if (!((seen >> i) & 1)) v[i] = 0xff800000u;
-        }
+        for (int c = 0; c < 4; ++c) {
+          uint32_t pk[16];
 #pragma unroll
-        for (int i = 0; i < 16; ++i) {
-          float p0 = fast_exp2(__uint_as_float(v[2 * i]) * p.scale_log2 - m_safe);
-          float p1 = fast_exp2(__uint_as_float(v[2 * i + 1]) * p.scale_log2 - m_safe);
-          if (!kWindow && need_mask) {
-            if (kbase + c * 32 + 2 * i > klimit) p0 = 0.f;
-            if (kbase + c * 32 + 2 * i + 1 > klimit) p1 = 0.f;
+          for (int i = 0; i < 16; ++i) {
+            const int k = c * 32 + 2 * i;
+            const float2 e = fma2(make_float2(__uint_as_float(v[k]), __uint_as_float(v[k + 1])), sc, off);
+            float2 pr = make_float2(fast_exp2(e.x), fast_exp2(e.y));
+            if (decltype(masked)::value) {
+              if (k > lim) pr.x = 0.f;
+              if (k + 1 > lim) pr.y = 0.f;
+            }
+            lsum += pr.x + pr.y;
+            pk[i] = pack_bf16(pr.x, pr.y);
           }
-          lsum += p0 + p1;
-          pk[i] = pack_bf16(p0, p1);
+          tmem_st16(s_addr + c * 16, pk);
         }
-        tmem_st16(s_addr + c * 16, pk);
-      }
+      };
+      if (!kWindow && need_mask) probabilities(AttnFlag<true>());
+      else probabilities(AttnFlag<false>());
       tmem_st_wait();
       l_run += lsum;
       tc_fence_before();
