@@ -541,24 +541,18 @@ def decode_append(qkv, qw, kw, positions, seq_of_token, slot_of_token, block_tab
     return q
 
 
-_decode_scratch: dict = {}
-
-
 def decode_attn(q, k_pages, v_pages, block_table, seq_lens, page_size, scale, splits=None):
     """q [B,H,HD] attends over each sequence's pages; returns [B,H,HD]."""
     B, H, HD = q.shape
     G = k_pages.shape[2]
     if splits is None:
-        # the per-key work is latency bound, so fill every SM with ~16 small CTAs, but keep at
-        # least 128 keys of cache capacity per split
-        cap = block_table.shape[1] * page_size
-        splits = max(1, min(32, -(-(148 * 16) // max(B * G, 1)), cap // 128))
-    key = (q.device.index, B, H, HD, splits)
-    sc = _decode_scratch.get(key)
-    if sc is None:
-        sc = (torch.empty(B * H * splits * HD, dtype=torch.float32, device=q.device),
-              torch.empty(B * H * splits * 2, dtype=torch.float32, device=q.device))
-        _decode_scratch[key] = sc
+        # two waves of the CTAs that fit an SM (one where eight heads share a row), at least 128 keys of capacity
+        # each.  32 sequences of 2048, 32 heads on 8, by splits 2 / 4 / 8 / 16: 75 69 71 80 us; one of 4096, by
+        # 8 / 16 / 32 / 48: 19.1 13.6 13.6 15.4; eight of 4096, 32 on 4, by 4 / 8 / 16 / 32: 41 35 39 48.
+        ctas = 1184 if H // G <= 4 else 296
+        splits = max(1, min(32, ctas // max(B * G, 1), block_table.shape[1] * page_size // 128))
+    sc = (torch.empty(B * H * splits * HD, dtype=torch.float32, device=q.device),
+          torch.empty(B * H * splits * 2, dtype=torch.float32, device=q.device))
     out = torch.empty_like(q)
     _call("ob_decode_attn", q.data_ptr(), k_pages.data_ptr(), v_pages.data_ptr(), block_table.data_ptr(),
           seq_lens.data_ptr(), B, H, G, HD, block_table.shape[1], page_size, splits, float(scale),

@@ -654,6 +654,27 @@ def test_attention_backward_shared_query_heads(HD, H, G, lens, splits):
     assert (dkv[:lead] == 3).all() and (dkv[inner.stop:] == 3).all()
 
 
+@pytest.mark.parametrize("R", [1, 2, 4, 8])
+@pytest.mark.parametrize("splits", [1, 3, 70])
+def test_decode_attention_lengths(R, splits):
+    """Lengths around the 32 keys of an iteration, an empty sequence, splits without keys; fp32 reference, one rounding to bf16
+    (2^-8) of outputs of size one."""
+    from omegalax_b200.ops import kernels as Kn, lib
+    torch.manual_seed(35)
+    G, HD, ps, lens = 2, 128, 64, [0, 1, 31, 32, 33, 200, 1000]
+    B, H, blocks = len(lens), 2 * R, 16
+    k, v = (torch.randn(B * blocks, ps, G, HD, device=_dev()).to(bf16) for _ in range(2))
+    table = torch.randperm(B * blocks, device=_dev()).to(torch.int32).view(B, blocks)
+    q = (torch.randn(B, H, HD, device=_dev()) * 3).to(bf16)
+    n = torch.tensor(lens, device=_dev(), dtype=torch.int32)
+    out = Kn.decode_attn(q, k, v, table, n, ps, HD ** -0.5, splits=splits)
+    _check(lib)
+    for b, m in enumerate(lens):
+        kb, vb = (t[table[b].long()].view(-1, G, HD)[:m].float().repeat_interleave(R, 1) for t in (k, v))
+        p = torch.softmax(torch.einsum("hd,shd->hs", q[b].float(), kb) * HD ** -0.5, -1)
+        torch.testing.assert_close(out[b].float(), torch.einsum("hs,shd->hd", p, vb), rtol=2.0 ** -8, atol=2.0 ** -10)
+
+
 def test_paged_decode_matches_full_forward():
     """Prefill a left-padded batch into the paged cache, then decode 6 steps with the paged
     kernels; every step's logits must agree with a full forward over the grown sequence."""
