@@ -19,7 +19,8 @@ class DecodeGraph:
         self.batch = batch            # the recorded step reads these tensors
         before = K.launch_count()
         self.graph = torch.cuda.CUDAGraph()
-        with torch.cuda.graph(self.graph):
+        # other threads go on allocating while this one records
+        with torch.cuda.graph(self.graph, capture_error_mode="thread_local"):
             self.out = model.run_layers(batch, cache)
         self.launches = K.launch_count() - before
         self.model = model
@@ -29,18 +30,19 @@ class DecodeGraph:
         return os.environ.get("OMEGALAX_B200_DECODE_GRAPH", "1") == "1"
 
     @staticmethod
-    def step(model, cache, batch):
-        """fp32 residual rows of a single-token batch; the tensor is reused by the next step."""
+    def step(model, cache, batch, key=None):
+        """Residual rows of a single-token batch; the tensor is reused by the next step.  A recording serves while
+        ``key`` (what the model runs and where its weights lie) compares equal."""
         state = cache.decode_graph
         if not DecodeGraph.enabled():
             return model.run_layers(batch, cache)
-        if state is None or state[0] is not model:
-            cache.decode_graph = (model, None)
+        if state is None or state[0] is not model or state[2] != key:
+            cache.decode_graph = (model, None, key)
             return model.run_layers(batch, cache)
         graph = state[1]
         if graph is None:
             graph = DecodeGraph(model, cache, batch)
-            cache.decode_graph = (model, graph)
+            cache.decode_graph = (model, graph, key)
         else:
             graph.batch.flat.copy_(batch.flat)
             K.add_launches(graph.launches)

@@ -31,27 +31,32 @@ class TokenBatch:
     def build(cache, tokens: list) -> "TokenBatch":
         """``tokens[b]``: 1-D int32 CPU tensor of sequence b's new tokens (possibly empty).  Pages must
         be reserved.  One host -> device copy."""
-        B, lens = cache.B, cache.seq_lens_host
+        B, lens, ps = cache.B, cache.seq_lens_host, cache.page_size
         n = [int(t.numel()) for t in tokens]
         single = max(n) == 1
         i32 = torch.int32
+        hist, count = torch.tensor(lens, dtype=i32), torch.tensor(n, dtype=i32)
+        new = torch.cat([t.to(i32) for t in tokens])
         if single:
-            ids = torch.tensor([int(t[0]) if k else -1 for t, k in zip(tokens, n)], dtype=i32)
-            pos = torch.tensor([lens[b] if n[b] else -1 for b in range(B)], dtype=i32)
-            row = torch.tensor([cache.flat_row_host(b, lens[b]) if n[b] else -1 for b in range(B)], dtype=i32)
+            has = count > 0
+            ids = torch.full((B,), -1, dtype=i32)
+            ids[has] = new
+            pos = torch.where(has, hist, -1)
             seq = torch.arange(B, dtype=i32)
             cu = torch.arange(B + 1, dtype=i32)
+            at = pos.clamp_min(0)
         else:
-            ids = torch.cat([t.to(i32) for t in tokens])
-            pos = torch.cat([torch.arange(lens[b], lens[b] + n[b], dtype=i32) for b in range(B)])
-            row = torch.cat([cache.flat_rows_host(b, lens[b], n[b]) for b in range(B)])
-            seq = torch.repeat_interleave(torch.arange(B, dtype=i32), torch.tensor(n))
+            ids = new
             cu = torch.tensor([0] + n, dtype=i32).cumsum(0).to(i32)
-        hist = torch.tensor(lens, dtype=i32)
+            seq = torch.repeat_interleave(torch.arange(B, dtype=i32), count)
+            at = pos = hist[seq] + torch.arange(len(new), dtype=i32) - cu[seq]
+        row = cache.block_table_host[seq.long(), (at // ps).long()] * ps + at % ps
+        if single:
+            row = torch.where(has, row, -1)
         parts = [ids, pos, row, seq, pos + 1, cu, hist]
         # every part starts on a 16-byte boundary of the one buffer that travels
         padded = [torch.cat([p, p.new_zeros(-p.numel() % 4)]) for p in parts]
-        flat = torch.cat(padded).to(cache.device)
+        flat = torch.cat(padded).to(cache.device, non_blocking=True)     # pageable memory is staged before the call returns
         out, at = [], 0
         for p, q in zip(parts, padded):
             out.append(flat[at:at + p.numel()])

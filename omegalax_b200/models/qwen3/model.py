@@ -9,14 +9,19 @@ from __future__ import annotations
 
 import dataclasses
 import math
+from types import SimpleNamespace
 
 import torch
+import torch.nn.functional as F
 from torch import nn
+from torch.nn.modules import module as _module_hooks
 
 from ...ops import functional as Fn
 from ...ops import moe as moe_ops
 from ...ops import reference as R
+from ...ops import lib
 from ...parallel import tp as tp_lib
+from ..decode_graph import DecodeGraph
 from .cache import LayerCache
 from .config import Qwen3Config
 from .norms import RMSNorm
@@ -280,6 +285,44 @@ class Qwen3(nn.Module):
     def logits(self, hidden):
         return self.lm_head(hidden)
 
+    def _recordable(self, cache):
+        """Key under which a recorded single-token step may be replayed: the modules that run and where weights and
+        pages lie.  None: hooks want to see every call, or experts are routed (their buffers follow the routing)."""
+        mods, ptrs = [], [t.data_ptr() for t in (cache.block_table, *cache.k_pages, *cache.v_pages)]
+        if _module_hooks._global_forward_hooks or _module_hooks._global_forward_pre_hooks or lib.debug_enabled():
+            return None
+        for m in self.modules():
+            if m._forward_hooks or m._forward_pre_hooks or getattr(m, "is_moe", False):
+                return None
+            mods.append(m)
+            ptrs.extend(p.data_ptr() for p in m._parameters.values() if p is not None)
+        return tuple(mods), tuple(ptrs)
+
+    @torch.no_grad()
+    def run_layers(self, batch, cache):
+        """Residual rows of one new token per sequence, after the last layer."""
+        from ...ops import kernels as K
+
+        x = self.embed(batch.ids)
+        for li, layer in enumerate(self.layers):
+            a, k, v = layer.attn, cache.k_pages[li], cache.v_pages[li]
+            q = K.decode_append(a.qkv_proj(layer.input_norm(x)), a.q_norm.weight, a.k_norm.weight, batch.slot, batch.seq, batch.slot,
+                                cache.block_table, cache.page_size, k, v, a.H, a.G, a.Kd, a.Kd, self.cfg.rope_theta, a.eps)
+            if batch.every:
+                o = K.decode_attn(q, k, v, cache.block_table, batch.lens, cache.page_size, a.scale)
+            else:
+                qb = torch.zeros(cache.B, a.H, a.Kd, dtype=q.dtype, device=q.device)
+                qb[batch.seq.long()] = q
+                o = K.decode_attn(qb, k, v, cache.block_table, batch.lens, cache.page_size, a.scale)[batch.seq.long()]
+            x = self._after_attention(layer, o, x)
+        return x
+
+    @staticmethod
+    def _after_attention(layer, o, x):
+        x = layer.attn.o_proj(o.reshape(x.shape[0], -1), residual=x)
+        y = layer.mlp(layer.post_norm(x), residual=x)
+        return y[0] if layer.is_moe else y
+
     @torch.no_grad()
     def decode_paged(self, token_ids, segment_ids, cache, select=None):
         """Prefill or one decode step against a ``PagedKVCache`` (CUDA bf16).  Only real tokens
@@ -290,56 +333,60 @@ class Qwen3(nn.Module):
 
         cfg = self.cfg
         B, T = token_ids.shape
-        dev = token_ids.device
-        real = segment_ids != 0
+        dev, ps, i32 = token_ids.device, cache.page_size, torch.int32
+        key = self._recordable(cache) if T == 1 else None
+        # The indices of the call are worked out on the host and travel in one copy: the ids are the only thing
+        # waited for.  A step of one token per sequence is then one graph launch (8 layers of 4096 channels: 3.1 ms of
+        # launches for 1.1 ms of kernels).
+        both = torch.stack((token_ids.to(i32), (segment_ids != 0).to(i32))).cpu()
+        real = both[1] != 0
         counts = real.sum(-1)
-        new_tokens = [int(c) for c in counts.tolist()]
+        new_tokens = counts.tolist()
         cache.reserve(new_tokens)
-        seq_of = torch.arange(B, device=dev)[:, None].expand(B, T)[real].to(torch.int32)
-        rank_in = (real.cumsum(-1) - 1)[real]
-        start = cache.seq_lens[seq_of.long()]
-        slot = (start + rank_in).to(torch.int32)
-        ids = token_ids[real]
-        x = self.embed(ids)
-        N = x.shape[0]
-        single = max(new_tokens) <= 1
+        cache.settle()
+        N, single = sum(new_tokens), max(new_tokens) <= 1
         if not single and any(cache.seq_lens_host[b] > 0 and new_tokens[b] > 0 for b in range(B)):
             raise NotImplementedError("multi-token calls are only supported on an empty cache (prefill)")
-        cu = torch.zeros(B + 1, dtype=torch.int32, device=dev)
-        cu[1:] = counts.cumsum(0)
-        sin, cos = R.rope_tables(slot, cfg.head_dim, cfg.rope_theta)
-        lens_after = (cache.seq_lens + counts.to(torch.int32)).contiguous()
-        rows = cache.flat_rows(seq_of, slot)
-        last = (cu[1:] - 1).long().clamp_min(0)
-        for li, layer in enumerate(self.layers):
-            a = layer.attn
-            h = layer.input_norm(x)
-            qkv = a.qkv_proj(h)
-            if single:
-                q = K.decode_append(qkv, a.q_norm.weight, a.k_norm.weight, slot, seq_of, slot, cache.block_table,
-                                    cache.page_size, cache.k_pages[li], cache.v_pages[li], a.H, a.G, a.Kd, a.Kd,
-                                    cfg.rope_theta, a.eps)
-                # every sequence contributes exactly one row in this mode
-                qb = torch.zeros(B, a.H, a.Kd, dtype=q.dtype, device=dev)
-                qb[seq_of.long()] = q
-                ob = K.decode_attn(qb, cache.k_pages[li], cache.v_pages[li], cache.block_table, lens_after,
-                                   cache.page_size, a.scale)
-                o = ob[seq_of.long()]
-            else:
-                q, k, v, _ = Fn.qk_norm_rope(qkv, a.q_norm.weight, a.k_norm.weight, sin, cos, a.H, a.G, a.Kd, eps=a.eps)
-                o = Fn.flash_attention(q, k, v, cu, T, scale=a.scale, causal=True)
-                cache.k_pages[li].view(-1, a.G, a.Kd).index_copy_(0, rows, k)
-                cache.v_pages[li].view(-1, a.G, a.Kd).index_copy_(0, rows, v.contiguous())
-            x = a.o_proj(o.reshape(N, a.H * a.Kd), residual=x)
-            hh = layer.post_norm(x)
-            x = layer.mlp(hh, residual=x)[0] if layer.is_moe else layer.mlp(hh, residual=x)
+        if N == 0:
+            return torch.zeros(0 if select is not None else B, cfg.emb_dim, dtype=self.embedder.weight.dtype, device=dev)
+        seq = real.nonzero()[:, 0]
+        hist = torch.tensor(cache.seq_lens_host)
+        slot = hist[seq] + (real.cumsum(-1) - 1)[real]
+        rows = cache.block_table_host[seq, slot // ps] * ps + slot % ps
+        cu = torch.cat([counts.new_zeros(1), counts.cumsum(0)])
+        has = counts.nonzero()[:, 0]
+        parts = dict(ids=both[0][real], seq=seq, slot=slot, rows=rows, cu=cu, lens=hist + counts, has=has, last=cu[has + 1] - 1)
+        # every part starts on a 16-byte boundary; pageable memory is staged before the copy returns
+        flat = torch.cat([F.pad(t.to(i32), (0, -t.numel() % 4)) for t in parts.values()]).to(dev, non_blocking=True)
+        batch, at = SimpleNamespace(flat=flat, every=single and N == B), 0
+        for name, t in parts.items():
+            setattr(batch, name, flat[at:at + t.numel()])
+            at += t.numel() + -t.numel() % 4
+        if batch.every and key is not None:
+            x = DecodeGraph.step(self, cache, batch, key)
+        elif single:
+            x = self.run_layers(batch, cache)
+        else:
+            x = self.embed(batch.ids)
+            sin, cos = R.rope_tables(batch.slot, cfg.head_dim, cfg.rope_theta)
+            for li, layer in enumerate(self.layers):
+                a = layer.attn
+                q, k, v, _ = Fn.qk_norm_rope(a.qkv_proj(layer.input_norm(x)), a.q_norm.weight, a.k_norm.weight, sin, cos, a.H, a.G,
+                                             a.Kd, eps=a.eps)
+                o = Fn.flash_attention(q, k, v, batch.cu, T, scale=a.scale, causal=True)
+                K.kv_store(k, v, batch.rows, cache.k_pages[li], cache.v_pages[li])
+                x = self._after_attention(layer, o, x)
         cache.advance(new_tokens)
-        x = self.final_norm(x)
         if select is not None:
-            return x[(select.to(dev) & real)[real]]
+            marked = (select.cpu() & real)[real].nonzero()[:, 0]
+            return self.final_norm(x[marked.to(dev)])
+        if batch.every:
+            return self.final_norm(x)
+        end = self.final_norm(x[batch.last.long()])
+        if has.numel() == B:
+            return end
         out = torch.zeros(B, x.shape[1], dtype=x.dtype, device=dev)
-        has = counts > 0
-        out[has] = x[last[has]]
+        out[batch.has.long()] = end
         return out
 
     def embed(self, token_ids):

@@ -17,3 +17,4 @@ class PagedKVCache(PagedSequences):
         shape = (self.num_pages, page_size, G, K)
         self.k_pages = [torch.zeros(shape, dtype=dtype, device=device) for _ in range(cfg.num_layers)]
         self.v_pages = [torch.zeros(shape, dtype=dtype, device=device) for _ in range(cfg.num_layers)]
+        self.decode_graph = None     # recorded single-token step

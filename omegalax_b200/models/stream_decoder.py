@@ -103,14 +103,22 @@ class StreamDecoder(nn.Module):
         layers keep.  Returns normed hidden rows: of every sequence's last new token [B, D] (zeros for
         sequences without one), or, with the bool mask ``select`` [B, T], of the marked tokens in order."""
         ids, real = token_ids.cpu(), segment_ids.cpu() != 0
-        tokens = [ids[b][real[b]].to(torch.int32) for b in range(cache.B)]
-        new = [int(t.numel()) for t in tokens]
+        new = real.sum(-1).tolist()
+        tokens = list(ids[real].to(torch.int32).split(new))
         cache.reserve(new)
+        cache.settle()
         if max(new, default=0) == 0:
             rows = 0 if select is not None else cache.B
             return torch.zeros(rows, self.cfg.width, dtype=self.embedder.weight.dtype, device=cache.device)
         batch = TokenBatch.build(cache, tokens)
-        x = DecodeGraph.step(self, cache, batch) if batch.single else self.run_layers(batch, cache)
+        if batch.single:
+            x = DecodeGraph.step(self, cache, batch)
+        else:
+            # A prompt's first tokens read a recurrent state of one or two products and norm what they read: next to
+            # nothing where query and key are nearly orthogonal.  So that such tokens do not depend on what they are
+            # batched with, prompts of these models keep one order of sums for all numbers of rows.
+            with S.whole_reductions(cache.recurrent):
+                x = self.run_layers(batch, cache)
         cache.advance(new)
         if select is None:
             if batch.single:

@@ -74,6 +74,34 @@ __global__ void decode_append_kernel(const bf16* __restrict__ qkv, const bf16* _
   }
 }
 
+// Keys and values of a prompt into their pages: row n of k and v (W channels, any pitch) to cache row rows[n].  blockIdx.y: 0 k, 1 v.
+// Four 16-byte groups of a thread are in flight.  8192 rows of 1024 channels: TIMEKV
+__global__ void __launch_bounds__(256)
+kv_store_kernel(const bf16* __restrict__ k, const bf16* __restrict__ v, long long ldk, long long ldv,
+                const int* __restrict__ rows, bf16* __restrict__ k_pages, bf16* __restrict__ v_pages, long long N, int W) {
+  constexpr int U = 4;
+  const bf16* src = blockIdx.y ? v : k;
+  bf16* dst = blockIdx.y ? v_pages : k_pages;
+  const long long ld = blockIdx.y ? ldv : ldk;
+  const int wv = W >> 3;
+  const long long total = N * wv, i0 = blockIdx.x * (256ll * U) + threadIdx.x;
+  uint4 x[U];
+  long long at[U];
+#pragma unroll
+  for (int t = 0; t < U; ++t) {
+    const long long i = i0 + t * 256;
+    if (i < total) {
+      const long long n = i / wv;
+      const int c = (int)(i - n * wv) * 8;
+      x[t] = *reinterpret_cast<const uint4*>(src + n * ld + c);
+      at[t] = (long long)rows[n] * W + c;
+    }
+  }
+#pragma unroll
+  for (int t = 0; t < U; ++t)
+    if (i0 + t * 256 < total) *reinterpret_cast<uint4*>(dst + at[t]) = x[t];
+}
+
 // Sums of V values over the 16 lanes of a half-warp: lane hl ends with value hl * V / 16 (V a power of two up to
 // 16).  Exchanging halves takes V - 1 + log2(16 / V) shuffles where a butterfly per value takes 4 V.
 template <int V>
@@ -336,6 +364,19 @@ int ob_decode_append(const void* qkv, const void* qw, const void* kw, const int*
     decode_append_kernel<false><<<(unsigned)blocks, 256, 0, s>>>(
         (const bf16*)qkv, (const bf16*)qw, (const bf16*)kw, positions, seq_of_token, slot_of_token, block_table,
         max_blocks, page_size, (bf16*)q_out, (bf16*)k_pages, (bf16*)v_pages, ntok, H, G, HD, rot, theta, eps);
+  OB_CHECK_LAUNCH();
+  return 0;
+}
+
+int ob_kv_store(const void* k, const void* v, long long ldk, long long ldv, const int* rows, void* k_pages, void* v_pages,
+                long long N, int W, cudaStream_t s) {
+  if (N <= 0 || W <= 0) return 0;
+  if ((W & 7) || (ldk & 7) || (ldv & 7)) return 6001;
+  if (((uintptr_t)k | (uintptr_t)v | (uintptr_t)k_pages | (uintptr_t)v_pages) & 15) return 6002;
+  const long long blocks = (N * (W / 8) + 1023) / 1024;
+  if (blocks > 0x7fffffff) return 6005;
+  kv_store_kernel<<<dim3((unsigned)blocks, 2), 256, 0, s>>>((const bf16*)k, (const bf16*)v, ldk, ldv, rows, (bf16*)k_pages,
+                                                            (bf16*)v_pages, N, W);
   OB_CHECK_LAUNCH();
   return 0;
 }

@@ -666,14 +666,14 @@ class _LinearCEFn(torch.autograd.Function):
         tgt_logit = torch.zeros(min(chunk, M), dtype=torch.float32, device=dev)
         lse = torch.empty(min(chunk, M), dtype=torch.float32, device=dev)
         fp32_stats = os.environ.get("OMEGALAX_B200_CE_STATS", "1") == "1" and h.shape[1] % 8 == 0
-        if fp32_stats and pg is None and M >= 2048:
+        if fp32_stats and pg is None and M >= 2560:
             # Rows without loss (prompts, padding) take no part in the head: the others are gathered and counted
             # on the device.  Chunks past the count return at once, so the chunk bounds need no host copy of it.
             # (With gradients that leave over NVLink the whole rows go on: that GEMM takes no count.  So do fewer than
-            # 2048 rows: such a step is bound by its launches, and 3 rows of 333 took 6.87 ms, counted 7.12.)
+            # 2560 rows: such a step is bound by its launches, and 3 rows of 333 took 6.87 ms, counted 7.12.)
             w = K._row_major_2d(w)
             count, rows, place, t32, mk = K.ce_supervised(mk, t32)
-            h = K.ce_gather(h, rows, count)
+            h, hs = K.ce_gather(h, rows, count, scale_t)
             dh = torch.zeros(M, D, dtype=torch.float32, device=dev) if need_grad else None
             for r0 in range(0, M, chunk):
                 r1 = min(M, r0 + chunk)
@@ -684,8 +684,8 @@ class _LinearCEFn(torch.autograd.Function):
                     K.ce_counted_grad_(logits[:n], t32[r0:r1], lse[:n], mk[r0:r1], scale_t, at)
                     K.gemm_counted(1, logits[:n], w, dh[r0:r1], at)
                     if dw is not None:
-                        K.gemm_counted(2, logits[:n], h[r0:r1], dw, at)
-            ctx.save_for_backward(dh, place)
+                        K.gemm_counted(2, logits[:n], hs[r0:r1], dw, at)
+            ctx.save_for_backward(dh, place, scale_t)
             ctx.counted, ctx.dw, ctx.w_dtype = True, None if mg is not None else dw, w.dtype
             return (loss_sum * scale_t).squeeze(0)
         ctx.counted = False
@@ -720,7 +720,7 @@ class _LinearCEFn(torch.autograd.Function):
         if dh is None:
             gh = None
         elif ctx.counted:
-            gh = K.ce_scatter(dh, ctx.saved_tensors[1], g.to(torch.float32).contiguous())
+            gh = K.ce_scatter(dh, ctx.saved_tensors[1], g.to(torch.float32).contiguous(), ctx.saved_tensors[2])
         else:
             gh = dh * g.to(dh.dtype)
         gw = None if dw is None else (dw * g).to(ctx.w_dtype)

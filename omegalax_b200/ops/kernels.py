@@ -342,11 +342,11 @@ _attn_scratch: dict = {}
 
 
 def attn_bwd_splits(tiles: int, H: int, G: int, steps: int) -> int:
-    """CTAs that share the query heads of a key tile: doubled while (tile, kv head) pairs leave SMs without a CTA, and
-    a CTA keeps sixteen steps of 64 queries.  32 heads on 4, one row of 4096 (128 pairs): 1062 us, with two CTAs
+    """CTAs that share the query heads of a key tile: doubled while (tile, kv head) pairs leave SMs without a second CTA,
+    and a CTA keeps sixteen steps of 64 queries.  32 heads on 4, one row of 4096 (128 pairs): 1062 us, with two CTAs
     580, with four 576; on 8, two rows of 4096 (512 pairs): 1076, 1147, 1289 (partial sums to store and add)."""
     n, R = 1, H // G
-    while tiles * G * n < 200 and R % (2 * n) == 0 and R // (2 * n) * steps >= 16:
+    while tiles * G * n < 250 and R % (2 * n) == 0 and R // (2 * n) * steps >= 16:
         n *= 2
     return n
 
@@ -369,7 +369,9 @@ def attn_bwd(q, k, v, o, lse, do, cu_seqlens, max_seqlen, scale, causal, dk_out=
         _attn_scratch[key] = scratch
     dq_acc, delta = scratch
     if splits is None:
-        splits = attn_bwd_splits(-(-int(max_seqlen) // 128) * (cu_seqlens.numel() - 1) * (Kd // 128), H, G, -(-int(max_seqlen) // 64))
+        B = cu_seqlens.numel() - 1     # empty sequences (no padding on the left) among them
+        tiles = min(-(-int(max_seqlen) // 128) * B, N // 128 + B)
+        splits = attn_bwd_splits(tiles * (Kd // 128), H, G, -(-int(max_seqlen) // 64))
     part = torch.empty(splits, 2, N, G * Kd, dtype=torch.float32, device=q.device) if splits > 1 else None
     st = lib.status_tensor(q.device)
     _call("ob_attn_bwd", q.data_ptr(), k.data_ptr(), v.data_ptr(), o.data_ptr(), do.data_ptr(),
@@ -424,24 +426,26 @@ def ce_supervised(mask, targets):
     return count, rows, place, tgt, mk
 
 
-def ce_gather(h, rows, count):
-    """The counted rows of h [M, D] first; what follows their next multiple of 64 stays unwritten."""
-    out = torch.empty_like(h)
-    _call("ob_ce_gather", h.data_ptr(), rows.data_ptr(), count.data_ptr(), out.data_ptr(), h.shape[0], h.shape[1],
-          lib.stream_ptr())
-    return out
+def ce_gather(h, rows, count, scale):
+    """The counted rows of h [M, D] first, and the same times what ``scale`` (fp32 [1]) is beyond a power of two; what
+    follows their next multiple of 64 stays unwritten."""
+    out, scaled = torch.empty_like(h), torch.empty_like(h)
+    _call("ob_ce_gather", h.data_ptr(), rows.data_ptr(), count.data_ptr(), scale.data_ptr(), out.data_ptr(), scaled.data_ptr(),
+          h.shape[0], h.shape[1], lib.stream_ptr())
+    return out, scaled
 
 
-def ce_scatter(dh, place, g):
-    """bf16 rows: g times row ``place`` of fp32 ``dh``, or zero."""
+def ce_scatter(dh, place, g, scale):
+    """bf16 rows: g and what ``scale`` is beyond a power of two times row ``place`` of fp32 ``dh``, or zero."""
     out = torch.empty(dh.shape, dtype=bf16, device=dh.device)
-    _call("ob_ce_scatter", dh.data_ptr(), place.data_ptr(), g.data_ptr(), out.data_ptr(), dh.shape[0], dh.shape[1],
+    _call("ob_ce_scatter", dh.data_ptr(), place.data_ptr(), g.data_ptr(), scale.data_ptr(), out.data_ptr(), dh.shape[0], dh.shape[1],
           lib.stream_ptr())
     return out
 
 
 def ce_counted_grad_(logits, targets, lse, mask, grad_scale, counted):
-    """Logits -> dlogits in place for the counted rows, zeros up to their next multiple of 64."""
+    """Logits -> dlogits over what ``grad_scale`` is beyond a power of two, in place for the counted rows; zeros up to
+    their next multiple of 64."""
     R, V = logits.shape
     _call("ob_ce_counted_grad", logits.data_ptr(), R, V, logits.stride(0), targets.data_ptr(), lse.data_ptr(), mask.data_ptr(),
           grad_scale.data_ptr(), counted[0].data_ptr(), counted[1], lib.stream_ptr())
@@ -539,6 +543,17 @@ def decode_append(qkv, qw, kw, positions, seq_of_token, slot_of_token, block_tab
           page_size, q.data_ptr(), k_pages.data_ptr(), v_pages.data_ptr(), n, H, G, HD, rot, float(theta),
           float(eps), int(one_plus), lib.stream_ptr())
     return q
+
+
+def kv_store(k, v, rows, k_pages, v_pages):
+    """k, v [N, G, HD] (row-strided views allowed) into rows ``rows`` (int32 [N]) of [*, G, HD] pages."""
+    N, G, HD = k.shape
+    lib.check_index("kv_store rows", rows, k_pages.numel() // (G * HD))
+    for t in (k, v):
+        if t.stride(2) != 1 or t.stride(1) != HD or t.dtype != k_pages.dtype:
+            raise ValueError("keys and values need contiguous heads in the type of the pages")
+    _call("ob_kv_store", k.data_ptr(), v.data_ptr(), k.stride(0), v.stride(0), rows.data_ptr(), k_pages.data_ptr(), v_pages.data_ptr(),
+          N, G * HD, lib.stream_ptr())
 
 
 def decode_attn(q, k_pages, v_pages, block_table, seq_lens, page_size, scale, splits=None):

@@ -7,6 +7,9 @@ exact single precision and its matrix products are cuBLAS SGEMMs.  There is no C
 """
 from __future__ import annotations
 
+import contextlib
+import threading
+
 import torch
 import torch.nn.functional as F
 
@@ -41,6 +44,19 @@ def _contig(*ts) -> None:
 
 
 # ----------------------------------------------------------------------------------------------- products
+_calls = threading.local()
+
+
+@contextlib.contextmanager
+def whole_reductions(on: bool = True):
+    """``project`` calls of this thread sum every reduction in one go, whatever the number of rows."""
+    before, _calls.whole = getattr(_calls, "whole", False), on
+    try:
+        yield
+    finally:
+        _calls.whole = before
+
+
 def project(x, w, *, out_dtype=None, into=None):
     """x [M, K] @ w [N, K]^T in ``out_dtype`` (default: that of x), or added into the fp32 rows
     ``into``.  bf16 products run on the tcgen05 GEMM; sizes it cannot address are zero-padded."""
@@ -49,15 +65,16 @@ def project(x, w, *, out_dtype=None, into=None):
             return into.addmm_(x, w.t())
         return x @ w.t()
     N, Kd = w.shape
+    few = False if getattr(_calls, "whole", False) else None
     if Kd % 8:
         x, w = F.pad(x, (0, 8 - Kd % 8)), F.pad(w, (0, 8 - Kd % 8))
     if into is not None:
         if N % 8 == 0:
-            return K.gemm(x, w, out=into, accumulate=True)
+            return K.gemm(x, w, out=into, accumulate=True, few=few)
         return into.add_(project(x, w, out_dtype=f32))
     if N % 8:
         w = F.pad(w, (0, 0, 0, 8 - N % 8))
-    y = K.gemm(x, w, out_dtype=out_dtype or bf16)
+    y = K.gemm(x, w, out_dtype=out_dtype or bf16, few=few)
     return y[:, :N] if N % 8 else y
 
 

@@ -47,5 +47,5 @@ def chunked_cross_entropy_loss(hidden_BTD, lm_head_VD, targets_BT, mask_BT, num_
     if h.is_cuda:
         # every chunk of rows adds into the whole fp32 gradient of the head: 4096 rows and more keep its
         # traffic (0.4 ms for 152k x 2048) under the time of the chunk's product (1.7 ms)
-        chunk = min(max(chunk, 4096 if rows >= 2048 else 1024), 8192)
+        chunk = min(max(chunk, 4096 if rows >= 2560 else 1024), 8192)
     return Fn.linear_cross_entropy(h, lm_head_VD, tgt, mask, scale, chunk=chunk)

@@ -353,6 +353,26 @@ def test_gemm_grouped_and_wgrad(pair):
         _assert_gemm_close(dw[e], ref, max(b - a, 1))
 
 
+@pytest.mark.parametrize("M", [1, 9, 1000])
+@pytest.mark.parametrize("D", [8, 1032, 2048, 4104, 8192])
+def test_rmsnorm_backward_rows(M, D):
+    """Fewer rows than CTAs, several rows per CTA, ragged columns; added to what dw holds.  dx is one rounding to bf16 of
+    values of size one (2^-8), dw a sum of M products in fp32; the normalisation is taken from x where it was not kept."""
+    from omegalax_b200.ops import kernels as Kn, lib
+    torch.manual_seed(36)
+    x, dy = (torch.randn(M, D, device=_dev()).to(bf16) for _ in range(2))
+    w = (1 + 0.1 * torch.randn(D, device=_dev())).to(bf16)
+    xr, wr = x.double().requires_grad_(True), w.double().requires_grad_(True)
+    (xr * torch.rsqrt(xr.square().mean(-1, keepdim=True) + 1e-6) * wr).backward(dy.double())
+    for rstd in (None, torch.rsqrt(x.float().square().mean(-1) + 1e-6)):
+        dw = torch.full((D,), 0.5, device=_dev())
+        dx = Kn.rmsnorm_bwd(dy, x, w, rstd, 1e-6, dw)
+        _check(lib)
+        torch.testing.assert_close(dx.double(), xr.grad, rtol=2.0 ** -8, atol=2.0 ** -10)
+        torch.testing.assert_close(dw.double() - 0.5, wr.grad, rtol=1e-4, atol=1e-5 * math.sqrt(M))
+    assert torch.equal(Kn.rmsnorm_bwd(dy, x, w, rstd, 1e-6, None), dx)
+
+
 @pytest.mark.parametrize("D", [64, 1024, 4096])
 @pytest.mark.parametrize("one_plus", [False, True])
 def test_rmsnorm(D, one_plus):
@@ -505,8 +525,8 @@ def test_linear_cross_entropy():
     assert _rel_err(w.grad, wr.grad) < 3e-2
 
 
-@pytest.mark.parametrize("M,n,chunk", [(2048, 0, 1024), (2050, 1, 1024), (2050, 63, 1024), (2050, 64, 1024), (2050, 1025, 1024),
-                                       (2112, 2112, 4096), (2500, 1537, 512)])
+@pytest.mark.parametrize("M,n,chunk", [(2560, 0, 1024), (2570, 1, 1024), (2570, 63, 1024), (2570, 64, 1024), (2570, 1025, 1024),
+                                       (2624, 2624, 4096), (3000, 1537, 512)])
 @pytest.mark.parametrize("main_grad", [False, True])
 def test_linear_cross_entropy_supervised_rows(M, n, chunk, main_grad):
     """Counts around the 64-row blocks of the weight gradient, the 512-row tiles and the chunks; V and D leave ragged tiles.
