@@ -660,13 +660,16 @@ class _LinearCEFn(torch.autograd.Function):
             dw = mg if mg is not None else torch.zeros(V, D, dtype=torch.float32, device=dev)
         t32 = targets.to(torch.int32).contiguous()
         mk = mask.to(torch.float32).contiguous()
+        fp32_stats = os.environ.get("OMEGALAX_B200_CE_STATS", "1") == "1" and h.shape[1] % 8 == 0
+        counted = fp32_stats and pg is None and M >= 2560
+        if counted:      # a chunk starts on a block of 64 rows, to which the gathered rows are filled up with zeros
+            chunk = -(-chunk // 64) * 64
         logits = torch.empty(min(chunk, M), V, dtype=bf16, device=dev)
         n_tiles = -(-V // 256)
         stats = torch.empty(min(chunk, M), n_tiles, 2, dtype=torch.float32, device=dev)
         tgt_logit = torch.zeros(min(chunk, M), dtype=torch.float32, device=dev)
         lse = torch.empty(min(chunk, M), dtype=torch.float32, device=dev)
-        fp32_stats = os.environ.get("OMEGALAX_B200_CE_STATS", "1") == "1" and h.shape[1] % 8 == 0
-        if fp32_stats and pg is None and M >= 2560:
+        if counted:
             # Rows without loss (prompts, padding) take no part in the head: the others are gathered and counted
             # on the device.  Chunks past the count return at once, so the chunk bounds need no host copy of it.
             # (With gradients that leave over NVLink the whole rows go on: that GEMM takes no count.  So do fewer than

@@ -559,6 +559,34 @@ def test_linear_cross_entropy_supervised_rows(M, n, chunk, main_grad):
         assert not dw.any()
 
 
+@pytest.mark.parametrize("n", [1030, 1031, 1088, 1089, 2061, 2112, 2570])
+def test_linear_cross_entropy_chunks_off_the_row_blocks(monkeypatch, n):
+    """Chunks that are no multiple of the 64-row blocks, with counts just past a chunk's start and on either side of a block's
+    edge: rows that nothing wrote must not reach the gradient, so they hold NaN here.  Tolerance as above."""
+    from omegalax_b200.ops import functional as Fn, kernels as Kn, lib
+    torch.manual_seed(37)
+    M, D, V = 2570, 264, 2056
+    h = torch.randn(M, D, device=_dev()).to(bf16).requires_grad_(True)
+    w = (torch.randn(V, D, device=_dev()) * 0.1).to(bf16).requires_grad_(True)
+    y = torch.randint(0, V, (M,), device=_dev(), dtype=torch.int32)
+    mask = torch.zeros(M, device=_dev())
+    mask[torch.randperm(M, device=_dev())[:n]] = 1
+    with monkeypatch.context() as mp:
+        mp.setattr(torch, "empty_like", lambda t, **kw: torch.full_like(t, float("nan"), **kw))
+        loss = Fn.linear_cross_entropy(h, w, y, mask, 1.0 / n, chunk=1030)
+    loss.backward()
+    _check(lib)
+    hr, wr = h.detach().double().requires_grad_(True), w.detach().double().requires_grad_(True)
+    ref = (torch.nn.functional.cross_entropy(hr @ wr.t(), y.long(), reduction="none") * mask).sum() / n
+    ref.backward()
+    assert abs(float(loss) - float(ref)) <= 1e-5 * abs(float(ref))
+    assert torch.isfinite(w.grad).all() and torch.isfinite(h.grad).all()
+    assert _rel_err(h.grad, hr.grad) < 3e-2 and _rel_err(w.grad, wr.grad) < 3e-2
+    with pytest.raises(lib.KernelError):      # a chunk that starts inside a block
+        Kn.gemm_counted(2, h.detach()[8:72, :256], h.detach()[8:72], torch.zeros(256, D, device=_dev()),
+                        (torch.tensor([72], dtype=torch.int32, device=_dev()), 8))
+
+
 def test_embedding_and_optimizer_kernels():
     from omegalax_b200.ops import kernels as Kn, lib
     torch.manual_seed(9)
