@@ -761,32 +761,20 @@ __global__ void __launch_bounds__(1024) ce_count_kernel(const float* __restrict_
 
 // dlogits are rounded to bf16, and the largest of a row, (p - 1) times the loss's scale, has nearly the same value
 // in every row: the rounding of the scale would be an error of one sign in all gradients (5e-4 at 2440 rows).
-// So dlogits carry the scale's power of two only; the rest, in [1, 2), goes into the rows of the weight
-// gradient's other operand and, in fp32, into the hidden rows' gradient.
-__device__ __forceinline__ float scale_pow2(float s) { return s != 0.f && isfinite(s) ? ldexpf(s < 0.f ? -1.f : 1.f, ilogbf(s)) : s; }
-__device__ __forceinline__ float scale_rest(float s) { return s != 0.f && isfinite(s) ? s / scale_pow2(s) : 1.f; }
+// So dlogits carry the scale's power of two only; the rest, in [1, 2), meets both gradients in fp32: the weight's as it
+// leaves the accumulator, the hidden rows' when they go back to their places.
 
-// Hidden rows in that order, and times the rest of the scale; the reduction of the weight gradient runs in blocks of
-// 64 rows, so the rows after the last one are zeroed that far.
+// Hidden rows in that order; the reduction of the weight gradient runs in blocks of 64 rows, so the rows
+// after the last one are zeroed that far.
 __global__ void ce_gather_kernel(const bf16* __restrict__ h, const int* __restrict__ rows, const int* __restrict__ count,
-                                 const float* __restrict__ scale, bf16* __restrict__ out, bf16* __restrict__ scaled, long long M,
-                                 int D) {
+                                 bf16* __restrict__ out, long long M, int D) {
   const int dv = D >> 3;
-  const float rest = scale_rest(*scale);
   const long long n = *count, end = min((n + 63) / 64 * 64, M);
   for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < end * dv; t += (long long)gridDim.x * blockDim.x) {
     const long long c = t / dv;
     const int i = (int)(t - c * dv);
-    uint4 x = make_uint4(0, 0, 0, 0);
-    if (c < n) x = reinterpret_cast<const uint4*>(h + (long long)rows[c] * D)[i];
-    reinterpret_cast<uint4*>(out + c * D)[i] = x;
-    uint32_t* u = &x.x;
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const float2 f = unpack_bf16(u[j]);
-      u[j] = pack_bf16(f.x * rest, f.y * rest);
-    }
-    reinterpret_cast<uint4*>(scaled + c * D)[i] = x;
+    reinterpret_cast<uint4*>(out + c * D)[i] =
+        c < n ? reinterpret_cast<const uint4*>(h + (long long)rows[c] * D)[i] : make_uint4(0, 0, 0, 0);
   }
 }
 
@@ -1202,11 +1190,10 @@ int ob_ce_count(const float* mask, const int* targets, long long M, int* rows, i
   return 0;
 }
 
-int ob_ce_gather(const void* h, const int* rows, const int* count, const float* scale, void* out, void* scaled, long long M, int D,
-                 cudaStream_t s) {
+int ob_ce_gather(const void* h, const int* rows, const int* count, void* out, long long M, int D, cudaStream_t s) {
   if (D % 8) return 6001;
   if (M <= 0) return 0;
-  ce_gather_kernel<<<grid_for(M * (D / 8), 256), 256, 0, s>>>((const bf16*)h, rows, count, scale, (bf16*)out, (bf16*)scaled, M, D);
+  ce_gather_kernel<<<grid_for(M * (D / 8), 256), 256, 0, s>>>((const bf16*)h, rows, count, (bf16*)out, M, D);
   OB_CHECK_LAUNCH();
   return 0;
 }

@@ -62,6 +62,8 @@ struct GemmArgs {
   // rows of C (rows_in_k 0) or the reduction (rows_in_k 1); the reduction is then cut on the device.
   const int* rows_dev;
   int rows_off, rows_in_k;
+  // with rows_in_k: the product times scale_rest(*scale_dev), in fp32 before it is added to C
+  const float* scale_dev;
   int* status;
 };
 

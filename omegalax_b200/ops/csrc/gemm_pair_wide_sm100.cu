@@ -356,6 +356,7 @@ gemm_bf16_pair_wide_kernel(const __grid_constant__ CUtensorMap tmA, const __grid
           if (do_ce) p.ce_stats[my_grow * p.num_n_blocks + (ti.c_col0 / kWideBN)] = make_float2(ce_m, ce_s);
         } else if (tma_out) {
           // fp32 store / accumulate: 32 columns (128 bytes per row) per bulk tensor store / reduce-add
+          const float rest = p.scale_dev ? scale_rest(__ldg(p.scale_dev)) : 1.f;
 #pragma unroll 1
           for (int c32 = 0; c32 < kWideBN / 32; ++c32) {
             uint32_t v[32];
@@ -365,6 +366,10 @@ gemm_bf16_pair_wide_kernel(const __grid_constant__ CUtensorMap tmA, const __grid
             } else {
 #pragma unroll
               for (int i = 0; i < 32; ++i) v[i] = 0;
+            }
+            if (p.scale_dev) {
+#pragma unroll
+              for (int i = 0; i < 32; ++i) v[i] = __float_as_uint(__uint_as_float(v[i]) * rest);
             }
             if (lane == 0) tma_store_wait_read<1>();
             __syncwarp();
@@ -397,6 +402,11 @@ gemm_bf16_pair_wide_kernel(const __grid_constant__ CUtensorMap tmA, const __grid
             } else {
 #pragma unroll
               for (int i = 0; i < 32; ++i) v[i] = 0;
+            }
+            if (p.scale_dev) {
+              const float rest = scale_rest(__ldg(p.scale_dev));
+#pragma unroll
+              for (int i = 0; i < 32; ++i) v[i] = __float_as_uint(__uint_as_float(v[i]) * rest);
             }
             const int col0 = ti.c_col0 + c * 32;
             const int ncols = min(32, ti.cols_valid - c * 32);

@@ -448,4 +448,8 @@ __device__ __forceinline__ float warp_max(float v) {
   return v;
 }
 
+// A scale s as a power of two of its sign times a rest in [1, 2); zero, infinity and NaN stay whole.
+__device__ __forceinline__ float scale_pow2(float s) { return s != 0.f && isfinite(s) ? ldexpf(s < 0.f ? -1.f : 1.f, ilogbf(s)) : s; }
+__device__ __forceinline__ float scale_rest(float s) { return s != 0.f && isfinite(s) ? s / scale_pow2(s) : 1.f; }
+
 }  // namespace ob

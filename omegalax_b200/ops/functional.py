@@ -676,7 +676,7 @@ class _LinearCEFn(torch.autograd.Function):
             # 2560 rows: such a step is bound by its launches, and 3 rows of 333 took 6.87 ms, counted 7.12.)
             w = K._row_major_2d(w)
             count, rows, place, t32, mk = K.ce_supervised(mk, t32)
-            h, hs = K.ce_gather(h, rows, count, scale_t)
+            h = K.ce_gather(h, rows, count)
             dh = torch.zeros(M, D, dtype=torch.float32, device=dev) if need_grad else None
             for r0 in range(0, M, chunk):
                 r1 = min(M, r0 + chunk)
@@ -687,7 +687,7 @@ class _LinearCEFn(torch.autograd.Function):
                     K.ce_counted_grad_(logits[:n], t32[r0:r1], lse[:n], mk[r0:r1], scale_t, at)
                     K.gemm_counted(1, logits[:n], w, dh[r0:r1], at)
                     if dw is not None:
-                        K.gemm_counted(2, logits[:n], hs[r0:r1], dw, at)
+                        K.gemm_counted(2, logits[:n], h[r0:r1], dw, at, scale=scale_t)
             ctx.save_for_backward(dh, place, scale_t)
             ctx.counted, ctx.dw, ctx.w_dtype = True, None if mg is not None else dw, w.dtype
             return (loss_sum * scale_t).squeeze(0)

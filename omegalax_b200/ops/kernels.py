@@ -426,13 +426,11 @@ def ce_supervised(mask, targets):
     return count, rows, place, tgt, mk
 
 
-def ce_gather(h, rows, count, scale):
-    """The counted rows of h [M, D] first, and the same times what ``scale`` (fp32 [1]) is beyond a power of two; what
-    follows their next multiple of 64 stays unwritten."""
-    out, scaled = torch.empty_like(h), torch.empty_like(h)
-    _call("ob_ce_gather", h.data_ptr(), rows.data_ptr(), count.data_ptr(), scale.data_ptr(), out.data_ptr(), scaled.data_ptr(),
-          h.shape[0], h.shape[1], lib.stream_ptr())
-    return out, scaled
+def ce_gather(h, rows, count):
+    """The counted rows of h [M, D] first, then zeros up to their next multiple of 64; what follows stays unwritten."""
+    out = torch.empty_like(h)
+    _call("ob_ce_gather", h.data_ptr(), rows.data_ptr(), count.data_ptr(), out.data_ptr(), h.shape[0], h.shape[1], lib.stream_ptr())
+    return out
 
 
 def ce_scatter(dh, place, g, scale):
@@ -451,10 +449,10 @@ def ce_counted_grad_(logits, targets, lse, mask, grad_scale, counted):
           grad_scale.data_ptr(), counted[0].data_ptr(), counted[1], lib.stream_ptr())
 
 
-def gemm_counted(kind: int, a, b, out, counted, ce=None):
+def gemm_counted(kind: int, a, b, out, counted, ce=None, scale=None):
     """The head's products when only the first ``counted[0]`` (int32 [1] on the device) - ``counted[1]`` rows
     of ``a`` hold anything.  kind 0: out bf16 = a b^T with the statistics ``ce``; kind 1: out fp32 += a b;
-    kind 2: out fp32 += a^T b."""
+    kind 2: out fp32 += a^T b, times what ``scale`` (fp32 [1]) is beyond a power of two."""
     (M, K) = (a.shape[1], a.shape[0]) if kind == 2 else a.shape
     N = b.shape[1] if kind else b.shape[0]
     ce_ptrs = (None, None, None) if ce is None else (ce[0].data_ptr(), ce[1].data_ptr(), ce[2].data_ptr())
@@ -464,7 +462,7 @@ def gemm_counted(kind: int, a, b, out, counted, ce=None):
         if t.stride(1) != 1:
             raise ValueError("row-major operands expected")
     _call("ob_gemm_counted_rows", kind, a.data_ptr(), b.data_ptr(), out.data_ptr(), M, N, K, a.stride(0), b.stride(0), out.stride(0),
-          counted[0].data_ptr(), counted[1], *ce_ptrs, lib.status_tensor(a.device).data_ptr(), lib.stream_ptr())
+          counted[0].data_ptr(), counted[1], *ce_ptrs, lib.ptr(scale), lib.status_tensor(a.device).data_ptr(), lib.stream_ptr())
     return out
 
 

@@ -33,7 +33,7 @@ _SIGS = {
     "ob_gemm_bf16_pair_peer_reduce": [P, P, P, I, I, I, I, I, L, L, L, I, I, I, I, P, P],
     "ob_gemm_bf16_pair": [P, P, P, P, I, I, I, L, L, L, L, I, I, I, P, P, P, P, P, P],
     "ob_gemm_few": [P, P, P, P, I, I, I, L, L, L, L, I, P, I, P, P],
-    "ob_gemm_counted_rows": [I, P, P, P, I, I, I, L, L, L, P, I, P, P, P, P, P],
+    "ob_gemm_counted_rows": [I, P, P, P, I, I, I, L, L, L, P, I, P, P, P, P, P, P],
     "ob_gemm_bf16_pair_ag": [P, P, P, P, P, I, I, I, L, L, I, I, I, I, I, P, c_uint, I, P, P],
     "ob_gemm_bf16_ag": [P, P, P, P, P, I, I, I, L, L, I, I, I, I, I, P, c_uint, I, P, P],
     "ob_gemm_bf16_peer_reduce": [P, P, P, I, I, I, I, I, L, L, L, I, I, I, I, P, P],
@@ -91,7 +91,7 @@ _SIGS = {
     "ob_sigmoid_gate_bwd": [P, P, P, P, P, L, I, I, L, L, P],
     "ob_ce_finish": [P, I, P, P, P, P, L, P, I, P],
     "ob_ce_count": [P, P, L, P, P, P, P, P, P],
-    "ob_ce_gather": [P, P, P, P, P, P, L, I, P],
+    "ob_ce_gather": [P, P, P, P, L, I, P],
     "ob_ce_scatter": [P, P, P, P, P, L, I, P],
     "ob_ce_counted_grad": [P, L, I, L, P, P, P, P, P, I, P],
     "ob_ce_vp_stats": [P, L, I, L, I, P, P, P, P, P],

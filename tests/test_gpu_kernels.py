@@ -587,6 +587,24 @@ def test_linear_cross_entropy_chunks_off_the_row_blocks(monkeypatch, n):
                         (torch.tensor([72], dtype=torch.int32, device=_dev()), 8))
 
 
+def test_linear_cross_entropy_rounds_only_dlogits():
+    """The weight gradient's operands are bf16 dlogits and the hidden rows as they are.  With one supervised row it is an outer
+    product, exact but for one fp32 rounding of the rest of the scale 1/3: columns over the row's elements agree to 2^-21."""
+    from omegalax_b200.ops import functional as Fn, lib
+    torch.manual_seed(38)
+    M, D, V = 2570, 264, 2056
+    h = torch.randn(M, D, device=_dev()).to(bf16).requires_grad_(True)
+    w = (torch.randn(V, D, device=_dev()) * 0.1).to(bf16).requires_grad_(True)
+    w.main_grad = torch.zeros(V, D, device=_dev())
+    mask = torch.zeros(M, device=_dev())
+    mask[1234] = 1
+    y = torch.randint(0, V, (M,), device=_dev(), dtype=torch.int32)
+    Fn.linear_cross_entropy(h, w, y, mask, 1.0 / 3).backward()
+    _check(lib)
+    ratio = w.main_grad.double() / h.detach()[1234].double()
+    assert ((ratio / ratio[:, :1] - 1).abs() < 2.0 ** -21).all()
+
+
 def test_embedding_and_optimizer_kernels():
     from omegalax_b200.ops import kernels as Kn, lib
     torch.manual_seed(9)
