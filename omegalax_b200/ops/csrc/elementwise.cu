@@ -1192,6 +1192,7 @@ int ob_ce_count(const float* mask, const int* targets, long long M, int* rows, i
 
 int ob_ce_gather(const void* h, const int* rows, const int* count, void* out, long long M, int D, cudaStream_t s) {
   if (D % 8) return 6001;
+  if (((uintptr_t)h | (uintptr_t)out) & 15) return 6002;
   if (M <= 0) return 0;
   ce_gather_kernel<<<grid_for(M * (D / 8), 256), 256, 0, s>>>((const bf16*)h, rows, count, (bf16*)out, M, D);
   OB_CHECK_LAUNCH();
