@@ -246,6 +246,10 @@ def vocab_parallel_head(cfg, tp_size: int) -> bool:
     return tp_size > 1 and not cfg.tie_word_embeddings and cfg.vocab_size % (8 * tp_size) == 0
 
 
+_STEP_METHODS = frozenset(("forward", "embed", "run_layers", "_after_attention"))
+_PLAIN = frozenset((int, float, bool))
+
+
 class Qwen3(nn.Module):
     """Returns the final hidden states (before lm_head) and the summed auxiliary loss; the
     lm_head is a separate projection applied by callers (loss, decode)."""
@@ -286,17 +290,29 @@ class Qwen3(nn.Module):
         return self.lm_head(hidden)
 
     def _recordable(self, cache):
-        """Key under which a recorded single-token step may be replayed: the modules that run and where weights and
-        pages lie.  None: hooks want to see every call, or experts are routed (their buffers follow the routing)."""
-        mods, ptrs = [], [t.data_ptr() for t in (cache.block_table, *cache.k_pages, *cache.v_pages)]
-        if _module_hooks._global_forward_hooks or _module_hooks._global_forward_pre_hooks or lib.debug_enabled():
+        """Key under which a recorded single-token step may be replayed: all that ``run_layers`` reads besides its batch, so that a
+        step whose key differs is recorded anew.  None: hooks or replaced methods want to see every call, experts are routed (their
+        buffers follow the routing), weights are gathered from other GPUs, or layer outputs are being stashed."""
+        if (_module_hooks._global_forward_hooks or _module_hooks._global_forward_pre_hooks or lib.debug_enabled()
+                or Fn._ACTIVE_STASH is not None):
             return None
-        for m in self.modules():
-            if m._forward_hooks or m._forward_pre_hooks or getattr(m, "is_moe", False):
+        key = [Fn.use_kernels(self.embedder.weight), Fn.library_mode(), self.cfg.rope_theta, cache.page_size, cache.B]
+        key += [t.data_ptr() for t in (cache.block_table, *cache.k_pages, *cache.v_pages)]
+        left = [self]
+        while left:
+            m = left.pop()
+            own = m.__dict__
+            if own["_forward_hooks"] or own["_forward_pre_hooks"] or own.get("is_moe") or not _STEP_METHODS.isdisjoint(own):
                 return None
-            mods.append(m)
-            ptrs.extend(p.data_ptr() for p in m._parameters.values() if p is not None)
-        return tuple(mods), tuple(ptrs)
+            key += (m, type(m).forward)
+            key += [v for v in own.values() if v.__class__ in _PLAIN]      # eps, scale, heads, ...
+            for p in own["_parameters"].values():
+                if p is not None:
+                    if hasattr(p, "ag_spec"):
+                        return None
+                    key += (p.data_ptr(), p.dtype, p.shape, p.stride())
+            left += [c for c in own["_modules"].values() if c is not None]
+        return key
 
     @torch.no_grad()
     def run_layers(self, batch, cache):
