@@ -261,16 +261,16 @@ __global__ void __launch_bounds__(256, 1) gdn_fwd_kernel(GdnArgs p) {
       float x[GC];
 #pragma unroll
       for (int i = 0; i < GC; ++i) {
-        float s[4] = {n_s[i * LDU + tid], 0.f, 0.f, 0.f};     // four chains: one would be 2016 dependent steps
+        float s = n_s[i * LDU + tid];
 #pragma unroll
         for (int q4 = 0; q4 < (i + 3) / 4; ++q4) {
           const float4 l = *reinterpret_cast<const float4*>(L_s + i * LDC_ + 4 * q4);
-          if (4 * q4 + 0 < i) s[0] = fmaf(-l.x, x[4 * q4 + 0], s[0]);
-          if (4 * q4 + 1 < i) s[1] = fmaf(-l.y, x[4 * q4 + 1], s[1]);
-          if (4 * q4 + 2 < i) s[2] = fmaf(-l.z, x[4 * q4 + 2], s[2]);
-          if (4 * q4 + 3 < i) s[3] = fmaf(-l.w, x[4 * q4 + 3], s[3]);
+          if (4 * q4 + 0 < i) s = fmaf(-l.x, x[4 * q4 + 0], s);
+          if (4 * q4 + 1 < i) s = fmaf(-l.y, x[4 * q4 + 1], s);
+          if (4 * q4 + 2 < i) s = fmaf(-l.z, x[4 * q4 + 2], s);
+          if (4 * q4 + 3 < i) s = fmaf(-l.w, x[4 * q4 + 3], s);
         }
-        x[i] = (s[0] + s[1]) + (s[2] + s[3]);
+        x[i] = s;
       }
       float* no = p.n_out ? p.n_out + (row0 * p.H + h) * U + u0 + tid : nullptr;
 #pragma unroll
@@ -410,16 +410,16 @@ __global__ void __launch_bounds__(256, 1) gdn_bwd_kernel(GdnArgs p) {
       float x[GC];
 #pragma unroll
       for (int i = GC - 1; i >= 0; --i) {
-        float s[4] = {dr_s[i * BLDU + tid], 0.f, 0.f, 0.f};
+        float s = dr_s[i * BLDU + tid];
 #pragma unroll
         for (int q4 = (i + 1) / 4; q4 < GC / 4; ++q4) {
           const float4 l = *reinterpret_cast<const float4*>(M_s + i * LDC_ + 4 * q4);
-          if (4 * q4 + 0 > i) s[0] = fmaf(-l.x, x[4 * q4 + 0], s[0]);
-          if (4 * q4 + 1 > i) s[1] = fmaf(-l.y, x[4 * q4 + 1], s[1]);
-          if (4 * q4 + 2 > i) s[2] = fmaf(-l.z, x[4 * q4 + 2], s[2]);
-          if (4 * q4 + 3 > i) s[3] = fmaf(-l.w, x[4 * q4 + 3], s[3]);
+          if (4 * q4 + 0 > i) s = fmaf(-l.x, x[4 * q4 + 0], s);
+          if (4 * q4 + 1 > i) s = fmaf(-l.y, x[4 * q4 + 1], s);
+          if (4 * q4 + 2 > i) s = fmaf(-l.z, x[4 * q4 + 2], s);
+          if (4 * q4 + 3 > i) s = fmaf(-l.w, x[4 * q4 + 3], s);
         }
-        x[i] = (s[0] + s[1]) + (s[2] + s[3]);
+        x[i] = s;
       }
       float* dvp = p.dv + (row0 * p.H + h) * U + u0 + tid;
 #pragma unroll
