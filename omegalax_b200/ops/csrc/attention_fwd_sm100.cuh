@@ -58,9 +58,6 @@ __device__ __forceinline__ uint32_t bits_between(int lo, int hi) {
   return upto & from;
 }
 
-template <bool V>
-struct AttnFlag { static constexpr bool value = V; };
-
 // two single-precision multiply-adds in one instruction
 __device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
   float2 d;
@@ -81,7 +78,7 @@ struct AttnFwdSmem {
   static constexpr int kTotal = kBarOff + 256 + 1024;
 };
 
-template <int QB, int VB, int KST, int VST, bool kWindow = false>
+template <int QB, int VB, int KST, int VST, bool kWindow, bool kOnce>
 __global__ void __launch_bounds__(kAttnThreads, 1)
 attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                 const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmQ2,
@@ -286,32 +283,53 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
       const bool need_mask = (kbase + 128 > seqlen) || (p.causal && kbase + 127 > q0 + w * 128) ||
                              (kWindow && p.window > 0 && kbase <= q0 + w * 128 + 127 - p.window);
       const int klimit = p.causal ? min(seqlen - 1, qpos) : seqlen - 1;  // last visible key
-      // The whole row of scores stays in registers between maximum and exponentials: four loads in flight and one wait,
-      // where two passes of four loads waited eight times (32 heads on 8, two rows of 4096: 404 us, now 360).
-      uint32_t v[128];
-#pragma unroll
-      for (int c = 0; c < 4; ++c) tmem_ld32(s_addr + c * 32, v + c * 32);
-      tmem_ld_wait();
       const int lim = klimit - kbase;      // last visible column
-      float mx4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
-      if (kWindow && need_mask) {          // hidden scores become -inf, their exponentials 0
+      float mx = -INFINITY;
+      uint32_t v[kOnce ? 128 : 1];
+      if constexpr (kOnce) {
+        // The whole row of scores stays in registers between maximum and exponentials: four loads in flight and one wait,
+        // where two passes of four loads wait eight times (32 heads on 8, two rows of 4096: 373 us, 339 so).
+        // Hidden scores become -inf, their exponentials 0, and a masked tile is like any other from there; a warp
+        // looks only at groups past the columns that its first row sees.
 #pragma unroll
-        for (int c = 0; c < 4; ++c) {
-          const uint32_t seen = bits_between(kfirst - kbase - c * 32, lim - c * 32);
+        for (int c = 0; c < 4; ++c) tmem_ld32(s_addr + c * 32, v + c * 32);
+        tmem_ld_wait();
+        if (need_mask) {
+          const int clear = __shfl_sync(0xffffffffu, lim, 0);
 #pragma unroll
-          for (int i = 0; i < 32; ++i)
-            if (!((seen >> i) & 1)) v[c * 32 + i] = 0xff800000u;
+          for (int c = 0; c < 4; ++c) {
+            if (kWindow || c * 32 + 31 > clear) {
+              const uint32_t seen = bits_between(kWindow ? kfirst - kbase - c * 32 : 0, lim - c * 32);
+#pragma unroll
+              for (int i = 0; i < 32; ++i)
+                if (!((seen >> i) & 1)) v[c * 32 + i] = 0xff800000u;
+            }
+          }
         }
-      }
-      if (!kWindow && need_mask) {
-#pragma unroll
-        for (int i = 0; i < 128; ++i)
-          if (i <= lim) mx4[i & 3] = fmaxf(mx4[i & 3], __uint_as_float(v[i]));
-      } else {
+        float mx4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
 #pragma unroll
         for (int i = 0; i < 128; ++i) mx4[i & 3] = fmaxf(mx4[i & 3], __uint_as_float(v[i]));
+        mx = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3]));
+      } else {
+#pragma unroll 1
+        for (int c = 0; c < 4; ++c) {
+          uint32_t u[32];
+          tmem_ld32(s_addr + c * 32, u);
+          tmem_ld_wait();
+          if (kWindow && need_mask) {
+            const uint32_t seen = bits_between(kfirst - kbase - c * 32, lim - c * 32);
+#pragma unroll
+            for (int i = 0; i < 32; ++i) mx = fmaxf(mx, (seen >> i) & 1 ? __uint_as_float(u[i]) : -INFINITY);
+          } else if (need_mask) {
+#pragma unroll
+            for (int i = 0; i < 32; ++i)
+              if (c * 32 + i <= lim) mx = fmaxf(mx, __uint_as_float(u[i]));
+          } else {
+#pragma unroll
+            for (int i = 0; i < 32; ++i) mx = fmaxf(mx, __uint_as_float(u[i]));
+          }
+        }
       }
-      const float mx = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3]));
       m_run = fmaxf(m_run, mx * p.scale_log2);
       // move the reference (and rescale O) only when some row of this warp needs it; the TMEM
       // accesses below are warp-wide, so the decision is too
@@ -339,9 +357,9 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
       }
       const float m_safe = (m_ref == -INFINITY) ? 0.f : m_ref;
       float lsum = 0.f;
-      const float2 sc = make_float2(p.scale_log2, p.scale_log2), off = make_float2(-m_safe, -m_safe);
       // probabilities, packed bf16 into the first 64 columns of S
-      auto probabilities = [&](auto masked) {
+      if constexpr (kOnce) {
+        const float2 sc = make_float2(p.scale_log2, p.scale_log2), off = make_float2(-m_safe, -m_safe);
 #pragma unroll
         for (int c = 0; c < 4; ++c) {
           uint32_t pk[16];
@@ -349,19 +367,39 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
           for (int i = 0; i < 16; ++i) {
             const int k = c * 32 + 2 * i;
             const float2 e = fma2(make_float2(__uint_as_float(v[k]), __uint_as_float(v[k + 1])), sc, off);
-            float2 pr = make_float2(fast_exp2(e.x), fast_exp2(e.y));
-            if (decltype(masked)::value) {
-              if (k > lim) pr.x = 0.f;
-              if (k + 1 > lim) pr.y = 0.f;
-            }
-            lsum += pr.x + pr.y;
-            pk[i] = pack_bf16(pr.x, pr.y);
+            const float p0 = fast_exp2(e.x), p1 = fast_exp2(e.y);
+            lsum += p0 + p1;
+            pk[i] = pack_bf16(p0, p1);
           }
           tmem_st16(s_addr + c * 16, pk);
         }
-      };
-      if (!kWindow && need_mask) probabilities(AttnFlag<true>());
-      else probabilities(AttnFlag<false>());
+      } else {
+#pragma unroll 1
+        for (int c = 0; c < 4; ++c) {
+          uint32_t u[32], pk[16];
+          tmem_ld32(s_addr + c * 32, u);
+          tmem_ld_wait();
+          uint32_t seen = 0xffffffffu;
+          if (kWindow && need_mask) seen = bits_between(kfirst - kbase - c * 32, lim - c * 32);
+          if (kWindow && seen != 0xffffffffu) {
+#pragma unroll
+            for (int i = 0; i < 32; ++i)
+              if (!((seen >> i) & 1)) u[i] = 0xff800000u;
+          }
+#pragma unroll
+          for (int i = 0; i < 16; ++i) {
+            float p0 = fast_exp2(__uint_as_float(u[2 * i]) * p.scale_log2 - m_safe);
+            float p1 = fast_exp2(__uint_as_float(u[2 * i + 1]) * p.scale_log2 - m_safe);
+            if (!kWindow && need_mask) {
+              if (c * 32 + 2 * i > lim) p0 = 0.f;
+              if (c * 32 + 2 * i + 1 > lim) p1 = 0.f;
+            }
+            lsum += p0 + p1;
+            pk[i] = pack_bf16(p0, p1);
+          }
+          tmem_st16(s_addr + c * 16, pk);
+        }
+      }
       tmem_st_wait();
       l_run += lsum;
       tc_fence_before();
@@ -419,17 +457,34 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
   }
 }
 
-template <int QB, int VB, int KST, int VST, bool kWindow = false>
-static int run_attn_fwd(const CUtensorMap& tmQ, const CUtensorMap& tmK, const CUtensorMap& tmV, const CUtensorMap& tmQ2,
-                        const CUtensorMap& tmK2, const AttnFwdArgs& a, int B, int max_seqlen, cudaStream_t stream) {
+template <int QB, int VB, int KST, int VST, bool kWindow, bool kOnce>
+static int launch_attn_tiles(const CUtensorMap& tmQ, const CUtensorMap& tmK, const CUtensorMap& tmV, const CUtensorMap& tmQ2,
+                             const CUtensorMap& tmK2, const AttnFwdArgs& a, int B, int max_seqlen, cudaStream_t stream) {
   using L = AttnFwdSmem<QB, VB, KST, VST>;
   static_assert(L::kTotal <= 227 * 1024, "shared memory");
-  auto kern = attn_fwd_kernel<QB, VB, KST, VST, kWindow>;
+  auto kern = attn_fwd_kernel<QB, VB, KST, VST, kWindow, kOnce>;
   OB_ENSURE_DYN_SMEM(kern, L::kTotal);
   dim3 grid((max_seqlen + 255) / 256, a.H, B);
   kern<<<grid, kAttnThreads, L::kTotal, stream>>>(tmQ, tmK, tmV, tmQ2, tmK2, a);
   OB_CHECK_LAUNCH();
   return 0;
+}
+
+// Scores in one pass (kOnce) or two.  One pass is the faster one per tile, but its code, unrolled over 128 columns, costs a causal
+// CTA of a few tiles more than it saves, and beside queries and keys of 192 channels it is the slower one.  In us by passes two / one,
+// 32 heads: 128 channels, 8 kv heads 8 x 256 22.4 25.9, 7 x 512 46.9 51.1, 8 x 1000 137 139, 1 x 1000 26.9 25.6, 1 x 4096 212 192,
+// without a mask 8 x 256 23.8 24.1; 192 channels 8 x 256 25.6 32.2, 8 x 1000 168 201, 2 x 4096 470 516; windows, 4 kv heads,
+// 8 x 256 23.9 23.4, 8 x 1000 140 131, window 128 97 95, 2 x 4096 375 331.  Heads of 64 gain from one pass at all lengths (8 x 256
+// 10.6 10.7, 1 x 1000 24.4 21.8).  A scale that is not positive does not keep -inf where it is: two passes, which
+// mask probabilities.
+template <int QB, int VB, int KST, int VST, bool kWindow = false>
+static int run_attn_fwd(const CUtensorMap& tmQ, const CUtensorMap& tmK, const CUtensorMap& tmV, const CUtensorMap& tmQ2,
+                        const CUtensorMap& tmK2, const AttnFwdArgs& a, int B, int max_seqlen, cudaStream_t stream) {
+  if constexpr (kWindow || QB <= 2) {
+    if (a.scale_log2 > 0.f && (kWindow || QB == 1 || !a.causal || max_seqlen > 896))
+      return launch_attn_tiles<QB, VB, KST, VST, kWindow, true>(tmQ, tmK, tmV, tmQ2, tmK2, a, B, max_seqlen, stream);
+  }
+  return launch_attn_tiles<QB, VB, KST, VST, kWindow, false>(tmQ, tmK, tmV, tmQ2, tmK2, a, B, max_seqlen, stream);
 }
 
 }  // namespace ob

@@ -605,6 +605,29 @@ def test_linear_cross_entropy_rounds_only_dlogits():
     assert ((ratio / ratio[:, :1] - 1).abs() < 2.0 ** -21).all()
 
 
+@pytest.mark.parametrize("HD", [64, 128])
+@pytest.mark.parametrize("causal", [True, False])
+@pytest.mark.parametrize("scale", [0.1, 0.0, -0.1])
+def test_attention_forward_edges_of_a_tile(HD, causal, scale):
+    """Sequences that end around the 32 columns of a group and the 128 of a tile, together in one call, and scales that keep or
+    turn the order of the scores: against fp32 with probabilities and outputs rounded to bf16 (2^-8 each of values of size one)."""
+    from omegalax_b200.ops import kernels as Kn, reference as R, lib
+    torch.manual_seed(39)
+    lens = [1, 31, 32, 33, 64, 97, 127, 128, 129, 161, 255, 256, 257, 390]
+    N, H, G = sum(lens), 4, 2
+    q, k, v = (torch.randn(N, n, HD, device=_dev()).to(bf16) for n in (H, G, G))
+    cu = torch.tensor([0] + torch.tensor(lens).cumsum(0).tolist(), device=_dev(), dtype=torch.int32)
+    o, lse = Kn.attn_fwd(q, k, v, cu, max(lens), scale, causal)
+    _check(lib)
+    torch.testing.assert_close(o.float(), R.attention_varlen(q.float(), k.float(), v.float(), cu, causal=causal, scale=scale),
+                               rtol=2.0 ** -7, atol=2.0 ** -7)
+    for a, b in zip(cu.tolist(), cu.tolist()[1:]):
+        s = torch.einsum("qhd,khd->hqk", q[a:b].float(), k[a:b].float().repeat_interleave(H // G, 1)) * scale
+        if causal:
+            s = s.masked_fill(torch.ones(b - a, b - a, device=_dev()).triu(1).bool(), float("-inf"))
+        torch.testing.assert_close(lse[:, a:b], torch.logsumexp(s, -1), rtol=1e-4, atol=1e-3)
+
+
 def test_embedding_and_optimizer_kernels():
     from omegalax_b200.ops import kernels as Kn, lib
     torch.manual_seed(9)
