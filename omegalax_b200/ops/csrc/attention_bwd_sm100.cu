@@ -23,9 +23,9 @@
 // Few kv heads leave few CTAs (one sequence of 3001 with 2 kv heads: 48 of 148 SMs, and a causal walk is up to
 // 24 times as long for the first tile as for the last).  Then `hsplit` CTAs share the query heads of a
 // (key tile, kv head); each stores fp32 partial sums and a second kernel adds them in order.  The grid is
-// flat with the tile index slowest, so the longest walks start first.  In us, before and after: 32 heads of 256 on 2,
-// one row of 3001: 6785, 1228; 32 heads of 128 on 4, one row of 4096: 1000, 531 (two shares); on 8, two rows of
-// 4096: 1324, 983 (one share: the order alone).
+// flat with the tile index slowest, so the longest walks start first.  In us for all of a backward call, before and after: 32 heads
+// of 256 on 2, one row of 3001 6856, 1378; 32 heads of 128 on 4, one row of 4096 1061, 575; on 8, two rows of 4096
+// (one share: the order alone) 1324, 1054.
 //
 // Heads of 256 (template HD = 256): dK and dV of a 128-key tile would need all 512 TMEM columns, so
 // the grid holds every CTA twice, once per 128-wide half `dh` of the head dimension.  Each pass computes

@@ -1,5 +1,5 @@
-"""Arguments that a launcher refuses before anything runs: plain integers stand for device pointers here, so no GPU is needed
-(and where one is there, nothing is launched)."""
+"""What is decided before a launch: arguments that are refused (plain integers stand for device pointers, so no GPU is needed, and
+where one is there, nothing is launched) and choices by size."""
 import pytest
 
 from omegalax_b200.ops import lib
@@ -11,3 +11,15 @@ A = 1 << 20      # an aligned address that is never read
 def test_row_gather_of_the_head_wants_16_byte_rows(h, out, D, code):
     """A contiguous view may start anywhere; the gather reads 16 bytes at a time, as the products it stands before do."""
     assert lib.load().ob_ce_gather(h, A, A, out, 128, D, None) == code
+
+
+@pytest.mark.parametrize("batch,rows,H,G,hd,causal,least,most", [
+    (7, 512, 32, 8, 128, True, 1, 1), (4, 800, 32, 8, 128, True, 1, 1), (7, 512, 32, 4, 128, False, 1, 1), (2, 1000, 16, 8, 128, False, 1, 1),
+    (1, 4096, 32, 8, 128, True, 1, 1), (2, 4096, 32, 8, 128, True, 1, 1), (1, 128, 16, 8, 128, True, 1, 1),
+    (1, 4096, 32, 4, 128, True, 2, 4), (1, 3001, 32, 2, 256, True, 4, 8), (1, 512, 64, 4, 128, False, 8, 8), (1, 1000, 16, 8, 128, True, 2, 2)])
+def test_ctas_share_a_key_tile_only_where_that_saves(batch, rows, H, G, hd, causal, least, most):
+    """Sizes at which sharing was measured to lose, and to win by the factors named in ``attn_bwd_splits``."""
+    from omegalax_b200.ops import kernels as K
+
+    tiles = min(-(-rows // 128) * batch, batch * rows // 128 + batch) * (hd // 128)
+    assert least <= K.attn_bwd_splits(tiles, H, G, -(-rows // 64), causal, batch * rows * G * hd) <= most
