@@ -210,10 +210,11 @@ gemm_few_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__
 
 // CTAs per panel: as many as the SMs take in one wave of two, with slices of at least four k-blocks.  M 1,
 // K 4096, in us by CTAs per panel 1 / 2 / 4 / 8: N 4096 22.5 13.7 10.3 10.8, N 6144 22.2 14.3 12.8 15.9,
-// N 24576 37.6 38.9 40.5 46.6.
+// N 24576 37.6 38.9 40.5 46.6.  Clusters of four and eight do not fill the last 40 of the 296 places, since the SMs of a GPC are no
+// whole number of them: 64 panels of 128 rows by four, K 1024, 10.8 us, 72 panels 16.8 (by two 10.6).
 static int few_splits(long long panels, int kblocks) {
   int s = 1;
-  while (s < 8 && panels * 2 * s <= 2 * num_sms() && kblocks / (2 * s) >= 4) s *= 2;
+  while (s < 8 && panels * 2 * s <= 2 * num_sms() - (s > 1 ? 40 : 0) && kblocks / (2 * s) >= 4) s *= 2;
   return s;
 }
 

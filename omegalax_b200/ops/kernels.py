@@ -72,8 +72,12 @@ def _use_few(M: int, N: int, K: int) -> bool:
     reads every weight once (N 4096, K 12288: 22 us for one row, 81 on 128 x 128 tiles; N 151936, K 4096: 191,
     516); above, while its 128 x 128 panels fit the SMs in one wave of two (M 500, N 6144, K 4096: 33 us against
     51; M 1000, N 6144: 64 against 55, beyond the wave).  Short reductions leave nothing to share out
-    (M 128, N 8192, K 512: 9.9 against 9.5)."""
-    return K > 0 and (M <= 64 or (K >= 768 and (M <= 128 or -(-M // 128) * -(-N // 128) <= 296)))
+    (M 128, N 8192, K 512: 9.9 against 9.5; K 768, M 2048, N 1024, whose panels are just one wave of the others: 11.7 against
+    10.4, while 192 panels, two waves of the others, take 13.3 against 15.5)."""
+    if M <= 64:
+        return K > 0
+    panels = -(-M // 128) * -(-N // 128)
+    return K >= 768 and (M <= 128 or panels <= 296) and (K >= 1024 or not 74 < panels <= 148)
 
 
 def gemm(a, b, *, a_mn: bool = False, b_mn: bool = False, out=None, out_dtype=bf16,

@@ -23,3 +23,11 @@ def test_ctas_share_a_key_tile_only_where_that_saves(batch, rows, H, G, hd, caus
 
     tiles = min(-(-rows // 128) * batch, batch * rows // 128 + batch) * (hd // 128)
     assert least <= K.attn_bwd_splits(tiles, H, G, -(-rows // 64), causal, batch * rows * G * hd) <= most
+
+
+@pytest.mark.parametrize("M,N,K,few", [(1, 8, 64, True), (64, 4096, 32, True), (65, 4096, 512, False), (2048, 1024, 768, False), (500, 6144, 768, True),
+                                       (2048, 1024, 1024, True), (1000, 6144, 4096, False), (128, 151936, 4096, True)])
+def test_products_of_few_rows_go_where_they_are_faster(M, N, K, few):
+    from omegalax_b200.ops import kernels
+
+    assert kernels._use_few(M, N, K) is few
