@@ -379,7 +379,7 @@ class Qwen3(nn.Module):
             setattr(batch, name, flat[at:at + t.numel()])
             at += t.numel() + -t.numel() % 4
         if batch.every and key is not None:
-            x = DecodeGraph.step(self, cache, batch, key)
+            x = DecodeGraph.step(self, cache, batch, key, alone=True)
         elif single:
             x = self.run_layers(batch, cache)
         else:

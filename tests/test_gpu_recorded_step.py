@@ -108,6 +108,7 @@ CHANGES = {
 @pytest.mark.parametrize("what", CHANGES)
 def test_a_change_between_steps_is_seen(served, monkeypatch, what):
     model, cfg = served
+    monkeypatch.setattr("omegalax_b200.models.decode_graph.other_threads", lambda: False)
     state = {k: v.clone() for k, v in model.state_dict().items()}
     got, _ = _run(model, cfg, True, monkeypatch, CHANGES[what])
     for k, v in model.state_dict().items():
@@ -122,6 +123,7 @@ def test_idle_sequences_and_two_caches(served, monkeypatch):
     from omegalax_b200.text import api
 
     model, cfg = served
+    monkeypatch.setattr("omegalax_b200.models.decode_graph.other_threads", lambda: False)
     more = _ids()[1].clone()
     more[5, 1] = 0
     got, _ = _run(model, cfg, True, monkeypatch, more=more)
@@ -146,6 +148,7 @@ def test_steps_on_two_streams(served, monkeypatch):
     from omegalax_b200.text import api
 
     model, cfg = served
+    monkeypatch.setattr("omegalax_b200.models.decode_graph.other_threads", lambda: False)
     want, _ = _run(model, cfg, False, monkeypatch)
     monkeypatch.setenv("OMEGALAX_B200_DECODE_GRAPH", "1")
     prompt, steps = _ids()
@@ -160,3 +163,41 @@ def test_steps_on_two_streams(served, monkeypatch):
     assert cache.decode_graph[1] is not None and cache.seq_lens.tolist() == [T + STEPS] * B
     for i, (a, b) in enumerate(zip(out, want)):
         assert torch.equal(a, b), f"call {i}"
+
+
+def test_nothing_is_recorded_beside_other_threads(served, monkeypatch):
+    """Two threads that decode, draw random numbers and wait for the device at the same time: as when every call is issued."""
+    import threading
+
+    from omegalax_b200.text import api
+
+    model, cfg = served
+    want, _ = _run(model, cfg, False, monkeypatch)
+    monkeypatch.setenv("OMEGALAX_B200_DECODE_GRAPH", "1")
+    got, errors, start = [[], []], [], threading.Barrier(2)
+
+    def serve(t):
+        try:
+            with torch.cuda.stream(torch.cuda.Stream()):
+                prompt, steps = _ids()
+                cache = api.make_cache(cfg, B, T, STEPS, device="cuda")
+                start.wait(30)
+                for ids in [prompt, *steps]:
+                    got[t].append(api.decode(model, cache, ids, 0, cfg)[0])
+                    torch.multinomial(torch.softmax(got[t][-1].float(), -1), 1)
+                    torch.cuda.synchronize()
+                assert cache.decode_graph is None or cache.decode_graph[1] is None
+        except BaseException as e:
+            errors.append(e)
+
+    torch.cuda.synchronize()
+    threads = [threading.Thread(target=serve, args=(t,)) for t in range(2)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join(120)
+    assert not errors and not any(t.is_alive() for t in threads)
+    torch.cuda.synchronize()
+    for t in range(2):
+        for i, (a, b) in enumerate(zip(got[t], want)):
+            assert torch.equal(a, b), f"thread {t} call {i}"
