@@ -115,9 +115,10 @@ class StreamDecoder(nn.Module):
             x = DecodeGraph.step(self, cache, batch)
         else:
             # A prompt's first tokens read a recurrent state of one or two products and norm what they read: next to
-            # nothing where query and key are nearly orthogonal.  So that such tokens do not depend on what they are
-            # batched with, prompts of these models keep one order of sums for all numbers of rows.
-            with S.whole_reductions(cache.recurrent):
+            # nothing where query and key are nearly orthogonal, and any difference in them is magnified.  So queries,
+            # keys and gates of a prompt are summed in the same order whatever it is batched with.  (The sums into the
+            # residual rows are not: the tile kernels cut long reductions by the number of rows.)
+            with S.tile_kernels(cache.recurrent):
                 x = self.run_layers(batch, cache)
         cache.advance(new)
         if select is None:

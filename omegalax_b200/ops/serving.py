@@ -48,13 +48,14 @@ _calls = threading.local()
 
 
 @contextlib.contextmanager
-def whole_reductions(on: bool = True):
-    """``project`` calls of this thread sum every reduction in one go, whatever the number of rows."""
-    before, _calls.whole = getattr(_calls, "whole", False), on
+def tile_kernels(on: bool = True):
+    """``project`` calls of this thread stay off the kernel for few rows.  A row's result in ``out_dtype`` is then one sum in one
+    order, whatever the number of rows; sums ``into`` given rows are still cut by their size."""
+    before, _calls.tiles = getattr(_calls, "tiles", False), on
     try:
         yield
     finally:
-        _calls.whole = before
+        _calls.tiles = before
 
 
 def project(x, w, *, out_dtype=None, into=None):
@@ -65,7 +66,7 @@ def project(x, w, *, out_dtype=None, into=None):
             return into.addmm_(x, w.t())
         return x @ w.t()
     N, Kd = w.shape
-    few = False if getattr(_calls, "whole", False) else None
+    few = False if getattr(_calls, "tiles", False) else None
     if Kd % 8:
         x, w = F.pad(x, (0, 8 - Kd % 8)), F.pad(w, (0, 8 - Kd % 8))
     if into is not None:

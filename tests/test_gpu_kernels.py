@@ -313,6 +313,19 @@ def test_gemm_few_rows(M, N, K, splits):
         _assert_gemm_close(Kn.gemm(x, w), ref, K)
 
 
+@pytest.mark.parametrize("N,K", [(16416, 4096), (512, 4096), (6144, 512)])
+def test_projections_off_the_few_row_kernel_do_not_depend_on_the_batch(N, K):
+    """A row's bf16 result is the same to the last bit alone and among others, whichever tile kernel the number of rows chooses."""
+    from omegalax_b200.ops import serving as S, lib
+    torch.manual_seed(40)
+    x, w = (torch.randn(n, K, device=_dev()).to(bf16) for n in (6000, N))
+    with S.tile_kernels():
+        whole = S.project(x, w)
+        for M in (1, 64, 65, 300, 1000, 2049):
+            assert torch.equal(S.project(x[:M], w), whole[:M]), M
+    _check(lib)
+
+
 @pytest.mark.parametrize("pair", [False, True])
 def test_gemm_grouped_and_wgrad(pair):
     """Grouped expert GEMMs (forward, input gradient, weight gradient) on the single-CTA kernel
