@@ -23,6 +23,16 @@ def supervised_count(mask_BT, group=None) -> torch.Tensor:
     return n
 
 
+def chunk_rows(rows: int, num_tiles: int) -> int:
+    """Rows of a chunk on the GPU: those of ``num_tiles`` tiles, between 1024 and 8192.  Every chunk adds into the whole fp32
+    gradient of the head (0.4 ms for 152k x 2048), so from 2560 rows on a chunk has 4096 at least, whose product takes 1.7 ms;
+    its bf16 logits are then up to 1.2 GB at 152k instead of 0.3.  More tiles than the default of eight ask for less memory, and
+    get it.  Beside the logits a step of 2560 rows and more holds the supervised hidden rows once more in bf16, and their
+    gradient in fp32 (4 bytes a channel and row) until the backward pass."""
+    least = 4096 if rows >= 2560 and num_tiles <= 8 else 1024
+    return min(max(-(-rows // max(num_tiles, 1)), least), 8192)
+
+
 def chunked_cross_entropy_loss(hidden_BTD, lm_head_VD, targets_BT, mask_BT, num_tiles: int = 8,
                                *, group=None, count: torch.Tensor | None = None):
     """Masked mean next-token NLL.  ``lm_head_VD`` is the [vocab, hidden] projection weight.
@@ -43,9 +53,5 @@ def chunked_cross_entropy_loss(hidden_BTD, lm_head_VD, targets_BT, mask_BT, num_
         count = supervised_count(mask_BT, group)
     scale = 1.0 / count.clamp_min(1.0)
     rows = h.shape[0]
-    chunk = max(1, -(-rows // max(num_tiles, 1)))
-    if h.is_cuda:
-        # every chunk of rows adds into the whole fp32 gradient of the head: 4096 rows and more keep its
-        # traffic (0.4 ms for 152k x 2048) under the time of the chunk's product (1.7 ms)
-        chunk = min(max(chunk, 4096 if rows >= 2560 else 1024), 8192)
+    chunk = chunk_rows(rows, num_tiles) if h.is_cuda else max(1, -(-rows // max(num_tiles, 1)))
     return Fn.linear_cross_entropy(h, lm_head_VD, tgt, mask, scale, chunk=chunk)

@@ -31,3 +31,11 @@ def test_products_of_few_rows_go_where_they_are_faster(M, N, K, few):
     from omegalax_b200.ops import kernels
 
     assert kernels._use_few(M, N, K) is few
+
+
+@pytest.mark.parametrize("rows,tiles,chunk", [(8192, 4, 4096), (32768, 4, 8192), (16384, 16, 1024), (4096, 64, 1024), (3000, 8, 4096),
+                                              (2559, 4, 1024), (100, 8, 1024), (24000, 12, 2000)])
+def test_more_tiles_than_the_default_bound_the_memory_of_the_head(rows, tiles, chunk):
+    from omegalax_b200.trainers.loss import chunk_rows
+
+    assert chunk_rows(rows, tiles) == chunk
