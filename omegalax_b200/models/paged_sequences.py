@@ -75,7 +75,8 @@ class PagedSequences:
             self._sent_on = (s.stream_id, s.device_index, s.device_type)
 
     def settle(self) -> None:
-        """Order the current stream after the copies that another stream was given."""
+        """Order the current stream after the copies that another stream was given.  Calls on the cache do so; who reads
+        ``block_table`` or ``seq_lens`` directly, on a stream of its own, calls it first."""
         if self._sent_on is not None:
             s = torch.cuda.current_stream(self._sent_on[1])
             if s.stream_id != self._sent_on[0]:
@@ -110,6 +111,7 @@ class PagedSequences:
 
     def flat_rows(self, seq_of_token, slot_of_token):
         """Row index into pages.view(num_pages * page_size, ...) of (sequence, slot) pairs (device tensors)."""
+        self.settle()
         blk = self.block_table[seq_of_token.long(), (slot_of_token // self.page_size).long()].long()
         return blk * self.page_size + (slot_of_token % self.page_size).long()
 

@@ -165,6 +165,25 @@ def test_steps_on_two_streams(served, monkeypatch):
         assert torch.equal(a, b), f"call {i}"
 
 
+def test_rows_of_pages_reserved_on_another_stream(served):
+    """``flat_rows`` on one stream sees the pages whose table is still on its way on another."""
+    from omegalax_b200.text import api
+
+    cache = api.make_cache(served[1], B, 200, 0, device="cuda")
+    seq = torch.arange(B, device="cuda").repeat_interleave(200)
+    slot = torch.arange(200, device="cuda").repeat(B)
+    work = torch.empty(1 << 28, device="cuda")
+    torch.cuda.synchronize()
+    with torch.cuda.stream(torch.cuda.Stream()):
+        for _ in range(10):
+            work.normal_()
+        cache.reserve([200] * B)
+    with torch.cuda.stream(torch.cuda.Stream()):
+        rows = cache.flat_rows(seq, slot)
+    torch.cuda.synchronize()
+    assert rows.tolist() == [r for b in range(B) for r in cache.flat_rows_host(b, 0, 200).tolist()]
+
+
 def test_nothing_is_recorded_beside_other_threads(served, monkeypatch):
     """Two threads that decode, draw random numbers and wait for the device at the same time: as when every call is issued."""
     import threading
