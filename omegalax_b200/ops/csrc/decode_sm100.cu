@@ -75,7 +75,8 @@ __global__ void decode_append_kernel(const bf16* __restrict__ qkv, const bf16* _
 }
 
 // Keys and values of a prompt into their pages: row n of k and v (W channels, any pitch) to cache row rows[n].  blockIdx.y: 0 k, 1 v.
-// Four 16-byte groups of a thread are in flight.  8192 rows of 1024 channels: TIMEKV
+// Four 16-byte groups of a thread are in flight.  8192 rows of 1024 channels, keys and values, L2 flushed: 17.4 us (67 MB: 3.9 TB/s),
+// where two indexed copies and one to close the gaps of v took 78.8.
 __global__ void __launch_bounds__(256)
 kv_store_kernel(const bf16* __restrict__ k, const bf16* __restrict__ v, long long ldk, long long ldv,
                 const int* __restrict__ rows, bf16* __restrict__ k_pages, bf16* __restrict__ v_pages, long long N, int W) {

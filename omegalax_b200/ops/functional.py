@@ -672,8 +672,12 @@ class _LinearCEFn(torch.autograd.Function):
         if counted:
             # Rows without loss (prompts, padding) take no part in the head: the others are gathered and counted
             # on the device.  Chunks past the count return at once, so the chunk bounds need no host copy of it.
-            # (With gradients that leave over NVLink the whole rows go on: that GEMM takes no count.  So do fewer than
-            # 2560 rows: such a step is bound by its launches, and 3 rows of 333 took 6.87 ms, counted 7.12.)
+            # With gradients that leave over NVLink the whole rows go on: that GEMM takes no count.
+            # The line at 2560 rows is drawn for results, not for time: at 152k x 1024, half of the rows supervised, counted
+            # rows take 695 us against 1286 at 512 rows, 711 against 1526 at 1000, 1424 against 4693 at 2500.  But they round
+            # differently (the loss scale's part beyond a power of two stays in fp32, the input gradient is a split sum),
+            # and in a small step, where few vocabulary rows get a gradient at all, single elements move by the rms of the
+            # whole gradient with any change in the order of sums.  Small steps keep the rounding they had.
             w = K._row_major_2d(w)
             count, rows, place, t32, mk = K.ce_supervised(mk, t32)
             h = K.ce_gather(h, rows, count)

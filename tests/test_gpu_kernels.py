@@ -777,6 +777,25 @@ def test_decode_attention_lengths(R, splits):
         torch.testing.assert_close(out[b].float(), torch.einsum("hs,shd->hd", p, vb), rtol=2.0 ** -8, atol=2.0 ** -10)
 
 
+@pytest.mark.parametrize("N", [1, 5, 1025])
+@pytest.mark.parametrize("G", [1, 3])
+def test_kv_store(N, G):
+    """Strided keys and values to scattered rows: a copy, and every other row stays as it was."""
+    from omegalax_b200.ops import kernels as Kn, lib
+    torch.manual_seed(41)
+    HD, rows = 128, 1100
+    qkv = torch.randn(N, (2 + 2 * G) * HD + 8, device=_dev()).to(bf16)
+    k, v = (qkv[:, (i + i * G) * HD: (i + i * G + G) * HD].unflatten(1, (G, HD)) for i in (0, 1))
+    pages = [torch.full((rows // 11, 11, G, HD), 3.0, device=_dev(), dtype=bf16) for _ in range(2)]
+    at = torch.randperm(rows, device=_dev())[:N].to(torch.int32)
+    Kn.kv_store(k, v, at, *pages)
+    _check(lib)
+    for src, dst in zip((k, v), pages):
+        want = torch.full((rows, G, HD), 3.0, device=_dev(), dtype=bf16)
+        want[at.long()] = src
+        assert torch.equal(dst.view(rows, G, HD), want)
+
+
 def test_paged_decode_matches_full_forward():
     """Prefill a left-padded batch into the paged cache, then decode 6 steps with the paged
     kernels; every step's logits must agree with a full forward over the grown sequence."""
