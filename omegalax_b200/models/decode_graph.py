@@ -15,6 +15,11 @@ import torch
 from ..ops import kernels as K
 
 
+# A recording that leaves less than this to the device gives the allocator's free memory back first: while one is made
+# the allocator cannot do so, and a step's temporaries come from memory of its own.
+_SPARE = 1 << 30
+
+
 def other_threads() -> bool:
     return threading.active_count() > 1
 
@@ -26,6 +31,8 @@ class DecodeGraph:
         self.graph = torch.cuda.CUDAGraph()
         # ``torch.cuda.graph`` would wait for the device and give the allocator's free memory back first, to be asked for
         # again: the second step of a fresh cache took 9.0 ms so and takes 5.1 (8 layers of 4096 channels; 3.1 call by call, 1.6 recorded)
+        if torch.cuda.mem_get_info()[0] < _SPARE:
+            torch.cuda.empty_cache()
         here, side = torch.cuda.current_stream(), torch.cuda.Stream()
         side.wait_stream(here)
         with torch.cuda.stream(side):

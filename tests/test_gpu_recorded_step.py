@@ -143,6 +143,26 @@ def test_idle_sequences_and_two_caches(served, monkeypatch):
             assert torch.equal(a, b)
 
 
+@pytest.mark.parametrize("free,times", [(1 << 20, 1), (1 << 34, 0)])
+def test_free_memory_of_the_allocator_is_given_back_where_a_recording_may_need_it(served, monkeypatch, free, times):
+    """While a step is recorded the allocator cannot empty itself: done before, where the device has little left (a stand-in says how much)."""
+    model, cfg = served
+    monkeypatch.setattr("omegalax_b200.models.decode_graph.other_threads", lambda: False)
+    want, _ = _run(model, cfg, False, monkeypatch, change=lambda m: lambda: None)
+    calls, empty = [], torch.cuda.empty_cache
+
+    def emptied():
+        calls.append(torch.cuda.is_current_stream_capturing())
+        empty()
+
+    monkeypatch.setattr(torch.cuda, "mem_get_info", lambda *a: (free, 1 << 37))
+    monkeypatch.setattr(torch.cuda, "empty_cache", emptied)
+    got, _ = _run(model, cfg, True, monkeypatch, change=lambda m: lambda: None)
+    assert calls == [False] * times
+    for i, (a, b) in enumerate(zip(got, want)):
+        assert torch.equal(a, b), f"call {i}"
+
+
 def test_steps_on_two_streams(served, monkeypatch):
     """Steps of one cache that take turns on two streams: each finds lengths, pages and recorded buffers as the last one left them."""
     from omegalax_b200.text import api
