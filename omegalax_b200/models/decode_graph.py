@@ -13,6 +13,7 @@ import threading
 import torch
 
 from ..ops import kernels as K
+from ..ops import lib
 
 
 # A recording that leaves less than this to the device gives the allocator's free memory back first: while one is made
@@ -39,8 +40,11 @@ class DecodeGraph:
             # other threads go on allocating while this one records
             self.graph.capture_begin(capture_error_mode="thread_local")
             try:
+                # no kernel of a step writes weights, so each may read its own ahead of the kernel before it
+                lib.call("ob_overlap_launches", 1)
                 self.out = model.run_layers(batch, cache)
             finally:
+                lib.call("ob_overlap_launches", 0)
                 self.graph.capture_end()
         here.wait_stream(side)
         self.launches = K.launch_count() - before

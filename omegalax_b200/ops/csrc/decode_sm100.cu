@@ -26,6 +26,7 @@ __global__ void decode_append_kernel(const bf16* __restrict__ qkv, const bf16* _
                                      bf16* __restrict__ q_out, bf16* __restrict__ k_pages,
                                      bf16* __restrict__ v_pages, long long ntok, int H, int G, int HD, int rot,
                                      float theta, float eps) {
+  grid_begin();
   const int lane = threadIdx.x & 31;
   const long long wid = (blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5;
   const int HH = H + 2 * G;
@@ -144,6 +145,7 @@ decode_attn_kernel(const bf16* __restrict__ q, const bf16* __restrict__ k_pages,
                    const int* __restrict__ block_table, const int* __restrict__ seq_lens, int max_blocks,
                    int page_size, int G, int splits, float scale, float* __restrict__ part_o,
                    float* __restrict__ part_ml) {
+  grid_begin();
   static_assert(HD == 128, "one half-warp covers a 128-channel row");
   constexpr int C = 8;    // channels per lane
   constexpr int NW = 8;   // half-warps per CTA
@@ -316,6 +318,7 @@ decode_attn_kernel(const bf16* __restrict__ q, const bf16* __restrict__ k_pages,
 // One CTA per head: the weights of the splits once, a lane each, then every channel's sum with its loads independent.
 __global__ void __launch_bounds__(128) decode_combine_kernel(const float* __restrict__ part_o, const float* __restrict__ part_ml,
                                                              bf16* __restrict__ out, int splits, int HD) {
+  grid_begin();
   __shared__ float w[64], sm[2];      // weights of the first 64 splits, maximum and denominator
   const long long bh = blockIdx.x;
   const float2* ml = reinterpret_cast<const float2*>(part_ml) + bh * splits;
@@ -358,11 +361,11 @@ int ob_decode_append(const void* qkv, const void* qw, const void* kw, const int*
   long long warps = ntok * (H + 2 * G);
   long long blocks = (warps * 32 + 255) / 256;
   if (one_plus)
-    decode_append_kernel<true><<<(unsigned)blocks, 256, 0, s>>>(
+    OB_LAUNCH(decode_append_kernel<true>, (unsigned)blocks, 256, 0, s, 
         (const bf16*)qkv, (const bf16*)qw, (const bf16*)kw, positions, seq_of_token, slot_of_token, block_table,
         max_blocks, page_size, (bf16*)q_out, (bf16*)k_pages, (bf16*)v_pages, ntok, H, G, HD, rot, theta, eps);
   else
-    decode_append_kernel<false><<<(unsigned)blocks, 256, 0, s>>>(
+    OB_LAUNCH(decode_append_kernel<false>, (unsigned)blocks, 256, 0, s, 
         (const bf16*)qkv, (const bf16*)qw, (const bf16*)kw, positions, seq_of_token, slot_of_token, block_table,
         max_blocks, page_size, (bf16*)q_out, (bf16*)k_pages, (bf16*)v_pages, ntok, H, G, HD, rot, theta, eps);
   OB_CHECK_LAUNCH();
@@ -392,14 +395,14 @@ int ob_decode_attn(const void* q, const void* k_pages, const void* v_pages, cons
   dim3 grid(B, G, splits);
 #define OB_DA(RR)                                                                                         \
   OB_ENSURE_DYN_SMEM((decode_attn_kernel<128, RR>), kDecodeRing);                                          \
-  decode_attn_kernel<128, RR><<<grid, 128, kDecodeRing, s>>>((const bf16*)q, (const bf16*)k_pages, (const bf16*)v_pages, \
+  OB_LAUNCH((decode_attn_kernel<128, RR>), grid, 128, kDecodeRing, s, (const bf16*)q, (const bf16*)k_pages, (const bf16*)v_pages, \
                                                     block_table, seq_lens, max_blocks, page_size, G, splits,   \
                                                     scale, part_o, part_ml)
   if (R == 1) { OB_DA(1); } else if (R == 2) { OB_DA(2); } else if (R == 4) { OB_DA(4); } else if (R == 8) { OB_DA(8); }
   else return 6005;
 #undef OB_DA
   OB_CHECK_LAUNCH();
-  decode_combine_kernel<<<(unsigned)(B * H), 128, 0, s>>>(part_o, part_ml, (bf16*)out, splits, HD);
+  OB_LAUNCH(decode_combine_kernel, (unsigned)(B * H), 128, 0, s, part_o, part_ml, (bf16*)out, splits, HD);
   OB_CHECK_LAUNCH();
   return 0;
 }

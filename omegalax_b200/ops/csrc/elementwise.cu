@@ -36,6 +36,8 @@ __global__ void rmsnorm_fwd_kernel(const bf16* __restrict__ x, const bf16* __res
   const long long row = blockIdx.x;
   const uint4* xr = reinterpret_cast<const uint4*>(x + row * D);
   const int nv = D >> 3;
+  for (int i = threadIdx.x; i < nv; i += blockDim.x) prefetch_l2(reinterpret_cast<const uint4*>(w) + i);
+  grid_begin();
   float ss = 0.f;
   for (int i = threadIdx.x; i < nv; i += blockDim.x) {
     uint4 q = xr[i];
@@ -188,6 +190,7 @@ rmsnorm_bwd_kernel(const bf16* __restrict__ dy, const bf16* __restrict__ x, cons
 // gu is [M, 2F] = [gate | up];  act = silu(gate) * up.
 __global__ void swiglu_fwd_kernel(const bf16* __restrict__ gu, bf16* __restrict__ act, long long M,
                                   int F) {
+  grid_begin();
   const int fv = F >> 3;
   const long long total = M * fv;
   for (long long idx = blockIdx.x * (long long)blockDim.x + threadIdx.x; idx < total;
@@ -832,6 +835,7 @@ __global__ void ce_counted_grad_kernel(bf16* __restrict__ logits, long long ld, 
 // ------------------------------------------------------------------ embedding (K13)
 __global__ void embedding_fwd_kernel(const int* __restrict__ ids, const bf16* __restrict__ table,
                                      bf16* __restrict__ out, long long M, int D) {
+  grid_begin();
   const int dv = D >> 3;
   for (long long idx = blockIdx.x * (long long)blockDim.x + threadIdx.x; idx < M * dv;
        idx += (long long)gridDim.x * blockDim.x) {
@@ -1025,10 +1029,10 @@ int ob_rmsnorm_fwd(const void* x, const void* w, void* y, float* rstd, long long
   if (M <= 0) return 0;
   int threads = D >= 2048 ? 256 : 128;
   if (one_plus)
-    rmsnorm_fwd_kernel<true><<<(unsigned)M, threads, 0, s>>>((const bf16*)x, (const bf16*)w,
+    OB_LAUNCH(rmsnorm_fwd_kernel<true>, (unsigned)M, threads, 0, s, (const bf16*)x, (const bf16*)w,
                                                              (bf16*)y, rstd, D, eps);
   else
-    rmsnorm_fwd_kernel<false><<<(unsigned)M, threads, 0, s>>>((const bf16*)x, (const bf16*)w,
+    OB_LAUNCH(rmsnorm_fwd_kernel<false>, (unsigned)M, threads, 0, s, (const bf16*)x, (const bf16*)w,
                                                               (bf16*)y, rstd, D, eps);
   OB_CHECK_LAUNCH();
   return 0;
@@ -1061,7 +1065,7 @@ int ob_rmsnorm_bwd(const void* dy, const void* x, const void* w, const float* rs
 int ob_swiglu_fwd(const void* gu, void* act, long long M, int F, cudaStream_t s) {
   if (F % 8) return 6001;
   if (M <= 0) return 0;
-  swiglu_fwd_kernel<<<grid_for(M * (F / 8), 256), 256, 0, s>>>((const bf16*)gu, (bf16*)act, M, F);
+  OB_LAUNCH(swiglu_fwd_kernel, grid_for(M * (F / 8), 256), 256, 0, s, (const bf16*)gu, (bf16*)act, M, F);
   OB_CHECK_LAUNCH();
   return 0;
 }
@@ -1239,7 +1243,7 @@ int ob_embedding_fwd(const int* ids, const void* table, void* out, long long M, 
                      cudaStream_t s) {
   if (D % 8) return 6001;
   if (M <= 0) return 0;
-  embedding_fwd_kernel<<<grid_for(M * (D / 8), 256), 256, 0, s>>>(ids, (const bf16*)table,
+  OB_LAUNCH(embedding_fwd_kernel, grid_for(M * (D / 8), 256), 256, 0, s, ids, (const bf16*)table,
                                                                   (bf16*)out, M, D);
   OB_CHECK_LAUNCH();
   return 0;

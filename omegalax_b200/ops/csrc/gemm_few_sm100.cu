@@ -66,6 +66,10 @@ gemm_few_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int splits = (int)gridDim.x, rank = (int)blockIdx.x;    // the cluster spans the x dimension
   const int n0 = blockIdx.y * 128, m0 = blockIdx.z * NB;
+  if (threadIdx.x == 0) {
+    tma_prefetch_desc(&tmW);
+    tma_prefetch_desc(&tmX);
+  }
   const int k_begin = rank * p.k_per_split, k_end = min(p.K, k_begin + p.k_per_split);
 
   if (threadIdx.x == 0) {
@@ -88,11 +92,18 @@ gemm_few_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__
 
   if (warp == 0) {
     if (lane == 0) {
-      tma_prefetch_desc(&tmW);
-      tma_prefetch_desc(&tmX);
-      int stage = 0;
-      uint32_t phase = 0;
-      for (int k0 = k_begin; k0 < k_end; k0 += BK) {
+      // the weights of the first stages are on their way while the kernel before, which gives X, still runs
+      const int ahead = min(kSt, (k_end - k_begin + BK - 1) / BK);
+      for (int i = 0; i < ahead; ++i) {
+        mbar_expect_tx(&full_bar[i], L::kStageBytes);
+        tma_load_2d(smem + i * L::kStageBytes, &tmW, &full_bar[i], k_begin + i * BK, n0);
+      }
+      grid_begin();
+      for (int i = 0; i < ahead; ++i)
+        tma_load_2d(smem + i * L::kStageBytes + L::kABytes, &tmX, &full_bar[i], k_begin + i * BK, m0);
+      int stage = ahead == kSt ? 0 : ahead;
+      uint32_t phase = ahead == kSt;
+      for (int k0 = k_begin + ahead * BK; k0 < k_end; k0 += BK) {
         if (!mbar_wait(&empty_bar[stage], phase ^ 1, abort_flag, p.status, OB_ERR_WAIT_EMPTY)) break;
         uint8_t* sw = smem + stage * L::kStageBytes;
         mbar_expect_tx(&full_bar[stage], L::kStageBytes);
@@ -148,6 +159,7 @@ gemm_few_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__
       tc_fence_before();
     }
   }
+  grid_wait();            // the threads that read the residual below
   __syncwarp();
   cluster_sync_all();     // every partial sum of the cluster is in place
   if (!*abort_flag) {
@@ -234,16 +246,8 @@ static int launch_few(const void* X, const void* W, FewArgs a, long long ldx, lo
   const int per = (kblocks + splits - 1) / splits;
   splits = (kblocks + per - 1) / per;     // every CTA has a slice
   a.k_per_split = per * BK;
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(splits, panels, mblocks);
-  cfg.blockDim = dim3(kGemmThreads, 1, 1);
-  cfg.dynamicSmemBytes = FewSmem<NB>::kTotal;
-  cfg.stream = stream;
-  cudaLaunchAttribute at[1];
-  at[0].id = cudaLaunchAttributeClusterDimension;
-  at[0].val.clusterDim.x = splits; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = 1;
-  cfg.attrs = at; cfg.numAttrs = 1;
-  const cudaError_t ce = cudaLaunchKernelEx(&cfg, kern, tmW, tmX, a);
+  const cudaError_t ce = launch(kern, dim3(splits, panels, mblocks), dim3(kGemmThreads), FewSmem<NB>::kTotal, stream, splits,
+                                tmW, tmX, a);
   if (ce != cudaSuccess) {
     (void)cudaGetLastError();
     return 1000 + (int)ce;
@@ -256,6 +260,13 @@ static int launch_few(const void* X, const void* W, FewArgs a, long long ldx, lo
 using namespace ob;
 
 extern "C" {
+
+// Launches of this thread that support it overlap with the kernel before them (1) or not (0).  The caller sees to it that no
+// kernel of the sequence writes what the one after it reads as weights.
+int ob_overlap_launches(int on) {
+  overlapped_launches() = on != 0;
+  return 0;
+}
 
 // C[M,N] (+)= X[M,K] W[N,K]^T (+ bias, residual): contract of ob_gemm_bf16 with K-major operands.
 // splits: CTAs per column panel (at most 8, fewer where the reduction has fewer slices; 0 chooses).

@@ -315,6 +315,7 @@ struct GlaStepArgs {
 // CTA = (head, sequence), 256 threads as R rows x (V / VW) column groups; VW = 4 needs V % 4 == 0.
 template <typename T, int VW>
 __global__ void __launch_bounds__(256) gla_step_kernel(const GlaStepArgs p) {
+  grid_begin();
   extern __shared__ float sm[];     // a[K], k[K], q[K], v[V], part[R*V]
   __shared__ float red[33];
   const int h = blockIdx.x, b = blockIdx.y, tid = threadIdx.x;
@@ -420,8 +421,8 @@ static int launch_step(const GlaStepArgs& a, int B, cudaStream_t s) {
   const int ncol = a.V / vw, R = 256 / ncol > 1 ? 256 / ncol : 1;
   const int smem = (3 * a.K + a.V + R * a.V) * 4;
   if (smem > 48 * 1024) return 6005;
-  if (vw == 4) gla_step_kernel<T, 4><<<grid, 256, smem, s>>>(a);
-  else gla_step_kernel<T, 1><<<grid, 256, smem, s>>>(a);
+  if (vw == 4) OB_LAUNCH((gla_step_kernel<T, 4>), grid, 256, smem, s, a);
+  else OB_LAUNCH((gla_step_kernel<T, 1>), grid, 256, smem, s, a);
   OB_CHECK_LAUNCH();
   return 0;
 }

@@ -32,6 +32,7 @@ struct LatentPrepArgs {
 
 template <typename T>
 __global__ void __launch_bounds__(256) latent_prepare_kernel(const LatentPrepArgs p) {
+  grid_begin();
   __shared__ float red[33];
   const int n = blockIdx.x;
   const int pos = p.pos[n];
@@ -89,6 +90,7 @@ template <typename T, typename O, bool VEC>
 __global__ void __launch_bounds__(128) latent_absorb_kernel(const T* __restrict__ q, long long ldq, int head_stride,
                                                             const T* __restrict__ uk, O* __restrict__ out, int N, int H,
                                                             int dim, int rank) {
+  grid_begin();
   extern __shared__ __align__(16) float sq[];   // [dim][8]
   __shared__ float part[4][8][128];
   const int h = blockIdx.y, n0 = blockIdx.z * 8, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -134,6 +136,7 @@ __global__ void __launch_bounds__(128) latent_absorb_kernel(const T* __restrict_
 template <typename T, bool VEC>
 __global__ void __launch_bounds__(256) latent_expand_kernel(const float* __restrict__ ol, const T* __restrict__ uv,
                                                             T* __restrict__ out, int N, int H, int vdim, int rank) {
+  grid_begin();
   extern __shared__ __align__(16) float so[];   // [8][rank padded to 4]
   const int h = blockIdx.y, n0 = blockIdx.z * 8, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int nn = min(8, N - n0), ld = (rank + 3) & ~3;
@@ -177,7 +180,7 @@ __global__ void __launch_bounds__(256) latent_expand_kernel(const float* __restr
 
 template <typename T>
 static int launch_prepare(const LatentPrepArgs& a, int N, cudaStream_t s) {
-  latent_prepare_kernel<T><<<N, 256, 0, s>>>(a);
+  OB_LAUNCH(latent_prepare_kernel<T>, N, 256, 0, s, a);
   OB_CHECK_LAUNCH();
   return 0;
 }
@@ -212,8 +215,8 @@ int ob_latent_absorb(const void* q, long long ldq, int head_stride, const void* 
     const long long qo = n0 * ldq, oo = (long long)n0 * H * rank;
 #define OB_ABSORB(T, O)                                                                                              \
   do {                                                                                                               \
-    if (vec) latent_absorb_kernel<T, O, true><<<grid, 128, smem, s>>>((const T*)q + qo, ldq, head_stride, (const T*)uk, (O*)out + oo, n, H, dim, rank); \
-    else latent_absorb_kernel<T, O, false><<<grid, 128, smem, s>>>((const T*)q + qo, ldq, head_stride, (const T*)uk, (O*)out + oo, n, H, dim, rank);    \
+    if (vec) OB_LAUNCH((latent_absorb_kernel<T, O, true>), grid, 128, smem, s, (const T*)q + qo, ldq, head_stride, (const T*)uk, (O*)out + oo, n, H, dim, rank); \
+    else OB_LAUNCH((latent_absorb_kernel<T, O, false>), grid, 128, smem, s, (const T*)q + qo, ldq, head_stride, (const T*)uk, (O*)out + oo, n, H, dim, rank);    \
   } while (0)
     if (fp32) OB_ABSORB(float, float);
     else if (out_bf16) OB_ABSORB(bf16, bf16);
@@ -237,8 +240,8 @@ int ob_latent_expand(const float* o_lat, const void* uv, void* out, int N, int H
 #define OB_EXPAND(T)                                                                                                 \
   do {                                                                                                               \
     T* o = (T*)out + (long long)n0 * H * vdim;                                                                       \
-    if (vec) latent_expand_kernel<T, true><<<grid, 256, smem, s>>>(ol, (const T*)uv, o, n, H, vdim, rank);           \
-    else latent_expand_kernel<T, false><<<grid, 256, smem, s>>>(ol, (const T*)uv, o, n, H, vdim, rank);              \
+    if (vec) OB_LAUNCH((latent_expand_kernel<T, true>), grid, 256, smem, s, ol, (const T*)uv, o, n, H, vdim, rank);           \
+    else OB_LAUNCH((latent_expand_kernel<T, false>), grid, 256, smem, s, ol, (const T*)uv, o, n, H, vdim, rank);              \
   } while (0)
     if (fp32) OB_EXPAND(float);
     else OB_EXPAND(bf16);

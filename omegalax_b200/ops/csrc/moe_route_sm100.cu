@@ -18,6 +18,7 @@ template <typename T, bool kSigmoid>
 __global__ void router_topk_kernel(const T* __restrict__ logits, long long ldl, float* __restrict__ probs,
                                    float* __restrict__ weights, int* __restrict__ idx, int* __restrict__ counts,
                                    long long M, int E, int k, int renorm) {
+  grid_begin();
   const int lane = threadIdx.x & 31;
   const long long row = (blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5;
   if (row >= M) return;
@@ -239,7 +240,7 @@ int ob_router_topk(const void* logits, float* probs, float* weights, int* idx, i
   if (E % 32 || E > 32 * kMaxEPL || E <= 0) return 6001;
   if (k <= 0 || k > kMaxTopK || k > E) return 6005;
   if (M <= 0) return 0;
-  router_topk_kernel<bf16, false><<<(unsigned)((M * 32 + 255) / 256), 256, 0, s>>>((const bf16*)logits, E, probs, weights,
+  OB_LAUNCH((router_topk_kernel<bf16, false>), (unsigned)((M * 32 + 255) / 256), 256, 0, s, (const bf16*)logits, E, probs, weights,
                                                                                    idx, counts, M, E, k, renorm);
   OB_CHECK_LAUNCH();
   return 0;
@@ -251,7 +252,7 @@ int ob_router_sigmoid_topk(const float* logits, long long ldl, float* weights, i
   if (E > 32 * kMaxEPL || E <= 0) return 6001;
   if (k <= 0 || k > kMaxTopK || k > E) return 6005;
   if (M <= 0) return 0;
-  router_topk_kernel<float, true><<<(unsigned)((M * 32 + 255) / 256), 256, 0, s>>>(logits, ldl, nullptr, weights, idx, nullptr,
+  OB_LAUNCH((router_topk_kernel<float, true>), (unsigned)((M * 32 + 255) / 256), 256, 0, s, logits, ldl, nullptr, weights, idx, nullptr,
                                                                                    M, E, k, 0);
   OB_CHECK_LAUNCH();
   return 0;

@@ -42,6 +42,7 @@ __global__ void __launch_bounds__(128) moe_gather_kernel(const T* __restrict__ h
 template <typename T, bool VEC>
 __global__ void __launch_bounds__(256) moe_sum_kernel(const T* __restrict__ y, const int* __restrict__ dest,
                                                       float* __restrict__ x, int k, int D, int max_rows) {
+  grid_begin();
   const long long m = blockIdx.y;
   const int i = (blockIdx.x * 256 + threadIdx.x) * (VEC ? 4 : 1);
   if (i >= D) return;
@@ -165,6 +166,7 @@ __device__ __forceinline__ void few_rows(const bf16* const* w, const bf16* const
 __global__ void __launch_bounds__(128) expert_up_few_kernel(const bf16* __restrict__ h, const bf16* __restrict__ W,
                                                             const int* __restrict__ idx, const float* __restrict__ weight,
                                                             bf16* __restrict__ act, int P, int k, int F, int K) {
+  grid_begin();
   __shared__ int list[kFewPairs], count;
   __shared__ __align__(16) float red[4][2][2][128];
   const int e = blockIdx.y, f0 = blockIdx.x * 16;
@@ -205,6 +207,7 @@ __global__ void __launch_bounds__(128) expert_up_few_kernel(const bf16* __restri
 __global__ void __launch_bounds__(128) expert_down_few_kernel(const bf16* __restrict__ act, const bf16* __restrict__ W,
                                                               const int* __restrict__ idx, float* __restrict__ y, int P, int D,
                                                               int F) {
+  grid_begin();
   __shared__ int list[kFewPairs], count;
   __shared__ __align__(16) float red[4][2][128];
   const int e = blockIdx.y, d0 = blockIdx.x * 16;
@@ -263,7 +266,7 @@ int ob_moe_sum(const void* y, const int* dest, float* x, int M, int k, int D, in
     const long long skip = dest ? 0 : (long long)m0 * k;
     float* xo = x + (long long)m0 * D;
     const int rows = max_rows - (int)skip;
-#define OB_SUM(T, V) moe_sum_kernel<T, V><<<grid, 256, 0, s>>>((const T*)y + skip * D, d, xo, k, D, rows)
+#define OB_SUM(T, V) OB_LAUNCH((moe_sum_kernel<T, V>), grid, 256, 0, s, (const T*)y + skip * D, d, xo, k, D, rows)
     if (y_fp32) { if (vec) OB_SUM(float, true); else OB_SUM(float, false); }
     else { if (vec) OB_SUM(bf16, true); else OB_SUM(bf16, false); }
 #undef OB_SUM
@@ -293,9 +296,9 @@ int ob_experts_few(const void* h, const int* idx, const float* weight, const voi
   if (P > kFewPairs || k <= 0 || E <= 0 || E > 65535) return 6005;
   if ((D & 7) || (F & 7)) return 6001;
   if ((((uintptr_t)h) | ((uintptr_t)gate_up) | ((uintptr_t)down) | ((uintptr_t)act)) & 15) return 6002;
-  expert_up_few_kernel<<<dim3((F + 15) / 16, E), 128, 0, s>>>((const bf16*)h, (const bf16*)gate_up, idx, weight, (bf16*)act, P, k, F, D);
+  OB_LAUNCH(expert_up_few_kernel, (dim3((F + 15) / 16, E)), 128, 0, s, (const bf16*)h, (const bf16*)gate_up, idx, weight, (bf16*)act, P, k, F, D);
   OB_CHECK_LAUNCH();
-  expert_down_few_kernel<<<dim3((D + 15) / 16, E), 128, 0, s>>>((const bf16*)act, (const bf16*)down, idx, y, P, D, F);
+  OB_LAUNCH(expert_down_few_kernel, (dim3((D + 15) / 16, E)), 128, 0, s, (const bf16*)act, (const bf16*)down, idx, y, P, D, F);
   OB_CHECK_LAUNCH();
   return 0;
 }

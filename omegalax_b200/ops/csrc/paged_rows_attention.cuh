@@ -153,6 +153,7 @@ constexpr float kLog2e = 1.4426950408889634f;
 // keys.  Output: warp w owns rank_pad / 8 = 8 * NT value columns for all heads of the block, in registers.
 template <int MT, int NT, bool kScoreValues, typename O>
 __global__ void __launch_bounds__(256) paged_decode_kernel(const PagedDecodeArgs p) {
+  grid_begin();
   extern __shared__ __align__(128) uint8_t smem[];
   constexpr int HB = 16 * MT;
   constexpr int RP = 64 * NT;
@@ -405,6 +406,7 @@ template <typename O>
 __global__ void __launch_bounds__(128) paged_combine_kernel(const float* __restrict__ part_o, const float* __restrict__ part_ml,
                                                             const bf16* __restrict__ sink, O* __restrict__ out, int H,
                                                             int rank, int splits) {
+  grid_begin();
   __shared__ float wgt[64];
   const int h = blockIdx.x, b = blockIdx.y;
   const float2* ml = (const float2*)part_ml + (long long)b * splits * H + h;
@@ -449,10 +451,10 @@ static int launch_paged_decode(const PagedDecodeArgs& a, int B, cudaStream_t s) 
   auto kern = paged_decode_kernel<MT, NT, kScoreValues, O>;
   OB_ENSURE_DYN_SMEM(kern, 227 * 1024);
   dim3 grid(a.splits, (a.group + 16 * MT - 1) / (16 * MT) * (a.H / a.group), B);
-  kern<<<grid, 256, smem, s>>>(a);
+  OB_LAUNCH(kern, grid, 256, smem, s, a);
   OB_CHECK_LAUNCH();
   if (a.splits > 1) {
-    paged_combine_kernel<O><<<dim3(a.H, B, (a.rank + 127) / 128), 128, 0, s>>>(a.part_o, a.part_ml, a.sink, (O*)a.out, a.H,
+    OB_LAUNCH(paged_combine_kernel<O>, (dim3(a.H, B, (a.rank + 127) / 128)), 128, 0, s, a.part_o, a.part_ml, a.sink, (O*)a.out, a.H,
                                                                                a.rank, a.splits);
     OB_CHECK_LAUNCH();
   }

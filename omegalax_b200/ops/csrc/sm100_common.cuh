@@ -45,6 +45,17 @@ __device__ __forceinline__ uint32_t smem_u32(const void* p) {
   return (uint32_t)__cvta_generic_to_shared(p);
 }
 
+// Kernels that may be launched overlapped (host_utils.h).  grid_wait(): the kernel before has ended and its writes are
+// visible; grid_next(): blocks of the kernel after may move in.  The order matters: who comes after this block's grid_next knows
+// that all grids before this one have ended, so weights may be read ahead of grid_wait().  Both do nothing in an ordinary launch.
+__device__ __forceinline__ void grid_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void grid_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void grid_begin() {
+  grid_wait();
+  grid_next();
+}
+__device__ __forceinline__ void prefetch_l2(const void* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
+
 __device__ __forceinline__ bool elect_one() {
   uint32_t pred = 0;
   asm volatile(

@@ -9,6 +9,7 @@ namespace ob {
 template <typename T>
 __global__ void embed_rows_kernel(const int* __restrict__ ids, const T* __restrict__ table, float* __restrict__ out,
                                   int V, int D, int* status) {
+  grid_begin();
   const int n = blockIdx.x;
   const int id = ids[n];
   float* o = out + (long long)n * D;
@@ -36,6 +37,11 @@ __global__ void __launch_bounds__(256) norm_rows_kernel(const float* __restrict_
   __shared__ float red[33];
   const float* xr = x + (long long)blockIdx.x * D;
   T* yr = y + (long long)blockIdx.x * D;
+  for (int c = threadIdx.x * 4; c < D; c += 1024) {
+    prefetch_l2(w + c);
+    if (kMean) prefetch_l2(b + c);
+  }
+  grid_begin();
   float4 v[NV];
   float s = 0.f;
 #pragma unroll
@@ -70,6 +76,7 @@ __global__ void __launch_bounds__(256) norm_rows_kernel(const float* __restrict_
 template <typename T, bool kMean>
 __global__ void __launch_bounds__(256) norm_rows_any_kernel(const float* __restrict__ x, const T* __restrict__ w,
                                                             const T* __restrict__ b, T* __restrict__ y, int D, float eps) {
+  grid_begin();
   __shared__ float red[33];
   const float* xr = x + (long long)blockIdx.x * D;
   T* yr = y + (long long)blockIdx.x * D;
@@ -102,6 +109,7 @@ __device__ __forceinline__ float gate_value(float z, float up) {
 template <typename T, bool kGelu, bool VEC>
 __global__ void __launch_bounds__(256) gated_act_kernel(const T* __restrict__ x, T* __restrict__ y, const int* __restrict__ rows,
                                                         long long M, int F) {
+  grid_begin();
   if (rows) M = min(M, (long long)*rows);
   const unsigned C = VEC ? F >> 3 : F;
   const long long n = M * C, stride = (long long)gridDim.x * 256;
@@ -124,6 +132,7 @@ __global__ void __launch_bounds__(256) gated_act_kernel(const T* __restrict__ x,
 
 template <typename T>
 __global__ void relu_sq_kernel(const T* __restrict__ x, T* __restrict__ y, long long n) {
+  grid_begin();
   const long long n4 = n >> 2;
   const long long stride = (long long)gridDim.x * blockDim.x;
   const long long t0 = (long long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -139,6 +148,7 @@ __global__ void relu_sq_kernel(const T* __restrict__ x, T* __restrict__ y, long 
 }
 
 __global__ void soft_cap_kernel(float* __restrict__ x, long long n, float cap) {
+  grid_begin();
   const long long stride = (long long)gridDim.x * blockDim.x;
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride)
     x[i] = cap * tanhf(x[i] / cap);
@@ -148,11 +158,11 @@ template <typename T, bool kMean>
 static int launch_norm(const float* x, const void* w, const void* b, void* y, int N, int D, float eps, cudaStream_t s) {
   const T *wt = (const T*)w, *bt = (const T*)b;
   T* yt = (T*)y;
-  if (D % 4 || D > 8192) norm_rows_any_kernel<T, kMean><<<N, 256, 0, s>>>(x, wt, bt, yt, D, eps);
-  else if (D <= 1024) norm_rows_kernel<T, 1, kMean><<<N, 256, 0, s>>>(x, wt, bt, yt, D, eps);
-  else if (D <= 2048) norm_rows_kernel<T, 2, kMean><<<N, 256, 0, s>>>(x, wt, bt, yt, D, eps);
-  else if (D <= 4096) norm_rows_kernel<T, 4, kMean><<<N, 256, 0, s>>>(x, wt, bt, yt, D, eps);
-  else norm_rows_kernel<T, 8, kMean><<<N, 256, 0, s>>>(x, wt, bt, yt, D, eps);
+  if (D % 4 || D > 8192) OB_LAUNCH((norm_rows_any_kernel<T, kMean>), N, 256, 0, s, x, wt, bt, yt, D, eps);
+  else if (D <= 1024) OB_LAUNCH((norm_rows_kernel<T, 1, kMean>), N, 256, 0, s, x, wt, bt, yt, D, eps);
+  else if (D <= 2048) OB_LAUNCH((norm_rows_kernel<T, 2, kMean>), N, 256, 0, s, x, wt, bt, yt, D, eps);
+  else if (D <= 4096) OB_LAUNCH((norm_rows_kernel<T, 4, kMean>), N, 256, 0, s, x, wt, bt, yt, D, eps);
+  else OB_LAUNCH((norm_rows_kernel<T, 8, kMean>), N, 256, 0, s, x, wt, bt, yt, D, eps);
   OB_CHECK_LAUNCH();
   return 0;
 }
@@ -172,8 +182,8 @@ extern "C" {
 int ob_embed_rows(const int* ids, const void* table, float* out, int N, int V, int D, int fp32, int* status,
                   cudaStream_t s) {
   if (N <= 0) return 0;
-  if (fp32) embed_rows_kernel<float><<<N, 256, 0, s>>>(ids, (const float*)table, out, V, D, status);
-  else embed_rows_kernel<bf16><<<N, 256, 0, s>>>(ids, (const bf16*)table, out, V, D, status);
+  if (fp32) OB_LAUNCH(embed_rows_kernel<float>, N, 256, 0, s, ids, (const float*)table, out, V, D, status);
+  else OB_LAUNCH(embed_rows_kernel<bf16>, N, 256, 0, s, ids, (const bf16*)table, out, V, D, status);
   OB_CHECK_LAUNCH();
   return 0;
 }
@@ -197,8 +207,8 @@ int ob_gated_act(const void* x, void* y, const int* rows, long long M, int F, in
   const unsigned grid = flat_grid(M * (vec ? F / 8 : F));
 #define OB_ACT(T, G)                                                                                  \
   do {                                                                                                \
-    if (vec) gated_act_kernel<T, G, true><<<grid, 256, 0, s>>>((const T*)x, (T*)y, rows, M, F);       \
-    else gated_act_kernel<T, G, false><<<grid, 256, 0, s>>>((const T*)x, (T*)y, rows, M, F);          \
+    if (vec) OB_LAUNCH((gated_act_kernel<T, G, true>), grid, 256, 0, s, (const T*)x, (T*)y, rows, M, F);       \
+    else OB_LAUNCH((gated_act_kernel<T, G, false>), grid, 256, 0, s, (const T*)x, (T*)y, rows, M, F);          \
   } while (0)
   if (fp32) { if (gelu) OB_ACT(float, true); else OB_ACT(float, false); }
   else { if (gelu) OB_ACT(bf16, true); else OB_ACT(bf16, false); }
@@ -209,15 +219,15 @@ int ob_gated_act(const void* x, void* y, const int* rows, long long M, int F, in
 
 int ob_relu_sq(const void* x, void* y, long long n, int fp32, cudaStream_t s) {
   if (n <= 0) return 0;
-  if (fp32) relu_sq_kernel<float><<<flat_grid(n / 4), 256, 0, s>>>((const float*)x, (float*)y, n);
-  else relu_sq_kernel<bf16><<<flat_grid(n / 4), 256, 0, s>>>((const bf16*)x, (bf16*)y, n);
+  if (fp32) OB_LAUNCH(relu_sq_kernel<float>, flat_grid(n / 4), 256, 0, s, (const float*)x, (float*)y, n);
+  else OB_LAUNCH(relu_sq_kernel<bf16>, flat_grid(n / 4), 256, 0, s, (const bf16*)x, (bf16*)y, n);
   OB_CHECK_LAUNCH();
   return 0;
 }
 
 int ob_soft_cap(float* x, long long n, float cap, cudaStream_t s) {
   if (n <= 0) return 0;
-  soft_cap_kernel<<<flat_grid(n), 256, 0, s>>>(x, n, cap);
+  OB_LAUNCH(soft_cap_kernel, flat_grid(n), 256, 0, s, x, n, cap);
   OB_CHECK_LAUNCH();
   return 0;
 }

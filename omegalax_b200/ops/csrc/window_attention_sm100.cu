@@ -38,6 +38,7 @@ __device__ __forceinline__ bool window_row_ok(const WindowPrepArgs& p, int n, in
 // from the sums of squares to the stores.  2 * pairs % 16, dim % 8, vdim % 8 == 0, 16-byte aligned rows.
 template <typename T, int NU>
 __global__ void __launch_bounds__(256) window_prepare_kernel(const WindowPrepArgs p) {
+  grid_begin();
   __shared__ float red[33];
   const int n = blockIdx.x;
   const int pos = p.pos[n], row = p.row[n];
@@ -120,6 +121,7 @@ __global__ void __launch_bounds__(256) window_prepare_kernel(const WindowPrepArg
 // any sizes
 template <typename T>
 __global__ void __launch_bounds__(256) window_prepare_any_kernel(const WindowPrepArgs p) {
+  grid_begin();
   __shared__ float red[33];
   const int n = blockIdx.x;
   const int pos = p.pos[n], row = p.row[n];
@@ -172,10 +174,10 @@ static int launch_window_prepare(const WindowPrepArgs& a, int N, cudaStream_t s)
   const uintptr_t bases = (uintptr_t)a.proj | (uintptr_t)a.norm_w | (uintptr_t)a.cache | (uintptr_t)a.v_first |
                           (uintptr_t)a.cos_t | (uintptr_t)a.sin_t;
   const bool vec = !((a.pairs | a.dim | a.vdim) & 7) && !((a.ldp | a.ldv | a.ldc) & 7) && !(bases & 15);
-  if (vec && units <= 256) window_prepare_kernel<T, 1><<<N, 256, 0, s>>>(a);
-  else if (vec && units <= 512) window_prepare_kernel<T, 2><<<N, 256, 0, s>>>(a);
-  else if (vec && units <= 1024) window_prepare_kernel<T, 4><<<N, 256, 0, s>>>(a);
-  else window_prepare_any_kernel<T><<<N, 256, 0, s>>>(a);
+  if (vec && units <= 256) OB_LAUNCH((window_prepare_kernel<T, 1>), N, 256, 0, s, a);
+  else if (vec && units <= 512) OB_LAUNCH((window_prepare_kernel<T, 2>), N, 256, 0, s, a);
+  else if (vec && units <= 1024) OB_LAUNCH((window_prepare_kernel<T, 4>), N, 256, 0, s, a);
+  else OB_LAUNCH(window_prepare_any_kernel<T>, N, 256, 0, s, a);
   OB_CHECK_LAUNCH();
   return 0;
 }
