@@ -49,10 +49,25 @@ class DecodeGraph:
         here.wait_stream(side)
         self.launches = K.launch_count() - before
         self.model = model
+        self.every = False            # the last call had a token for every sequence, as far as the model says so
+        self.asked, self.arrived = None, torch.cuda.Event()     # what a step that runs ahead asks the device for (pinned)
 
     @staticmethod
     def enabled() -> bool:
         return os.environ.get("OMEGALAX_B200_DECODE_GRAPH", "1") == "1"
+
+    @staticmethod
+    def recorded(model, cache, key) -> "DecodeGraph | None":
+        """The recording that a step with this key would replay."""
+        state = cache.decode_graph
+        if state is None or state[0] is not model or state[1] is None or state[2] != key or not DecodeGraph.enabled():
+            return None
+        return state[1]
+
+    def replay(self):
+        K.add_launches(self.launches)
+        self.graph.replay()
+        return self.out
 
     @staticmethod
     def step(model, cache, batch, key=None, alone: bool = False):
@@ -72,8 +87,7 @@ class DecodeGraph:
                 return model.run_layers(batch, cache)
             graph = DecodeGraph(model, cache, batch)
             cache.decode_graph = (model, graph, key)
-        else:
-            graph.batch.flat.copy_(batch.flat)
-            K.add_launches(graph.launches)
-        graph.graph.replay()
-        return graph.out
+            graph.graph.replay()
+            return graph.out
+        graph.batch.flat.copy_(batch.flat)
+        return graph.replay()

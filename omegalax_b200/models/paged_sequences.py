@@ -65,6 +65,24 @@ class PagedSequences:
         if changed:
             self._send(self.block_table, self.block_table_host.clamp_min(0))
 
+    def reserve_ahead(self):
+        """Pages for one more token of every sequence, before it is known which of them get one: the sequences that were given a
+        page, or None (and nothing is reserved) where one is full or the pages do not suffice."""
+        want = [b for b, n in enumerate(self.seq_lens_host) if n // self.page_size >= self.blocks_held[b]]
+        if len(want) > len(self.allocator.free) or any(self.blocks_held[b] >= self.max_blocks for b in want):
+            return None
+        self.reserve([1] * self.B)
+        return want
+
+    def take_back(self, seqs: list[int]) -> None:
+        """Undo ``reserve_ahead``: the free list is as it was."""
+        for b in reversed(seqs):
+            j = self.blocks_held[b] = self.blocks_held[b] - 1
+            self.allocator.release([self.block_table_host[b, j]])
+            self.block_table_host[b, j] = -1
+        if seqs:
+            self._send(self.block_table, self.block_table_host.clamp_min(0))
+
     def _send(self, dst, host) -> None:
         # The copy of pageable memory returns when it is staged: a blocking one would wait for the step in flight,
         # and the device would idle while the host prepares the next (64 sequences: 0.7 of 3.6 ms).

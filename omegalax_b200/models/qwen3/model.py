@@ -339,6 +339,46 @@ class Qwen3(nn.Module):
         y = layer.mlp(layer.post_norm(x), residual=x)
         return y[0] if layer.is_moe else y
 
+    @staticmethod
+    def _indices(ids, real, cache):
+        """Indices of a call's tokens (host [B, T]: ids, and which of them are tokens): parts by name, and all of them in one
+        buffer, where every part starts on a 16-byte boundary."""
+        ps, counts = cache.page_size, real.sum(-1)
+        seq = real.nonzero()[:, 0]
+        hist = torch.tensor(cache.seq_lens_host)
+        slot = hist[seq] + (real.cumsum(-1) - 1)[real]
+        rows = cache.block_table_host[seq, slot // ps] * ps + slot % ps
+        cu = torch.cat([counts.new_zeros(1), counts.cumsum(0)])
+        has = counts.nonzero()[:, 0]
+        parts = dict(ids=ids[real], seq=seq, slot=slot, rows=rows, cu=cu, lens=hist + counts, has=has, last=cu[has + 1] - 1)
+        return parts, torch.cat([F.pad(t.to(torch.int32), (0, -t.numel() % 4)) for t in parts.values()])
+
+    def _run_ahead(self, graph, both, cache):
+        """A recorded step before the host knows the ids (``both``: ids and marks [2, B, 1] on the device), for callers that had a
+        token for every sequence the last time.  Where that holds again the device goes on without a gap: one sequence
+        of 4096 tokens, 8 layers of 4096 channels, spent 0.25 of 1.33 ms waiting for the host.  Returns the residual rows; or, where a
+        sequence got no token, None and ``both`` on the host, with the cache as it was: what was written for such
+        a sequence lies behind its last token, where its next one will go, and its id counted as 0."""
+        pages = cache.reserve_ahead()
+        if pages is None:
+            return None, both
+        if graph.asked is None:
+            graph.asked = torch.empty(both.shape, dtype=both.dtype, pin_memory=True)
+        graph.asked.copy_(both, non_blocking=True)
+        graph.arrived.record()
+        cache.settle()
+        one = torch.ones(cache.B, 1, dtype=torch.bool)
+        graph.batch.flat.copy_(self._indices(one.to(torch.int32), one, cache)[1], non_blocking=True)
+        torch.mul(both[0], both[1], out=graph.batch.ids.view(-1, 1))
+        x = graph.replay()
+        graph.arrived.synchronize()
+        if bool(graph.asked[1].all()):
+            cache.advance([1] * cache.B)
+            return x, both
+        graph.every = False
+        cache.take_back(pages)
+        return None, graph.asked.clone()
+
     @torch.no_grad()
     def decode_paged(self, token_ids, segment_ids, cache, select=None):
         """Prefill or one decode step against a ``PagedKVCache`` (CUDA bf16).  Only real tokens
@@ -349,12 +389,18 @@ class Qwen3(nn.Module):
 
         cfg = self.cfg
         B, T = token_ids.shape
-        dev, ps, i32 = token_ids.device, cache.page_size, torch.int32
+        dev = token_ids.device
         key = self._recordable(cache) if T == 1 else None
         # The indices of the call are worked out on the host and travel in one copy: the ids are the only thing
         # waited for.  A step of one token per sequence is then one graph launch (8 layers of 4096 channels: 3.1 ms of
         # launches for 1.1 ms of kernels).
-        both = torch.stack((token_ids.to(i32), (segment_ids != 0).to(i32))).cpu()
+        both = torch.stack((token_ids.to(torch.int32), (segment_ids != 0).to(torch.int32)))
+        graph = DecodeGraph.recorded(self, cache, key) if key is not None and select is None else None
+        if graph is not None and graph.every and B == cache.B and dev == graph.batch.flat.device:
+            x, both = self._run_ahead(graph, both, cache)
+            if x is not None:
+                return self.final_norm(x)
+        both = both.cpu()
         real = both[1] != 0
         counts = real.sum(-1)
         new_tokens = counts.tolist()
@@ -365,21 +411,18 @@ class Qwen3(nn.Module):
             raise NotImplementedError("multi-token calls are only supported on an empty cache (prefill)")
         if N == 0:
             return torch.zeros(0 if select is not None else B, cfg.emb_dim, dtype=self.embedder.weight.dtype, device=dev)
-        seq = real.nonzero()[:, 0]
-        hist = torch.tensor(cache.seq_lens_host)
-        slot = hist[seq] + (real.cumsum(-1) - 1)[real]
-        rows = cache.block_table_host[seq, slot // ps] * ps + slot % ps
-        cu = torch.cat([counts.new_zeros(1), counts.cumsum(0)])
-        has = counts.nonzero()[:, 0]
-        parts = dict(ids=both[0][real], seq=seq, slot=slot, rows=rows, cu=cu, lens=hist + counts, has=has, last=cu[has + 1] - 1)
-        # every part starts on a 16-byte boundary; pageable memory is staged before the copy returns
-        flat = torch.cat([F.pad(t.to(i32), (0, -t.numel() % 4)) for t in parts.values()]).to(dev, non_blocking=True)
-        batch, at = SimpleNamespace(flat=flat, every=single and N == B), 0
+        parts, flat = self._indices(both[0], real, cache)
+        has = parts["has"]
+        # pageable memory is staged before the copy returns
+        batch, at = SimpleNamespace(flat=flat.to(dev, non_blocking=True), every=single and N == B), 0
         for name, t in parts.items():
-            setattr(batch, name, flat[at:at + t.numel()])
+            setattr(batch, name, batch.flat[at:at + t.numel()])
             at += t.numel() + -t.numel() % 4
         if batch.every and key is not None:
             x = DecodeGraph.step(self, cache, batch, key, alone=True)
+            graph = DecodeGraph.recorded(self, cache, key)
+            if graph is not None:
+                graph.every = True
         elif single:
             x = self.run_layers(batch, cache)
         else:

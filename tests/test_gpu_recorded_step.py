@@ -143,6 +143,32 @@ def test_idle_sequences_and_two_caches(served, monkeypatch):
             assert torch.equal(a, b)
 
 
+def test_a_step_that_runs_ahead_of_its_ids_leaves_the_cache_as_it_was(served, monkeypatch):
+    """Sequences without a token at steps that need new pages, a cache that is full, and one whose pages are all taken: logits, lengths,
+    pages and free list as when every step waits for its ids."""
+    from omegalax_b200.text import api
+
+    model, cfg = served
+    monkeypatch.setattr("omegalax_b200.models.decode_graph.other_threads", lambda: False)
+    steps = torch.randint(1, 1024, (14, B, 1), generator=torch.Generator().manual_seed(1)).cuda()
+    steps[4, 1] = steps[9, 0] = steps[10] = 0      # 20 + 4 tokens fill three pages of 8, 20 + 12 four
+    seen = []
+    for recorded in (True, False):
+        monkeypatch.setenv("OMEGALAX_B200_DECODE_GRAPH", "1" if recorded else "0")
+        cache = api.make_cache(cfg, B, T, 12, device="cuda", page_size=8, num_pages=B * 4)
+        out = [api.decode(model, cache, _ids()[0], 0, cfg)[0]]
+        for ids in steps:
+            try:
+                out.append(api.decode(model, cache, ids, 0, cfg)[0].clone())
+            except RuntimeError as e:
+                out.append(torch.tensor([len(str(e))]))
+            out.append(torch.tensor(cache.allocator.free + cache.seq_lens_host + cache.blocks_held))
+            out.append(cache.block_table_host.clone())
+        seen.append(out)
+    for i, (a, b) in enumerate(zip(*seen)):
+        assert torch.equal(a.cpu(), b.cpu()), i
+
+
 @pytest.mark.parametrize("free,times", [(1 << 20, 1), (1 << 34, 0)])
 def test_free_memory_of_the_allocator_is_given_back_where_a_recording_may_need_it(served, monkeypatch, free, times):
     """While a step is recorded the allocator cannot empty itself: done before, where the device has little left (a stand-in says how much)."""
