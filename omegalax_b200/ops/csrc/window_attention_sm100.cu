@@ -6,6 +6,7 @@
 //                           rewritten in place (prompts attend to the packed rows)
 //
 // Attention over the pages is that of paged_rows_attention.cuh with c = value and r = key.
+#include "decode_rows.cuh"
 #include "paged_rows_attention.cuh"
 
 namespace ob {
@@ -217,6 +218,15 @@ int ob_window_decode(const void* q, long long ldq, const void* cache, long long 
                      int G, int dim, int vdim, int window, int splits, float scale, cudaStream_t s) {
   if (B <= 0) return 0;
   if (G <= 0 || H % G) return 6005;
+  if (dim == 128 && vdim == 128 && H / G <= 8) {
+    DecodeRowsArgs a = {};
+    a.q = (const bf16*)q; a.ldq = ldq;
+    a.v = (const bf16*)cache; a.k = a.v + 128; a.pitch = ldc; a.head = 256;
+    a.table = table; a.len = len; a.max_blocks = max_blocks; a.page_size = page_size;
+    a.sink = (const bf16*)sink; a.part_o = part_o; a.part_ml = part_ml; a.out = (bf16*)out;
+    a.H = H; a.G = G; a.splits = splits; a.window = window; a.scale = scale;
+    return launch_decode_rows(a, B, s);
+  }
   PagedDecodeArgs a = {nullptr, (const bf16*)q, (const bf16*)cache, len, table, part_o, part_ml, (const bf16*)sink, out, ldq,
                        ldc, dim, H, H / G, vdim, dim, max_blocks, page_size, splits, window, scale * kLog2e};
   return dispatch_paged_decode<false, bf16>(a, B, s);

@@ -574,16 +574,19 @@ def kv_store(k, v, rows, k_pages, v_pages):
           N, G * HD, lib.stream_ptr())
 
 
+def decode_splits(blocks: int, keys: int) -> int:
+    """CTAs that share a sequence's keys: as many as fit at once, two on an SM, with at least 128 keys of capacity each.  In us by
+    splits, alone: 32 sequences of 2048 on 8 key heads 1 / 2 / 4: 48 54 62; one of 4096, 8 / 16 / 32 / 48: 13.8 11.3 11.8 16.2; eight of
+    4096 on 4, 4 / 8 / 16: 23.8 19.9 25.1; 64 of 1000 on 4, 1 / 2: 28.9 36.6."""
+    return max(1, min(32, 296 // max(blocks, 1), keys // 128))
+
+
 def decode_attn(q, k_pages, v_pages, block_table, seq_lens, page_size, scale, splits=None):
     """q [B,H,HD] attends over each sequence's pages; returns [B,H,HD]."""
     B, H, HD = q.shape
     G = k_pages.shape[2]
     if splits is None:
-        # two waves of the CTAs that fit an SM (one where eight heads share a row), at least 128 keys of capacity
-        # each.  32 sequences of 2048, 32 heads on 8, by splits 2 / 4 / 8 / 16: 75 69 71 80 us; one of 4096, by
-        # 8 / 16 / 32 / 48: 19.1 13.6 13.6 15.4; eight of 4096, 32 on 4, by 4 / 8 / 16 / 32: 41 35 39 48.
-        ctas = 1184 if H // G <= 4 else 296
-        splits = max(1, min(32, ctas // max(B * G, 1), block_table.shape[1] * page_size // 128))
+        splits = decode_splits(B * G, block_table.shape[1] * page_size)
     sc = (torch.empty(B * H * splits * HD, dtype=torch.float32, device=q.device),
           torch.empty(B * H * splits * 2, dtype=torch.float32, device=q.device))
     out = torch.empty_like(q)

@@ -359,7 +359,8 @@ def window_decode(q, cache, seen, block_table, page_size: int, H: int, G: int, d
     B = q.shape[0]
     if splits is None:
         keys = block_table.shape[1] * page_size
-        splits = window_decode_splits(B, H, G, min(keys, window) if window else keys)
+        keys = min(keys, window) if window else keys
+        splits = K.decode_splits(B * G, keys) if dim == vdim == 128 and H // G <= 8 else window_decode_splits(B, H, G, keys)
     part_o = part_ml = None
     if splits > 1:
         part_o = torch.empty(B * splits * H * vdim, dtype=f32, device=q.device)

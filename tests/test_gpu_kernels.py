@@ -777,6 +777,29 @@ def test_decode_attention_lengths(R, splits):
         torch.testing.assert_close(out[b].float(), torch.einsum("hs,shd->hd", p, vb), rtol=2.0 ** -8, atol=2.0 ** -10)
 
 
+@pytest.mark.parametrize("R,window", [(8, 0), (8, 100), (3, 16), (1, 1)])
+@pytest.mark.parametrize("splits", [1, 5, 70])
+def test_decode_attention_window_and_sink(R, window, splits):
+    """Lengths around the 16 keys of a group, windows that start inside one, any number of heads up to eight on a key head, pages of 24;
+    double precision, one rounding to bf16 (2^-8) of outputs of size one."""
+    from omegalax_b200.ops import lib, serving as S
+    torch.manual_seed(36)
+    G, ps, lens = 2, 24, [0, 1, 15, 16, 17, 33, 500]
+    B, H, blocks = len(lens), 2 * R, 21
+    store = torch.randn(B * blocks * ps, G * 256 + 8, device=_dev()).to(bf16)
+    table = torch.randperm(B * blocks, device=_dev()).to(torch.int32).view(B, blocks)
+    q, sink = (torch.randn(B, H * 128 + 8, device=_dev()) * 2).to(bf16)[:, :H * 128], torch.randn(H, device=_dev()).to(bf16)
+    n = torch.tensor(lens, device=_dev(), dtype=torch.int32)
+    out = S.window_decode(q, store, n, table, ps, H, G, 128, 128, 128 ** -0.5, window, sink=sink, splits=min(splits, 64))
+    _check(lib)
+    for b, m in enumerate(lens):
+        rows = store.view(-1, ps, store.shape[1])[table[b].long()].view(blocks * ps, -1)[max(0, m - (window or m)):m, :G * 256].double()
+        v, k = (t.repeat_interleave(R, 1) for t in rows.view(-1, G, 256).split(128, -1))
+        s = torch.einsum("hd,shd->hs", q[b].double().view(H, 128), k) * 128 ** -0.5
+        p = torch.softmax(torch.cat([s, sink.double()[:, None]], -1), -1)[:, :-1]
+        torch.testing.assert_close(out[b].double().view(H, 128), torch.einsum("hs,shd->hd", p, v), rtol=2.0 ** -8, atol=2.0 ** -10)
+
+
 @pytest.mark.parametrize("N", [1, 5, 1025])
 @pytest.mark.parametrize("G", [1, 3])
 def test_kv_store(N, G):
