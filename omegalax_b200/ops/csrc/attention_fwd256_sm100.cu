@@ -34,6 +34,7 @@ struct AttnFwd256Args {
   int causal;
   float scale_log2;
   int* status;
+  int B, qblocks;      // sequences and 128-row blocks of the longest one
 };
 
 struct AttnFwd256Smem {
@@ -68,12 +69,11 @@ attn_fwd256_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
 
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
-  const int b = blockIdx.z;
-  const int h = blockIdx.y;
+  const int h = blockIdx.x % p.H, b = blockIdx.x / p.H % p.B;
   const int g = h / (p.H / p.G);
   const int seq_start = __ldg(p.cu_seqlens + b);
   const int seqlen = __ldg(p.cu_seqlens + b + 1) - seq_start;
-  const int qblk = (int)gridDim.x - 1 - (int)blockIdx.x;   // heaviest query blocks first
+  const int qblk = p.qblocks - 1 - (int)(blockIdx.x / p.H / p.B);   // heaviest query blocks of all heads first
   const int q0 = qblk * 128;
   if (q0 >= seqlen) return;
   const int n_kv_total = (seqlen + 127) >> 7;
@@ -314,8 +314,10 @@ int launch_attn_fwd256(const void* q, const void* k, const void* v, void* out, f
   a.H = H; a.G = G; a.causal = causal;
   a.scale_log2 = scale * 1.4426950408889634f;
   a.status = status;
-  dim3 grid((max_seqlen + 127) / 128, H, B);
-  attn_fwd256_kernel<<<grid, kF256Threads, AttnFwd256Smem::kTotal, stream>>>(tmQ, tmK, tmV, a);
+  a.B = B; a.qblocks = (max_seqlen + 127) / 128;
+  const long long ctas = (long long)a.qblocks * H * B;
+  if (ctas > 0x7fffffff) return 6005;
+  attn_fwd256_kernel<<<(unsigned)ctas, kF256Threads, AttnFwd256Smem::kTotal, stream>>>(tmQ, tmK, tmV, a);
   OB_CHECK_LAUNCH();
   return 0;
 }
