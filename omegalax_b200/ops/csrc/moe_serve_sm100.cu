@@ -3,15 +3,12 @@
 //
 // Prompts sort (token, slot) pairs by expert (moe_route_sm100.cu), gather the scaled rows, run the
 // grouped tcgen05 GEMM (or, for fp32 and sizes it cannot address, expert_rows_any_kernel) and sum.
-// Few pairs (decoding) skip the sort: a CTA of the *_few kernels owns 16 output features of one expert,
-// finds the pairs routed to it and streams the expert's weights past them on mma.sync tiles, weights as
-// the 16-row operand and up to 16 pairs as columns, so that every weight is read once.
+// Few pairs per expert (decoding, short prompts) have a plan of their own, without padding, and kernels that stream each used
+// expert's weights once past the pairs routed to it.
 #include "host_utils.h"
 #include "serve_common.cuh"
 
 namespace ob {
-
-constexpr int kFewPairs = 2048;      // most (token, slot) pairs of the *_few kernels
 
 // ------------------------------------------------------------------------------------------------ row movement
 // xs[dest[p]] = w[p] * h[p / k]
@@ -107,133 +104,284 @@ __global__ void __launch_bounds__(256) expert_rows_any_kernel(const T* __restric
 }
 
 // ------------------------------------------------------------------------------------------------ few pairs
-__device__ __forceinline__ void mma_bf16(float* c, uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
-  asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
-               : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
-               : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
-}
+// Pairs in the order of their experts, and units: at most `cap` consecutive pairs of one expert.
+//   order [P]  pairs by expert (in any order within one: a pair's results do not depend on its place)
+//   unit [2 * max]  first place in the order, expert << 8 | pairs - 1;  count: number of units
+// One CTA; ids outside 0 ... E - 1 belong to no unit.
+constexpr int kPlanExperts = 8192;      // counted in shared memory; more of them in `wide` [E]
 
-// The pairs routed to expert e, in any order (results do not depend on it).
-__device__ __forceinline__ int find_pairs(const int* __restrict__ idx, int P, int e, int* list, int* count) {
-  if (threadIdx.x == 0) *count = 0;
+__global__ void __launch_bounds__(1024) expert_units_kernel(const int* __restrict__ idx, int P, int E, int cap, int* __restrict__ order,
+                                                            int* __restrict__ unit, int* __restrict__ count, int* wide) {
+  extern __shared__ int near[];
+  __shared__ int part[2][32];
+  int* hist = wide ? wide : near;      // [E] pairs, then the next free place
+  grid_begin();
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  for (int e = tid; e < E; e += 1024) hist[e] = 0;
   __syncthreads();
-  for (int i = threadIdx.x; i < P; i += 128)
-    if (idx[i] == e) list[atomicAdd(count, 1)] = i;
+  for (int i = tid; i < P; i += 1024)
+    if ((unsigned)idx[i] < (unsigned)E) atomicAdd(hist + idx[i], 1);
   __syncthreads();
-  return *count;
-}
-
-// acc[t][c] += 16 rows of NW weight matrices (w[t], pitch K) times up to 16 columns, over this warp's quarter of
-// K.  Column g of block c is the row x[c] of its lane group.  The four lanes of a group hold 8 consecutive
-// channels each; both operands use that order, so a pair of MMAs consumes a 32-channel chunk with one
-// 16-byte load per operand row.  K % 8 == 0.
-template <int NW>
-__device__ __forceinline__ void few_rows(const bf16* const* w, const bf16* const* x, bool two, int K, int warp, int tq,
-                                         float (&acc)[NW][2][4]) {
-  constexpr int U = 4;                     // chunks in flight
-  const uint4 zero = make_uint4(0, 0, 0, 0);
-  for (int k0 = warp * 32 * U; k0 < K; k0 += 4 * 32 * U) {
-    uint4 a[U][NW][2], b[U][2];
+  // places and units before the experts of this thread: inclusive sums over the threads, less its own
+  const int per = (E + 1023) / 1024, lo = tid * per, hi = min(lo + per, E);
+  int np = 0, nu = 0;
+  for (int e = lo; e < hi; ++e) {
+    np += hist[e];
+    nu += (hist[e] + cap - 1) / cap;
+  }
+  int sp = np, su = nu;
 #pragma unroll
-    for (int u = 0; u < U; ++u) {
-      const int k = k0 + u * 32 + tq * 8;
-      const bool in = k < K;
+  for (int o = 1; o < 32; o *= 2) {
+    const int x = __shfl_up_sync(0xffffffffu, sp, o), y = __shfl_up_sync(0xffffffffu, su, o);
+    if (lane >= o) { sp += x; su += y; }
+  }
+  if (lane == 31) { part[0][warp] = sp; part[1][warp] = su; }
+  __syncthreads();
+  if (warp == 0) {
+    int x = part[0][lane], y = part[1][lane];
 #pragma unroll
-      for (int t = 0; t < NW; ++t) {
-        a[u][t][0] = in ? __ldg(reinterpret_cast<const uint4*>(w[2 * t] + k)) : zero;
-        a[u][t][1] = in ? __ldg(reinterpret_cast<const uint4*>(w[2 * t + 1] + k)) : zero;
-      }
-#pragma unroll
-      for (int c = 0; c < 2; ++c) b[u][c] = in && x[c] && (c == 0 || two) ? *reinterpret_cast<const uint4*>(x[c] + k) : zero;
+    for (int o = 1; o < 32; o *= 2) {
+      const int a = __shfl_up_sync(0xffffffffu, x, o), b = __shfl_up_sync(0xffffffffu, y, o);
+      if (lane >= o) { x += a; y += b; }
     }
-#pragma unroll
-    for (int u = 0; u < U; ++u)
-#pragma unroll
-      for (int c = 0; c < 2; ++c) {
-        if (c == 1 && !two) break;
-#pragma unroll
-        for (int t = 0; t < NW; ++t) {
-          mma_bf16(acc[t][c], a[u][t][0].x, a[u][t][1].x, a[u][t][0].y, a[u][t][1].y, b[u][c].x, b[u][c].y);
-          mma_bf16(acc[t][c], a[u][t][0].z, a[u][t][1].z, a[u][t][0].w, a[u][t][1].w, b[u][c].z, b[u][c].w);
+    part[0][lane] = x;
+    part[1][lane] = y;
+    if (lane == 31) *count = y;
+  }
+  __syncthreads();
+  sp += (warp ? part[0][warp - 1] : 0) - np;
+  su += (warp ? part[1][warp - 1] : 0) - nu;
+  for (int e = lo; e < hi; ++e) {
+    const int n = hist[e];
+    hist[e] = sp;
+    for (int f = 0; f < n; f += cap, ++su) {
+      unit[2 * su] = sp + f;
+      unit[2 * su + 1] = e << 8 | (min(cap, n - f) - 1);
+    }
+    sp += n;
+  }
+  __syncthreads();
+  for (int i = tid; i < P; i += 1024)
+    if ((unsigned)idx[i] < (unsigned)E) order[atomicAdd(hist + idx[i], 1)] = i;
+}
+
+// xs[place] = h[order[place] / k]; one warp per row, D % 8 == 0.  Places past the pairs that have an expert hold no pair.
+__global__ void __launch_bounds__(256) expert_rows_kernel(const bf16* __restrict__ h, const int* __restrict__ idx, const int* __restrict__ order,
+                                                          bf16* __restrict__ xs, int P, int E, int k, int D) {
+  grid_begin();
+  const int place = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+  if (place >= P) return;
+  const int pr = order[place];
+  if ((unsigned)pr >= (unsigned)P || (unsigned)idx[pr] >= (unsigned)E) return;
+  const uint4* src = reinterpret_cast<const uint4*>(h + (long long)(pr / k) * D);
+  uint4* dst = reinterpret_cast<uint4*>(xs + (long long)place * D);
+#pragma unroll 4
+  for (int i = lane; i < D / 8; i += 32) dst[i] = src[i];
+}
+
+// The used experts' weights stream past their pairs: 128 rows of W on the M side of the MMA, the NB (16 ... 128) pairs of a unit on
+// its N side.  Persistent, one CTA per SM with about 200 KB of tiles in flight across its tasks (unit x 128 rows), so that only the first
+// tile of a CTA waits for memory; accumulators alternate between two ranges of TMEM.  kUp: 64 features' gate rows and their up
+// rows are one tile; out = silu(s g) (s u) in the order of the pairs, s the weight of the pair (the products are linear in the
+// input, so its scale is applied to them).  Otherwise out[pair] = fp32 rows.
+// Bound by reading the weights (128 experts of 768, width 2048, 8 per token: 1.21 GB, 184 us).  In us, whole experts with plan and sum, a
+// CTA per 16 rows that looked for its pairs before and now, 64 tokens: 255, 209 (5.8 TB/s); against padded
+// tiles, 500 tokens: 300, 239; 1000: 311, 287; 2000: 370, 443.
+// Roles (192 threads): warp 0 TMA, warp 1 TMEM and MMA, warps 2 ... 5 empty the accumulators.  Every wait is bounded.
+struct ExpertArgs {
+  const int *unit, *count, *order;
+  const float* weight;
+  void* out;
+  int rows, K;      // rows of the output, length of the reduction
+  int* status;
+};
+
+template <int NB>
+struct ExpertSmem {
+  static constexpr int kABytes = 128 * 64 * 2, kStageBytes = kABytes + NB * 128;
+  static constexpr int kStages = 200 * 1024 / kStageBytes;
+  static constexpr int kPairOff = kStages * kStageBytes;      // up products on their way to the warps with the gates
+  static constexpr int kBarOff = kPairOff + 2 * 16 * 64 * 4;
+  static constexpr int kTotal = kBarOff + 512 + 1024;
+};
+
+template <int NB, bool kUp>
+__global__ void __launch_bounds__(192, 1) experts_few_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUtensorMap tmX,
+                                                             const ExpertArgs p) {
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
+  using L = ExpertSmem<NB>;
+  constexpr int kSt = L::kStages, kCols = 2 * NB < 32 ? 32 : 2 * NB, kPanel = kUp ? 64 : 128;
+  uint64_t* full = (uint64_t*)(smem + L::kBarOff);
+  uint64_t *empty = full + kSt, *tfull = empty + kSt, *tempty = tfull + 2;
+  uint32_t* tmem_slot = (uint32_t*)(tempty + 2);
+  volatile int* abort_flag = (volatile int*)(tmem_slot + 1);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  if (threadIdx.x == 0) {
+    tma_prefetch_desc(&tmW);
+    tma_prefetch_desc(&tmX);
+    for (int i = 0; i < kSt; ++i) {
+      mbar_init(&full[i], 1);
+      mbar_init(&empty[i], 1);
+    }
+    for (int i = 0; i < 2; ++i) {
+      mbar_init(&tfull[i], 1);
+      mbar_init(&tempty[i], 4);
+    }
+    *abort_flag = 0;
+    mbar_fence_init();
+  }
+  if (warp == 1) {
+    tmem_alloc(tmem_slot, kCols);
+    tmem_relinquish();
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem_base = *tmem_slot;
+  grid_begin();
+  const int units = *p.count, panels = (p.rows + kPanel - 1) / kPanel, tasks = units * panels;
+  const int kblocks = (p.K + 63) / 64;
+
+  if (warp == 0) {
+    if (lane == 0) {
+      int stage = 0;
+      uint32_t phase = 0;
+      bool ok = true;
+      for (int t = blockIdx.x; t < tasks && ok; t += gridDim.x) {
+        const int u = t % units, r0 = t / units * kPanel;      // panels of one expert's units side by side: read once
+        const int first = p.unit[2 * u], e = p.unit[2 * u + 1] >> 8;
+        const int w0 = (kUp ? 2 * e : e) * p.rows + r0;
+        for (int k = 0; k < kblocks; ++k) {
+          ok = mbar_wait(&empty[stage], phase ^ 1, abort_flag, p.status, OB_ERR_WAIT_EMPTY);
+          if (!ok) break;
+          uint8_t* sw = smem + stage * L::kStageBytes;
+          mbar_expect_tx(&full[stage], L::kStageBytes);
+          if (kUp) {
+            tma_load_2d(sw, &tmW, &full[stage], k * 64, w0);
+            tma_load_2d(sw + L::kABytes / 2, &tmW, &full[stage], k * 64, w0 + p.rows);
+          } else {
+            tma_load_2d(sw, &tmW, &full[stage], k * 64, w0);
+          }
+          tma_load_2d(sw + L::kABytes, &tmX, &full[stage], k * 64, first);
+          if (++stage == kSt) {
+            stage = 0;
+            phase ^= 1;
+          }
         }
       }
+    }
+  } else if (warp == 1) {
+    if (lane == 0) {
+      constexpr uint32_t idesc = make_idesc_bf16(128, NB, 0, 0);
+      int stage = 0, buf = 0;
+      uint32_t phase = 0, tphase = 0;
+      bool ok = true;
+      for (int t = blockIdx.x; t < tasks && ok; t += gridDim.x) {
+        ok = mbar_wait(&tempty[buf], tphase ^ 1, abort_flag, p.status, OB_ERR_WAIT_TMEM_EMPTY);
+        if (!ok) break;
+        tc_fence_after();
+        for (int k = 0; k < kblocks; ++k) {
+          ok = mbar_wait(&full[stage], phase, abort_flag, p.status, OB_ERR_WAIT_FULL);
+          if (!ok) break;
+          tc_fence_after();
+          const uint32_t sw = smem_u32(smem + stage * L::kStageBytes), sx = sw + L::kABytes;
+#pragma unroll
+          for (int j = 0; j < 4; ++j)
+            umma_ss(tmem_base + buf * NB, make_smem_desc(sw + j * 32, 16, 1024), make_smem_desc(sx + j * 32, 16, 1024), idesc,
+                    (k | j) ? 1u : 0u);
+          umma_commit(&empty[stage]);
+          if (++stage == kSt) {
+            stage = 0;
+            phase ^= 1;
+          }
+        }
+        if (!ok) break;
+        umma_commit(&tfull[buf]);
+        if (buf) tphase ^= 1;
+        buf ^= 1;
+      }
+    }
+  } else {
+    const int quad = warp & 3, row = quad * 32 + lane;      // TMEM lane = row of the tile
+    float* pair = (float*)(smem + L::kPairOff);             // [2][16 pairs][64 features]
+    int buf = 0, pb = 0;
+    uint32_t tphase = 0;
+    bool ok = true;
+    for (int t = blockIdx.x; t < tasks && ok; t += gridDim.x) {
+      const int u = t % units, r = t / units * kPanel + (kUp ? row & 63 : row);
+      const int first = p.unit[2 * u], n = (p.unit[2 * u + 1] & 255) + 1;
+      ok = mbar_wait(&tfull[buf], tphase, abort_flag, p.status, OB_ERR_WAIT_TMEM_FULL);
+      if (kUp) ok = named_bar_and(1, 128, ok);      // the exchange below takes all four warps
+      if (!ok) break;
+      tc_fence_after();
+      const uint32_t taddr = tmem_base + buf * NB + ((uint32_t)(quad * 32) << 16);
+#pragma unroll 1
+      for (int c = 0; c < n; c += 16) {
+        uint32_t v[16];
+        tmem_ld16(taddr + c, v);
+        const int my = c + (lane & 15) < n ? p.order[first + c + (lane & 15)] : 0;      // a lane knows one pair
+        const float mw = kUp ? p.weight[my] : 0.f;
+        tmem_ld_wait();
+        if (kUp) {
+          float* x = pair + pb * 16 * 64;
+          pb ^= 1;
+          if (quad >= 2) {
+#pragma unroll
+            for (int i = 0; i < 16; ++i) x[i * 64 + (row & 63)] = __uint_as_float(v[i]);
+          }
+          named_bar_and(1, 128, true);      // a buffer is written again two rounds later, past the next barrier
+          if (quad < 2) {
+#pragma unroll
+            for (int i = 0; i < 16; ++i) {
+              const float s = __shfl_sync(0xffffffffu, mw, i);
+              if (c + i < n && r < p.rows)
+                ((bf16*)p.out)[(long long)(first + c + i) * p.rows + r] =
+                    __float2bfloat16(silu_f(__uint_as_float(v[i]) * s) * (x[i * 64 + row] * s));
+            }
+          }
+        } else {
+#pragma unroll
+          for (int i = 0; i < 16; ++i) {
+            const int pr = __shfl_sync(0xffffffffu, my, i);
+            if (c + i < n && r < p.rows) ((float*)p.out)[(long long)pr * p.rows + r] = __uint_as_float(v[i]);
+          }
+        }
+      }
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&tempty[buf]);
+      if (buf) tphase ^= 1;
+      buf ^= 1;
+    }
+  }
+  tc_fence_before();
+  __syncthreads();
+  if (*abort_flag) {   // copies that may still be in flight land before shared memory is released
+    const long long t0 = clock64();
+    while (clock64() - t0 < 2000000) __nanosleep(1000);
+    __syncthreads();
+  }
+  if (warp == 1) {
+    tc_fence_after();
+    tmem_dealloc(tmem_base, kCols);
   }
 }
 
-// act[p, f] = silu(s W_gate h) * (s W_up h), s = weight of pair p, for the pairs of expert blockIdx.y and the
-// features f of block blockIdx.x; W [E][gate F rows | up F rows][K].  The products are linear in the input,
-// so its scale is applied to them.
-__global__ void __launch_bounds__(128) expert_up_few_kernel(const bf16* __restrict__ h, const bf16* __restrict__ W,
-                                                            const int* __restrict__ idx, const float* __restrict__ weight,
-                                                            bf16* __restrict__ act, int P, int k, int F, int K) {
-  grid_begin();
-  __shared__ int list[kFewPairs], count;
-  __shared__ __align__(16) float red[4][2][2][128];
-  const int e = blockIdx.y, f0 = blockIdx.x * 16;
-  const int n = find_pairs(idx, P, e, list, &count);
-  if (n == 0) return;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, tq = lane & 3;
-  const bf16* we = W + (long long)e * 2 * F * K;
-  const int r0 = min(f0 + g, F - 1), r1 = min(f0 + g + 8, F - 1);
-  const bf16* w[4] = {we + (long long)r0 * K, we + (long long)r1 * K, we + (long long)(F + r0) * K, we + (long long)(F + r1) * K};
-  for (int p0 = 0; p0 < n; p0 += 16) {
-    const bf16* x[2];
-#pragma unroll
-    for (int c = 0; c < 2; ++c) x[c] = p0 + c * 8 + g < n ? h + (long long)(list[p0 + c * 8 + g] / k) * K : nullptr;
-    float acc[2][2][4] = {};
-    few_rows<2>(w, x, n - p0 > 8, K, warp, tq, acc);
-    __syncthreads();           // the sums of the round before are read
-#pragma unroll
-    for (int t = 0; t < 2; ++t)
-#pragma unroll
-      for (int c = 0; c < 2; ++c) store4(&red[warp][t][c][lane * 4], make_float4(acc[t][c][0], acc[t][c][1], acc[t][c][2], acc[t][c][3]));
-    __syncthreads();
-    // element i of a 16 x 8 block: lane i / 4's value i % 4 = (row g + 8 (v >> 1), column 2 tq + (v & 1))
-#pragma unroll
-    for (int c = 0; c < 2; ++c) {
-      const int i = threadIdx.x, ln = i >> 2, v = i & 3;
-      const int f = f0 + (ln >> 2) + 8 * (v >> 1), q = p0 + c * 8 + (ln & 3) * 2 + (v & 1);
-      if (f >= F || q >= n) continue;
-      const int pr = list[q];
-      const float s = weight[pr];
-      const float gt = ((red[0][0][c][i] + red[1][0][c][i]) + (red[2][0][c][i] + red[3][0][c][i])) * s;
-      const float up = ((red[0][1][c][i] + red[1][1][c][i]) + (red[2][1][c][i] + red[3][1][c][i])) * s;
-      act[(long long)pr * F + f] = __float2bfloat16(silu_f(gt) * up);
-    }
-  }
-}
-
-// y[p, d] = W_down[d, :] act[p, :] for the pairs of expert blockIdx.y; W [E][D][F]
-__global__ void __launch_bounds__(128) expert_down_few_kernel(const bf16* __restrict__ act, const bf16* __restrict__ W,
-                                                              const int* __restrict__ idx, float* __restrict__ y, int P, int D,
-                                                              int F) {
-  grid_begin();
-  __shared__ int list[kFewPairs], count;
-  __shared__ __align__(16) float red[4][2][128];
-  const int e = blockIdx.y, d0 = blockIdx.x * 16;
-  const int n = find_pairs(idx, P, e, list, &count);
-  if (n == 0) return;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, tq = lane & 3;
-  const bf16* we = W + (long long)e * D * F;
-  const bf16* w[2] = {we + (long long)min(d0 + g, D - 1) * F, we + (long long)min(d0 + g + 8, D - 1) * F};
-  for (int p0 = 0; p0 < n; p0 += 16) {
-    const bf16* x[2];
-#pragma unroll
-    for (int c = 0; c < 2; ++c) x[c] = p0 + c * 8 + g < n ? act + (long long)list[p0 + c * 8 + g] * F : nullptr;
-    float acc[1][2][4] = {};
-    few_rows<1>(w, x, n - p0 > 8, F, warp, tq, acc);
-    __syncthreads();
-#pragma unroll
-    for (int c = 0; c < 2; ++c) store4(&red[warp][c][lane * 4], make_float4(acc[0][c][0], acc[0][c][1], acc[0][c][2], acc[0][c][3]));
-    __syncthreads();
-#pragma unroll
-    for (int c = 0; c < 2; ++c) {
-      const int i = threadIdx.x, ln = i >> 2, v = i & 3;
-      const int d = d0 + (ln >> 2) + 8 * (v >> 1), q = p0 + c * 8 + (ln & 3) * 2 + (v & 1);
-      if (d >= D || q >= n) continue;
-      y[(long long)list[q] * D + d] = (red[0][c][i] + red[1][c][i]) + (red[2][c][i] + red[3][c][i]);
-    }
-  }
+template <int NB, bool kUp>
+static int launch_experts(const void* X, const void* W, const ExpertArgs& a, int P, int E, cudaStream_t s) {
+  CUtensorMap tmW, tmX;
+  int e = make_tmap_2d(&tmX, X, P, a.K, a.K, NB, 64);
+  if (e) return 2000 + e;
+  e = make_tmap_2d(&tmW, W, (uint64_t)E * (kUp ? 2 : 1) * a.rows, a.K, a.K, kUp ? 64 : 128, 64);
+  if (e) return 3000 + e;
+  auto kern = experts_few_kernel<NB, kUp>;
+  OB_ENSURE_DYN_SMEM(kern, ExpertSmem<NB>::kTotal);
+  const long long most = (long long)P * ((a.rows + (kUp ? 63 : 127)) / (kUp ? 64 : 128));      // no more tasks than that
+  const unsigned grid = (unsigned)(most < num_sms() ? most : num_sms());
+  (void)launch(kern, dim3(grid), dim3(192), ExpertSmem<NB>::kTotal, s, 0, tmW, tmX, a);
+  OB_CHECK_LAUNCH();
+  return 0;
 }
 
 }  // namespace ob
@@ -288,19 +436,34 @@ int ob_expert_rows_any(const void* A, const void* W, void* C, const int* offsets
   return 0;
 }
 
-// Experts of P = M * k pairs, P <= 2048, bf16: h [M, D], idx / weight [P], gate_up [E, 2F, D], down [E, D, F];
-// scratch act bf16 [P, F]; y fp32 [P, D].  D, F multiples of 8.
-int ob_experts_few(const void* h, const int* idx, const float* weight, const void* gate_up, const void* down, void* act,
-                   float* y, int P, int k, int E, int D, int F, cudaStream_t s) {
+// Experts of P = M * k pairs, bf16, for few pairs per expert: h [M, D], idx / weight [P], gate_up [E, 2F, D], down [E, D, F];
+// scratch xs [P, D], act [P, F] bf16, plan int32 [1 + 3 * P], and E more with over 8192 experts; y fp32 [P, D].  D, F multiples of 8.
+// cap: pairs of a unit (16, 32, 64 or 128).
+int ob_experts_few(const void* h, const int* idx, const float* weight, const void* gate_up, const void* down, void* xs, void* act,
+                   int* plan, float* y, int P, int k, int E, int D, int F, int cap, int* status, cudaStream_t s) {
   if (P <= 0) return 0;
-  if (P > kFewPairs || k <= 0 || E <= 0 || E > 65535) return 6005;
+  if (k <= 0 || E <= 0 || E > 65535 || D <= 0 || F <= 0 || (long long)E * 2 * (D > F ? D : F) > 0x7fffffff) return 6005;
   if ((D & 7) || (F & 7)) return 6001;
-  if ((((uintptr_t)h) | ((uintptr_t)gate_up) | ((uintptr_t)down) | ((uintptr_t)act)) & 15) return 6002;
-  OB_LAUNCH(expert_up_few_kernel, (dim3((F + 15) / 16, E)), 128, 0, s, (const bf16*)h, (const bf16*)gate_up, idx, weight, (bf16*)act, P, k, F, D);
+  if ((((uintptr_t)h) | ((uintptr_t)gate_up) | ((uintptr_t)down) | ((uintptr_t)act) | ((uintptr_t)xs)) & 15) return 6002;
+  int *count = plan, *order = plan + 1, *unit = order + P;
+  const bool wide = E > kPlanExperts;
+  OB_LAUNCH(expert_units_kernel, 1, 1024, wide ? 0 : E * 4, s, idx, P, E, cap, order, unit, count, wide ? unit + 2 * (size_t)P : (int*)nullptr);
   OB_CHECK_LAUNCH();
-  OB_LAUNCH(expert_down_few_kernel, (dim3((D + 15) / 16, E)), 128, 0, s, (const bf16*)act, (const bf16*)down, idx, y, P, D, F);
+  OB_LAUNCH(expert_rows_kernel, (unsigned)((P + 7) / 8), 256, 0, s, (const bf16*)h, idx, (const int*)order, (bf16*)xs, P, E, k, D);
   OB_CHECK_LAUNCH();
-  return 0;
+  const ExpertArgs up = {unit, count, order, weight, act, F, D, status}, dn = {unit, count, order, weight, y, D, F, status};
+#define OB_EXPERTS(NB)                                              \
+  do {                                                              \
+    const int e = launch_experts<NB, true>(xs, gate_up, up, P, E, s); \
+    if (e) return e;                                                \
+    return launch_experts<NB, false>(act, down, dn, P, E, s);       \
+  } while (0)
+  if (cap == 16) OB_EXPERTS(16);
+  if (cap == 32) OB_EXPERTS(32);
+  if (cap == 64) OB_EXPERTS(64);
+  if (cap == 128) OB_EXPERTS(128);
+#undef OB_EXPERTS
+  return 6005;
 }
 
 }  // extern "C"

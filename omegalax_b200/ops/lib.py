@@ -68,7 +68,7 @@ _SIGS = {
     "ob_moe_gather": [P, P, P, P, L, I, I, I, I, P],
     "ob_moe_sum": [P, P, P, I, I, I, I, I, P],
     "ob_expert_rows_any": [P, P, P, P, I, I, I, I, I, P],
-    "ob_experts_few": [P, P, P, P, P, P, P, I, I, I, I, I, P],
+    "ob_experts_few": [P, P, P, P, P, P, P, P, P, I, I, I, I, I, I, P, P],
     "ob_decode_append": [P, P, P, P, P, P, P, I, I, P, P, P, L, I, I, I, I, F, F, I, P],
     "ob_kv_store": [P, P, L, L, P, P, P, L, I, P],
     "ob_decode_attn": [P, P, P, P, P, I, I, I, I, I, I, I, F, P, P, P, P],

@@ -254,6 +254,27 @@ def test_experts_on_every_path(dtype, M_, E, k, D, F):
         close(into - cu(base), want - base.double(), dtype, k=2)
 
 
+@pytest.mark.parametrize("cap,E,D,F", [(16, 6, 136, 72), (32, 6, 136, 72), (64, 6, 136, 72), (128, 6, 136, 72), (16, 9000, 16, 8)])
+def test_experts_of_few_pairs(monkeypatch, cap, E, D, F):
+    """Units of one expert cut at every size, experts with one pair and none, rows and columns that no tile divides."""
+    monkeypatch.setattr(S, "experts_few_cap", lambda *a: cap)
+    M_, k = 150, 2
+    h, gu, down = rnd(1, M_, D, dtype=bf16), rnd(2, E, 2 * F, D, dtype=bf16) * D ** -0.5, rnd(3, E, D, F, dtype=bf16) * F ** -0.5
+    idx = torch.stack([torch.zeros(M_, dtype=i32), torch.arange(M_, dtype=i32) // 16 % 3 + 1], -1)      # 150, 54, 48, 48, 0, 0 pairs
+    idx[7, 1] = E - 1
+    w = torch.rand(M_, k, generator=gen(5)) * 0.9 + 0.1
+    base = torch.randn(M_, D, generator=gen(6))
+    want = base.double().clone()
+    for m in range(M_):
+        for e, a in zip(idx[m].tolist(), w[m].double()):
+            x = a * h[m].double()
+            want[m] += (O.silu(gu[e, :F].double() @ x) * (gu[e, F:].double() @ x)) @ down[e].double().t()
+    into = cu(base.clone())
+    S.experts_into(cu(h), cu(w), cu(idx), cu(gu), cu(down), "silu", into, few=True)
+    done()
+    close(into - cu(base), want - base.double(), bf16, k=2)
+
+
 # ------------------------------------------------------------------------------------------ whole models
 MODELS = {"even": M.EVEN, "odd": M.ODD}
 ALL = pytest.mark.parametrize("name", list(MODELS))
