@@ -521,17 +521,23 @@ def embedding_bwd_peer(ids, dy, peer_ptrs, rows_per_rank: int):
           int(rows_per_rank), ids32.numel(), d2.shape[1], lib.stream_ptr())
 
 
-def sumsq(g, out):
-    _call("ob_sumsq", g.data_ptr(), g.numel(), out.data_ptr(), lib.stream_ptr())
+def sumsq(g, out, used=None):
+    """out += sum of squares of g; ``used`` (uint8, ``used_blocks``) says of every 128 elements whether one is not zero."""
+    _call("ob_sumsq", g.data_ptr(), g.numel(), out.data_ptr(), lib.ptr(used), lib.stream_ptr())
+
+
+def used_blocks(g):
+    return torch.empty(-(-g.numel() // 1024) * 8, dtype=torch.uint8, device=g.device)
 
 
 def adamw(p, m, v, g, p16, *, lr, b1, b2, eps, wd, step, grad_mul=1.0, norm_sq=None,
-          max_norm=0.0, zero_grad=True):
+          max_norm=0.0, zero_grad=True, used=None):
+    """``used``: what ``sumsq`` found in g as it is now."""
     bc1 = 1.0 - b1 ** step
     bc2 = 1.0 - b2 ** step
     _call("ob_adamw", p.data_ptr(), m.data_ptr(), v.data_ptr(), g.data_ptr(), lib.ptr(p16),
           p.numel(), float(lr), float(b1), float(b2), float(eps), float(wd), float(bc1),
-          float(bc2), float(grad_mul), lib.ptr(norm_sq), float(max_norm), int(zero_grad),
+          float(bc2), float(grad_mul), lib.ptr(norm_sq), float(max_norm), int(zero_grad), lib.ptr(used),
           lib.stream_ptr())
 
 

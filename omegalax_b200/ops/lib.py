@@ -114,8 +114,8 @@ _SIGS = {
     "ob_embedding_fwd": [P, P, P, L, I, P],
     "ob_embedding_bwd": [P, P, P, L, I, I, I, P],
     "ob_embedding_bwd_peer": [P, P, P, I, I, L, I, P],
-    "ob_sumsq": [P, L, P, P],
-    "ob_adamw": [P, P, P, P, P, L, F, F, F, F, F, c_double, c_double, F, P, F, I, P],
+    "ob_sumsq": [P, L, P, P, P],
+    "ob_adamw": [P, P, P, P, P, L, F, F, F, F, F, c_double, c_double, F, P, F, I, P, P],
     "ob_cast_f32_bf16": [P, P, L, P],
     "ob_transpose_bf16": [P, P, I, I, L, L, P],
     "ob_l2_flush": [P, L, P],

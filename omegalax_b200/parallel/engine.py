@@ -261,6 +261,7 @@ class TrainEngine:
         else:
             self.compute_shard = self._alloc_compute_shard(n)
         self.norm_sq = torch.zeros(1, dtype=torch.float32, device=dev)
+        self._grad_used = None      # which blocks of the gradient are not zero, as the norm found them
         if self.W > 1:
             layer_like = [u for u in self.units if u.name.startswith("layers.")]
             self._ring_numel = max((u.full_numel for u in layer_like), default=0)
@@ -586,7 +587,9 @@ class TrainEngine:
                 dist.all_reduce(self.norm_sq, group=self.group)
             return self.norm_sq
         if self.use_cuda_kernels:
-            K.sumsq(self.grad, self.norm_sq)
+            if self._grad_used is None:
+                self._grad_used = K.used_blocks(self.grad)
+            K.sumsq(self.grad, self.norm_sq, self._grad_used)
         else:
             acc = torch.zeros((), dtype=torch.float64, device=self.device)
             for off in range(0, self.grad.numel(), _TORCH_CHUNK):   # bounded temporaries on large shards
@@ -620,7 +623,7 @@ class TrainEngine:
             p16 = None if self.compute_shard is self.master else self.compute_shard
             K.adamw(self.master, self.exp_avg, self.exp_avg_sq, self.grad, p16, lr=lr, b1=b1, b2=b2,
                     eps=self.eps, wd=self.wd, step=self.step_count, grad_mul=gmul, norm_sq=nsq,
-                    max_norm=self.max_grad_norm, zero_grad=True)
+                    max_norm=self.max_grad_norm, zero_grad=True, used=self._grad_used if self.TP == 1 else None)
         else:
             mul = torch.full((), gmul, dtype=torch.float32, device=self.device)
             if self.max_grad_norm > 0:

@@ -777,6 +777,27 @@ def test_decode_attention_lengths(R, splits):
         torch.testing.assert_close(out[b].float(), torch.einsum("hs,shd->hd", p, vb), rtol=2.0 ** -8, atol=2.0 ** -10)
 
 
+@pytest.mark.parametrize("n", [1, 511, 513, 4099, 1 << 20])
+def test_adamw_passes_over_zero_gradients(n):
+    """Blocks of 128 gradients that are all zero are neither read nor cleared: the same update to the bit, and gradients end as zeros."""
+    from omegalax_b200.ops import kernels as Kn, lib
+    torch.manual_seed(42)
+    g = torch.randn(n, device=_dev()) * (torch.rand(-(-n // 128), device=_dev()) < 0.3).repeat_interleave(128)[:n]
+    g[-1] = 1.0
+    p, m, v = (torch.randn(n, device=_dev()) for _ in range(3))
+    nsq, used = torch.zeros(1, device=_dev()), Kn.used_blocks(g)
+    Kn.sumsq(g, nsq, used)
+    torch.testing.assert_close(nsq.double(), g.double().square().sum().view(1), rtol=1e-5, atol=0)
+    outs = []
+    for u in (None, used):
+        t = [x.clone() for x in (p, m, v.abs(), g)] + [torch.zeros(n, dtype=bf16, device=_dev())]
+        Kn.adamw(*t, lr=1e-2, b1=0.9, b2=0.999, eps=1e-8, wd=0.01, step=3, norm_sq=nsq, max_norm=1.0, used=u)
+        assert not t[3].any()
+        outs.append(t)
+    _check(lib)
+    assert all(torch.equal(a, b) for a, b in zip(*outs))
+
+
 @pytest.mark.parametrize("R,window", [(8, 0), (8, 100), (3, 16), (1, 1)])
 @pytest.mark.parametrize("splits", [1, 5, 70])
 def test_decode_attention_window_and_sink(R, window, splits):
