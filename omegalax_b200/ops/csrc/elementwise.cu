@@ -188,9 +188,11 @@ rmsnorm_bwd_kernel(const bf16* __restrict__ dy, const bf16* __restrict__ x, cons
 
 // ------------------------------------------------------------------ SwiGLU (K5)
 // gu is [M, 2F] = [gate | up];  act = silu(gate) * up.
-__global__ void swiglu_fwd_kernel(const bf16* __restrict__ gu, bf16* __restrict__ act, long long M,
+// rows (may be null): a device count of the rows that matter, the first ones.
+__global__ void swiglu_fwd_kernel(const bf16* __restrict__ gu, bf16* __restrict__ act, const int* __restrict__ rows, long long M,
                                   int F) {
   grid_begin();
+  if (rows) M = min(M, (long long)*rows);
   const int fv = F >> 3;
   const long long total = M * fv;
   for (long long idx = blockIdx.x * (long long)blockDim.x + threadIdx.x; idx < total;
@@ -216,7 +218,8 @@ __global__ void swiglu_fwd_kernel(const bf16* __restrict__ gu, bf16* __restrict_
 // dgu may be gu itself (no __restrict__ on the two): every thread reads its eight gate and up
 // values before it writes the gradients to the same places, and no other thread touches them.
 __global__ void swiglu_bwd_kernel(const bf16* gu, const bf16* __restrict__ dact, bf16* dgu,
-                                  bf16* __restrict__ act_out, long long M, int F) {
+                                  bf16* __restrict__ act_out, const int* __restrict__ rows, long long M, int F) {
+  if (rows) M = min(M, (long long)*rows);
   const int fv = F >> 3;
   const long long total = M * fv;
   for (long long idx = blockIdx.x * (long long)blockDim.x + threadIdx.x; idx < total;
@@ -1084,20 +1087,20 @@ int ob_rmsnorm_bwd(const void* dy, const void* x, const void* w, const float* rs
   return 0;
 }
 
-int ob_swiglu_fwd(const void* gu, void* act, long long M, int F, cudaStream_t s) {
+int ob_swiglu_fwd(const void* gu, void* act, const int* rows, long long M, int F, cudaStream_t s) {
   if (F % 8) return 6001;
   if (M <= 0) return 0;
-  OB_LAUNCH(swiglu_fwd_kernel, grid_for(M * (F / 8), 256), 256, 0, s, (const bf16*)gu, (bf16*)act, M, F);
+  OB_LAUNCH(swiglu_fwd_kernel, grid_for(M * (F / 8), 256), 256, 0, s, (const bf16*)gu, (bf16*)act, rows, M, F);
   OB_CHECK_LAUNCH();
   return 0;
 }
 
-int ob_swiglu_bwd(const void* gu, const void* dact, void* dgu, void* act_out, long long M, int F,
+int ob_swiglu_bwd(const void* gu, const void* dact, void* dgu, void* act_out, const int* rows, long long M, int F,
                   cudaStream_t s) {
   if (F % 8) return 6001;
   if (M <= 0) return 0;
   swiglu_bwd_kernel<<<grid_for(M * (F / 8), 256), 256, 0, s>>>(
-      (const bf16*)gu, (const bf16*)dact, (bf16*)dgu, (bf16*)act_out, M, F);
+      (const bf16*)gu, (const bf16*)dact, (bf16*)dgu, (bf16*)act_out, rows, M, F);
   OB_CHECK_LAUNCH();
   return 0;
 }

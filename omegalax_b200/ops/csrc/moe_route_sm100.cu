@@ -177,6 +177,16 @@ __global__ void moe_dest_kernel(const int* __restrict__ idx, const int* __restri
   dest[p] = (e >= 0 && e < E) ? offsets[e] + atomicAdd(cursor + e, 1) : -1;   // -1: dropped by the row movers
 }
 
+// The rows of [R, D] that fill a segment up to the next one: zeros.  CTA (expert, every gridDim.y-th row).
+__global__ void __launch_bounds__(256) moe_fill_kernel(const int* __restrict__ counts, const int* __restrict__ offsets,
+                                                       bf16* __restrict__ rows, int D) {
+  const int e = blockIdx.x, end = offsets[e + 1];
+  for (int r = offsets[e] + counts[e] + blockIdx.y; r < end; r += gridDim.y) {
+    uint4* d = reinterpret_cast<uint4*>(rows + (long long)r * D);
+    for (int i = threadIdx.x; i < D / 8; i += 256) d[i] = make_uint4(0, 0, 0, 0);
+  }
+}
+
 // Expert-parallel plan.  allc [W][E] holds every rank's pick counts.  For expert e owned by rank
 // e / El: start[e] = (first row of e inside its owner's receive buffer) + (rows that lower ranks
 // send to e); offsets_local [El+1] are the padded segment boundaries of this rank's own experts;
@@ -284,6 +294,15 @@ int ob_moe_plan(const int* idx, int* counts, int* offsets, int* cursor, int* des
     moe_dest_kernel<<<(unsigned)((P + 255) / 256), 256, 0, s>>>(idx, offsets, cursor, dest, P, E);
     OB_CHECK_LAUNCH();
   }
+  return 0;
+}
+
+// rows bf16 [offsets[E], D]: the rows between the counts[e] of expert e and the end of its segment become zeros
+int ob_moe_fill(const int* counts, const int* offsets, void* rows, int E, int D, cudaStream_t s) {
+  if (E <= 0) return 0;
+  if ((D & 7) || (((uintptr_t)rows) & 15)) return 6001;
+  moe_fill_kernel<<<dim3(E, 32), 256, 0, s>>>(counts, offsets, (bf16*)rows, D);
+  OB_CHECK_LAUNCH();
   return 0;
 }
 

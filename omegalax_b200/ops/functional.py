@@ -370,20 +370,21 @@ def gather4(table, idx_N4, w_N4):
 # ----------------------------------------------------------------------------- swiglu
 class _SwiGLUFn(torch.autograd.Function):
     @staticmethod
-    def forward(ctx, gu):
-        ctx.save_for_backward(gu)
-        return K.swiglu_fwd(gu)
+    def forward(ctx, gu, rows):
+        ctx.save_for_backward(gu, rows)
+        return K.swiglu_fwd(gu, rows)
 
     @staticmethod
     def backward(ctx, dact):
-        (gu,) = ctx.saved_tensors
-        return K.swiglu_bwd(gu, dact)
+        gu, rows = ctx.saved_tensors
+        return K.swiglu_bwd(gu, dact, rows=rows), None
 
 
-def swiglu(gu):
-    """gu = [gate | up] on the last dim -> silu(gate) * up."""
+def swiglu(gu, rows=None):
+    """gu = [gate | up] on the last dim -> silu(gate) * up.  ``rows`` (an int32 count on the device): kernels leave the rows
+    from there on unwritten."""
     if use_kernels(gu) and gu.shape[-1] % 16 == 0:
-        return _SwiGLUFn.apply(gu.contiguous())
+        return _SwiGLUFn.apply(gu.contiguous(), rows)
     return R.swiglu(gu)
 
 

@@ -280,16 +280,17 @@ def rmsnorm_bwd(dy, x, w, rstd, eps, dw_out, one_plus=False):
     return dx.view(x.shape)
 
 
-def swiglu_fwd(gu):
+def swiglu_fwd(gu, rows=None):
+    """silu(gate) * up; ``rows`` (int32, on the device): only so many rows matter, the others stay unwritten."""
     g2 = gu.reshape(-1, gu.shape[-1])
     F = g2.shape[1] // 2
     act = torch.empty(g2.shape[0], F, dtype=gu.dtype, device=gu.device)
-    _call("ob_swiglu_fwd", g2.data_ptr(), act.data_ptr(), g2.shape[0], F, lib.stream_ptr())
+    _call("ob_swiglu_fwd", g2.data_ptr(), act.data_ptr(), lib.ptr(rows), g2.shape[0], F, lib.stream_ptr())
     return act.view(*gu.shape[:-1], F)
 
 
-def swiglu_bwd(gu, dact, with_act: bool = False, inplace: bool = False):
-    """Gradient of silu(gate) * up; ``with_act`` also returns the activation itself, recomputed in
+def swiglu_bwd(gu, dact, with_act: bool = False, inplace: bool = False, rows=None):
+    """Gradient of silu(gate) * up (``rows`` as in ``swiglu_fwd``); ``with_act`` also returns the activation itself, recomputed in
     the same pass (for a caller that did not keep it); ``inplace`` writes the gradient over
     ``gu`` (contiguous), for a caller that is the last reader of it."""
     g2 = gu.reshape(-1, gu.shape[-1])
@@ -301,7 +302,7 @@ def swiglu_bwd(gu, dact, with_act: bool = False, inplace: bool = False):
         raise ValueError("swiglu_bwd(inplace=True) needs a contiguous [gate | up] tensor")
     dgu = g2 if inplace else torch.empty_like(g2)
     act = torch.empty(g2.shape[0], F, dtype=gu.dtype, device=gu.device) if with_act else None
-    _call("ob_swiglu_bwd", g2.data_ptr(), d2.data_ptr(), dgu.data_ptr(), lib.ptr(act), g2.shape[0], F,
+    _call("ob_swiglu_bwd", g2.data_ptr(), d2.data_ptr(), dgu.data_ptr(), lib.ptr(act), lib.ptr(rows), g2.shape[0], F,
           lib.stream_ptr())
     return (dgu.view(gu.shape), act) if with_act else dgu.view(gu.shape)
 
@@ -697,9 +698,9 @@ def router_topk_bwd(probs, w, idx, dw, dprobs, renorm):
     return dlogits
 
 
-def moe_plan(idx32, E, pad=128, counts=None):
-    """idx [M,k] int32 -> offsets [E+1] int32 (segments padded to ``pad``), dest [M*k] int32.
-    ``counts`` [E] int32 may carry the histogram already (from the router)."""
+def moe_plan(idx32, E, pad=128, counts=None, with_counts: bool = False):
+    """idx [M,k] int32 -> offsets [E+1] int32 (segments padded to ``pad``), dest [M*k] int32, and ``with_counts`` the
+    histogram [E].  ``counts`` [E] int32 may carry it already (from the router)."""
     have = counts is not None
     if not have:
         counts = torch.empty(E, dtype=torch.int32, device=idx32.device)
@@ -709,7 +710,13 @@ def moe_plan(idx32, E, pad=128, counts=None):
     dest = torch.empty(Pn, dtype=torch.int32, device=idx32.device)
     _call("ob_moe_plan", idx32.data_ptr(), counts.data_ptr(), offsets.data_ptr(), cursor.data_ptr(), dest.data_ptr(), Pn,
           E, pad, int(not have), lib.stream_ptr())
-    return offsets, dest
+    return (offsets, dest, counts) if with_counts else (offsets, dest)
+
+
+def moe_fill_(rows, counts, offsets):
+    """Zeros in the rows of [R, D] between an expert's ``counts`` and the end of its segment."""
+    _call("ob_moe_fill", counts.data_ptr(), offsets.data_ptr(), rows.data_ptr(), counts.numel(), rows.shape[1], lib.stream_ptr())
+    return rows
 
 
 def gather_rows(src, idx32):

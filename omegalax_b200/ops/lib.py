@@ -99,6 +99,7 @@ _SIGS = {
     "ob_ce_vp_grad": [P, L, I, L, I, P, P, P, P, P],
     "ob_moe_count": [P, P, L, I, P],
     "ob_ep_plan": [P, P, P, P, P, P, P, L, I, I, I, I, I, P],
+    "ob_moe_fill": [P, P, P, I, I, P],
     "ob_moe_plan": [P, P, P, P, P, L, I, I, I, P],
     "ob_gdn_fwd": [P] * 10 + [I] * 6 + [P],
     "ob_gdn_bwd": [P] * 15 + [I] * 6 + [P],
@@ -106,8 +107,8 @@ _SIGS = {
     "ob_conv1d_silu_bwd": [P, P, P, P, P, I, I, I, I, P],
     "ob_rmsnorm_fwd": [P, P, P, P, L, I, F, I, P],
     "ob_rmsnorm_bwd": [P, P, P, P, P, P, L, I, F, I, P],
-    "ob_swiglu_fwd": [P, P, L, I, P],
-    "ob_swiglu_bwd": [P, P, P, P, L, I, P],
+    "ob_swiglu_fwd": [P, P, P, L, I, P],
+    "ob_swiglu_bwd": [P, P, P, P, P, L, I, P],
     "ob_qknorm_rope_fwd": [P, P, P, P, P, P, P, L, I, I, I, I, F, I, I, P],
     "ob_qknorm_rope_bwd": [P, P, P, P, P, P, P, P, P, P, L, I, I, I, I, F, I, I, P],
     "ob_ce_fwd_bwd": [P, L, L, I, P, P, P, P, P, I, P],

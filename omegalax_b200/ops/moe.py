@@ -160,7 +160,7 @@ def expert_mlp_permuted(xp, w_gate_up, w_down, offsets, out=None):
     """SwiGLU expert MLP on rows already grouped by expert (padded layout).  ``out`` may name
     the buffer that receives the result (e.g. the exchange buffer the combine step reads)."""
     gu = grouped_linear(xp, w_gate_up, offsets)
-    act = Fn.swiglu(gu)
+    act = Fn.swiglu(gu, offsets[-1:])
     return grouped_linear(act, w_down, offsets, out)
 
 
@@ -192,8 +192,9 @@ def _pull_rows(buf, rank0, src_row, M, k, weights=None, want_out=True, grad=None
 
 class _LocalDispatch(torch.autograd.Function):
     @staticmethod
-    def forward(ctx, x, dest, src_tok, rank0, cap, k):
-        xp = torch.zeros(cap, x.shape[1], dtype=x.dtype, device=x.device)   # padding rows stay zero
+    def forward(ctx, x, dest, src_tok, rank0, cap, k, counts, offsets):
+        # rows that fill a segment are zero; those after the last segment are never read
+        xp = K.moe_fill_(torch.empty(cap, x.shape[1], dtype=x.dtype, device=x.device), counts, offsets)
         _push_rows(xp, x, src_tok, rank0, dest, None)
         ctx.save_for_backward(dest, rank0)
         ctx.M, ctx.k = x.shape[0], k
@@ -203,26 +204,26 @@ class _LocalDispatch(torch.autograd.Function):
     def backward(ctx, d_xp):
         dest, rank0 = ctx.saved_tensors
         dx, _ = _pull_rows(d_xp.contiguous(), rank0, dest, ctx.M, ctx.k)
-        return dx, None, None, None, None, None
+        return dx, None, None, None, None, None, None, None
 
 
 class _LocalCombine(torch.autograd.Function):
     @staticmethod
-    def forward(ctx, yp, weights, dest, src_tok, rank0):
+    def forward(ctx, yp, weights, dest, src_tok, rank0, counts, offsets):
         M, k = weights.shape
         y, _ = _pull_rows(yp, rank0, dest, M, k, weights=weights.reshape(-1))
-        ctx.save_for_backward(yp, weights, dest, src_tok, rank0)
+        ctx.save_for_backward(yp, weights, dest, src_tok, rank0, counts, offsets)
         return y
 
     @staticmethod
     def backward(ctx, dy):
-        yp, weights, dest, src_tok, rank0 = ctx.saved_tensors
+        yp, weights, dest, src_tok, rank0, counts, offsets = ctx.saved_tensors
         M, k = weights.shape
         dy = dy.contiguous()
         _, dots = _pull_rows(yp, rank0, dest, M, k, want_out=False, grad=dy)
-        d_yp = torch.zeros_like(yp)
+        d_yp = K.moe_fill_(torch.empty_like(yp), counts, offsets)
         _push_rows(d_yp, dy, src_tok, rank0, dest, weights.reshape(-1))
-        return d_yp, dots.view(M, k), None, None, None
+        return d_yp, dots.view(M, k), None, None, None, None, None
 
 
 def moe_mlp(x, weights, idx, w_gate_up, w_down):
@@ -232,13 +233,13 @@ def moe_mlp(x, weights, idx, w_gate_up, w_down):
     E = w_gate_up.shape[0]
     k = idx.shape[1]
     if Fn.use_kernels(x) and w_gate_up.dtype == bf16 and D % 64 == 0:
-        offsets, dest = K.moe_plan(idx.to(torch.int32).contiguous(), E, PAD)
+        offsets, dest, counts = K.moe_plan(idx.to(torch.int32).contiguous(), E, PAD, with_counts=True)
         cap = (M * k + E * (PAD - 1) + PAD - 1) // PAD * PAD
         src_tok = torch.arange(M, device=x.device, dtype=torch.int32).repeat_interleave(k)
         rank0 = torch.zeros(M * k, dtype=torch.int32, device=x.device)
-        xp = _LocalDispatch.apply(x.contiguous(), dest, src_tok, rank0, cap, k)
+        xp = _LocalDispatch.apply(x.contiguous(), dest, src_tok, rank0, cap, k, counts, offsets)
         yp = expert_mlp_permuted(xp, w_gate_up, w_down, offsets)
-        return _LocalCombine.apply(yp, weights.contiguous().float(), dest, src_tok, rank0)
+        return _LocalCombine.apply(yp, weights.contiguous().float(), dest, src_tok, rank0, counts, offsets)
     out = torch.zeros(M, D, dtype=torch.float32, device=x.device)
     for e in range(E):
         tok, slot = torch.nonzero(idx == e, as_tuple=True)

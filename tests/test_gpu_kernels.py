@@ -798,6 +798,44 @@ def test_adamw_passes_over_zero_gradients(n):
     assert all(torch.equal(a, b) for a, b in zip(*outs))
 
 
+@pytest.mark.parametrize("M,k,D", [(1, 1, 8), (37, 8, 264), (50, 10, 1024), (9, 16, 256), (5, 20, 72)])
+def test_token_rows_pulled_and_dotted(M, k, D):
+    """Weighted sums of a token's rows and their products with its gradient, rows that were dropped among them; fp32 reference, one
+    rounding to bf16 of the sums, fp32 sums of D products."""
+    from omegalax_b200.ops import moe
+    torch.manual_seed(43)
+    rows = M * k + 3
+    buf, g = torch.randn(rows, D, device=_dev()).to(bf16), torch.randn(M, D, device=_dev()).to(bf16)
+    at = torch.randperm(rows, device=_dev())[:M * k].to(torch.int32)
+    at[::7] = -1
+    w, zero = torch.rand(M * k, device=_dev()), torch.zeros(M * k, dtype=torch.int32, device=_dev())
+    x = torch.where(at[:, None] >= 0, buf[at.clamp_min(0).long()].double(), 0.0).view(M, k, D)
+    for weights in (None, w):
+        for want_out, grad in ((True, None), (False, g), (True, g)):
+            out, dots = moe._pull_rows(buf, zero, at, M, k, weights=weights, want_out=want_out, grad=grad)
+            if want_out:
+                ref = (x * (1.0 if weights is None else weights.double().view(M, k, 1))).sum(1)
+                torch.testing.assert_close(out.double(), ref, rtol=2.0 ** -8, atol=k * 2.0 ** -20)
+            if grad is not None:
+                torch.testing.assert_close(dots.double().view(M, k), torch.einsum("mkd,md->mk", x, g.double()), rtol=1e-5, atol=D * 2.0 ** -20)
+
+
+@pytest.mark.parametrize("M,k,E", [(1, 1, 3), (300, 2, 5), (64, 4, 130)])
+def test_segments_are_filled_with_zeros(M, k, E):
+    """Only the rows between an expert's pairs and the next segment, where a GEMM reads them."""
+    from omegalax_b200.ops import kernels as Kn, lib
+    torch.manual_seed(44)
+    idx = torch.rand(M, E, device=_dev()).topk(k, -1).indices.to(torch.int32)
+    offsets, dest, counts = Kn.moe_plan(idx, E, 256, with_counts=True)
+    rows = torch.full((int(offsets[-1]) + 256, 72), 3.0, dtype=bf16, device=_dev())
+    Kn.moe_fill_(rows, counts, offsets)
+    _check(lib)
+    used = torch.zeros(rows.shape[0], dtype=torch.bool, device=_dev())
+    used[dest.long()] = True
+    used[int(offsets[-1]):] = True
+    assert (rows[used] == 3).all() and not rows[~used].any() and torch.equal(counts.long(), torch.bincount(idx.reshape(-1), minlength=E))
+
+
 @pytest.mark.parametrize("R,window", [(8, 0), (8, 100), (3, 16), (1, 1)])
 @pytest.mark.parametrize("splits", [1, 5, 70])
 def test_decode_attention_window_and_sink(R, window, splits):
