@@ -579,15 +579,16 @@ int ob_gemm_bf16_pair(const void* A, const void* B, void* C, const void* residua
 // whoever fills rows up to blocks of 64 counts them from row 0 of all rows, and the blocks read here start at rows_off.
 int ob_gemm_counted_rows(int kind, const void* A, const void* B, void* C, int M, int N, int K, long long lda,
                          long long ldb, long long ldc, const int* rows_dev, int rows_off, const int* ce_targets,
-                         void* ce_stats, float* ce_tgt, const float* scale, int* status, cudaStream_t stream) {
+                         void* ce_stats, float* ce_tgt, const float* scale, int accumulate, int* status, cudaStream_t stream) {
   if (M <= 0 || N <= 0 || K <= 0) return 0;
   if ((lda & 7) || (ldb & 7)) return 6001;
   if ((((uintptr_t)A) & 15) || (((uintptr_t)B) & 15)) return 6002;
   if (kind < 0 || kind > 2 || rows_dev == nullptr || (kind == 0) != (ce_stats != nullptr) || (scale && kind != 2)) return 6005;
   if (rows_off < 0 || (rows_off & 63)) return 6005;
+  if (!accumulate && (kind != 2 || (((uintptr_t)C) & 15) || (ldc & 3))) return 6005;
   GemmArgs g = {};
   g.M = M; g.N = N; g.K = K; g.mode = 0;
-  g.C = C; g.ldc = ldc; g.out_mode = kind == 0 ? 0 : 2;
+  g.C = C; g.ldc = ldc; g.out_mode = kind == 0 ? 0 : accumulate ? 2 : 1;
   g.ce_targets = ce_targets; g.ce_stats = (float2*)ce_stats; g.ce_tgt = ce_tgt;
   g.rows_dev = rows_dev; g.rows_off = rows_off; g.rows_in_k = kind == 2; g.scale_dev = scale;
   g.status = status;

@@ -60,7 +60,7 @@ __device__ __forceinline__ WideWork wide_work(const GemmArgs& p, int pairs) {
   const int n = min(max(__ldg(p.rows_dev) - p.rows_off, 0), p.rows_in_k ? p.K : p.M);
   if (p.rows_in_k) w.K = n;
   else w.num_m_blocks = (n + 511) / 512;
-  w.total_tiles = n > 0 ? w.num_m_blocks * p.num_n_blocks : 0;
+  w.total_tiles = n > 0 || (p.rows_in_k && p.out_mode == 1) ? w.num_m_blocks * p.num_n_blocks : 0;      // an empty sum is stored too
   const int kb = (w.K + BK - 1) / BK;
   w.k_splits = 1;
   w.k_per_split = kb * BK;

@@ -470,10 +470,10 @@ def ce_counted_grad_(logits, targets, lse, mask, grad_scale, counted):
           grad_scale.data_ptr(), counted[0].data_ptr(), counted[1], lib.stream_ptr())
 
 
-def gemm_counted(kind: int, a, b, out, counted, ce=None, scale=None):
+def gemm_counted(kind: int, a, b, out, counted, ce=None, scale=None, accumulate: bool = True):
     """The head's products when only the first ``counted[0]`` (int32 [1] on the device) - ``counted[1]`` rows
     of ``a`` hold anything.  kind 0: out bf16 = a b^T with the statistics ``ce``; kind 1: out fp32 += a b;
-    kind 2: out fp32 += a^T b, times what ``scale`` (fp32 [1]) is beyond a power of two."""
+    kind 2: out fp32 += a^T b, times what ``scale`` (fp32 [1]) is beyond a power of two (without ``accumulate``: =)."""
     (M, K) = (a.shape[1], a.shape[0]) if kind == 2 else a.shape
     N = b.shape[1] if kind else b.shape[0]
     ce_ptrs = (None, None, None) if ce is None else (ce[0].data_ptr(), ce[1].data_ptr(), ce[2].data_ptr())
@@ -483,7 +483,8 @@ def gemm_counted(kind: int, a, b, out, counted, ce=None, scale=None):
         if t.stride(1) != 1:
             raise ValueError("row-major operands expected")
     _call("ob_gemm_counted_rows", kind, a.data_ptr(), b.data_ptr(), out.data_ptr(), M, N, K, a.stride(0), b.stride(0), out.stride(0),
-          counted[0].data_ptr(), counted[1], *ce_ptrs, lib.ptr(scale), lib.status_tensor(a.device).data_ptr(), lib.stream_ptr())
+          counted[0].data_ptr(), counted[1], *ce_ptrs, lib.ptr(scale), int(accumulate or kind != 2), lib.status_tensor(a.device).data_ptr(),
+          lib.stream_ptr())
     return out
 
 

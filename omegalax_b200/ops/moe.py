@@ -144,7 +144,7 @@ class _GroupedLinearFn(torch.autograd.Function):
         if ctx.needs_input_grad[1]:
             mg = getattr(ctx.w_ref, "main_grad", None)
             if mg is not None:
-                K.gemm_grouped_wgrad(dy, x, offsets, mg, accumulate=True, pair=_PAIR)
+                K.gemm_grouped_wgrad(dy, x, offsets, mg, accumulate=not Fn.first_gradient(ctx.w_ref), pair=_PAIR)
             else:
                 dwf = torch.zeros(w.shape, dtype=torch.float32, device=w.device)
                 K.gemm_grouped_wgrad(dy, x, offsets, dwf, accumulate=False, pair=_PAIR)

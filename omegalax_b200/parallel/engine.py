@@ -64,6 +64,7 @@ class ParamSlot:
     shard_world: int = 1       # number of ranks the parameter is cut over (1 when replicated) ...
     shard_rank: int = 0        # ... and which piece this rank holds
     ep_product: bool = False   # experts cut over shard group x tensor-parallel group (every rank of the job)
+    old_grad: bool = False     # its gradient is left as it is by the optimizer and stored over by the next step's first product
 
 
 @dataclasses.dataclass
@@ -349,8 +350,44 @@ class TrainEngine:
                     u.resident = True
         if hasattr(self.model, "layer_runner"):
             self.model.layer_runner = self.run_layer
+        # One rank: gradients of experts and (untied) head are whole products, written by ``first_gradient``'s callers.
+        head = getattr(getattr(self.model, "lm_head", None), "weight", None)
+        tied = any(type(m).__name__ == "Embedding" and getattr(m, "weight", None) is head for m in self.model.modules())
+        if self.use_cuda_kernels and self.W == 1 and self.TP == 1 and self.compute_dtype == bf16:
+            for u in self.units:
+                for s in u.slots:
+                    name = s.pname.rsplit(".", 1)[-1]
+                    s.old_grad = name in ("experts_gate_up", "experts_down") or (s.param is head and not tied)
+        self._grad_runs = self._clearing_runs()
         self._layer_units = {id(u.modules[0]): u for u in self.units if u.name.startswith("layers.")}
         self._layer_by_index = {int(u.name.split(".")[1]): u for u in self.units if u.name.startswith("layers.")}
+
+    def _clearing_runs(self):
+        """(start, end, clear) over the flat shard: where the optimizer clears gradients and where it leaves them, in whole
+        blocks of the ``used`` map."""
+        left: list = []      # [start, end) of neighbours whose gradients stay
+        for u in self.units:
+            for s in u.slots:
+                if s.old_grad:
+                    lo = u.shard_base + s.shard_off
+                    if left and lo - left[-1][1] < 8:      # nothing but padding between them
+                        left[-1][1] = lo + s.shard_numel
+                    else:
+                        left.append([lo, lo + s.shard_numel])
+        runs, at = [], 0
+        for lo, hi in left:
+            lo, hi = -(-lo // 128) * 128, hi // 128 * 128
+            if hi > lo:
+                runs += [(at, lo, True)] * (lo > at) + [(lo, hi, False)]
+                at = hi
+        return runs + [(at, self.total_shard, True)] * (self.total_shard > at)
+
+    def _settle_grads(self):
+        """Every ``main_grad`` is that of this step from here on: one that no product has written is zero."""
+        for u in self.units:
+            for s in u.slots:
+                if s.old_grad:
+                    Fn.clear_old_gradient(s.param)
 
     def _bind(self, u: Unit, full: torch.Tensor, full_grad: torch.Tensor | None):
         for s in u.slots:
@@ -536,6 +573,7 @@ class TrainEngine:
         for s in u.slots:
             p = s.param
             if p.grad is not None:
+                Fn.clear_old_gradient(p)
                 p.main_grad.add_(p.grad.to(torch.float32).view(p.main_grad.shape))   # local experts: [E/W, ...]
                 p.grad = None
         if self.W > 1 and not u.resident:
@@ -549,12 +587,14 @@ class TrainEngine:
             for s in u.slots:
                 p = s.param
                 if p.grad is not None:
+                    Fn.clear_old_gradient(p)
                     p.main_grad.add_(p.grad.to(torch.float32).view(s.shape))
                     p.grad = None
             if self.W > 1 and u.resident:
                 self._reduce_scatter(u, u.full_grad)
         if self.comm_kind == "p2p":
             self._barrier()  # every peer's gradient contributions to this shard have landed
+        self._settle_grads()
         self.micro_steps += 1
 
     def _tp_sync_grads(self):
@@ -569,6 +609,7 @@ class TrainEngine:
     # ------------------------------------------------------------------ optimizer
     def grad_norm_sq(self) -> torch.Tensor:
         """Squared global gradient norm (unscaled accumulated gradients) as a device scalar."""
+        self._settle_grads()
         self.norm_sq.zero_()
         if self.TP > 1:
             # tp-sharded slices add up over tp ranks, replicated parameters count once
@@ -621,9 +662,15 @@ class TrainEngine:
         b1, b2 = self.betas
         if self.use_cuda_kernels:
             p16 = None if self.compute_shard is self.master else self.compute_shard
-            K.adamw(self.master, self.exp_avg, self.exp_avg_sq, self.grad, p16, lr=lr, b1=b1, b2=b2,
-                    eps=self.eps, wd=self.wd, step=self.step_count, grad_mul=gmul, norm_sq=nsq,
-                    max_norm=self.max_grad_norm, zero_grad=True, used=self._grad_used if self.TP == 1 else None)
+            used = self._grad_used if self.TP == 1 else None
+            for lo, hi, clear in self._grad_runs:
+                K.adamw(self.master[lo:hi], self.exp_avg[lo:hi], self.exp_avg_sq[lo:hi], self.grad[lo:hi],
+                        None if p16 is None else p16[lo:hi], lr=lr, b1=b1, b2=b2, eps=self.eps, wd=self.wd, step=self.step_count,
+                        grad_mul=gmul, norm_sq=nsq, max_norm=self.max_grad_norm, zero_grad=clear,
+                        used=None if used is None else used[lo // 128:])
+            for u in self.units:
+                for s in u.slots:
+                    s.param.grad_is_old = s.old_grad
         else:
             mul = torch.full((), gmul, dtype=torch.float32, device=self.device)
             if self.max_grad_norm > 0:

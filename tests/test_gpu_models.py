@@ -177,6 +177,49 @@ def test_training_engine_reduces_loss(name):
     assert losses[-1] < losses[0] - 0.05, losses
 
 
+@pytest.mark.parametrize("M", [192, 1700])      # the head on whole rows, and on the supervised ones
+@pytest.mark.parametrize("name", ["qwen3-dense", "qwen3-moe"])
+def test_gradients_that_the_optimizer_leaves(name, M):
+    """Gradients of experts and head stay behind the optimizer and are stored over: accumulated batches, a batch without supervised
+    rows, a step without any backward pass and one that reads the gradients give the moments of an engine that clears them all (to
+    sums by atomics: the learning rate is zero, as Adam's division would turn the rounding of gradients near zero into whole steps)."""
+    from omegalax_b200.ops import lib
+    from omegalax_b200.parallel import mesh as mesh_lib
+    from omegalax_b200.trainers import text as trainer
+
+    dev, runs = _dev(), []
+    for clear in (False, True):
+        mesh_lib.set_default_mesh(None)
+        tcfg = trainer.TrainConfig(batch_size=2, seq_len=M, num_steps=8, learning_rate=0.0, max_grad_norm=1.0)
+        model, cfg = trainer.init_model(_configs()[name], 0, tp_size=1, fsdp_size=1, dp_size=1, meta=True)
+        opt = trainer.build_optimizer(model, tcfg, device=dev)
+        left = [s for u in opt.units for s in u.slots if s.old_grad]
+        assert len(left) == (5 if name == "qwen3-moe" else 1) and [r[2] for r in opt._grad_runs].count(False) == len(left) // 2 + 1
+        if clear:
+            for s in left:
+                s.old_grad = False
+            opt._grad_runs = [(0, opt.total_shard, True)]
+        g = torch.Generator().manual_seed(5)
+        seen = []
+        for masks in ((1, 1), (1,), (), (0,), (1,)):
+            for m in masks:
+                tok = torch.randint(1, cfg.vocab_size, (2, M), generator=g, dtype=torch.int32).to(dev)
+                ce, aux, _ = trainer._loss_and_count(model, cfg, {"token_ids_BT": tok, "attention_mask_BT": torch.ones_like(tok),
+                                                                  "loss_mask_BT": torch.full_like(tok, m)}, 0, None)
+                (ce + aux).backward()
+                opt.finish_backward()
+            if not masks:
+                opt.finish_backward()
+            norm = opt.grad_norm_sq().clone()
+            grads = [s.param.main_grad.clone() for s in left]
+            opt.optimizer_step(lr=0.0, grad_accum=max(1, len(masks)))
+            seen += [norm, *grads, opt.exp_avg.clone()]
+        runs.append(seen)
+    lib.check_status()
+    for i, (a, b) in enumerate(zip(*runs)):
+        assert torch.isfinite(a).all() and float((a - b).norm()) <= 1e-3 * float(b.norm()) + 1e-12, i
+
+
 def test_remat_policies_follow_the_same_loss_curve(monkeypatch):
     """full / selective / auto rematerialisation compute the same step: the stashed or replayed
     tensors are the ones a full re-run would produce.  "auto" gets a budget that lets every layer
