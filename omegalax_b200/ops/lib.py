@@ -101,8 +101,8 @@ _SIGS = {
     "ob_ep_plan": [P, P, P, P, P, P, P, L, I, I, I, I, I, P],
     "ob_moe_fill": [P, P, P, I, I, P],
     "ob_moe_plan": [P, P, P, P, P, L, I, I, I, P],
-    "ob_gdn_fwd": [P] * 10 + [I] * 6 + [P],
-    "ob_gdn_bwd": [P] * 15 + [I] * 6 + [P],
+    "ob_gdn_fwd": [P] * 13 + [I] * 8 + [P],
+    "ob_gdn_bwd": [P] * 22 + [I] * 8 + [P],
     "ob_conv1d_silu_fwd": [P, P, P, I, I, I, I, P],
     "ob_conv1d_silu_bwd": [P, P, P, P, P, I, I, I, I, P],
     "ob_rmsnorm_fwd": [P, P, P, P, L, I, F, I, P],
