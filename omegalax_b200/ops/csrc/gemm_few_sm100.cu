@@ -220,14 +220,17 @@ gemm_few_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__
   }
 }
 
-// CTAs per panel: as many as the SMs take in one wave of two, with slices of at least four k-blocks.  M 1,
-// K 4096, in us by CTAs per panel 1 / 2 / 4 / 8: N 4096 22.5 13.7 10.3 10.8, N 6144 22.2 14.3 12.8 15.9,
-// N 24576 37.6 38.9 40.5 46.6.  Clusters of four and eight do not fill the last 40 of the 296 places, since the SMs of a GPC are no
-// whole number of them: 64 panels of 128 rows by four, K 1024, 10.8 us, 72 panels 16.8 (by two 10.6).
+// CTAs per panel: as many as the SMs take in one wave of two, with slices of at least four k-blocks (six where they are no power
+// of two).  The more of the panel's weights wait in the rings when X arrives, the better, but clusters of more than two do not
+// fill the last 46 of the 296 places, since the SMs of a GPC are no whole number of them (four: the last 40).  In a chain with
+// norms, in us by CTAs per panel: N 6144, K 4096, M 1 2: 15.5, 4: 14.0, 5: 13.1, 6: 18.0; N 10240, M 64 2: 23.4, 3: 21.8, 4: 27.9;
+// N 4096, K 12288, M 32 4: 27.1, 7: 25.7, 8: 33.8; N 24576 1: 37.6, 2: 39.3.  Short slices lose: N 9216, K 1024, M 32 2: 9.6, 3: 10.5.
 static int few_splits(long long panels, int kblocks) {
-  int s = 1;
-  while (s < 8 && panels * 2 * s <= 2 * num_sms() - (s > 1 ? 40 : 0) && kblocks / (2 * s) >= 4) s *= 2;
-  return s;
+  for (int s = 8; s > 1; --s) {
+    const bool two = (s & (s - 1)) == 0;
+    if (panels * s <= (s == 2 ? 2 * num_sms() : 2 * num_sms() - (s == 4 ? 40 : 46)) && kblocks / s >= (two ? 4 : 6)) return s;
+  }
+  return 1;
 }
 
 template <int NB>
