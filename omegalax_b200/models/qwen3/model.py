@@ -246,6 +246,7 @@ def vocab_parallel_head(cfg, tp_size: int) -> bool:
     return tp_size > 1 and not cfg.tie_word_embeddings and cfg.vocab_size % (8 * tp_size) == 0
 
 
+_FORWARDS = {c: c.forward for c in (Linear, RMSNorm, Attention, MLP, DecoderLayer)}
 _STEP_METHODS = frozenset(("forward", "embed", "run_layers", "_after_attention"))
 _PLAIN = frozenset((int, float, bool))
 
@@ -319,10 +320,15 @@ class Qwen3(nn.Module):
         """Residual rows of one new token per sequence, after the last layer."""
         from ...ops import kernels as K
 
-        x = self.embed(batch.ids)
+        x, squares = self.embed(batch.ids), None
+        fused = self._plain_step(cache, x)
         for li, layer in enumerate(self.layers):
             a, k, v = layer.attn, cache.k_pages[li], cache.v_pages[li]
-            q = K.decode_append(a.qkv_proj(layer.input_norm(x)), a.q_norm.weight, a.k_norm.weight, batch.slot, batch.seq, batch.slot,
+            if squares is None:
+                qkv = a.qkv_proj(layer.input_norm(x))
+            else:
+                qkv = K.gemm_step(x, a.qkv_proj.weight, norm=(layer.input_norm.weight, layer.input_norm.eps, squares))
+            q = K.decode_append(qkv, a.q_norm.weight, a.k_norm.weight, batch.slot, batch.seq, batch.slot,
                                 cache.block_table, cache.page_size, k, v, a.H, a.G, a.Kd, a.Kd, self.cfg.rope_theta, a.eps)
             if batch.every:
                 o = K.decode_attn(q, k, v, cache.block_table, batch.lens, cache.page_size, a.scale)
@@ -330,8 +336,42 @@ class Qwen3(nn.Module):
                 qb = torch.zeros(cache.B, a.H, a.Kd, dtype=q.dtype, device=q.device)
                 qb[batch.seq.long()] = q
                 o = K.decode_attn(qb, k, v, cache.block_table, batch.lens, cache.page_size, a.scale)[batch.seq.long()]
-            x = self._after_attention(layer, o, x)
+            if fused:
+                n, m, sums = layer.post_norm, layer.mlp, x.shape[0] <= 32
+                x = K.gemm_step(o.reshape(x.shape[0], -1), a.o_proj.weight, residual=x, squares=sums)
+                x, squares = x if sums else (x, None)
+                if sums:
+                    h = K.gemm_step(x, m.gate_up_proj.weight, norm=(n.weight, n.eps, squares), act=True)
+                else:
+                    h = K.gemm_step(n(x), m.gate_up_proj.weight, act=True)
+                x = K.gemm_step(h, m.down_proj.weight, residual=x, squares=sums and li + 1 < len(self.layers))
+                x, squares = x if x.__class__ is tuple else (x, None)
+            else:
+                x = self._after_attention(layer, o, x)
         return x
+
+    def _plain_step(self, cache, x):
+        """Whether the products of a step may take norms, activation and sums of squares along: nothing wants to see the modules'
+        calls, and all of them are dense and of this file's classes."""
+        D = self.cfg.emb_dim
+        if (x.shape[0] > 64 or x.dtype != torch.bfloat16 or not Fn.use_kernels(x) or Fn.library_mode() or self.tp_size > 1 or D % 128
+                or self._recordable(cache) is None):
+            return False
+        for la in self.layers:
+            a, m = la.attn, la.mlp
+            if not (type(la) is DecoderLayer and type(a) is Attention and type(m) is MLP):
+                return False
+            for n in (la.input_norm, la.post_norm):
+                if type(n) is not RMSNorm or n.one_plus or n.scale_in_dtype:
+                    return False
+            linears = (a.qkv_proj, a.o_proj, m.gate_up_proj, m.down_proj)
+            if any(type(p) is not Linear or p.bias is not None or hasattr(p.weight, "main_grad") or p.weight.shape[0] % 128
+                   or p.weight.shape[1] % 64 for p in linears):
+                return False
+            for p in (la.input_norm, la.post_norm, *linears):
+                if p.weight.dtype != torch.bfloat16 or not p.weight.is_contiguous() or p.weight.data_ptr() % 16:
+                    return False
+        return all(c.forward is f for c, f in _FORWARDS.items())
 
     @staticmethod
     def _after_attention(layer, o, x):

@@ -28,6 +28,13 @@ struct FewArgs {
   const bf16* bias;
   int vec;                 // C (and residual) rows take 4-element accesses
   int* status;
+  // in a decode step (ob_gemm_step)
+  const bf16 *X, *norm_w;  // kNorm: rows of X, weights of the norm that they pass on their way to shared memory
+  const float* squares;    // kNorm: [M, K / 128] sums of squares of X by panels of 128 columns
+  float* squares_out;      // or null: the same of C
+  long long ldx;
+  float eps;
+  int act;                 // W is [gate | up]: C = silu(gate) * up, N / 2 columns
 };
 
 template <int NB>
@@ -49,7 +56,72 @@ __device__ __forceinline__ float4 ld_cluster_v4(uint32_t addr) {
   return v;
 }
 
+// One stage's rows of X (NB x 64), normalised: 128 threads, 16 bytes of NB / 16 rows each, in the layout that TMA would
+// leave (128-byte rows, 16-byte groups exchanged by the row's last three bits).  Loads run kAhead stages ahead, since a stage of
+// weights passes in 0.5 us and a load takes one (two ahead, 32 rows: 47 us for N 24576, K 4096, four: 40).
 template <int NB>
+__device__ __forceinline__ void few_norm_rows(const FewArgs& p, uint8_t* smem, uint64_t* full_bar, uint64_t* empty_bar,
+                                              volatile int* abort_flag, int m0, int k_begin, int k_end) {
+  using L = FewSmem<NB>;
+  constexpr int kR = NB / 16, kAhead = NB == 16 ? 6 : 4;
+  const int t = threadIdx.x - 64, r0 = t >> 3, c = t & 7, n = (k_end - k_begin) / BK;
+  const bf16* w = p.norm_w + k_begin + c * 8;
+  uint4 wq[kAhead], xq[kAhead][kR];
+  auto load = [&](int j, int i) {
+    if (i >= n) return;
+    wq[j] = *reinterpret_cast<const uint4*>(w + i * BK);
+#pragma unroll
+    for (int r = 0; r < kR; ++r) {
+      const int m = m0 + r0 + 16 * r;
+      xq[j][r] = m < p.M ? *reinterpret_cast<const uint4*>(p.X + m * p.ldx + k_begin + c * 8 + i * BK) : make_uint4(0, 0, 0, 0);
+    }
+  };
+#pragma unroll
+  for (int j = 0; j < kAhead; ++j) load(j, j);
+  float rstd[kR];
+#pragma unroll
+  for (int r = 0; r < kR; ++r) {      // the eight threads of a row
+    const int m = min(m0 + r0 + 16 * r, p.M - 1), parts = p.K >> 7;
+    float s = 0.f;
+    for (int i = c; i < parts; i += 8) s += p.squares[(long long)m * parts + i];
+#pragma unroll
+    for (int o = 1; o < 8; o <<= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    rstd[r] = rsqrtf(s / (float)p.K + p.eps);
+  }
+  int stage = 0;
+  uint32_t phase = 0;
+  for (int i0 = 0; i0 < n; i0 += kAhead) {
+#pragma unroll
+    for (int j = 0; j < kAhead; ++j) {
+      if (i0 + j >= n) break;
+      if (!mbar_wait(&empty_bar[stage], phase ^ 1, abort_flag, p.status, OB_ERR_WAIT_EMPTY)) return;
+      uint8_t* sx = smem + stage * L::kStageBytes + L::kABytes;
+      const uint32_t g[4] = {wq[j].x, wq[j].y, wq[j].z, wq[j].w};
+#pragma unroll
+      for (int r = 0; r < kR; ++r) {
+        const uint32_t u[4] = {xq[j][r].x, xq[j][r].y, xq[j][r].z, xq[j][r].w};
+        uint32_t o[4];
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          const float2 x = unpack_bf16(u[e]), y = unpack_bf16(g[e]);
+          o[e] = pack_bf16(x.x * rstd[r] * y.x, x.y * rstd[r] * y.y);
+        }
+        const int row = r0 + 16 * r;
+        *reinterpret_cast<uint4*>(sx + row * 128 + ((c ^ (row & 7)) << 4)) = make_uint4(o[0], o[1], o[2], o[3]);
+      }
+      load(j, i0 + j + kAhead);
+      fence_proxy_async_smem();
+      __syncwarp();
+      if ((threadIdx.x & 31) == 0) mbar_arrive(&full_bar[stage]);
+      if (++stage == L::kStages) {
+        stage = 0;
+        phase ^= 1;
+      }
+    }
+  }
+}
+
+template <int NB, bool kNorm>
 __global__ void __launch_bounds__(kGemmThreads, 2)
 gemm_few_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUtensorMap tmX, const FewArgs p) {
   extern __shared__ uint8_t smem_raw[];
@@ -65,7 +137,7 @@ gemm_few_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int splits = (int)gridDim.x, rank = (int)blockIdx.x;    // the cluster spans the x dimension
-  const int n0 = blockIdx.y * 128, m0 = blockIdx.z * NB;
+  const int n0 = blockIdx.y * (p.act ? 64 : 128), m0 = blockIdx.z * NB;
   if (threadIdx.x == 0) {
     tma_prefetch_desc(&tmW);
     tma_prefetch_desc(&tmX);
@@ -74,7 +146,7 @@ gemm_few_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__
 
   if (threadIdx.x == 0) {
     for (int i = 0; i < kSt; ++i) {
-      mbar_init(&full_bar[i], 1);
+      mbar_init(&full_bar[i], kNorm ? 5 : 1);      // the copies, and the four warps that bring X
       mbar_init(&empty_bar[i], 1);
     }
     mbar_init(done_bar, 1);
@@ -92,23 +164,24 @@ gemm_few_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__
 
   if (warp == 0) {
     if (lane == 0) {
+      auto load_w = [&](int stage, int k0) {
+        uint8_t* sw = smem + stage * L::kStageBytes;
+        mbar_expect_tx(&full_bar[stage], kNorm ? L::kABytes : L::kStageBytes);
+        tma_load_2d(sw, &tmW, &full_bar[stage], k0, n0);
+        if (p.act) tma_load_2d(sw + L::kABytes / 2, &tmW, &full_bar[stage], k0, p.N / 2 + n0);
+      };
       // the weights of the first stages are on their way while the kernel before, which gives X, still runs
       const int ahead = min(kSt, (k_end - k_begin + BK - 1) / BK);
-      for (int i = 0; i < ahead; ++i) {
-        mbar_expect_tx(&full_bar[i], L::kStageBytes);
-        tma_load_2d(smem + i * L::kStageBytes, &tmW, &full_bar[i], k_begin + i * BK, n0);
-      }
+      for (int i = 0; i < ahead; ++i) load_w(i, k_begin + i * BK);
       grid_begin();
-      for (int i = 0; i < ahead; ++i)
+      for (int i = 0; i < ahead && !kNorm; ++i)
         tma_load_2d(smem + i * L::kStageBytes + L::kABytes, &tmX, &full_bar[i], k_begin + i * BK, m0);
       int stage = ahead == kSt ? 0 : ahead;
       uint32_t phase = ahead == kSt;
       for (int k0 = k_begin + ahead * BK; k0 < k_end; k0 += BK) {
         if (!mbar_wait(&empty_bar[stage], phase ^ 1, abort_flag, p.status, OB_ERR_WAIT_EMPTY)) break;
-        uint8_t* sw = smem + stage * L::kStageBytes;
-        mbar_expect_tx(&full_bar[stage], L::kStageBytes);
-        tma_load_2d(sw, &tmW, &full_bar[stage], k0, n0);
-        tma_load_2d(sw + L::kABytes, &tmX, &full_bar[stage], k0, m0);
+        load_w(stage, k0);
+        if (!kNorm) tma_load_2d(smem + stage * L::kStageBytes + L::kABytes, &tmX, &full_bar[stage], k0, m0);
         if (++stage == kSt) {
           stage = 0;
           phase ^= 1;
@@ -144,6 +217,10 @@ gemm_few_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__
     // output column, so a warp's stores cover 128 consecutive bytes
     float* part = reinterpret_cast<float*>(smem);
     const int quad = warp & 3;
+    if constexpr (kNorm) {
+      grid_wait();
+      few_norm_rows<NB>(p, smem, full_bar, empty_bar, abort_flag, m0, k_begin, k_end);
+    }
     if (mbar_wait(done_bar, 0, abort_flag, p.status, OB_ERR_WAIT_TMEM_FULL)) {
       __syncwarp();
       tc_fence_after();
@@ -172,9 +249,20 @@ gemm_few_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__
         const float4 t = ld_cluster_v4(mapa_shared(mine + m * 512, r));
         s.x += t.x; s.y += t.y; s.z += t.z; s.w += t.w;
       }
-      if (ncol <= 0) continue;
       float v[4] = {s.x, s.y, s.z, s.w};
       const long long row = m0 + m;
+      if (p.act) {      // lanes 0..15 gate, 16..31 up, rounded as products of their own would be
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          v[i] = __bfloat162float(__float2bfloat16(v[i]));
+          const float u = __shfl_down_sync(0xffffffffu, v[i], 16);
+          v[i] = v[i] / (1.f + __expf(-v[i])) * u;
+        }
+        if (lane < 16)
+          *reinterpret_cast<uint2*>((bf16*)p.C + row * p.ldc + col) = make_uint2(pack_bf16(v[0], v[1]), pack_bf16(v[2], v[3]));
+        continue;
+      }
+      if (ncol <= 0) continue;
       if (p.bias) {
 #pragma unroll
         for (int i = 0; i < 4; ++i) if (i < ncol) v[i] += __bfloat162float(p.bias[col + i]);
@@ -191,6 +279,11 @@ gemm_few_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__
       }
       if (p.out_mode == 0) {
         bf16* cp = (bf16*)p.C + row * p.ldc + col;
+        if (p.squares_out) {      // N % 128 == 0: all lanes are here
+          const float2 a = unpack_bf16(pack_bf16(v[0], v[1])), b = unpack_bf16(pack_bf16(v[2], v[3]));
+          const float ss = warp_sum(a.x * a.x + a.y * a.y + b.x * b.x + b.y * b.y);
+          if (lane == 0) p.squares_out[row * (p.N >> 7) + blockIdx.y] = ss;
+        }
         if (p.vec && ncol == 4) *reinterpret_cast<uint2*>(cp) = make_uint2(pack_bf16(v[0], v[1]), pack_bf16(v[2], v[3]));
         else for (int i = 0; i < ncol; ++i) cp[i] = __float2bfloat16(v[i]);
       } else {
@@ -233,14 +326,14 @@ static int few_splits(long long panels, int kblocks) {
   return 1;
 }
 
-template <int NB>
+template <int NB, bool kNorm = false>
 static int launch_few(const void* X, const void* W, FewArgs a, long long ldx, long long ldw, int splits, cudaStream_t stream) {
   CUtensorMap tmW, tmX;
   int e = make_tmap_2d(&tmX, X, a.M, a.K, ldx, NB, BK);
   if (e) return 2000 + e;
-  e = make_tmap_2d(&tmW, W, a.N, a.K, ldw, 128, BK);
+  e = make_tmap_2d(&tmW, W, a.N, a.K, ldw, a.act ? 64 : 128, BK);
   if (e) return 3000 + e;
-  auto kern = gemm_few_kernel<NB>;
+  auto kern = gemm_few_kernel<NB, kNorm>;
   OB_ENSURE_DYN_SMEM(kern, FewSmem<NB>::kTotal);
   const int panels = (a.N + 127) / 128, mblocks = (a.M + NB - 1) / NB, kblocks = (a.K + BK - 1) / BK;
   if (panels > 65535 || mblocks > 65535) return 6005;
@@ -292,6 +385,42 @@ int ob_gemm_few(const void* X, const void* W, void* C, const void* residual, int
   if (M <= 64) OB_FEW(64);
   OB_FEW(128);
 #undef OB_FEW
+}
+
+// The same for the rows of a decode step, with what stands beside its products (each was a launch of 3 to 5 us in a chain
+// where every kernel waits for the one before: 8 layers of 4096 channels, one sequence of 4096 tokens 1001 -> 957 us, 32 of 2048
+// 1440 -> 1412; a norm and its product of N 24576, 32 rows, with the activation 42.5 -> 40.0, the product alone 37.6).
+// norm_w with squares [M, K / 128] (sums of squares of X by panels of 128 columns; eps): X passes an RMS norm on its way, M <= 32.
+// squares_out [M, N / 128] or null: the same sums of C as stored.  act: W is [gate | up], C [M, N / 2] = silu(gate) * up of
+// the rounded products.  Rounding and order are those of ob_rmsnorm_fwd and ob_swiglu_fwd but for the order of a sum of squares.
+int ob_gemm_step(const void* X, const void* W, void* C, const void* residual, int M, int N, int K, long long ldx, long long ldw,
+                 long long ldc, long long ldr, const void* norm_w, const float* squares, float eps, float* squares_out, int act,
+                 int* status, cudaStream_t stream) {
+  if (M <= 0 || N <= 0) return 0;
+  if (K <= 0) return 6005;
+  if ((ldx & 7) || (ldw & 7)) return 6001;
+  if ((((uintptr_t)X) & 15) || (((uintptr_t)W) & 15)) return 6002;
+  FewArgs a = {};
+  a.M = M; a.N = N; a.K = K;
+  a.C = C; a.ldc = ldc;
+  a.residual = (const bf16*)residual; a.ldr = ldr;
+  a.vec = !(ldc & 3) && !((uintptr_t)C & 7) && (!residual || (!(ldr & 3) && !((uintptr_t)residual & 7)));
+  a.X = (const bf16*)X; a.ldx = ldx;
+  a.norm_w = (const bf16*)norm_w; a.squares = squares; a.eps = eps;
+  a.squares_out = squares_out;
+  a.act = act;
+  a.status = status;
+  if (act && ((N & 127) || residual || squares_out || !a.vec)) return 6005;
+  if (squares_out && (N & 127)) return 6005;
+  if (norm_w) {
+    if (M > 32 || !squares || (K & 127) || ((uintptr_t)norm_w & 15)) return 6005;
+    if (M <= 16) return launch_few<16, true>(X, W, a, ldx, ldw, 0, stream);
+    return launch_few<32, true>(X, W, a, ldx, ldw, 0, stream);
+  }
+  if (M <= 16) return launch_few<16>(X, W, a, ldx, ldw, 0, stream);
+  if (M <= 32) return launch_few<32>(X, W, a, ldx, ldw, 0, stream);
+  if (M <= 64) return launch_few<64>(X, W, a, ldx, ldw, 0, stream);
+  return launch_few<128>(X, W, a, ldx, ldw, 0, stream);
 }
 
 }  // extern "C"

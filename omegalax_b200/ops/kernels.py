@@ -145,6 +145,21 @@ def gemm(a, b, *, a_mn: bool = False, b_mn: bool = False, out=None, out_dtype=bf
     return out
 
 
+def gemm_step(x, w, *, residual=None, norm=None, squares: bool = False, act: bool = False):
+    """C = x w^T (+ residual) of a decode step's few rows (x [M,K], w [N,K], bf16, contiguous), with what stands beside
+    the product.  ``norm`` = (weight [K], eps, sums): x passes an RMS norm first, whose sums of squares by panels of 128
+    columns are ``sums`` (M <= 32, K % 128 == 0).  ``squares``: returns (C, such sums of C) (N % 128 == 0).  ``act``: w is
+    [gate | up] (N % 128 == 0) and C = silu(gate) * up."""
+    M, K = x.shape
+    N = w.shape[0]
+    out = torch.empty(M, N // 2 if act else N, dtype=bf16, device=x.device)
+    sums = torch.empty(M, N // 128, dtype=torch.float32, device=x.device) if squares else None
+    weight, eps, given = (None, 0.0, None) if norm is None else norm
+    _call("ob_gemm_step", x.data_ptr(), w.data_ptr(), out.data_ptr(), lib.ptr(residual), M, N, K, K, K, out.shape[1], N, lib.ptr(weight),
+          lib.ptr(given), float(eps), lib.ptr(sums), int(act), lib.status_tensor(x.device).data_ptr(), lib.stream_ptr())
+    return (out, sums) if squares else out
+
+
 def gemm_peer_reduce(a, b, peer_ptrs, rows_per_peer: int, ldc: int, *, a_mn=False, b_mn=False, bf16_out=False,
                      pair: bool | None = None, slot: int | None = None):
     """GEMM whose result rows are added into buffers owned by other GPUs (``peer_ptrs[r]`` holds

@@ -33,6 +33,7 @@ _SIGS = {
     "ob_gemm_bf16_pair_peer_reduce": [P, P, P, I, I, I, I, I, L, L, L, I, I, I, I, P, P],
     "ob_gemm_bf16_pair": [P, P, P, P, I, I, I, L, L, L, L, I, I, I, P, P, P, P, P, P],
     "ob_overlap_launches": [I],
+    "ob_gemm_step": [P, P, P, P, I, I, I, L, L, L, L, P, P, F, P, I, P, P],
     "ob_gemm_few": [P, P, P, P, I, I, I, L, L, L, L, I, P, I, P, P],
     "ob_gemm_counted_rows": [I, P, P, P, I, I, I, L, L, L, P, I, P, P, P, P, I, P, P],
     "ob_gemm_bf16_pair_ag": [P, P, P, P, P, I, I, I, L, L, I, I, I, I, I, P, c_uint, I, P, P],

@@ -836,6 +836,35 @@ def test_segments_are_filled_with_zeros(M, k, E):
     assert (rows[used] == 3).all() and not rows[~used].any() and torch.equal(counts.long(), torch.bincount(idx.reshape(-1), minlength=E))
 
 
+@pytest.mark.parametrize("M,N,K", [(1, 6144, 4096), (5, 128, 128), (16, 384, 1152), (17, 256, 2048), (32, 1024, 640), (33, 768, 512),
+                                   (64, 128, 1024)])
+def test_products_of_a_step_take_norm_and_activation_along(M, N, K):
+    """Against the same in launches of their own.  Sums of squares: fp32 sums of 128 squares, within 128 roundings.  The
+    activation: the same bits.  The norm: another order of its sum of squares moves single values of x by one bf16 step at most,
+    and a product of K such by less than one step of the largest output."""
+    from omegalax_b200.ops import kernels as Kn, lib
+    torch.manual_seed(M)
+    x = 3 * torch.randn(M, K, device=_dev(), dtype=torch.bfloat16)
+    w = (torch.randn(N, K, device=_dev()) * K ** -0.5).to(torch.bfloat16)
+    weight = torch.randn(K, device=_dev(), dtype=torch.bfloat16)
+    r = torch.randn(M, N, device=_dev(), dtype=torch.bfloat16)
+    plain = Kn.gemm(x, w, few=True)
+    c, sums = Kn.gemm_step(x, w, residual=r, squares=True)
+    assert torch.equal(c, Kn.gemm(x, w, residual=r, few=True))
+    exact = c.double().square().view(M, -1, 128).sum(-1)
+    assert bool(((sums - exact).abs() <= exact * 128 * 2.0 ** -24).all())
+    assert torch.equal(Kn.gemm_step(x, w, act=True), Kn.swiglu_fwd(plain))
+    if M > 32:
+        return _check(lib)
+    given = x.double().square().view(M, -1, 128).sum(-1).float()
+    want = Kn.gemm(Kn.rmsnorm_fwd(x, weight, 1e-6)[0], w, few=True)
+    for act in (False, True):
+        got = Kn.gemm_step(x, w, norm=(weight, 1e-6, given), act=act).float()
+        ref = (Kn.swiglu_fwd(want) if act else want).float()
+        assert float((got - ref).abs().max()) <= float(ref.abs().max()) * 2.0 ** -7
+    _check(lib)
+
+
 @pytest.mark.parametrize("R,window", [(8, 0), (8, 100), (3, 16), (1, 1)])
 @pytest.mark.parametrize("splits", [1, 5, 70])
 def test_decode_attention_window_and_sink(R, window, splits):
