@@ -13,8 +13,10 @@ from __future__ import annotations
 
 import hashlib
 import os
+import shutil
 import subprocess
 import sys
+import sysconfig
 from concurrent.futures import ThreadPoolExecutor
 from pathlib import Path
 
@@ -106,5 +108,42 @@ def build(force: bool = False, verbose: bool = False, debug: bool = False, group
     return out_lib
 
 
+def launch_module() -> Path:
+    """Where ``csrc/launch_module.cpp`` is built for this interpreter."""
+    return HERE / f"_launch{sysconfig.get_config_var('EXT_SUFFIX') or '.so'}"
+
+
+def launch_stamp() -> Path:
+    return BUILD / "launch" / "stamp.txt"
+
+
+def build_launch_module(table: str, signatures: str) -> Path | None:
+    """Build the module that calls the launchers of ``table`` (lines for table.inc); ``signatures`` names their state.  None
+    where there is no C++ compiler or no headers of Python: the launchers are then called through ctypes."""
+    out, gen = launch_module(), BUILD / "launch"
+    include = sysconfig.get_paths()["include"]
+    cxx = os.environ.get("CXX") or shutil.which("g++") or shutil.which("c++")
+    if not cxx or not os.path.exists(os.path.join(include, "Python.h")):
+        return None
+    gen.mkdir(parents=True, exist_ok=True)
+    # under names of this process first: others may build or load the same
+    inc = gen / str(os.getpid())
+    inc.mkdir(exist_ok=True)
+    (inc / "table.inc").write_text(table)
+    tmp = inc / out.name
+    cmd = [cxx, "-O2", "-std=c++17", "-shared", "-fPIC", f'-DSIGNATURES="{signatures}"', "-I", include, "-I", str(inc),
+           str(CSRC / "launch_module.cpp"), "-o", str(tmp)]
+    res = subprocess.run(cmd, capture_output=True, text=True)
+    if res.returncode != 0:
+        raise RuntimeError(f"{cxx} failed for launch_module.cpp:\n{res.stderr}")
+    os.replace(tmp, out)
+    shutil.rmtree(inc, ignore_errors=True)
+    launch_stamp().write_text(signatures)
+    return out
+
+
 if __name__ == "__main__":
     print(build(force="--force" in sys.argv, verbose="-v" in sys.argv, debug="--debug" in sys.argv))
+    from omegalax_b200.ops import lib
+
+    lib.build_launch_module()

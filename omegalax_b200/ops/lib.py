@@ -7,6 +7,8 @@ silently to another implementation on CUDA tensors).
 from __future__ import annotations
 
 import ctypes
+import hashlib
+import importlib.util
 import os
 from ctypes import c_double, c_float, c_int, c_longlong, c_void_p
 from pathlib import Path
@@ -124,12 +126,53 @@ _SIGS = {
 }
 
 
+_FAST = dict(_SIGS)      # the launchers that csrc/launch_module.cpp knows
+
+
 class KernelError(RuntimeError):
     pass
 
 
 def available() -> bool:
     return LIB_PATH.exists()
+
+
+_TYPE = {P: "P", I: "I", L: "L", F: "F", c_uint: "U", c_double: "D"}
+_launch = None        # call of the module that stands in for ctypes, or None
+
+
+def _launch_table() -> tuple[str, str]:
+    """Lines of table.inc for the launchers of this file, and a name of what they and the module's source are."""
+    from . import build as _build
+
+    lines = "".join(f"SIG({n}, {', '.join(_TYPE[t] for t in sig)})\n" for n, sig in sorted(_FAST.items()))
+    return lines, hashlib.sha256(lines.encode() + (_build.CSRC / "launch_module.cpp").read_bytes()).hexdigest()
+
+
+def build_launch_module() -> None:
+    """Build the module that calls the launchers, where it is not the one of these signatures."""
+    from . import build as _build
+
+    table, state = _launch_table()
+    stamp = _build.launch_stamp()
+    if not (_build.launch_module().exists() and stamp.exists() and stamp.read_text() == state):
+        _build.build_launch_module(table, state)
+
+
+def _load_launch_module():
+    """The module for this interpreter and these signatures, built first where this process may; None: ctypes."""
+    from . import build as _build
+
+    if os.environ.get("OMEGALAX_B200_NO_BUILD") != "1":
+        build_launch_module()
+    path, stamp = _build.launch_module(), _build.launch_stamp()
+    state = _launch_table()[1]
+    if not (path.exists() and stamp.exists() and stamp.read_text() == state):
+        return None
+    spec = importlib.util.spec_from_file_location("_launch", path)
+    mod = importlib.util.module_from_spec(spec)
+    spec.loader.exec_module(mod)
+    return mod if mod.signatures == state else None
 
 
 def load(group: str | None = None):
@@ -160,11 +203,17 @@ def load(group: str | None = None):
 
 
 def _bind(lib):
+    global _launch
     for name, sig in _SIGS.items():
         if hasattr(lib, name):
             fn = getattr(lib, name)
             fn.argtypes = sig
             fn.restype = c_int
+    mod = _load_launch_module()
+    if mod is not None:
+        for name in _FAST:
+            mod.bind(name, ctypes.cast(getattr(lib, name), c_void_p).value if hasattr(lib, name) else 0)
+        _launch = mod.call
     if hasattr(lib, "ob_gemm_pair_tune"):
         lib.ob_gemm_pair_tune.argtypes = [c_int, c_int, c_int]
         lib.ob_gemm_pair_tune.restype = None
@@ -302,9 +351,11 @@ def check_canaries() -> None:
 
 def call(name: str, *args) -> None:
     lib = _lib if _lib is not None else load()
-    if _partial and not hasattr(lib, name):
-        lib = load()
-    rc = getattr(lib, name)(*args)
+    rc = _launch(name, *args) if _launch is not None else None
+    if rc is None:
+        if _partial and not hasattr(lib, name):
+            lib = load()
+        rc = getattr(lib, name)(*args)
     if rc != 0:
         raise KernelError(f"{name} failed with code {rc}")
 

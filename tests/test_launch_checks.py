@@ -39,3 +39,35 @@ def test_more_tiles_than_the_default_bound_the_memory_of_the_head(rows, tiles, c
     from omegalax_b200.trainers.loss import chunk_rows
 
     assert chunk_rows(rows, tiles) == chunk
+
+
+def test_launch_module_converts_arguments_as_ctypes_does(monkeypatch):
+    """Calls that the launchers answer on the host: same code, same kind of error, for numbers of each type and for what only
+    ctypes takes."""
+    import ctypes
+
+    from omegalax_b200.ops import lib
+
+    if not lib.available():
+        pytest.skip("no library")
+    lib.load()
+    if lib._launch is None:
+        pytest.skip("no C++ compiler or no headers of Python")
+    fast = lib._launch
+    buf = (ctypes.c_char * 16)()
+    cases = [("ob_gemm_few", (None, 0, 0, None, True, 1, 0, 8, 8, 1 << 40, 0, 0, None, 0, None, 0)),     # a size of zero
+             ("ob_gemm_few", (None, 0, 0, None, 1 << 32, 1, 8, 8, 8, 8, 0, 0, None, 0, None, 0)),        # rows cut to 32 bits: none
+             ("ob_gemm_few", (None, 0, 0, None, 1, 1, 8, 7, 8, 8, 0, 0, None, 0, None, 0)),              # a pitch refused
+             ("ob_gemm_few", (buf, 0, 0, None, 1, 1, 8, 7, 8, 8, 0, 0, None, 0, None, 0)),               # a pointer as an object
+             ("ob_gemm_step", (8, 16, 16, None, 1, 8, 8, 8, 8, 8, 8, None, None, 1, None, 0, None, 0)),  # an int for a float
+             ("ob_gemm_few", (1, 2)), ("ob_gemm_few", (None, 0, 0, None, 1.5, 1, 8, 8, 8, 8, 0, 0, None, 0, None, 0))]
+    for name, args in cases:
+        seen = []
+        for call in (fast, None):
+            monkeypatch.setattr(lib, "_launch", call)
+            try:
+                seen.append(lib.call(name, *args))
+            except Exception as e:
+                seen.append((type(e), str(e)))
+        assert seen[0] == seen[1], (name, args, seen)
+    assert fast("ob_gemm_few", *cases[2][1]) == 6001 and fast(*[cases[3][0], *cases[3][1]]) is None and fast("ob_unknown", 1) is None
