@@ -16,7 +16,6 @@ from __future__ import annotations
 import math
 
 import torch
-import torch.nn.functional as F
 from torch import nn
 
 from ...ops import functional as Fn
@@ -109,14 +108,7 @@ class GatedDeltaNet(nn.Module):
         b = self.in_proj_b(x)
         a = self.in_proj_a(x)
         mixed = Fn.causal_conv1d_silu(mixed, self.conv_weight)
-        q, k, v = torch.split(mixed, [self.key_dim, self.key_dim, self.value_dim], dim=-1)
-        q = q.reshape(B, T, self.nk, self.ak)
-        k = k.reshape(B, T, self.nk, self.ak)
-        v = v.reshape(B, T, self.nv, self.av)
-        beta = torch.sigmoid(b.float()).view(B, T, self.nv)
-        g = (-torch.exp(self.A_log.float()) * F.softplus(a.float() + self.dt_bias.float())).view(B, T, self.nv)
-        core = Fn.gated_delta_rule(q, k, v, g, beta)               # key heads are shared by nv/nk value heads
-
+        core = Fn.delta_rows(mixed, b, a, -torch.exp(self.A_log.float()), self.dt_bias.float(), self.nk, self.ak, self.nv, self.av)
         core = self.norm(core.reshape(-1, self.av), z.reshape(-1, self.av))
         if tp is not None:
             return tp_lib.row_parallel_linear(core.reshape(B * T, self.value_dim), self.out_proj.weight, residual, tp)

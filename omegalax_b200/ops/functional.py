@@ -925,6 +925,40 @@ class _GatedDeltaRuleFn(torch.autograd.Function):
         return dq, dk, dv, dg, dbeta, ds0, None
 
 
+class _DeltaRowsFn(torch.autograd.Function):
+    """The rule between bf16 rows: norms, gates and padding before it, the cast behind it."""
+
+    @staticmethod
+    def forward(ctx, mixed, b, a, neg_a, dt, Hk, H, U):
+        rows = (mixed, b, a, neg_a, dt)
+        inputs = K.gdn_rows_in(*rows, Hk, H, U)
+        save = any(ctx.needs_input_grad[:5])
+        o, n_out, states, _ = K.gdn_fwd(*inputs, save=save)
+        if save:
+            ctx.save_for_backward(*rows, *inputs, n_out, states)
+        return K.gdn_rows_cast(o, mixed.shape[1])
+
+    @staticmethod
+    def backward(ctx, dy):
+        saved = ctx.saved_tensors
+        rows, inputs, (n_out, states) = saved[:5], saved[5:10], saved[10:]
+        d_o = K.gdn_rows_cast(dy.contiguous(), n_out.shape[1])
+        grads = K.gdn_bwd(*inputs, n_out, states, d_o)[:5]
+        return *K.gdn_rows_in_bwd(*rows, *grads), None, None, None
+
+
+def delta_rows(mixed, b, a, neg_a, dt_bias, Hk: int, A: int, H: int, U: int):
+    """Gated delta rule of mixed [B,T,2 Hk A + H U] = [q | k | v] with beta = sigmoid(b) and g = neg_a softplus(a + dt_bias); b, a
+    [B*T,H], neg_a and dt_bias fp32 [H].  Returns [B,T,H,U]."""
+    B, T = mixed.shape[:2]
+    if use_kernels(mixed) and b.dtype == a.dtype == bf16 and A == 128 and U % 64 == 0 and T > 0:
+        return _DeltaRowsFn.apply(mixed.contiguous(), b.contiguous(), a.contiguous(), neg_a.contiguous(), dt_bias.contiguous(), Hk, H, U)
+    q, k, v = torch.split(mixed, [Hk * A, Hk * A, H * U], dim=-1)
+    beta = torch.sigmoid(b.float()).view(B, T, H)
+    g = (neg_a * F.softplus(a.float() + dt_bias)).view(B, T, H)
+    return gated_delta_rule(q.reshape(B, T, Hk, A), k.reshape(B, T, Hk, A), v.reshape(B, T, H, U), g, beta)
+
+
 def gated_delta_rule(q, k, v, g, beta, chunk: int = 64, initial_state=None, output_final_state=False):
     """Chunked gated delta rule (fp32 inside); q,k [B,T,Hk,A] with Hk dividing H, v [B,T,H,U],
     g/beta [B,T,H].  Key heads are shared by groups of H/Hk value heads."""

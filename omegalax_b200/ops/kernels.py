@@ -679,6 +679,40 @@ def gdn_bwd(q, k, v, g, beta, n_out, states, d_o, d_sfinal=None, want_ds0=False)
     return dq, dk, dv, dg, dbeta, ds0
 
 
+def gdn_rows_in(mixed, b, a, neg_a, dt, Hk: int, H: int, U: int, eps: float = 1e-6):
+    """Inputs of ``gdn_fwd`` from bf16 rows: mixed [B,T,(2 Hk) 128 + H U] = [q | k | v], b and a [B*T,H]; neg_a, dt fp32 [H].
+    q (scaled by 128^-1/2) and k are normed, v cast, beta = sigmoid(b), g = neg_a softplus(a + dt); T is padded to whole chunks
+    with zeros."""
+    B, T = mixed.shape[:2]
+    Tp = -(-T // 64) * 64
+    new = lambda *shape: torch.empty(B, Tp, *shape, dtype=torch.float32, device=mixed.device)  # noqa: E731
+    q, k, v, g, beta = new(Hk, 128), new(Hk, 128), new(H, U), new(H), new(H)
+    _call("ob_gdn_rows_in", mixed.data_ptr(), b.data_ptr(), a.data_ptr(), neg_a.data_ptr(), dt.data_ptr(), q.data_ptr(), k.data_ptr(),
+          v.data_ptr(), g.data_ptr(), beta.data_ptr(), B, T, Tp, Hk, H, H * U, 128 ** -0.5, float(eps), lib.stream_ptr())
+    return q, k, v, g, beta
+
+
+def gdn_rows_in_bwd(mixed, b, a, neg_a, dt, dq, dk, dv, dg, dbeta, eps: float = 1e-6):
+    """Gradients (dmixed, db, da, dneg_a, ddt)."""
+    B, T = mixed.shape[:2]
+    Tp, Hk, H = dq.shape[1], dq.shape[2], dv.shape[2]
+    dmixed, db, da = torch.empty_like(mixed), torch.empty_like(b), torch.empty_like(a)
+    da32, dneg = (torch.empty(B * T, H, dtype=torch.float32, device=mixed.device) for _ in range(2))
+    _call("ob_gdn_rows_in_bwd", mixed.data_ptr(), b.data_ptr(), a.data_ptr(), neg_a.data_ptr(), dt.data_ptr(), dq.data_ptr(), dk.data_ptr(),
+          dv.data_ptr(), dg.data_ptr(), dbeta.data_ptr(), dmixed.data_ptr(), db.data_ptr(), da.data_ptr(), da32.data_ptr(), dneg.data_ptr(),
+          B, T, Tp, Hk, H, H * dv.shape[3], 128 ** -0.5, float(eps), lib.stream_ptr())
+    return dmixed, db, da, dneg.sum(0), da32.sum(0)
+
+
+def gdn_rows_cast(x, T: int):
+    """fp32 [B,Tp,H,U] -> bf16 [B,T,H,U] (rows past T dropped), or bf16 [B,T',H,U] -> fp32 [B,T,H,U] (zeros past T')."""
+    B, t, H, U = x.shape
+    pad = x.dtype == bf16
+    y = torch.empty(B, T, H, U, dtype=torch.float32 if pad else bf16, device=x.device)
+    _call("ob_gdn_rows_cast", x.data_ptr(), y.data_ptr(), B, min(t, T), max(t, T), H * U, int(pad), lib.stream_ptr())
+    return y
+
+
 def gated_rmsnorm_fwd(x, z, w, eps):
     M, D = x.shape
     y = torch.empty_like(x)

@@ -104,6 +104,9 @@ _SIGS = {
     "ob_ep_plan": [P, P, P, P, P, P, P, L, I, I, I, I, I, P],
     "ob_moe_fill": [P, P, P, I, I, P],
     "ob_moe_plan": [P, P, P, P, P, L, I, I, I, P],
+    "ob_gdn_rows_in": [P] * 10 + [I] * 6 + [F, F, P],
+    "ob_gdn_rows_in_bwd": [P] * 15 + [I] * 6 + [F, F, P],
+    "ob_gdn_rows_cast": [P, P, I, I, I, I, I, P],
     "ob_gdn_fwd": [P] * 13 + [I] * 8 + [P],
     "ob_gdn_bwd": [P] * 22 + [I] * 8 + [P],
     "ob_conv1d_silu_fwd": [P, P, P, I, I, I, I, P],

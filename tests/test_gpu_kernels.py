@@ -1192,6 +1192,38 @@ def test_gated_delta_rule_strong_decay_against_fp64_recurrence():
         assert ek < max(5e-4, 5 * er), (name, ek, er)
 
 
+@pytest.mark.parametrize("B,T,Hk,H,U", [(1, 1, 1, 1, 64), (2, 63, 2, 4, 128), (1, 64, 1, 3, 64), (3, 130, 16, 32, 128), (1, 200, 9, 9, 64)])
+def test_rows_into_the_delta_rule_and_out(B, T, Hk, H, U):
+    """Against the same from separate operations: fp32 between the same two roundings to bf16, so values differ by one bf16 step
+    (2^-8) at most, sums over the rows (fp32) by far less."""
+    from omegalax_b200.ops import functional as Fn, lib
+    torch.manual_seed(T)
+    dev, A = _dev(), 128
+    mixed = torch.randn(B, T, 2 * Hk * A + H * U, device=dev).to(bf16)
+    b, a = (2 * torch.randn(2, B * T, H, device=dev)).to(bf16)
+    a[0, 0] = 30.0      # past the line where softplus is its argument
+    neg_a, dt = -torch.rand(H, device=dev) * 4, torch.randn(H, device=dev)
+    dy = torch.randn(B, T, H, U, device=dev).to(bf16)
+
+    def run(fused):
+        m, bb, aa, na, d = (t.clone().requires_grad_() for t in (mixed, b, a, neg_a, dt))
+        if fused:
+            y = Fn.delta_rows(m, bb, aa, na, d, Hk, A, H, U)
+        else:
+            q, k, v = torch.split(m, [Hk * A, Hk * A, H * U], dim=-1)
+            g = (na * torch.nn.functional.softplus(aa.float() + d)).view(B, T, H)
+            y = Fn.gated_delta_rule(q.reshape(B, T, Hk, A), k.reshape(B, T, Hk, A), v.reshape(B, T, H, U), g,
+                                    torch.sigmoid(bb.float()).view(B, T, H))
+        y.backward(dy)
+        return [y.detach()] + [t.grad for t in (m, bb, aa, na, d)]
+
+    for name, got, want in zip(("y", "mixed", "b", "a", "neg_a", "dt"), run(True), run(False)):
+        assert got.dtype == want.dtype and got.shape == want.shape, name
+        err, size = float((got.double() - want.double()).norm()), float(want.double().norm())
+        assert err <= size * 2.0 ** -8, (name, err, size)
+    _check(lib)
+
+
 def test_gather_scatter_gelu_kernels():
     from omegalax_b200.ops import functional as Fn, reference as R, lib
     torch.manual_seed(2)
