@@ -307,14 +307,15 @@ __global__ void qknorm_rope_fwd_kernel(const bf16* __restrict__ qkv, const bf16*
   }
 }
 
-// Backward: dq_rot/dk_rot -> un-rotate -> per-head RMSNorm backward -> written into the
-// q and k slices of dqkv [M, (H+2G)*K]; dqw / dkw accumulate with fp32 atomics.
+// Backward: dq_rot/dk_rot -> un-rotate -> per-head RMSNorm backward -> the q and k slices of dqkv
+// [M, (H+2G)*K]; dqw / dkw accumulate with fp32 atomics.  v and gate slices: dv, dgate (null: zeros).
 template <bool kOnePlus>
 __global__ void qknorm_rope_bwd_kernel(const bf16* __restrict__ qkv, const bf16* __restrict__ qw,
                                        const bf16* __restrict__ kw, const float* __restrict__ cosT,
                                        const float* __restrict__ sinT,
                                        const bf16* __restrict__ dq_rot,
-                                       const bf16* __restrict__ dk_rot, bf16* __restrict__ dqkv,
+                                       const bf16* __restrict__ dk_rot, const bf16* __restrict__ dv,
+                                       const bf16* __restrict__ dgate, bf16* __restrict__ dqkv,
                                        float* __restrict__ dqw, float* __restrict__ dkw,
                                        long long M, int H, int G, int K, int rot, float eps,
                                        int q_in_stride_heads, int rows_per_block) {
@@ -323,21 +324,25 @@ __global__ void qknorm_rope_bwd_kernel(const bf16* __restrict__ qkv, const bf16*
   __syncthreads();
   const int lane = threadIdx.x & 31;
   const int warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
-  const int HG = H + G;
+  const int QH = H * q_in_stride_heads, HT = QH + 2 * G;
   const int half = rot >> 1;
-  const long long row_stride = (long long)H * K * q_in_stride_heads + 2ll * G * K;
   const long long m0 = (long long)blockIdx.x * rows_per_block;
   const long long m1 = min(M, m0 + rows_per_block);
-  for (long long item = m0 * HG + warp; item < m1 * HG; item += nwarps) {
-    const long long m = item / HG;
-    const int h = (int)(item - m * HG);
-    const bool is_q = h < H;
-    const long long in_off = is_q ? (long long)h * K * q_in_stride_heads
-                                  : (long long)H * K * q_in_stride_heads + (long long)(h - H) * K;
-    const bf16* src = qkv + m * row_stride + in_off;
+  for (long long item = m0 * HT + warp; item < m1 * HT; item += nwarps) {
+    const long long m = item / HT;
+    const int part = (int)(item - m * HT);
+    const bool is_q = part < QH;
+    const int h = is_q ? part / q_in_stride_heads : part - QH + H;
+    const bf16* src = qkv + item * K;
+    bf16* ddst = dqkv + item * K;
+    if (is_q ? part % q_in_stride_heads != 0 : part >= QH + G) {
+      const bf16* from = is_q ? dgate : dv;
+      if (from) from += (is_q ? m * H + h : m * G + (part - QH - G)) * K;
+      for (int i = lane; i < K; i += 32) ddst[i] = from ? from[i] : __float2bfloat16(0.f);
+      continue;
+    }
     const bf16* w = is_q ? qw : kw;
     const bf16* dsrc = is_q ? dq_rot + (m * H + h) * K : dk_rot + (m * G + (h - H)) * K;
-    bf16* ddst = dqkv + m * row_stride + in_off;
     float* dws = dw_sm + (is_q ? 0 : K);
     const float* cr = cosT + m * half;
     const float* sr = sinT + m * half;
@@ -403,105 +408,194 @@ __global__ void qknorm_rope_bwd_kernel(const bf16* __restrict__ qkv, const bf16*
     for (int i = threadIdx.x; i < K; i += blockDim.x) atomicAdd(dkw + i, dw_sm[K + i]);
 }
 
-// Fast path for head_dim 128 with full rotation (Qwen3 / Qwen3-VL text): every lane owns the
-// channel pairs (2l, 2l+1) and (64+2l, 65+2l), i.e. both partners of its rotations, so a head
-// is read once with 4-byte accesses, and the weight gradients are accumulated in registers over
-// all the (row, head) items a warp visits.
-__device__ __forceinline__ float bf16r(float x) { return __bfloat162float(__float2bfloat16(x)); }
-
-template <bool kOnePlus>
-__global__ void qknorm_rope_fwd128_kernel(const bf16* __restrict__ qkv, const bf16* __restrict__ qw,
-                                          const bf16* __restrict__ kw, const float* __restrict__ cosT,
-                                          const float* __restrict__ sinT, bf16* __restrict__ q_out,
-                                          bf16* __restrict__ k_out, long long M, int H, int G, float eps) {
-  constexpr int K = 128;
-  const int lane = threadIdx.x & 31;
-  const long long wid = (blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5;
-  const int HG = H + G;
-  if (wid >= M * HG) return;
-  const long long m = wid / HG;
-  const int h = (int)(wid - m * HG);
-  const bool is_q = h < H;
-  const bf16* src = qkv + m * (long long)(H + 2 * G) * K + (long long)h * K;
-  const bf16* w = is_q ? qw : kw;
-  bf16* dst = is_q ? q_out + (m * H + h) * K : k_out + (m * G + (h - H)) * K;
-  const float2 a = unpack_bf16(*reinterpret_cast<const uint32_t*>(src + 2 * lane));
-  const float2 b = unpack_bf16(*reinterpret_cast<const uint32_t*>(src + 64 + 2 * lane));
-  float ss = a.x * a.x + a.y * a.y + b.x * b.x + b.y * b.y;
-  ss = warp_sum(ss);
-  const float rstd = w ? rsqrtf(ss / (float)K + eps) : 1.f;
-  float2 wa = make_float2(1.f, 1.f), wb = wa;
-  if (w) {
-    wa = unpack_bf16(*reinterpret_cast<const uint32_t*>(w + 2 * lane));
-    wb = unpack_bf16(*reinterpret_cast<const uint32_t*>(w + 64 + 2 * lane));
-    if (kOnePlus) { wa.x += 1.f; wa.y += 1.f; wb.x += 1.f; wb.y += 1.f; }
+// The same for heads of 16 L channels, L = 4, 8, 16, rot % 16 == 0, everything on 16-byte boundaries: L lanes have a head, each
+// two vectors of eight channels.  The first rot / 16 of them hold both partners of their rotations (channels 8 j ... and rot / 2 + 8 j
+// ...), the others 16 that are not rotated, so every head is read once in 16-byte accesses.  Bound by HBM.  With 4-byte accesses, a
+// warp per head, and v and gate left to zero filling, copies and an addition (100 us more), in us from launch to end, L2 flushed, before
+// and now, forward and backward: 8192 rows, 32 heads on 8 of 128 76 and 104, 56 and 91; 3001 of 32 on 2 of 256, rot 64, with gates 64 and
+// 356, 42 and 104; 999 of 16 on 8 of 128 26 and 30, 19 and 22.
+struct HeadLane {
+  int a, b;         // first channels of the lane's vectors
+  bool turns;
+  __device__ __forceinline__ HeadLane(int j, int rot) : turns(16 * j < rot) {
+    a = turns ? 8 * j : 16 * j;
+    b = turns ? (rot >> 1) + 8 * j : a + 8;
   }
-  const float2 c = *reinterpret_cast<const float2*>(cosT + m * 64 + 2 * lane);
-  const float2 sn = *reinterpret_cast<const float2*>(sinT + m * 64 + 2 * lane);
-  const float x1a = bf16r(a.x * rstd * wa.x), x1b = bf16r(a.y * rstd * wa.y);
-  const float x2a = bf16r(b.x * rstd * wb.x), x2b = bf16r(b.y * rstd * wb.y);
-  *reinterpret_cast<uint32_t*>(dst + 2 * lane) = pack_bf16(x1a * c.x - x2a * sn.x, x1b * c.y - x2b * sn.y);
-  *reinterpret_cast<uint32_t*>(dst + 64 + 2 * lane) = pack_bf16(x2a * c.x + x1a * sn.x, x2b * c.y + x1b * sn.y);
+};
+__device__ __forceinline__ void unpack8(uint4 q, float* v) {
+  const uint32_t u[4] = {q.x, q.y, q.z, q.w};
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const float2 f = unpack_bf16(u[i]);
+    v[2 * i] = f.x;
+    v[2 * i + 1] = f.y;
+  }
+}
+__device__ __forceinline__ uint4 pack8(const float* v) {
+  return make_uint4(pack_bf16(v[0], v[1]), pack_bf16(v[2], v[3]), pack_bf16(v[4], v[5]), pack_bf16(v[6], v[7]));
+}
+template <int L>
+__device__ __forceinline__ float head_sum(float x) {
+#pragma unroll
+  for (int o = 1; o < L; o <<= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
+  return x;
+}
+__device__ __forceinline__ float bf16r(float x) { return __bfloat162float(__float2bfloat16(x)); }
+// weights (1 without one) and the row's cosines and sines of a lane
+template <bool kOnePlus>
+__device__ __forceinline__ void head_factors(const bf16* w, const float* cosT, const float* sinT, long long m, int rot, const HeadLane& h,
+                                             float* wa, float* wb, float* c, float* sn) {
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    wa[i] = wb[i] = c[i] = 1.f;
+    sn[i] = 0.f;
+  }
+  if (w) {
+    unpack8(*reinterpret_cast<const uint4*>(w + h.a), wa);
+    unpack8(*reinterpret_cast<const uint4*>(w + h.b), wb);
+    if (kOnePlus) {
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        wa[i] += 1.f;
+        wb[i] += 1.f;
+      }
+    }
+  }
+  if (h.turns) {
+    const float4 *cp = reinterpret_cast<const float4*>(cosT + m * (rot >> 1) + h.a), *sp = reinterpret_cast<const float4*>(sinT + m * (rot >> 1) + h.a);
+    const float4 c0 = cp[0], c1 = cp[1], s0 = sp[0], s1 = sp[1];
+    c[0] = c0.x; c[1] = c0.y; c[2] = c0.z; c[3] = c0.w; c[4] = c1.x; c[5] = c1.y; c[6] = c1.z; c[7] = c1.w;
+    sn[0] = s0.x; sn[1] = s0.y; sn[2] = s0.z; sn[3] = s0.w; sn[4] = s1.x; sn[5] = s1.y; sn[6] = s1.z; sn[7] = s1.w;
+  }
 }
 
-template <bool kOnePlus>
-__global__ void qknorm_rope_bwd128_kernel(const bf16* __restrict__ qkv, const bf16* __restrict__ qw,
-                                          const bf16* __restrict__ kw, const float* __restrict__ cosT,
-                                          const float* __restrict__ sinT, const bf16* __restrict__ dq_rot,
-                                          const bf16* __restrict__ dk_rot, bf16* __restrict__ dqkv,
-                                          float* __restrict__ dqw, float* __restrict__ dkw, long long M, int H,
-                                          int G, float eps) {
-  constexpr int K = 128;
-  __shared__ float red[8][2 * K];
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const long long nwarps = (long long)gridDim.x * (blockDim.x >> 5);
+template <int L, bool kOnePlus>
+__global__ void __launch_bounds__(256)
+qknorm_rope_fwd_vec_kernel(const bf16* __restrict__ qkv, const bf16* __restrict__ qw, const bf16* __restrict__ kw,
+                           const float* __restrict__ cosT, const float* __restrict__ sinT, bf16* __restrict__ q_out,
+                           bf16* __restrict__ k_out, long long M, int H, int G, int rot, float eps, int q_in_stride_heads) {
+  constexpr int K = 16 * L;
+  const HeadLane at(threadIdx.x % L, rot);
   const int HG = H + G;
-  const long long row_stride = (long long)(H + 2 * G) * K;
-  float gq[4] = {0.f, 0.f, 0.f, 0.f}, gk[4] = {0.f, 0.f, 0.f, 0.f};
-  for (long long item = blockIdx.x * (long long)(blockDim.x >> 5) + warp; item < M * HG; item += nwarps) {
-    const long long m = item / HG;
-    const int h = (int)(item - m * HG);
-    const bool is_q = h < H;
-    const bf16* src = qkv + m * row_stride + (long long)h * K;
-    const bf16* w = is_q ? qw : kw;
-    const bf16* dsrc = is_q ? dq_rot + (m * H + h) * K : dk_rot + (m * G + (h - H)) * K;
-    bf16* ddst = dqkv + m * row_stride + (long long)h * K;
-    const float2 a = unpack_bf16(*reinterpret_cast<const uint32_t*>(src + 2 * lane));
-    const float2 b = unpack_bf16(*reinterpret_cast<const uint32_t*>(src + 64 + 2 * lane));
-    const float2 da = unpack_bf16(*reinterpret_cast<const uint32_t*>(dsrc + 2 * lane));
-    const float2 db = unpack_bf16(*reinterpret_cast<const uint32_t*>(dsrc + 64 + 2 * lane));
-    const float2 c = *reinterpret_cast<const float2*>(cosT + m * 64 + 2 * lane);
-    const float2 sn = *reinterpret_cast<const float2*>(sinT + m * 64 + 2 * lane);
-    float ss = a.x * a.x + a.y * a.y + b.x * b.x + b.y * b.y;
-    ss = warp_sum(ss);
-    const float rstd = w ? rsqrtf(ss / (float)K + eps) : 1.f;
-    float2 wa = make_float2(1.f, 1.f), wb = wa;
-    if (w) {
-      wa = unpack_bf16(*reinterpret_cast<const uint32_t*>(w + 2 * lane));
-      wb = unpack_bf16(*reinterpret_cast<const uint32_t*>(w + 64 + 2 * lane));
-      if (kOnePlus) { wa.x += 1.f; wa.y += 1.f; wb.x += 1.f; wb.y += 1.f; }
-    }
-    // un-rotate: gradient w.r.t. the normalised, weighted values
-    const float n1a = da.x * c.x + db.x * sn.x, n1b = da.y * c.y + db.y * sn.y;
-    const float n2a = db.x * c.x - da.x * sn.x, n2b = db.y * c.y - da.y * sn.y;
-    if (w) {
-      float* gw = is_q ? gq : gk;
-      gw[0] = fmaf(n1a * a.x, rstd, gw[0]); gw[1] = fmaf(n1b * a.y, rstd, gw[1]);
-      gw[2] = fmaf(n2a * b.x, rstd, gw[2]); gw[3] = fmaf(n2b * b.y, rstd, gw[3]);
-    }
-    float dot = n1a * wa.x * a.x + n1b * wa.y * a.y + n2a * wb.x * b.x + n2b * wb.y * b.y;
-    dot = warp_sum(dot);
-    const float cc = w ? dot * rstd * rstd * rstd / (float)K : 0.f;
-    *reinterpret_cast<uint32_t*>(ddst + 2 * lane) = pack_bf16(n1a * wa.x * rstd - a.x * cc, n1b * wa.y * rstd - a.y * cc);
-    *reinterpret_cast<uint32_t*>(ddst + 64 + 2 * lane) = pack_bf16(n2a * wb.x * rstd - b.x * cc, n2b * wb.y * rstd - b.y * cc);
+  const long long item = (blockIdx.x * 256ll + threadIdx.x) / L;
+  const bool live = item < M * HG;      // the shuffles want every lane
+  const long long m = live ? item / HG : 0;
+  const int h = live ? (int)(item - m * HG) : 0;
+  const bool is_q = h < H;
+  const bf16* src = qkv + (m * ((long long)H * q_in_stride_heads + 2 * G) +
+                           (is_q ? (long long)h * q_in_stride_heads : (long long)H * q_in_stride_heads + h - H)) * K;
+  const bf16* w = is_q ? qw : kw;
+  float a[8], b[8], wa[8], wb[8], c[8], sn[8], ss = 0.f;
+  unpack8(*reinterpret_cast<const uint4*>(src + at.a), a);
+  unpack8(*reinterpret_cast<const uint4*>(src + at.b), b);
+  head_factors<kOnePlus>(w, cosT, sinT, m, rot, at, wa, wb, c, sn);
+#pragma unroll
+  for (int i = 0; i < 8; ++i) ss += a[i] * a[i] + b[i] * b[i];
+  ss = head_sum<L>(ss);
+  if (!live) return;
+  const float rstd = w ? rsqrtf(ss / (float)K + eps) : 1.f;
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    const float x1 = bf16r(a[i] * rstd * wa[i]), x2 = bf16r(b[i] * rstd * wb[i]);
+    a[i] = x1 * c[i] - x2 * sn[i];
+    b[i] = x2 * c[i] + x1 * sn[i];
   }
-  float* r = red[warp];
-  r[2 * lane] = gq[0]; r[2 * lane + 1] = gq[1]; r[64 + 2 * lane] = gq[2]; r[65 + 2 * lane] = gq[3];
-  r[K + 2 * lane] = gk[0]; r[K + 2 * lane + 1] = gk[1]; r[K + 64 + 2 * lane] = gk[2]; r[K + 65 + 2 * lane] = gk[3];
+  bf16* dst = is_q ? q_out + (m * H + h) * K : k_out + (m * G + (h - H)) * K;
+  *reinterpret_cast<uint4*>(dst + at.a) = pack8(a);
+  *reinterpret_cast<uint4*>(dst + at.b) = pack8(b);
+}
+
+// All heads of a row of dqkv: gate and v heads are copies of dgate [M,H,K] and dv [M,G,K] (null: zeros).
+template <int L, bool kOnePlus>
+__global__ void __launch_bounds__(256)
+qknorm_rope_bwd_vec_kernel(const bf16* __restrict__ qkv, const bf16* __restrict__ qw, const bf16* __restrict__ kw,
+                           const float* __restrict__ cosT, const float* __restrict__ sinT, const bf16* __restrict__ dq_rot,
+                           const bf16* __restrict__ dk_rot, const bf16* __restrict__ dv, const bf16* __restrict__ dgate,
+                           bf16* __restrict__ dqkv, float* __restrict__ dqw, float* __restrict__ dkw, long long M, int H, int G, int rot,
+                           float eps, int q_in_stride_heads) {
+  constexpr int K = 16 * L;
+  __shared__ float red[8][2 * K];
+  const HeadLane at(threadIdx.x % L, rot);
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int QH = H * q_in_stride_heads, HT = QH + 2 * G;
+  float gq[16] = {}, gk[16] = {};
+  const long long items = M * HT, step = gridDim.x * (256ll / L);
+  for (long long first = blockIdx.x * (256ll / L) + warp * (32 / L); first < items; first += step) {
+    const long long item = first + lane / L;
+    const bool live = item < items;
+    const long long m = live ? item / HT : 0;
+    const int h = live ? (int)(item - m * HT) : 0;
+    bf16* ddst = dqkv + (m * HT + h) * K;
+    const bool is_q = h < QH, norm = live && (is_q ? h % q_in_stride_heads == 0 : h < QH + G);
+    float ss = 0.f, dot = 0.f, rstd = 1.f, a[8], b[8], n1[8], n2[8], wa[8], wb[8];
+    const bf16* w = is_q ? qw : kw;
+    if (norm) {
+      const bf16* src = qkv + (m * HT + h) * K;
+      const bf16* dsrc = is_q ? dq_rot + (m * H + h / q_in_stride_heads) * K : dk_rot + (m * G + (h - QH)) * K;
+      float c[8], sn[8], da[8], db[8];
+      unpack8(*reinterpret_cast<const uint4*>(src + at.a), a);
+      unpack8(*reinterpret_cast<const uint4*>(src + at.b), b);
+      unpack8(*reinterpret_cast<const uint4*>(dsrc + at.a), da);
+      unpack8(*reinterpret_cast<const uint4*>(dsrc + at.b), db);
+      head_factors<kOnePlus>(w, cosT, sinT, m, rot, at, wa, wb, c, sn);
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {      // un-rotate: gradient of the normalised, weighted values
+        ss += a[i] * a[i] + b[i] * b[i];
+        n1[i] = da[i] * c[i] + db[i] * sn[i];
+        n2[i] = db[i] * c[i] - da[i] * sn[i];
+        dot += n1[i] * wa[i] * a[i] + n2[i] * wb[i] * b[i];
+      }
+    } else if (live) {
+      const bf16* from = is_q ? dgate : dv;
+      if (from) from += is_q ? (m * H + h / q_in_stride_heads) * K : (m * G + (h - QH - G)) * K;
+      const uint4 zero = make_uint4(0, 0, 0, 0);
+      *reinterpret_cast<uint4*>(ddst + at.a) = from ? *reinterpret_cast<const uint4*>(from + at.a) : zero;
+      *reinterpret_cast<uint4*>(ddst + at.b) = from ? *reinterpret_cast<const uint4*>(from + at.b) : zero;
+    }
+    ss = head_sum<L>(ss);
+    dot = head_sum<L>(dot);
+    if (!norm) continue;
+    if (w) {
+      rstd = rsqrtf(ss / (float)K + eps);
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        if (is_q) {
+          gq[i] = fmaf(n1[i] * a[i], rstd, gq[i]);
+          gq[8 + i] = fmaf(n2[i] * b[i], rstd, gq[8 + i]);
+        } else {
+          gk[i] = fmaf(n1[i] * a[i], rstd, gk[i]);
+          gk[8 + i] = fmaf(n2[i] * b[i], rstd, gk[8 + i]);
+        }
+      }
+    }
+    const float cc = w ? dot * rstd * rstd * rstd / (float)K : 0.f;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      n1[i] = n1[i] * wa[i] * rstd - a[i] * cc;
+      n2[i] = n2[i] * wb[i] * rstd - b[i] * cc;
+    }
+    *reinterpret_cast<uint4*>(ddst + at.a) = pack8(n1);
+    *reinterpret_cast<uint4*>(ddst + at.b) = pack8(n2);
+  }
+  __syncwarp();
+#pragma unroll
+  for (int i = 0; i < 16; ++i) {      // the heads of a warp
+#pragma unroll
+    for (int o = L; o < 32; o <<= 1) {
+      gq[i] += __shfl_xor_sync(0xffffffffu, gq[i], o);
+      gk[i] += __shfl_xor_sync(0xffffffffu, gk[i], o);
+    }
+    if (lane < L) {
+      const int ch = i < 8 ? at.a + i : at.b + i - 8;
+      red[warp][ch] = gq[i];
+      red[warp][K + ch] = gk[i];
+    }
+  }
   __syncthreads();
-  for (int i = threadIdx.x; i < 2 * K; i += blockDim.x) {
+  for (int i = threadIdx.x; i < 2 * K; i += 256) {
     float sacc = 0.f;
-    for (int wi = 0; wi < (int)(blockDim.x >> 5); ++wi) sacc += red[wi][i];
+#pragma unroll
+    for (int wi = 0; wi < 8; ++wi) sacc += red[wi][i];
     if (i < K) { if (qw && dqw) atomicAdd(dqw + i, sacc); }
     else if (kw && dkw) atomicAdd(dkw + i - K, sacc);
   }
@@ -1105,53 +1199,57 @@ int ob_swiglu_bwd(const void* gu, const void* dact, void* dgu, void* act_out, co
   return 0;
 }
 
+// Sizes and alignment of the vector kernels: their L, or 0.
+static int qknorm_lanes(int K, int rot, const void* const* ptrs, int n) {
+  uintptr_t any = 0;
+  for (int i = 0; i < n; ++i) any |= (uintptr_t)ptrs[i];
+  return (K == 64 || K == 128 || K == 256) && rot >= 0 && rot <= K && !(rot & 15) && !(any & 15) ? K / 16 : 0;
+}
+
 int ob_qknorm_rope_fwd(const void* qkv, const void* qw, const void* kw, const float* cosT,
                        const float* sinT, void* q_out, void* k_out, long long M, int H, int G,
                        int K, int rot, float eps, int one_plus, int q_stride_heads,
                        cudaStream_t s) {
   if (M <= 0) return 0;
-  long long warps = M * (H + G);
-  int threads = 256;
-  long long blocks = (warps * 32 + threads - 1) / threads;
-  if (K == 128 && rot == 128 && q_stride_heads == 1) {
-    if (one_plus)
-      qknorm_rope_fwd128_kernel<true><<<(unsigned)blocks, threads, 0, s>>>(
-          (const bf16*)qkv, (const bf16*)qw, (const bf16*)kw, cosT, sinT, (bf16*)q_out, (bf16*)k_out, M, H, G, eps);
-    else
-      qknorm_rope_fwd128_kernel<false><<<(unsigned)blocks, threads, 0, s>>>(
-          (const bf16*)qkv, (const bf16*)qw, (const bf16*)kw, cosT, sinT, (bf16*)q_out, (bf16*)k_out, M, H, G, eps);
-    OB_CHECK_LAUNCH();
-    return 0;
+  const void* ptrs[] = {qkv, qw, kw, cosT, sinT, q_out, k_out};
+  const int lanes = qknorm_lanes(K, rot, ptrs, 7);
+  const int threads = 256;
+#define OB_QKNORM_FWD(kern, blocks, ...)                                                                                       \
+  kern<<<(unsigned)(blocks), threads, 0, s>>>((const bf16*)qkv, (const bf16*)qw, (const bf16*)kw, cosT, sinT, (bf16*)q_out, \
+                                              (bf16*)k_out, M, H, G, __VA_ARGS__)
+#define OB_QKNORM_FWD_VEC(L)                                                                                                     \
+  if (lanes == L) {                                                                                                              \
+    const long long blocks = (M * (H + G) * L + threads - 1) / threads;                                                          \
+    if (one_plus) OB_QKNORM_FWD((qknorm_rope_fwd_vec_kernel<L, true>), blocks, rot, eps, q_stride_heads);                        \
+    else OB_QKNORM_FWD((qknorm_rope_fwd_vec_kernel<L, false>), blocks, rot, eps, q_stride_heads);                                \
   }
-  if (one_plus)
-    qknorm_rope_fwd_kernel<true><<<(unsigned)blocks, threads, 0, s>>>(
-        (const bf16*)qkv, (const bf16*)qw, (const bf16*)kw, cosT, sinT, (bf16*)q_out, (bf16*)k_out,
-        M, H, G, K, rot, eps, q_stride_heads);
-  else
-    qknorm_rope_fwd_kernel<false><<<(unsigned)blocks, threads, 0, s>>>(
-        (const bf16*)qkv, (const bf16*)qw, (const bf16*)kw, cosT, sinT, (bf16*)q_out, (bf16*)k_out,
-        M, H, G, K, rot, eps, q_stride_heads);
+  OB_QKNORM_FWD_VEC(4) else OB_QKNORM_FWD_VEC(8) else OB_QKNORM_FWD_VEC(16) else {
+    const long long blocks = (M * (H + G) * 32 + threads - 1) / threads;
+    if (one_plus) OB_QKNORM_FWD(qknorm_rope_fwd_kernel<true>, blocks, K, rot, eps, q_stride_heads);
+    else OB_QKNORM_FWD(qknorm_rope_fwd_kernel<false>, blocks, K, rot, eps, q_stride_heads);
+  }
   OB_CHECK_LAUNCH();
   return 0;
 }
 
+// dqkv of all heads; dv [M,G,K] and dgate [M,H,K] (q_stride_heads 2) are copied to their places, null: zeros.
 int ob_qknorm_rope_bwd(const void* qkv, const void* qw, const void* kw, const float* cosT,
-                       const float* sinT, const void* dq_rot, const void* dk_rot, void* dqkv,
+                       const float* sinT, const void* dq_rot, const void* dk_rot, const void* dv, const void* dgate, void* dqkv,
                        float* dqw, float* dkw, long long M, int H, int G, int K, int rot,
                        float eps, int one_plus, int q_stride_heads, cudaStream_t s) {
   if (M <= 0) return 0;
   const int threads = 256;
-  if (K == 128 && rot == 128 && q_stride_heads == 1) {
-    long long want = (M * (H + G) + 7) / 8;
-    const unsigned nb = (unsigned)(want < (long long)num_sms() * 8 ? want : (long long)num_sms() * 8);
-    if (one_plus)
-      qknorm_rope_bwd128_kernel<true><<<nb, threads, 0, s>>>(
-          (const bf16*)qkv, (const bf16*)qw, (const bf16*)kw, cosT, sinT, (const bf16*)dq_rot, (const bf16*)dk_rot,
-          (bf16*)dqkv, dqw, dkw, M, H, G, eps);
-    else
-      qknorm_rope_bwd128_kernel<false><<<nb, threads, 0, s>>>(
-          (const bf16*)qkv, (const bf16*)qw, (const bf16*)kw, cosT, sinT, (const bf16*)dq_rot, (const bf16*)dk_rot,
-          (bf16*)dqkv, dqw, dkw, M, H, G, eps);
+  const void* ptrs[] = {qkv, qw, kw, cosT, sinT, dq_rot, dk_rot, dv, dgate, dqkv};
+  const int lanes = qknorm_lanes(K, rot, ptrs, 10);
+#define OB_QKNORM_BWD_VEC(L, P)                                                                                                    \
+  qknorm_rope_bwd_vec_kernel<L, P><<<(unsigned)min(((long long)M * (H * q_stride_heads + 2 * G) * L + 255) / 256, (long long)num_sms() * 8), \
+                                     threads, 0, s>>>((const bf16*)qkv, (const bf16*)qw, (const bf16*)kw, cosT, sinT,           \
+                                                      (const bf16*)dq_rot, (const bf16*)dk_rot, (const bf16*)dv, (const bf16*)dgate, \
+                                                      (bf16*)dqkv, dqw, dkw, M, H, G, rot, eps, q_stride_heads)
+  if (lanes == 4) { if (one_plus) OB_QKNORM_BWD_VEC(4, true); else OB_QKNORM_BWD_VEC(4, false); }
+  else if (lanes == 8) { if (one_plus) OB_QKNORM_BWD_VEC(8, true); else OB_QKNORM_BWD_VEC(8, false); }
+  else if (lanes == 16) { if (one_plus) OB_QKNORM_BWD_VEC(16, true); else OB_QKNORM_BWD_VEC(16, false); }
+  if (lanes) {
     OB_CHECK_LAUNCH();
     return 0;
   }
@@ -1161,12 +1259,12 @@ int ob_qknorm_rope_bwd(const void* qkv, const void* qw, const void* kw, const fl
   if (one_plus)
     qknorm_rope_bwd_kernel<true><<<(unsigned)blocks, threads, sm, s>>>(
         (const bf16*)qkv, (const bf16*)qw, (const bf16*)kw, cosT, sinT, (const bf16*)dq_rot,
-        (const bf16*)dk_rot, (bf16*)dqkv, dqw, dkw, M, H, G, K, rot, eps, q_stride_heads,
+        (const bf16*)dk_rot, (const bf16*)dv, (const bf16*)dgate, (bf16*)dqkv, dqw, dkw, M, H, G, K, rot, eps, q_stride_heads,
         rows_per_block);
   else
     qknorm_rope_bwd_kernel<false><<<(unsigned)blocks, threads, sm, s>>>(
         (const bf16*)qkv, (const bf16*)qw, (const bf16*)kw, cosT, sinT, (const bf16*)dq_rot,
-        (const bf16*)dk_rot, (bf16*)dqkv, dqw, dkw, M, H, G, K, rot, eps, q_stride_heads,
+        (const bf16*)dk_rot, (const bf16*)dv, (const bf16*)dgate, (bf16*)dqkv, dqw, dkw, M, H, G, K, rot, eps, q_stride_heads,
         rows_per_block);
   OB_CHECK_LAUNCH();
   return 0;

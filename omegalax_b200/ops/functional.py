@@ -496,22 +496,34 @@ def embedding(ids, table):
 
 
 # ----------------------------------------------------------------------------- qk-norm + rope
+def _value_and_gate(qkv, H: int, G: int, Kd: int, q_stride_heads: int):
+    M, width = qkv.shape[0], H * Kd * q_stride_heads
+    gate = qkv[:, :width].view(M, H, 2, Kd)[:, :, 1] if q_stride_heads == 2 else None
+    return qkv[:, width + G * Kd:].view(M, G, Kd), gate
+
+
 class _QKNormRopeFn(torch.autograd.Function):
+    """q, k, v and the gates (or None) of a fused projection; v and the gates are views of it, and belong to the node so that its
+    backward writes the whole gradient in one pass."""
+
     @staticmethod
     def forward(ctx, qkv, qw, kw, cos, sin, H, G, Kd, rot, eps, one_plus, q_stride_heads):
         q, k = K.qknorm_rope_fwd(qkv, qw, kw, cos, sin, H, G, Kd, rot, eps, one_plus, q_stride_heads)
         ctx.save_for_backward(qkv, qw, kw, cos, sin)
         ctx.cfg = (H, G, Kd, rot, eps, one_plus, q_stride_heads)
         ctx.qw_ref, ctx.kw_ref = qw, kw
-        return q, k
+        ctx.set_materialize_grads(False)
+        return q, k, *_value_and_gate(qkv, H, G, Kd, q_stride_heads)
 
     @staticmethod
-    def backward(ctx, dq, dk):
+    def backward(ctx, dq, dk, dv, dgate):
         qkv, qw, kw, cos, sin = ctx.saved_tensors
         H, G, Kd, rot, eps, one_plus, qs = ctx.cfg
-        dqkv = torch.zeros_like(qkv) if qs != 1 else torch.empty_like(qkv)
-        if qs == 1:
-            dqkv.view(qkv.shape[0], H + 2 * G, Kd)[:, H + G:].zero_()
+        M = qkv.shape[0]
+        dq = qkv.new_zeros(M, H, Kd) if dq is None else dq.contiguous()
+        dk = qkv.new_zeros(M, G, Kd) if dk is None else dk.contiguous()
+        dv, dgate = (None if t is None else t.contiguous() for t in (dv, dgate))
+        dqkv = torch.empty_like(qkv, memory_format=torch.contiguous_format)
         dqw = dkw = None
         qmg = getattr(ctx.qw_ref, "main_grad", None) if qw is not None else None
         kmg = getattr(ctx.kw_ref, "main_grad", None) if kw is not None else None
@@ -520,8 +532,7 @@ class _QKNormRopeFn(torch.autograd.Function):
             dkw_buf = kmg if kmg is not None else torch.zeros(Kd, dtype=torch.float32, device=qkv.device)
         else:
             dqw_buf = dkw_buf = None
-        K.qknorm_rope_bwd(qkv, qw, kw, cos, sin, dq.contiguous(), dk.contiguous(), dqkv, dqw_buf,
-                          dkw_buf, H, G, Kd, rot, eps, one_plus, qs)
+        K.qknorm_rope_bwd(qkv, qw, kw, cos, sin, dq, dk, dqkv, dqw_buf, dkw_buf, H, G, Kd, rot, eps, one_plus, qs, dv, dgate)
         if qw is not None and qmg is None:
             dqw = dqw_buf.to(qw.dtype)
         if kw is not None and kmg is None:
@@ -542,14 +553,9 @@ def qk_norm_rope(qkv, qw, kw, sin, cos, H: int, G: int, Kd: int, rot: int | None
     rot = Kd if rot is None else rot
     M = qkv.shape[0]
     qw_total = H * Kd * q_stride_heads
-    v = qkv[:, qw_total + G * Kd:].view(M, G, Kd)
-    gate = None
-    if q_stride_heads == 2:
-        gate = qkv[:, :qw_total].view(M, H, 2, Kd)[:, :, 1]
     if use_kernels(qkv) and (qw is None or qw.dtype == bf16):
-        q, k = _QKNormRopeFn.apply(qkv, qw, kw, cos.contiguous(), sin.contiguous(), H, G, Kd, rot,
-                                   eps, one_plus, q_stride_heads)
-        return q, k, v, gate
+        return _QKNormRopeFn.apply(qkv, qw, kw, cos.contiguous(), sin.contiguous(), H, G, Kd, rot, eps, one_plus, q_stride_heads)
+    v, gate = _value_and_gate(qkv, H, G, Kd, q_stride_heads)
     if q_stride_heads == 2:
         q = qkv[:, :qw_total].view(M, H, 2, Kd)[:, :, 0]
     else:

@@ -333,10 +333,11 @@ def qknorm_rope_fwd(qkv, qw, kw, cos, sin, H, G, K, rot, eps, one_plus=False, q_
 
 
 def qknorm_rope_bwd(qkv, qw, kw, cos, sin, dq, dk, dqkv, dqw, dkw, H, G, K, rot, eps,
-                    one_plus=False, q_stride_heads=1):
+                    one_plus=False, q_stride_heads=1, dv=None, dgate=None):
+    """All of dqkv: its v and gate heads are ``dv`` and ``dgate`` (zeros without)."""
     M = qkv.shape[0]
     _call("ob_qknorm_rope_bwd", qkv.data_ptr(), lib.ptr(qw), lib.ptr(kw), cos.data_ptr(),
-          sin.data_ptr(), dq.data_ptr(), dk.data_ptr(), dqkv.data_ptr(), lib.ptr(dqw),
+          sin.data_ptr(), dq.data_ptr(), dk.data_ptr(), lib.ptr(dv), lib.ptr(dgate), dqkv.data_ptr(), lib.ptr(dqw),
           lib.ptr(dkw), M, H, G, K, rot, float(eps), int(one_plus), q_stride_heads,
           lib.stream_ptr())
 

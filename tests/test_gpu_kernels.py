@@ -481,6 +481,45 @@ def test_qknorm_rope(Kd, rot, qs):
     assert _rel_err(qw.grad, qw_r.grad) < 3e-2 and _rel_err(kw.grad, kw_r.grad) < 3e-2
 
 
+@pytest.mark.parametrize("M,H,G,Kd,rot,qs,weights", [
+    (1, 1, 1, 64, 64, 1, False), (7, 3, 1, 64, 32, 1, True), (37, 5, 2, 128, 128, 1, True), (600, 16, 2, 128, 64, 2, True),
+    (33, 3, 1, 256, 64, 2, True), (9, 2, 2, 256, 0, 1, True), (11, 3, 1, 96, 96, 1, True), (5, 2, 1, 128, 24, 2, True)])
+@pytest.mark.parametrize("unused", [False, True])
+def test_qknorm_rope_gradient_of_the_whole_projection(M, H, G, Kd, rot, qs, weights, unused):
+    """Forward against fp32, one rounding (2^-8) before the rotation, whose terms have size four, and one behind it; v and gate gradients are the
+    same bits, or zeros where nobody used them; q and k gradients, of size four, one rounding; weight gradients fp32 sums of M heads."""
+    from omegalax_b200.ops import functional as Fn, reference as R, lib
+    torch.manual_seed(M)
+    dev = _dev()
+    qkv = torch.randn(M, (H * qs + 2 * G) * Kd, device=dev).to(bf16).requires_grad_()
+    ws = [(1 + 0.1 * torch.randn(Kd, device=dev)).to(bf16).requires_grad_() for _ in range(2)] if weights else [None, None]
+    sin, cos = R.rope_tables(torch.arange(M, device=dev), rot, 1e4) if rot else (torch.zeros(M, 0, device=dev),) * 2
+    outs = [t for t in Fn.qk_norm_rope(qkv, *ws, sin, cos, H, G, Kd, rot=rot, one_plus=qs == 2, q_stride_heads=qs) if t is not None]
+    grads = [torch.randn(t.shape, device=dev).to(bf16) for t in outs]
+    n = 2 if unused else len(outs)
+    torch.autograd.backward(outs[:n], grads[:n])
+    _check(lib)
+    ref, wr = qkv.detach().double().requires_grad_(), [None if w is None else w.detach().double().requires_grad_() for w in ws]
+    if rot:
+        want = [t for t in Fn.qk_norm_rope(ref, *wr, sin.double(), cos.double(), H, G, Kd, rot=rot, one_plus=qs == 2, q_stride_heads=qs)
+                if t is not None]
+    else:
+        heads = ref.view(M, -1, Kd)
+        want = [R.rmsnorm(heads[:, :H], wr[0], 1e-6, False), R.rmsnorm(heads[:, H:H + G], wr[1], 1e-6, False)]
+    torch.autograd.backward(want[:2], [g.double() for g in grads[:2]])
+    for got, t in zip(outs[:2], want):
+        assert float((got.double() - t).norm()) <= float(t.norm()) * 2.0 ** -7
+    dq, whole = qkv.grad.view(M, -1, Kd), ref.grad.view(M, -1, Kd)
+    normed = [h for h in range(H * qs + G) if h >= H * qs or h % qs == 0]
+    assert float((dq[:, normed].double() - whole[:, normed]).norm()) <= float(whole[:, normed].norm()) * 2.0 ** -8
+    copies = [dq[:, H * qs + G:]] + ([dq[:, 1:H * qs:2]] if qs == 2 else [])
+    for got, g in zip(copies, grads[2:]):
+        assert torch.equal(got, torch.zeros_like(g) if unused else g)
+    for w, r in zip(ws, wr):
+        if w is not None:
+            assert float((w.grad.double() - r.grad).norm()) <= float(r.grad.norm()) * 2.0 ** -7
+
+
 @pytest.mark.parametrize("HD", [128, 64])
 @pytest.mark.parametrize("causal", [True, False])
 @pytest.mark.parametrize("T", [128, 384, 1000])
