@@ -81,8 +81,16 @@ class VisionAttention(nn.Module):
 
     @scoped("vision_attention")
     def forward(self, x, cos, sin, cu_seqlens, max_seqlen: int):
-        N = x.shape[0]
-        qkv = self.qkv(x).view(N, 3, self.H, self.Kd)
+        """``cos``, ``sin`` [N, head_dim], or their first halves (the second ones are the same)."""
+        N, half = x.shape[0], self.Kd // 2
+        qkv = self.qkv(x)
+        if Fn.use_kernels(qkv) and self.Kd in (64, 128, 256):
+            q, k, v, _ = Fn.qk_norm_rope(qkv, None, None, sin[:, :half], cos[:, :half], self.H, self.H, self.Kd)
+            o = Fn.flash_attention(q, k, v, cu_seqlens, max_seqlen, scale=self.scale, causal=False)
+            return self.proj(o.reshape(N, self.H * self.Kd))
+        if cos.shape[-1] == half:
+            cos, sin = torch.cat([cos, cos], dim=-1), torch.cat([sin, sin], dim=-1)
+        qkv = qkv.view(N, 3, self.H, self.Kd)
         q = apply_vision_rope(qkv[:, 0], cos, sin).contiguous()
         k = apply_vision_rope(qkv[:, 1], cos, sin).contiguous()
         v = qkv[:, 2].contiguous()
@@ -189,6 +197,8 @@ class VisionTower(nn.Module):
         x = self.patch_embed(pixel_values.to(self.pos_embed.dtype))
         x = x + self.interpolated_pos_embed(grid, dev).to(x.dtype)
         cos, sin = self.rotary(grid, dev)
+        if Fn.use_kernels(x):      # once for all blocks, for kernels that read half a head's angles
+            cos, sin = (t[:, :t.shape[1] // 2].contiguous() for t in (cos, sin))
         if cu_seqlens is None:
             cu_seqlens = vision_cu_seqlens(grid, dev)
         max_len = max(h * w for _, h, w in grid)

@@ -153,6 +153,31 @@ def _few(w):
     return False if hasattr(w, "main_grad") else None
 
 
+def _column_sum(x):
+    if use_kernels(x) and x.is_contiguous() and x.shape[1] % 8 == 0 and x.data_ptr() % 16 == 0 and x.numel():
+        return K.column_sum(x)
+    return x.sum(0)
+
+
+class _ColumnMeanFn(torch.autograd.Function):
+    @staticmethod
+    def forward(ctx, x):
+        ctx.rows = x.shape[0]
+        return K.column_sum(x, 1.0 / x.shape[0])
+
+    @staticmethod
+    def backward(ctx, d):
+        return (d / ctx.rows).expand(ctx.rows, -1)
+
+
+def column_mean(x):
+    """x.mean(0) of fp32 rows."""
+    if (x.is_cuda and x.dtype == torch.float32 and x.dim() == 2 and x.numel() and x.shape[1] % 8 == 0 and x.data_ptr() % 16 == 0
+            and os.environ.get("OMEGALAX_B200_REFERENCE_OPS") != "1" and not library_mode()):
+        return _ColumnMeanFn.apply(x.contiguous())
+    return x.mean(0)
+
+
 class _LinearFn(torch.autograd.Function):
     @staticmethod
     def forward(ctx, x, w, residual, y_pre=None, bias=None):
@@ -191,7 +216,7 @@ class _LinearFn(torch.autograd.Function):
                 lambda mg: K.gemm(dy2, x2, a_mn=True, b_mn=True, out=mg, accumulate=True),
                 lambda: K.gemm(dy2, x2, a_mn=True, b_mn=True),
             )
-        db = dy2.sum(0) if (ctx.has_bias and ctx.needs_input_grad[4]) else None
+        db = _column_sum(dy2) if (ctx.has_bias and ctx.needs_input_grad[4]) else None
         return dx, dw, (dy if ctx.has_res else None), None, db
 
 

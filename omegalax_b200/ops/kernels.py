@@ -322,6 +322,14 @@ def swiglu_bwd(gu, dact, with_act: bool = False, inplace: bool = False, rows=Non
     return (dgu.view(gu.shape), act) if with_act else dgu.view(gu.shape)
 
 
+def column_sum(x, scale: float = 1.0):
+    """scale * x.sum(0) of a contiguous bf16 or fp32 matrix with a multiple of eight columns; fp32 sums."""
+    M, N = x.shape
+    out = torch.empty(N, dtype=x.dtype, device=x.device)
+    _call("ob_column_sum", x.data_ptr(), out.data_ptr(), M, N, int(x.dtype == bf16), float(scale), lib.stream_ptr())
+    return out
+
+
 def qknorm_rope_fwd(qkv, qw, kw, cos, sin, H, G, K, rot, eps, one_plus=False, q_stride_heads=1):
     M = qkv.shape[0]
     q = torch.empty(M, H, K, dtype=qkv.dtype, device=qkv.device)

@@ -115,6 +115,7 @@ _SIGS = {
     "ob_rmsnorm_bwd": [P, P, P, P, P, P, L, I, F, I, P],
     "ob_swiglu_fwd": [P, P, P, L, I, P],
     "ob_swiglu_bwd": [P, P, P, P, P, L, I, P],
+    "ob_column_sum": [P, P, L, I, I, F, P],
     "ob_qknorm_rope_fwd": [P, P, P, P, P, P, P, L, I, I, I, I, F, I, I, P],
     "ob_qknorm_rope_bwd": [P, P, P, P, P, P, P, P, P, P, P, P, L, I, I, I, I, F, I, I, P],
     "ob_ce_fwd_bwd": [P, L, L, I, P, P, P, P, P, I, P],

@@ -84,7 +84,7 @@ def load_balance_loss_qwen3(probs, idx, num_experts: int, coef: float, group=Non
     counts = torch.zeros(num_experts, dtype=torch.float32, device=probs.device)
     counts.scatter_add_(0, idx.reshape(-1), torch.ones(idx.numel(), dtype=torch.float32, device=probs.device))
     if group is None or coef == 0.0:
-        return coef * num_experts * torch.sum((counts / M) * probs.mean(0))
+        return coef * num_experts * torch.sum((counts / M) * Fn.column_mean(probs))
     stats, W = _global_sum(torch.cat([counts, probs.float().sum(0)]), group)
     counts_g, psum_g = stats[:num_experts].detach(), stats[num_experts:]
     return coef * num_experts * torch.sum((counts_g / (M * W)) * (psum_g / (M * W)))
@@ -94,7 +94,7 @@ def load_balance_loss_sq(probs, num_experts: int, coef: float, group=None):
     """coef * sum_e (mean prob of e - 1/E)^2 (omegalax/models/qwen3_5/model.py:172-174); with
     ``group`` the mean is over the tokens of every data rank."""
     if group is None or coef == 0.0:
-        return coef * torch.sum((probs.mean(0) - 1.0 / num_experts) ** 2)
+        return coef * torch.sum((Fn.column_mean(probs) - 1.0 / num_experts) ** 2)
     psum_g, W = _global_sum(probs.float().sum(0), group)
     return coef * torch.sum((psum_g / (probs.shape[0] * W) - 1.0 / num_experts) ** 2)
 

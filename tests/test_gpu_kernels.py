@@ -481,6 +481,22 @@ def test_qknorm_rope(Kd, rot, qs):
     assert _rel_err(qw.grad, qw_r.grad) < 3e-2 and _rel_err(kw.grad, kw_r.grad) < 3e-2
 
 
+@pytest.mark.parametrize("M,N", [(1, 8), (31, 72), (129, 64), (1000, 32), (3136, 1024), (5000, 4096)])
+def test_column_sum(M, N):
+    """fp32 sums of M values of size one: M roundings of 2^-24 of the sum of sizes, one of the result; the mean's gradient."""
+    from omegalax_b200.ops import functional as Fn, kernels as Kn, lib
+    torch.manual_seed(M)
+    x = torch.randn(M, N, device=_dev())
+    for t, step in ((x, 2.0 ** -24), (x.to(bf16), 2.0 ** -8)):
+        got, want, size = Kn.column_sum(t, 0.5).double(), 0.5 * t.double().sum(0), 0.5 * t.double().abs().sum(0)
+        assert bool(((got - want).abs() <= size * M * 2.0 ** -24 + want.abs() * step).all())
+        assert torch.equal(Kn.column_sum(t), Kn.column_sum(t))
+    y = x.clone().requires_grad_()
+    Fn.column_mean(y).square().sum().backward()
+    torch.testing.assert_close(y.grad, (2 * x.mean(0) / M).expand(M, -1), rtol=1e-4, atol=1e-6 / M)
+    _check(lib)
+
+
 @pytest.mark.parametrize("M,H,G,Kd,rot,qs,weights", [
     (1, 1, 1, 64, 64, 1, False), (7, 3, 1, 64, 32, 1, True), (37, 5, 2, 128, 128, 1, True), (600, 16, 2, 128, 64, 2, True),
     (33, 3, 1, 256, 64, 2, True), (9, 2, 2, 256, 0, 1, True), (11, 3, 1, 96, 96, 1, True), (5, 2, 1, 128, 24, 2, True)])
