@@ -25,7 +25,7 @@ class SquaredReluMLP(nn.Module):
         self.down = Projection(cfg.ff, width, device=device, dtype=dtype)
 
     def forward(self, h, x):
-        self.down(S.relu_squared(self.up(h).contiguous()), into=x)
+        self.down(self.up.relu_squared(h), into=x)
 
 
 @dataclasses.dataclass(frozen=True)

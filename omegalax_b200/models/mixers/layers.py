@@ -5,6 +5,7 @@ import math
 
 import torch
 from torch import nn
+from torch.nn.modules import module as _module_hooks
 
 from ...ops import serving as S
 
@@ -23,6 +24,18 @@ class Projection(nn.Module):
 
     def forward(self, x, out_dtype=None, into=None):
         return S.project(x, self.weight, out_dtype=out_dtype, into=into)
+
+    def relu_squared(self, x):
+        """max(., 0)^2 of the product, in one launch where nothing wants to see the call of the module."""
+        if not (type(self).forward is not _PROJECT or "forward" in self.__dict__ or self._forward_hooks or self._forward_pre_hooks
+                or _module_hooks._global_forward_hooks or _module_hooks._global_forward_pre_hooks):
+            y = S.project_relu_squared(x, self.weight)
+            if y is not None:
+                return y
+        return S.relu_squared(self(x).contiguous())
+
+
+_PROJECT = Projection.forward
 
 
 class LayerNorm(nn.Module):

@@ -27,6 +27,7 @@ struct GemmArgs {
   const bf16* residual;
   long long ldr;
   const bf16* bias;          // optional [N]: added to every row before the store (bf16 / fp32 store modes)
+  int squares;               // 512 x 256 tile kernel, bf16 output: C = max(., 0)^2 of the product rounded to bf16
   // Cross-entropy statistics (512 x 256 tile kernel, bf16 output): for every row and every
   // 256-column tile the maximum of the fp32 logits and the sum of exp(logit - maximum) go to
   // ce_stats[row * num_n_blocks + tile] and the fp32 logit of the row's target column to

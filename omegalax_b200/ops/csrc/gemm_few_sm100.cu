@@ -34,7 +34,7 @@ struct FewArgs {
   float* squares_out;      // or null: the same of C
   long long ldx;
   float eps;
-  int act;                 // W is [gate | up]: C = silu(gate) * up, N / 2 columns
+  int act;                 // 1: W is [gate | up], C = silu(gate) * up, N / 2 columns; 2: C = max(., 0)^2
 };
 
 template <int NB>
@@ -137,7 +137,7 @@ gemm_few_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int splits = (int)gridDim.x, rank = (int)blockIdx.x;    // the cluster spans the x dimension
-  const int n0 = blockIdx.y * (p.act ? 64 : 128), m0 = blockIdx.z * NB;
+  const int n0 = blockIdx.y * (p.act == 1 ? 64 : 128), m0 = blockIdx.z * NB;
   if (threadIdx.x == 0) {
     tma_prefetch_desc(&tmW);
     tma_prefetch_desc(&tmX);
@@ -168,7 +168,7 @@ gemm_few_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__
         uint8_t* sw = smem + stage * L::kStageBytes;
         mbar_expect_tx(&full_bar[stage], kNorm ? L::kABytes : L::kStageBytes);
         tma_load_2d(sw, &tmW, &full_bar[stage], k0, n0);
-        if (p.act) tma_load_2d(sw + L::kABytes / 2, &tmW, &full_bar[stage], k0, p.N / 2 + n0);
+        if (p.act == 1) tma_load_2d(sw + L::kABytes / 2, &tmW, &full_bar[stage], k0, p.N / 2 + n0);
       };
       // the weights of the first stages are on their way while the kernel before, which gives X, still runs
       const int ahead = min(kSt, (k_end - k_begin + BK - 1) / BK);
@@ -251,7 +251,7 @@ gemm_few_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__
       }
       float v[4] = {s.x, s.y, s.z, s.w};
       const long long row = m0 + m;
-      if (p.act) {      // lanes 0..15 gate, 16..31 up, rounded as products of their own would be
+      if (p.act == 1) {      // lanes 0..15 gate, 16..31 up, rounded as products of their own would be
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
           v[i] = __bfloat162float(__float2bfloat16(v[i]));
@@ -263,6 +263,13 @@ gemm_few_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__
         continue;
       }
       if (ncol <= 0) continue;
+      if (p.act == 2) {
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          v[i] = fmaxf(__bfloat162float(__float2bfloat16(v[i])), 0.f);
+          v[i] *= v[i];
+        }
+      }
       if (p.bias) {
 #pragma unroll
         for (int i = 0; i < 4; ++i) if (i < ncol) v[i] += __bfloat162float(p.bias[col + i]);
@@ -331,7 +338,7 @@ static int launch_few(const void* X, const void* W, FewArgs a, long long ldx, lo
   CUtensorMap tmW, tmX;
   int e = make_tmap_2d(&tmX, X, a.M, a.K, ldx, NB, BK);
   if (e) return 2000 + e;
-  e = make_tmap_2d(&tmW, W, a.N, a.K, ldw, a.act ? 64 : 128, BK);
+  e = make_tmap_2d(&tmW, W, a.N, a.K, ldw, a.act == 1 ? 64 : 128, BK);
   if (e) return 3000 + e;
   auto kern = gemm_few_kernel<NB, kNorm>;
   OB_ENSURE_DYN_SMEM(kern, FewSmem<NB>::kTotal);
@@ -391,8 +398,8 @@ int ob_gemm_few(const void* X, const void* W, void* C, const void* residual, int
 // where every kernel waits for the one before: 8 layers of 4096 channels, one sequence of 4096 tokens 1001 -> 957 us, 32 of 2048
 // 1440 -> 1412; a norm and its product of N 24576, 32 rows, with the activation 42.5 -> 40.0, the product alone 37.6).
 // norm_w with squares [M, K / 128] (sums of squares of X by panels of 128 columns; eps): X passes an RMS norm on its way, M <= 32.
-// squares_out [M, N / 128] or null: the same sums of C as stored.  act: W is [gate | up], C [M, N / 2] = silu(gate) * up of
-// the rounded products.  Rounding and order are those of ob_rmsnorm_fwd and ob_swiglu_fwd but for the order of a sum of squares.
+// squares_out [M, N / 128] or null: the same sums of C as stored.  act 1: W is [gate | up], C [M, N / 2] = silu(gate) * up of
+// the rounded products; 2: C = max(., 0)^2 of them.  Rounding and order are those of ob_rmsnorm_fwd and ob_swiglu_fwd but for the order of a sum of squares.
 int ob_gemm_step(const void* X, const void* W, void* C, const void* residual, int M, int N, int K, long long ldx, long long ldw,
                  long long ldc, long long ldr, const void* norm_w, const float* squares, float eps, float* squares_out, int act,
                  int* status, cudaStream_t stream) {
@@ -410,7 +417,7 @@ int ob_gemm_step(const void* X, const void* W, void* C, const void* residual, in
   a.squares_out = squares_out;
   a.act = act;
   a.status = status;
-  if (act && ((N & 127) || residual || squares_out || !a.vec)) return 6005;
+  if (act < 0 || act > 2 || (act && (residual || squares_out)) || (act == 1 && ((N & 127) || !a.vec))) return 6005;
   if (squares_out && (N & 127)) return 6005;
   if (norm_w) {
     if (M > 32 || !squares || (K & 127) || ((uintptr_t)norm_w & 15)) return 6005;

@@ -570,6 +570,30 @@ int ob_gemm_bf16_pair(const void* A, const void* B, void* C, const void* residua
   return launch_pair<true, false>(A, B, g, a_rows, a_cols, lda, b_rows, b_cols, ldb, stream);
 }
 
+// Whether ob_gemm_relu_sq covers a product: where ob_gemm_bf16_pair would take the 512 x 256 tiles.
+int ob_gemm_relu_sq_fits(int M, int N, int K) {
+  GemmArgs g = {};
+  g.M = M; g.N = N; g.K = K;
+  return M > 0 && N > 0 && K > 0 && !(K & 7) && !(N & 7) && want_wide(g);
+}
+
+// C [M,N] = max(X W^T, 0)^2, bf16, X [M,K], W [N,K]: the bits of the product and of ob_relu_sq after it, without the way through
+// memory in between (in us, two launches and one: 4096 x 12288, K 2048
+// 187 150; 8192 x 18432, K 4096 1091 900; 16 rows, on the kernel for few, 38.9 35.0).  SwiGLU gains nothing this way: its exponentials hold up the
+// accumulators, which these tiles have once (8192 x 24576, K 4096: 1365 in two launches, 1441 in one).
+int ob_gemm_relu_sq(const void* X, const void* W, void* C, int M, int N, int K, long long ldx, long long ldw, long long ldc,
+                    int* status, cudaStream_t stream) {
+  if (M <= 0 || N <= 0) return 0;
+  if ((ldx & 7) || (ldw & 7) || (ldc & 7)) return 6001;
+  if (((uintptr_t)X | (uintptr_t)W | (uintptr_t)C) & 15) return 6002;
+  if (K <= 0) return 6005;
+  GemmArgs g = {};
+  g.M = M; g.N = N; g.K = K;
+  g.C = C; g.ldc = ldc; g.squares = 1;
+  g.status = status;
+  return launch_pair_wide(X, W, g, ldx, ldw, 0, 0, pick_gm(2 * K), 0, stream);
+}
+
 // The three products of the fused linear + cross-entropy over rows that the device counted: the first
 // n = *rows_dev - rows_off of the `rows` rows given here hold anything.
 //   kind 0  C bf16 [rows, N] = A [rows, K] B [N, K]^T, with the softmax statistics of ob_gemm_bf16_pair

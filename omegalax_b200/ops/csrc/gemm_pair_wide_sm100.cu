@@ -102,6 +102,19 @@ __device__ __forceinline__ void st_shared_v4(uint32_t addr, uint32_t a, uint32_t
   asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(a), "r"(b), "r"(c), "r"(d) : "memory");
 }
 
+// Two outputs: rounded, and squared where they are positive if asked (the product of two bf16 values, rounded once, is what the
+// rounded fp32 product is)
+__device__ __forceinline__ uint32_t wide_pair(uint32_t a, uint32_t b, bool squares) {
+  uint32_t r = pack_bf16(__uint_as_float(a), __uint_as_float(b));
+  if (squares) {
+    __nv_bfloat162 v = *reinterpret_cast<__nv_bfloat162*>(&r);
+    v = __hmax2(v, __float2bfloat162_rn(0.f));
+    v = __hmul2(v, v);
+    r = *reinterpret_cast<uint32_t*>(&v);
+  }
+  return r;
+}
+
 template <bool A_MN, bool B_MN>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kGemmThreads, 1)
 gemm_bf16_pair_wide_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
@@ -265,6 +278,7 @@ gemm_bf16_pair_wide_kernel(const __grid_constant__ CUtensorMap tmA, const __grid
         if (tma_out && p.out_mode == 0) {
           // bf16: 64 columns (128 bytes per row) per bulk tensor store
           const long long my_grow = (long long)slab_row0 + lane;
+          const bool squares = p.squares != 0;
           const bool do_ce = p.ce_stats != nullptr && my_grow < p.M;
           const int tgt = do_ce ? __ldg(p.ce_targets + my_grow) : -1;
           float ce_m = -INFINITY, ce_s = 0.f;
@@ -332,17 +346,17 @@ gemm_bf16_pair_wide_kernel(const __grid_constant__ CUtensorMap tmA, const __grid
 #pragma unroll
             for (int c = 0; c < 4; ++c)
               st_shared_v4(base + (((uint32_t)c ^ sw) << 4),
-                           pack_bf16(__uint_as_float(v0[c * 8 + 0]), __uint_as_float(v0[c * 8 + 1])),
-                           pack_bf16(__uint_as_float(v0[c * 8 + 2]), __uint_as_float(v0[c * 8 + 3])),
-                           pack_bf16(__uint_as_float(v0[c * 8 + 4]), __uint_as_float(v0[c * 8 + 5])),
-                           pack_bf16(__uint_as_float(v0[c * 8 + 6]), __uint_as_float(v0[c * 8 + 7])));
+                           wide_pair(v0[c * 8 + 0], v0[c * 8 + 1], squares),
+                           wide_pair(v0[c * 8 + 2], v0[c * 8 + 3], squares),
+                           wide_pair(v0[c * 8 + 4], v0[c * 8 + 5], squares),
+                           wide_pair(v0[c * 8 + 6], v0[c * 8 + 7], squares));
 #pragma unroll
             for (int c = 0; c < 4; ++c)
               st_shared_v4(base + (((uint32_t)(c + 4) ^ sw) << 4),
-                           pack_bf16(__uint_as_float(v1[c * 8 + 0]), __uint_as_float(v1[c * 8 + 1])),
-                           pack_bf16(__uint_as_float(v1[c * 8 + 2]), __uint_as_float(v1[c * 8 + 3])),
-                           pack_bf16(__uint_as_float(v1[c * 8 + 4]), __uint_as_float(v1[c * 8 + 5])),
-                           pack_bf16(__uint_as_float(v1[c * 8 + 6]), __uint_as_float(v1[c * 8 + 7])));
+                           wide_pair(v1[c * 8 + 0], v1[c * 8 + 1], squares),
+                           wide_pair(v1[c * 8 + 2], v1[c * 8 + 3], squares),
+                           wide_pair(v1[c * 8 + 4], v1[c * 8 + 5], squares),
+                           wide_pair(v1[c * 8 + 6], v1[c * 8 + 7], squares));
             fence_proxy_async_smem();
             __syncwarp();
             const int col0 = ti.c_col0 + cc * 64;
@@ -513,6 +527,7 @@ static int launch_wide(const void* A, const void* B, GemmArgs args, long long a_
   if (args.rows_dev == nullptr && pairs > args.total_tiles * args.k_splits) pairs = args.total_tiles * args.k_splits;
   if (pairs <= 0 || args.total_tiles <= 0) return 0;
   if (args.ce_stats != nullptr && !(tma_out && args.out_mode == 0)) return 6008;   // statistics live in the TMA bf16 epilogue
+  if (args.squares && (!tma_out || args.out_mode != 0)) return 6008;
   kern<<<2 * pairs, kGemmThreads, WideSmem::kTotal, stream>>>(tmA, tmB, tmC, args, tma_out);
   OB_CHECK_LAUNCH();
   return 0;

@@ -145,19 +145,34 @@ def gemm(a, b, *, a_mn: bool = False, b_mn: bool = False, out=None, out_dtype=bf
     return out
 
 
-def gemm_step(x, w, *, residual=None, norm=None, squares: bool = False, act: bool = False):
+def gemm_step(x, w, *, residual=None, norm=None, squares: bool = False, act: int = 0):
     """C = x w^T (+ residual) of a decode step's few rows (x [M,K], w [N,K], bf16, contiguous), with what stands beside
     the product.  ``norm`` = (weight [K], eps, sums): x passes an RMS norm first, whose sums of squares by panels of 128
-    columns are ``sums`` (M <= 32, K % 128 == 0).  ``squares``: returns (C, such sums of C) (N % 128 == 0).  ``act``: w is
-    [gate | up] (N % 128 == 0) and C = silu(gate) * up."""
+    columns are ``sums`` (M <= 32, K % 128 == 0).  ``squares``: returns (C, such sums of C) (N % 128 == 0).  ``act`` 1: w is
+    [gate | up] (N % 128 == 0) and C = silu(gate) * up; 2: C = max(., 0)^2."""
     M, K = x.shape
     N = w.shape[0]
-    out = torch.empty(M, N // 2 if act else N, dtype=bf16, device=x.device)
+    out = torch.empty(M, N // 2 if act == 1 else N, dtype=bf16, device=x.device)
     sums = torch.empty(M, N // 128, dtype=torch.float32, device=x.device) if squares else None
     weight, eps, given = (None, 0.0, None) if norm is None else norm
     _call("ob_gemm_step", x.data_ptr(), w.data_ptr(), out.data_ptr(), lib.ptr(residual), M, N, K, K, K, out.shape[1], N, lib.ptr(weight),
           lib.ptr(given), float(eps), lib.ptr(sums), int(act), lib.status_tensor(x.device).data_ptr(), lib.stream_ptr())
     return (out, sums) if squares else out
+
+
+def gemm_relu_sq(x, w, few: bool | None = None):
+    """max(x w^T, 0)^2 without the product in memory, or None where the kernels that ``gemm`` takes for these sizes do not have
+    it: few rows do, and the 512 x 256 tiles."""
+    x, w = _row_major_2d(x), _row_major_2d(w)
+    (M, K), N = x.shape, w.shape[0]
+    if K % 8 == 0 and (_use_few(M, N, K) if few is None else few):
+        return gemm_step(x, w, act=2) if x.is_contiguous() and w.is_contiguous() else None
+    if not _use_pair(M, N, K) or not lib.load().ob_gemm_relu_sq_fits(M, N, K):
+        return None
+    out = torch.empty(M, N, dtype=bf16, device=x.device)
+    _call("ob_gemm_relu_sq", x.data_ptr(), w.data_ptr(), out.data_ptr(), M, N, K, x.stride(0), w.stride(0), N,
+          lib.status_tensor(x.device).data_ptr(), lib.stream_ptr())
+    return out
 
 
 def gemm_peer_reduce(a, b, peer_ptrs, rows_per_peer: int, ldc: int, *, a_mn=False, b_mn=False, bf16_out=False,

@@ -79,6 +79,13 @@ def project(x, w, *, out_dtype=None, into=None):
     return y[:, :N] if N % 8 else y
 
 
+def project_relu_squared(x, w):
+    """max(x w^T, 0)^2 without the product in memory, or None where the kernels do not have it."""
+    if _same(x, w) or w.shape[0] % 8 or w.shape[1] % 8:
+        return None
+    return K.gemm_relu_sq(x, w, few=False if getattr(_calls, "tiles", False) else None)
+
+
 # ----------------------------------------------------------------------------------------------- row ops
 def embed_rows(ids32, table):
     """fp32 rows of ``table``; id -1 gives a zero row, any other id outside the table an error status."""

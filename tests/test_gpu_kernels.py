@@ -891,6 +891,23 @@ def test_segments_are_filled_with_zeros(M, k, E):
     assert (rows[used] == 3).all() and not rows[~used].any() and torch.equal(counts.long(), torch.bincount(idx.reshape(-1), minlength=E))
 
 
+@pytest.mark.parametrize("M,N,K,fits", [(1, 256, 64, True), (33, 136, 512, True), (100, 384, 1024, True), (300, 512, 256, False),
+                                        (2500, 15368, 256, True), (4097, 8448, 328, True), (513, 75784, 264, True)])
+def test_squared_relu_of_a_product_has_the_bits_of_both_operations(M, N, K, fits):
+    """Few rows, the 512 x 256 tiles (297 of them and more, remainders in each direction), and sizes left to two operations."""
+    from omegalax_b200.ops import kernels as Kn, lib, serving as S
+    torch.manual_seed(M)
+    x = 2 * torch.randn(M, K, device=_dev()).to(bf16)
+    w = (torch.randn(N, K, device=_dev()) * K ** -0.5).to(bf16)
+    x[0, 0] = float("inf")      # an infinity or, where w is zero, a NaN that counts as zero
+    w[3, 0] = 0.0
+    y = Kn.gemm_relu_sq(x, w, few=False if fits is False else None)
+    assert (y is not None) == fits
+    if fits:
+        assert torch.equal(y, S.relu_squared(Kn.gemm(x, w)))
+    _check(lib)
+
+
 @pytest.mark.parametrize("M,N,K", [(1, 6144, 4096), (5, 128, 128), (16, 384, 1152), (17, 256, 2048), (32, 1024, 640), (33, 768, 512),
                                    (64, 128, 1024)])
 def test_products_of_a_step_take_norm_and_activation_along(M, N, K):
