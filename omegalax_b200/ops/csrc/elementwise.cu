@@ -434,11 +434,20 @@ __device__ __forceinline__ void unpack8(uint4 q, float* v) {
 __device__ __forceinline__ uint4 pack8(const float* v) {
   return make_uint4(pack_bf16(v[0], v[1]), pack_bf16(v[2], v[3]), pack_bf16(v[4], v[5]), pack_bf16(v[6], v[7]));
 }
+// Sums over a head of products of a lane's channel pairs u (2 u, 2 u + 1 of both vectors), in the order of a warp whose 32 lanes have a pair
+// each (heads of 128): halves of the pairs' lanes first, then the pairs of a lane.  Rounding of the normed values to bf16 hangs on the
+// last bit of this sum, and a model's gradients on that; this order is the one that its tolerances were measured with.  The four pairs
+// change hands on the way, so it takes 3 + log2 L shuffles.
 template <int L>
-__device__ __forceinline__ float head_sum(float x) {
+__device__ __forceinline__ float head_sum(const float (&p)[4]) {
+  const bool high = threadIdx.x & (L / 2), odd = threadIdx.x & (L / 4);
+  const float x0 = (high ? p[2] : p[0]) + __shfl_xor_sync(0xffffffffu, high ? p[0] : p[2], L / 2);
+  const float x1 = (high ? p[3] : p[1]) + __shfl_xor_sync(0xffffffffu, high ? p[1] : p[3], L / 2);
+  float s = (odd ? x1 : x0) + __shfl_xor_sync(0xffffffffu, odd ? x0 : x1, L / 4);
 #pragma unroll
-  for (int o = 1; o < L; o <<= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
-  return x;
+  for (int o = L / 8; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+  s += __shfl_xor_sync(0xffffffffu, s, L / 2);
+  return s + __shfl_xor_sync(0xffffffffu, s, L / 4);
 }
 __device__ __forceinline__ float bf16r(float x) { return __bfloat162float(__float2bfloat16(x)); }
 // weights (1 without one) and the row's cosines and sines of a lane
@@ -485,13 +494,13 @@ qknorm_rope_fwd_vec_kernel(const bf16* __restrict__ qkv, const bf16* __restrict_
   const bf16* src = qkv + (m * ((long long)H * q_in_stride_heads + 2 * G) +
                            (is_q ? (long long)h * q_in_stride_heads : (long long)H * q_in_stride_heads + h - H)) * K;
   const bf16* w = is_q ? qw : kw;
-  float a[8], b[8], wa[8], wb[8], c[8], sn[8], ss = 0.f;
+  float a[8], b[8], wa[8], wb[8], c[8], sn[8], squares[4];
   unpack8(*reinterpret_cast<const uint4*>(src + at.a), a);
   unpack8(*reinterpret_cast<const uint4*>(src + at.b), b);
   head_factors<kOnePlus>(w, cosT, sinT, m, rot, at, wa, wb, c, sn);
 #pragma unroll
-  for (int i = 0; i < 8; ++i) ss += a[i] * a[i] + b[i] * b[i];
-  ss = head_sum<L>(ss);
+  for (int i = 0; i < 8; i += 2) squares[i / 2] = a[i] * a[i] + a[i + 1] * a[i + 1] + b[i] * b[i] + b[i + 1] * b[i + 1];
+  const float ss = head_sum<L>(squares);
   if (!live) return;
   const float rstd = w ? rsqrtf(ss / (float)K + eps) : 1.f;
 #pragma unroll
@@ -527,7 +536,7 @@ qknorm_rope_bwd_vec_kernel(const bf16* __restrict__ qkv, const bf16* __restrict_
     const int h = live ? (int)(item - m * HT) : 0;
     bf16* ddst = dqkv + (m * HT + h) * K;
     const bool is_q = h < QH, norm = live && (is_q ? h % q_in_stride_heads == 0 : h < QH + G);
-    float ss = 0.f, dot = 0.f, rstd = 1.f, a[8], b[8], n1[8], n2[8], wa[8], wb[8];
+    float squares[4] = {}, dots[4] = {}, rstd = 1.f, a[8], b[8], n1[8], n2[8], wa[8], wb[8];
     const bf16* w = is_q ? qw : kw;
     if (norm) {
       const bf16* src = qkv + (m * HT + h) * K;
@@ -540,10 +549,13 @@ qknorm_rope_bwd_vec_kernel(const bf16* __restrict__ qkv, const bf16* __restrict_
       head_factors<kOnePlus>(w, cosT, sinT, m, rot, at, wa, wb, c, sn);
 #pragma unroll
       for (int i = 0; i < 8; ++i) {      // un-rotate: gradient of the normalised, weighted values
-        ss += a[i] * a[i] + b[i] * b[i];
         n1[i] = da[i] * c[i] + db[i] * sn[i];
         n2[i] = db[i] * c[i] - da[i] * sn[i];
-        dot += n1[i] * wa[i] * a[i] + n2[i] * wb[i] * b[i];
+      }
+#pragma unroll
+      for (int i = 0; i < 8; i += 2) {
+        squares[i / 2] = a[i] * a[i] + a[i + 1] * a[i + 1] + b[i] * b[i] + b[i + 1] * b[i + 1];
+        dots[i / 2] = n1[i] * wa[i] * a[i] + n1[i + 1] * wa[i + 1] * a[i + 1] + n2[i] * wb[i] * b[i] + n2[i + 1] * wb[i + 1] * b[i + 1];
       }
     } else if (live) {
       const bf16* from = is_q ? dgate : dv;
@@ -552,8 +564,7 @@ qknorm_rope_bwd_vec_kernel(const bf16* __restrict__ qkv, const bf16* __restrict_
       *reinterpret_cast<uint4*>(ddst + at.a) = from ? *reinterpret_cast<const uint4*>(from + at.a) : zero;
       *reinterpret_cast<uint4*>(ddst + at.b) = from ? *reinterpret_cast<const uint4*>(from + at.b) : zero;
     }
-    ss = head_sum<L>(ss);
-    dot = head_sum<L>(dot);
+    const float ss = head_sum<L>(squares), dot = head_sum<L>(dots);
     if (!norm) continue;
     if (w) {
       rstd = rsqrtf(ss / (float)K + eps);

@@ -481,6 +481,29 @@ def test_qknorm_rope(Kd, rot, qs):
     assert _rel_err(qw.grad, qw_r.grad) < 3e-2 and _rel_err(kw.grad, kw_r.grad) < 3e-2
 
 
+@pytest.mark.parametrize("M,H,G", [(999, 16, 8), (5, 3, 1)])
+def test_qk_norm_sums_squares_in_the_order_of_a_warp(M, H, G):
+    """Heads of 128: the same bits as lanes of two channels of either half that exchange their sums, 16 lanes apart first.  Squares of
+    bf16 are exact in fp32, so every addition here is one rounding there."""
+    from omegalax_b200.ops import functional as Fn, lib
+    torch.manual_seed(M)
+    dev = _dev()
+    qkv = torch.randn(M, (H + 2 * G) * 128, device=dev).to(bf16)
+    ws = [(1 + 0.1 * torch.randn(128, device=dev)).to(bf16) for _ in range(2)]
+    cos, sin = torch.ones(M, 64, device=dev), torch.zeros(M, 64, device=dev)
+    got = Fn.qk_norm_rope(qkv, *ws, sin, cos, H, G, 128, eps=1e-6)[:2]
+    _check(lib)
+    x = qkv.view(M, -1, 128)[:, :H + G].float()
+    a, b = x[..., :64].unflatten(-1, (32, 2)).square(), x[..., 64:].unflatten(-1, (32, 2)).square()
+    s = ((a[..., 0] + a[..., 1]) + b[..., 0]) + b[..., 1]
+    lane = torch.arange(32, device=dev)
+    for apart in (16, 8, 4, 2, 1):
+        s = s + s[..., lane ^ apart]
+    y = x * torch.rsqrt(s[..., :1] / 128 + 1e-6)
+    for t, w, heads in zip(got, ws, (y[:, :H], y[:, H:])):
+        assert torch.equal(t, (heads * w.float()).to(bf16))
+
+
 @pytest.mark.parametrize("M,N", [(1, 8), (31, 72), (129, 64), (1000, 32), (3136, 1024), (5000, 4096)])
 def test_column_sum(M, N):
     """fp32 sums of M values of size one: M roundings of 2^-24 of the sum of sizes, one of the result; the mean's gradient."""
