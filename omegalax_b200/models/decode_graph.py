@@ -40,7 +40,7 @@ class DecodeGraph:
             # other threads go on allocating while this one records
             self.graph.capture_begin(capture_error_mode="thread_local")
             try:
-                # no kernel of a step writes weights, so each may read its own ahead of the kernel before it
+                # no kernel of a step writes parameters, so products may read theirs ahead of the kernel before them
                 lib.call("ob_overlap_launches", 1)
                 self.out = model.run_layers(batch, cache)
             finally:

@@ -35,6 +35,7 @@ struct FewArgs {
   long long ldx;
   float eps;
   int act;                 // 1: W is [gate | up], C = silu(gate) * up, N / 2 columns; 2: C = max(., 0)^2
+  int ahead;               // W may be read while the kernel before still runs
 };
 
 template <int NB>
@@ -170,10 +171,12 @@ gemm_few_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__
         tma_load_2d(sw, &tmW, &full_bar[stage], k0, n0);
         if (p.act == 1) tma_load_2d(sw + L::kABytes / 2, &tmW, &full_bar[stage], k0, p.N / 2 + n0);
       };
-      // the weights of the first stages are on their way while the kernel before, which gives X, still runs
+      // The weights of the first stages are on their way while the kernel before, which gives X, still runs: parameters, that is.
+      // Weights that the call itself made (padded, of another type) may come from that very kernel.
+      if (!p.ahead) grid_begin();
       const int ahead = min(kSt, (k_end - k_begin + BK - 1) / BK);
       for (int i = 0; i < ahead; ++i) load_w(i, k_begin + i * BK);
-      grid_begin();
+      if (p.ahead) grid_begin();
       for (int i = 0; i < ahead && !kNorm; ++i)
         tma_load_2d(smem + i * L::kStageBytes + L::kABytes, &tmX, &full_bar[i], k_begin + i * BK, m0);
       int stage = ahead == kSt ? 0 : ahead;
@@ -362,24 +365,32 @@ static int launch_few(const void* X, const void* W, FewArgs a, long long ldx, lo
 
 using namespace ob;
 
+namespace {
+constexpr int kReadAhead = 4;
+}
+
 extern "C" {
 
-// Launches of this thread that support it overlap with the kernel before them (1) or not (0).  The caller sees to it that no
-// kernel of the sequence writes what the one after it reads as weights.
+// Launches of this thread that support it overlap with the kernel before them (1) or not (0).
 int ob_overlap_launches(int on) {
   overlapped_launches() = on != 0;
   return 0;
 }
 
-// C[M,N] (+)= X[M,K] W[N,K]^T (+ bias, residual): contract of ob_gemm_bf16 with K-major operands.
+// C[M,N] (+)= X[M,K] W[N,K]^T (+ bias, residual): contract of ob_gemm_bf16 with K-major operands.  out_mode + kReadAhead: no kernel
+// of an overlapped sequence writes W.
 // splits: CTAs per column panel (at most 8, fewer where the reduction has fewer slices; 0 chooses).
 int ob_gemm_few(const void* X, const void* W, void* C, const void* residual, int M, int N, int K, long long ldx, long long ldw,
                 long long ldc, long long ldr, int out_mode, const void* bias, int splits, int* status, cudaStream_t stream) {
   if (M <= 0 || N <= 0) return 0;
+  FewArgs a = {};
+  if (out_mode & kReadAhead) {
+    a.ahead = 1;
+    out_mode -= kReadAhead;
+  }
   if (K <= 0 || out_mode < 0 || out_mode > 2) return 6005;
   if ((ldx & 7) || (ldw & 7)) return 6001;
   if ((((uintptr_t)X) & 15) || (((uintptr_t)W) & 15)) return 6002;
-  FewArgs a = {};
   a.M = M; a.N = N; a.K = K;
   a.C = C; a.ldc = ldc; a.out_mode = out_mode;
   a.residual = (const bf16*)residual; a.ldr = ldr;
@@ -399,7 +410,7 @@ int ob_gemm_few(const void* X, const void* W, void* C, const void* residual, int
 // 1440 -> 1412; a norm and its product of N 24576, 32 rows, with the activation 42.5 -> 40.0, the product alone 37.6).
 // norm_w with squares [M, K / 128] (sums of squares of X by panels of 128 columns; eps): X passes an RMS norm on its way, M <= 32.
 // squares_out [M, N / 128] or null: the same sums of C as stored.  act 1: W is [gate | up], C [M, N / 2] = silu(gate) * up of
-// the rounded products; 2: C = max(., 0)^2 of them.  Rounding and order are those of ob_rmsnorm_fwd and ob_swiglu_fwd but for the order of a sum of squares.
+// the rounded products; 2: C = max(., 0)^2 of them; + kReadAhead as above.  Rounding and order are those of ob_rmsnorm_fwd and ob_swiglu_fwd but for the order of a sum of squares.
 int ob_gemm_step(const void* X, const void* W, void* C, const void* residual, int M, int N, int K, long long ldx, long long ldw,
                  long long ldc, long long ldr, const void* norm_w, const float* squares, float eps, float* squares_out, int act,
                  int* status, cudaStream_t stream) {
@@ -408,6 +419,10 @@ int ob_gemm_step(const void* X, const void* W, void* C, const void* residual, in
   if ((ldx & 7) || (ldw & 7)) return 6001;
   if ((((uintptr_t)X) & 15) || (((uintptr_t)W) & 15)) return 6002;
   FewArgs a = {};
+  if (act & kReadAhead) {
+    a.ahead = 1;
+    act -= kReadAhead;
+  }
   a.M = M; a.N = N; a.K = K;
   a.C = C; a.ldc = ldc;
   a.residual = (const bf16*)residual; a.ldr = ldr;

@@ -105,7 +105,7 @@ inline int num_sms() {
 // launches of 2 to 30 us, and starting up, first loads and draining are a good part of each: 8 layers of 4096 channels, one sequence of
 // 4096 tokens 1323 -> 1256 us, Letitar 16 x 2048 1317 -> 1276, Difedra 64 x 1000 2510 -> 2453.
 // Off outside of a recording: in eager calls the host is what a step waits for, and there the kernels may follow
-// anything that writes their weights.
+// anything that writes their parameters.
 inline bool& overlapped_launches() {
   static thread_local bool on = false;
   return on;

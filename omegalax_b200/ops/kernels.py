@@ -80,6 +80,13 @@ def _use_few(M: int, N: int, K: int) -> bool:
     return K >= 768 and (M <= 128 or panels <= 296) and (K >= 1024 or not 74 < panels <= 148)
 
 
+def _read_ahead(w) -> int:
+    """4 where the kernel for few rows may read these weights while the kernel before it still runs (recorded steps): those that no
+    kernel of a step writes, parameters.  A tensor that the call made (padded, cast, computed by a parametrization) may come from that
+    very kernel."""
+    return 4 if isinstance(w, torch.nn.Parameter) else 0
+
+
 def gemm(a, b, *, a_mn: bool = False, b_mn: bool = False, out=None, out_dtype=bf16,
          accumulate: bool = False, residual=None, bn: int = 0, pair: bool | None = None, bias=None,
          ce=None, few: bool | None = None, splits: int = 0):
@@ -124,7 +131,7 @@ def gemm(a, b, *, a_mn: bool = False, b_mn: bool = False, out=None, out_dtype=bf
         few = bn == 0 and pair is None and ce is None and not (a_mn or b_mn) and _use_few(M, N, K)
     if few:
         _call("ob_gemm_few", a.data_ptr(), b.data_ptr(), out.data_ptr(), res_ptr, M, N, K, a.stride(0), b.stride(0), out.stride(0),
-              ldr, mode, lib.ptr(bias), splits, st.data_ptr(), lib.stream_ptr())
+              ldr, mode | _read_ahead(b), lib.ptr(bias), splits, st.data_ptr(), lib.stream_ptr())
         return out
     if pair is None:
         pair = bn == 0 and _use_pair(M, N, K, wgrad=a_mn and b_mn)
@@ -156,7 +163,7 @@ def gemm_step(x, w, *, residual=None, norm=None, squares: bool = False, act: int
     sums = torch.empty(M, N // 128, dtype=torch.float32, device=x.device) if squares else None
     weight, eps, given = (None, 0.0, None) if norm is None else norm
     _call("ob_gemm_step", x.data_ptr(), w.data_ptr(), out.data_ptr(), lib.ptr(residual), M, N, K, K, K, out.shape[1], N, lib.ptr(weight),
-          lib.ptr(given), float(eps), lib.ptr(sums), int(act), lib.status_tensor(x.device).data_ptr(), lib.stream_ptr())
+          lib.ptr(given), float(eps), lib.ptr(sums), int(act) | _read_ahead(w), lib.status_tensor(x.device).data_ptr(), lib.stream_ptr())
     return (out, sums) if squares else out
 
 

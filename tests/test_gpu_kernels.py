@@ -481,6 +481,30 @@ def test_qknorm_rope(Kd, rot, qs):
     assert _rel_err(qw.grad, qw_r.grad) < 3e-2 and _rel_err(kw.grad, kw_r.grad) < 3e-2
 
 
+def test_weights_padded_in_a_recorded_step_are_those_of_the_step():
+    """The padding kernel stands right before the product that reads what it wrote; all products of the recording take their
+    weights from one pool.  The same launches one by one give the same bits."""
+    from omegalax_b200.ops import lib, serving as S
+    torch.manual_seed(3)
+    x = torch.randn(8, 1000, device=_dev()).to(bf16)
+    ws = [torch.nn.Parameter(torch.randn(n, 1000, device=_dev()).to(bf16), requires_grad=False) for n in (60, 100, 64, 250, 60, 1028)]
+    many = [S.project(x, w) for w in ws]      # attributes of the kernels are set before the recording
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        lib.call("ob_overlap_launches", 1)
+        try:
+            many = [S.project(x, w) for w in ws]
+        finally:
+            lib.call("ob_overlap_launches", 0)
+    for _ in range(10):
+        for w in ws:
+            w.normal_()
+        graph.replay()
+        for y, w in zip(many, ws):
+            assert torch.equal(y, S.project(x, w))
+    _check(lib)
+
+
 @pytest.mark.parametrize("M,H,G", [(999, 16, 8), (5, 3, 1)])
 def test_qk_norm_sums_squares_in_the_order_of_a_warp(M, H, G):
     """Heads of 128: the same bits as lanes of two channels of either half that exchange their sums, 16 lanes apart first.  Squares of

@@ -71,3 +71,30 @@ def test_launch_module_converts_arguments_as_ctypes_does(monkeypatch):
                 seen.append((type(e), str(e)))
         assert seen[0] == seen[1], (name, args, seen)
     assert fast("ob_gemm_few", *cases[2][1]) == 6001 and fast(*[cases[3][0], *cases[3][1]]) is None and fast("ob_unknown", 1) is None
+
+
+@pytest.mark.parametrize("N,K,made", [(64, 128, False), (60, 128, True), (64, 100, True), (60, 100, True), (64, 128, True)])
+def test_products_read_ahead_what_no_kernel_of_a_step_writes(monkeypatch, N, K, made):
+    """Weights that a call pads, or that are no parameters, are read when the kernel before has ended."""
+    import torch
+
+    from omegalax_b200.ops import kernels, serving
+
+    seen = []
+    monkeypatch.setattr(kernels, "_call", lambda name, *args: seen.append((name, args)))
+    monkeypatch.setattr(lib, "status_tensor", lambda device: torch.zeros(4, dtype=torch.int32))
+    monkeypatch.setattr(lib, "stream_ptr", lambda: 0)
+    monkeypatch.setattr(serving, "_same", lambda *ts: 0)
+    x, w = torch.zeros(3, K, dtype=torch.bfloat16), torch.nn.Parameter(torch.zeros(N, K, dtype=torch.bfloat16))
+    if made and N % 8 == K % 8 == 0:
+        w = w * 2
+    with torch.no_grad():
+        serving.project(x, w)
+        serving.project(x, w, into=torch.zeros(3, N))
+        if K % 8 == 0:
+            kernels.gemm_step(x, w, act=2)
+            kernels.gemm_relu_sq(x, w)
+    flags = [args[{"ob_gemm_few": 11, "ob_gemm_step": 15}[name]] & 4 for name, args in seen]
+    # a step's product is called with the weights as they are
+    want = [0 if made else 4] * 2 + [4 if isinstance(w, torch.nn.Parameter) else 0] * (2 if K % 8 == 0 else 0)
+    assert flags == want
