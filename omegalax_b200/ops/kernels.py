@@ -174,7 +174,7 @@ def gemm_relu_sq(x, w, few: bool | None = None):
     (M, K), N = x.shape, w.shape[0]
     if K % 8 == 0 and (_use_few(M, N, K) if few is None else few):
         return gemm_step(x, w, act=2) if x.is_contiguous() and w.is_contiguous() else None
-    if not _use_pair(M, N, K) or not lib.load().ob_gemm_relu_sq_fits(M, N, K):
+    if not _use_pair(M, N, K) or not lib.ask("ob_gemm_relu_sq_fits", M, N, K):
         return None
     out = torch.empty(M, N, dtype=bf16, device=x.device)
     _call("ob_gemm_relu_sq", x.data_ptr(), w.data_ptr(), out.data_ptr(), M, N, K, x.stride(0), w.stride(0), N,

@@ -366,6 +366,14 @@ def call(name: str, *args) -> None:
         raise KernelError(f"{name} failed with code {rc}")
 
 
+def ask(name: str, *args) -> int:
+    """What a function of the library answers on the host, from the group of kernels that is loaded where it is one of them."""
+    lib = _lib if _lib is not None else load()
+    if _partial and not hasattr(lib, name):
+        lib = load()
+    return getattr(lib, name)(*args)
+
+
 def ptr(t):
     if t is None:
         return None

@@ -98,3 +98,24 @@ def test_products_read_ahead_what_no_kernel_of_a_step_writes(monkeypatch, N, K, 
     # a step's product is called with the weights as they are
     want = [0 if made else 4] * 2 + [4 if isinstance(w, torch.nn.Parameter) else 0] * (2 if K % 8 == 0 else 0)
     assert flags == want
+
+
+def test_a_group_of_kernels_answers_for_itself(monkeypatch, tmp_path):
+    """With one group loaded and no complete library, a prompt's squared ReLU asks that group which tiles fit."""
+    import torch
+
+    from omegalax_b200.ops import build, kernels
+
+    if not lib.available():
+        pytest.skip("no library")
+    assert {"gemm_pair_sm100", "gemm_pair_wide_sm100"} <= set(build.GROUPS["latent_serving"])
+    lib.load()
+    monkeypatch.setattr(lib, "_partial", True)
+    monkeypatch.setattr(lib, "LIB_PATH", tmp_path / "none.so")
+    monkeypatch.setenv("OMEGALAX_B200_NO_BUILD", "1")
+    seen = []
+    monkeypatch.setattr(kernels, "_call", lambda name, *args: seen.append(name))
+    monkeypatch.setattr(lib, "status_tensor", lambda device: torch.zeros(4, dtype=torch.int32))
+    monkeypatch.setattr(lib, "stream_ptr", lambda: 0)
+    y = kernels.gemm_relu_sq(torch.zeros(8192, 256, dtype=torch.bfloat16), torch.zeros(4864, 256, dtype=torch.bfloat16))
+    assert y.shape == (8192, 4864) and seen == ["ob_gemm_relu_sq"]
