@@ -13,6 +13,7 @@ from __future__ import annotations
 
 import hashlib
 import os
+import shlex
 import shutil
 import subprocess
 import sys
@@ -114,7 +115,8 @@ def launch_module() -> Path:
 
 
 def launch_stamp() -> Path:
-    return BUILD / "launch" / "stamp.txt"
+    """Signatures that the module of this interpreter was built for."""
+    return BUILD / "launch" / f"{launch_module().name}.txt"
 
 
 def build_launch_module(table: str, signatures: str) -> Path | None:
@@ -122,7 +124,7 @@ def build_launch_module(table: str, signatures: str) -> Path | None:
     where there is no C++ compiler or no headers of Python: the launchers are then called through ctypes."""
     out, gen = launch_module(), BUILD / "launch"
     include = sysconfig.get_paths()["include"]
-    cxx = os.environ.get("CXX") or shutil.which("g++") or shutil.which("c++")
+    cxx = shlex.split(os.environ.get("CXX", "")) or [c for c in (shutil.which("g++") or shutil.which("c++"),) if c]
     if not cxx or not os.path.exists(os.path.join(include, "Python.h")):
         return None
     gen.mkdir(parents=True, exist_ok=True)
@@ -131,13 +133,15 @@ def build_launch_module(table: str, signatures: str) -> Path | None:
     inc.mkdir(exist_ok=True)
     (inc / "table.inc").write_text(table)
     tmp = inc / out.name
-    cmd = [cxx, "-O2", "-std=c++17", "-shared", "-fPIC", f'-DSIGNATURES="{signatures}"', "-I", include, "-I", str(inc),
+    cmd = [*cxx, "-O2", "-std=c++17", "-shared", "-fPIC", f'-DSIGNATURES="{signatures}"', "-I", include, "-I", str(inc),
            str(CSRC / "launch_module.cpp"), "-o", str(tmp)]
-    res = subprocess.run(cmd, capture_output=True, text=True)
-    if res.returncode != 0:
-        raise RuntimeError(f"{cxx} failed for launch_module.cpp:\n{res.stderr}")
-    os.replace(tmp, out)
-    shutil.rmtree(inc, ignore_errors=True)
+    try:
+        res = subprocess.run(cmd, capture_output=True, text=True)
+        if res.returncode != 0:
+            raise RuntimeError(f"{' '.join(cxx)} failed for launch_module.cpp:\n{res.stderr}")
+        os.replace(tmp, out)
+    finally:
+        shutil.rmtree(inc, ignore_errors=True)
     launch_stamp().write_text(signatures)
     return out
 

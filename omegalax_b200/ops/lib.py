@@ -10,6 +10,7 @@ import ctypes
 import hashlib
 import importlib.util
 import os
+import warnings
 from ctypes import c_double, c_float, c_int, c_longlong, c_void_p
 from pathlib import Path
 
@@ -166,18 +167,23 @@ def build_launch_module() -> None:
 
 
 def _load_launch_module():
-    """The module for this interpreter and these signatures, built first where this process may; None: ctypes."""
+    """The module for this interpreter and these signatures, built first where this process may; None: ctypes, also where that
+    fails (no compiler that works, a tree that cannot be written to)."""
     from . import build as _build
 
-    if os.environ.get("OMEGALAX_B200_NO_BUILD") != "1":
-        build_launch_module()
-    path, stamp = _build.launch_module(), _build.launch_stamp()
-    state = _launch_table()[1]
-    if not (path.exists() and stamp.exists() and stamp.read_text() == state):
+    try:
+        if os.environ.get("OMEGALAX_B200_NO_BUILD") != "1":
+            build_launch_module()
+        path, stamp = _build.launch_module(), _build.launch_stamp()
+        state = _launch_table()[1]
+        if not (path.exists() and stamp.exists() and stamp.read_text() == state):
+            return None
+        spec = importlib.util.spec_from_file_location("_launch", path)
+        mod = importlib.util.module_from_spec(spec)
+        spec.loader.exec_module(mod)
+    except (OSError, RuntimeError, ImportError) as e:
+        warnings.warn(f"kernels are launched through ctypes, which costs 2 us a call: {e}", RuntimeWarning, stacklevel=2)
         return None
-    spec = importlib.util.spec_from_file_location("_launch", path)
-    mod = importlib.util.module_from_spec(spec)
-    spec.loader.exec_module(mod)
     return mod if mod.signatures == state else None
 
 

@@ -119,3 +119,43 @@ def test_a_group_of_kernels_answers_for_itself(monkeypatch, tmp_path):
     monkeypatch.setattr(lib, "stream_ptr", lambda: 0)
     y = kernels.gemm_relu_sq(torch.zeros(8192, 256, dtype=torch.bfloat16), torch.zeros(4864, 256, dtype=torch.bfloat16))
     assert y.shape == (8192, 4864) and seen == ["ob_gemm_relu_sq"]
+
+
+@pytest.mark.parametrize("trouble", ["compiler fails", "compiler is missing", "tree is read-only"])
+def test_without_the_launch_module_the_library_loads_all_the_same(monkeypatch, tmp_path, trouble):
+    """Where the module cannot be built, launchers are called through ctypes; to build it is an error only for who asks for that."""
+    from omegalax_b200.ops import build
+
+    if not lib.available():
+        pytest.skip("no library")
+    monkeypatch.delenv("OMEGALAX_B200_NO_BUILD", raising=False)
+    monkeypatch.setenv("CXX", {"compiler fails": "/bin/false", "compiler is missing": str(tmp_path / "none"), "tree is read-only": "g++"}[trouble])
+    monkeypatch.setattr(build, "launch_module", lambda: tmp_path / "_launch.so")
+    monkeypatch.setattr(build, "BUILD", tmp_path / "build")
+    if trouble == "tree is read-only":
+        (tmp_path / "build").write_text("no folder can be made here")
+    monkeypatch.setattr(lib, "_lib", None)
+    monkeypatch.setattr(lib, "_launch", None)
+    with pytest.warns(RuntimeWarning, match="ctypes"):
+        lib.load()
+    assert lib._launch is None
+    with pytest.raises(lib.KernelError, match="6001"):
+        lib.call("ob_gemm_few", None, 0, 0, None, 1, 1, 8, 7, 8, 8, 0, 0, None, 0, None, 0)
+    with pytest.raises((OSError, RuntimeError)):
+        lib.build_launch_module()
+
+
+def test_the_compiler_of_the_launch_module_may_have_arguments(monkeypatch, tmp_path):
+    import os
+    import shutil
+    import sysconfig
+
+    from omegalax_b200.ops import build
+
+    if not shutil.which("g++") or not os.path.exists(os.path.join(sysconfig.get_paths()["include"], "Python.h")):
+        pytest.skip("no C++ compiler or no headers of Python")
+    monkeypatch.setenv("CXX", "env g++")
+    monkeypatch.setattr(build, "launch_module", lambda: tmp_path / "_launch.so")
+    monkeypatch.setattr(build, "BUILD", tmp_path / "build")
+    lib.build_launch_module()
+    assert (tmp_path / "_launch.so").exists() and build.launch_stamp().read_text() == lib._launch_table()[1]
