@@ -79,12 +79,15 @@ class VisionAttention(nn.Module):
         self.proj = Linear(dim, dim, bias=True, **kw)
         self.scale = self.Kd ** -0.5
 
+    def rotates_in_kernel(self, x) -> bool:
+        return Fn.use_kernels(x) and self.Kd in (64, 128, 256)
+
     @scoped("vision_attention")
     def forward(self, x, cos, sin, cu_seqlens, max_seqlen: int):
         """``cos``, ``sin`` [N, head_dim], or their first halves (the second ones are the same)."""
         N, half = x.shape[0], self.Kd // 2
         qkv = self.qkv(x)
-        if Fn.use_kernels(qkv) and self.Kd in (64, 128, 256):
+        if self.rotates_in_kernel(qkv):
             q, k, v, _ = Fn.qk_norm_rope(qkv, None, None, sin[:, :half], cos[:, :half], self.H, self.H, self.Kd)
             o = Fn.flash_attention(q, k, v, cu_seqlens, max_seqlen, scale=self.scale, causal=False)
             return self.proj(o.reshape(N, self.H * self.Kd))
@@ -197,7 +200,7 @@ class VisionTower(nn.Module):
         x = self.patch_embed(pixel_values.to(self.pos_embed.dtype))
         x = x + self.interpolated_pos_embed(grid, dev).to(x.dtype)
         cos, sin = self.rotary(grid, dev)
-        if Fn.use_kernels(x):      # once for all blocks, for kernels that read half a head's angles
+        if all(blk.attn.rotates_in_kernel(x) for blk in self.blocks):      # once for all blocks: the kernel reads half a head's angles
             cos, sin = (t[:, :t.shape[1] // 2].contiguous() for t in (cos, sin))
         if cu_seqlens is None:
             cu_seqlens = vision_cu_seqlens(grid, dev)

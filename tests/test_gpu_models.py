@@ -313,3 +313,18 @@ def test_qwen3_vl_kernels_match_reference_ops():
     bad = [(n, float((gk[n] - gr[n]).norm() / (gr[n].norm() + 1e-6))) for n in gk if float(gr[n].norm()) > 1e-4]
     bad = [b for b in bad if b[1] > 0.2]
     assert not bad, bad[:8]
+
+
+@pytest.mark.parametrize("width", [64, 72])
+def test_vision_heads_get_the_tables_that_their_kernels_read(width):
+    """Halves of the angles for heads that rotate in a kernel, whole tables for others, which would put halves together in every block."""
+    from omegalax_b200.models.vision_common import VisionTower
+
+    torch.manual_seed(0)
+    tower = VisionTower(depth=2, hidden_size=2 * width, intermediate_size=256, num_heads=2, patch_size=4, temporal_patch_size=2, spatial_merge_size=2,
+                        in_channels=3, out_hidden_size=128, num_position_embeddings=64, device="cuda", dtype=torch.bfloat16)
+    seen = []
+    for blk in tower.blocks:
+        blk.attn.register_forward_pre_hook(lambda m, args: seen.append(args[1].shape[-1]))
+    y = tower(torch.randn(64, tower.in_features, device="cuda"), torch.tensor([[1, 8, 8]]))
+    assert seen == [width // 2 if width == 64 else width] * 2 and bool(y.isfinite().all())
