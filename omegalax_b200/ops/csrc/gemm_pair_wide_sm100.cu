@@ -54,6 +54,22 @@ struct WideWork {
   int K, num_m_blocks, total_tiles, k_splits, k_per_split;
 };
 
+// Slices of the reduction: fewest k-blocks on the longest path, where emptying a tile costs as much as
+// about eight k-blocks (512 x 256 fp32 through the TMA unit: 4 us) and a slice has at least sixteen.
+__host__ __device__ __forceinline__ void wide_slices(int tiles, int kb, int pairs, int& splits, int& k_per_split) {
+  int best = 0x7fffffff;
+  for (int s = 1; s <= 32; ++s) {
+    const int per = (kb + s - 1) / s;
+    if (s > 1 && per < 16) break;
+    const int cost = ((tiles * ((kb + per - 1) / per) + pairs - 1) / pairs) * (per + 8);
+    if (cost < best) {
+      best = cost;
+      k_per_split = per * BK;
+      splits = (kb + per - 1) / per;
+    }
+  }
+}
+
 __device__ __forceinline__ WideWork wide_work(const GemmArgs& p, int pairs) {
   WideWork w = {p.K, p.num_m_blocks, p.total_tiles, p.k_splits, p.k_per_split};
   if (p.rows_dev == nullptr) return w;
@@ -65,19 +81,7 @@ __device__ __forceinline__ WideWork wide_work(const GemmArgs& p, int pairs) {
   w.k_splits = 1;
   w.k_per_split = kb * BK;
   if (p.out_mode != 2) return w;
-  // Slices of the reduction: fewest k-blocks on the longest path, where emptying a tile costs as much as
-  // about eight k-blocks (512 x 256 fp32 through the TMA unit: 4 us) and a slice has at least sixteen.
-  int best = 0x7fffffff;
-  for (int s = 1; s <= 32; ++s) {
-    const int per = (kb + s - 1) / s;
-    if (s > 1 && per < 16) break;
-    const int cost = ((w.total_tiles * ((kb + per - 1) / per) + pairs - 1) / pairs) * (per + 8);
-    if (cost < best) {
-      best = cost;
-      w.k_per_split = per * BK;
-      w.k_splits = (kb + per - 1) / per;
-    }
-  }
+  wide_slices(w.total_tiles, kb, pairs, w.k_splits, w.k_per_split);
   return w;
 }
 
@@ -452,6 +456,53 @@ gemm_bf16_pair_wide_kernel(const __grid_constant__ CUtensorMap tmA, const __grid
 }
 
 template <bool A_MN, bool B_MN>
+static int wide_shared_memory() {
+  static bool attr_set[64] = {};
+  int dev = 0;
+  cudaGetDevice(&dev);
+  if (dev < 0 || dev >= 64) dev = 0;
+  if (!attr_set[dev]) {
+    cudaError_t ce = cudaFuncSetAttribute(gemm_bf16_pair_wide_kernel<A_MN, B_MN>, cudaFuncAttributeMaxDynamicSharedMemorySize, WideSmem::kTotal);
+    if (ce != cudaSuccess) return 4000 + (int)ce;
+    attr_set[dev] = true;
+  }
+  return 0;
+}
+
+// Clusters of two that can be resident at once (one CTA per SM), once wide_shared_memory() is done.
+template <bool A_MN, bool B_MN>
+static int wide_pairs() {
+  static int max_pairs = 0;
+  if (max_pairs == 0) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(num_sms(), 1, 1);
+    cfg.blockDim = dim3(kGemmThreads, 1, 1);
+    cfg.dynamicSmemBytes = WideSmem::kTotal;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = 2; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = 1;
+    cfg.attrs = at; cfg.numAttrs = 1;
+    int n = 0;
+    if (cudaOccupancyMaxActiveClusters(&n, gemm_bf16_pair_wide_kernel<A_MN, B_MN>, &cfg) != cudaSuccess || n <= 0) n = num_sms() / 2;
+    (void)cudaGetLastError();
+    max_pairs = n;
+  }
+  return max_pairs;
+}
+
+// Whether a counted weight gradient (A [K, M], B [K, N]) is one sum per element, whatever part of the K rows counts.
+int wide_counted_one_sum(int M, int N, int K) {
+  if (wide_shared_memory<true, true>()) return 0;
+  const int tiles = ((M + 511) / 512) * ((N + kWideBN - 1) / kWideBN), pairs = wide_pairs<true, true>();
+  for (int kb = 1; kb <= (K + BK - 1) / BK; ++kb) {
+    int splits = 1, per = 0;
+    wide_slices(tiles, kb, pairs, splits, per);
+    if (splits > 1) return 0;
+  }
+  return 1;
+}
+
+template <bool A_MN, bool B_MN>
 static int launch_wide(const void* A, const void* B, GemmArgs args, long long a_rows, long long a_cols, long long lda,
                        long long b_rows, long long b_cols, long long ldb, int gm, int forced_splits,
                        cudaStream_t stream) {
@@ -475,31 +526,8 @@ static int launch_wide(const void* A, const void* B, GemmArgs args, long long a_
     }
   }
   auto kern = gemm_bf16_pair_wide_kernel<A_MN, B_MN>;
-  static bool attr_set[64] = {};
-  int dev = 0;
-  cudaGetDevice(&dev);
-  if (dev < 0 || dev >= 64) dev = 0;
-  if (!attr_set[dev]) {
-    cudaError_t ce = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, WideSmem::kTotal);
-    if (ce != cudaSuccess) return 4000 + (int)ce;
-    attr_set[dev] = true;
-  }
-  static int max_pairs = 0;   // clusters of two that can be resident at once (one CTA per SM)
-  if (max_pairs == 0) {
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(num_sms(), 1, 1);
-    cfg.blockDim = dim3(kGemmThreads, 1, 1);
-    cfg.dynamicSmemBytes = WideSmem::kTotal;
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeClusterDimension;
-    at[0].val.clusterDim.x = 2; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = 1;
-    cfg.attrs = at; cfg.numAttrs = 1;
-    int n = 0;
-    if (cudaOccupancyMaxActiveClusters(&n, kern, &cfg) != cudaSuccess || n <= 0) n = num_sms() / 2;
-    (void)cudaGetLastError();
-    max_pairs = n;
-  }
-  int pairs = max_pairs;
+  if (int ce = wide_shared_memory<A_MN, B_MN>()) return ce;
+  int pairs = wide_pairs<A_MN, B_MN>();
   args.raster_gm = gm;
   // reduction slices (reducing output modes only): fewest that fill the last wave to 95 %
   args.k_splits = 1;

@@ -708,16 +708,16 @@ class _LinearCEFn(torch.autograd.Function):
         dw = None
         if need_grad and w.requires_grad and pg is None:
             dw = mg if mg is not None else torch.empty(V, D, dtype=torch.float32, device=dev)
-        first = dw is not None and (mg is None or first_gradient(w))      # the first chunk's product is stored, the others are added
-        if first and (D % 8 or M == 0):
-            dw.zero_()
-            first = False
         t32 = targets.to(torch.int32).contiguous()
         mk = mask.to(torch.float32).contiguous()
         fp32_stats = os.environ.get("OMEGALAX_B200_CE_STATS", "1") == "1" and h.shape[1] % 8 == 0
         counted = fp32_stats and pg is None and M >= 2560
         if counted:      # a chunk starts on a block of 64 rows, to which the gathered rows are filled up with zeros
             chunk = -(-chunk // 64) * 64
+        first = dw is not None and (mg is None or first_gradient(w))      # the first chunk's product is stored, the others are added
+        if first and (D % 8 or M == 0 or dw.data_ptr() % 16 or not K.head_gradient_is_one_sum(V, D, min(chunk, M), counted)):
+            dw.zero_()
+            first = False
         logits = torch.empty(min(chunk, M), V, dtype=bf16, device=dev)
         n_tiles = -(-V // 256)
         stats = torch.empty(min(chunk, M), n_tiles, 2, dtype=torch.float32, device=dev)

@@ -516,6 +516,12 @@ def ce_counted_grad_(logits, targets, lse, mask, grad_scale, counted):
           grad_scale.data_ptr(), counted[0].data_ptr(), counted[1], lib.stream_ptr())
 
 
+def head_gradient_is_one_sum(V: int, D: int, rows: int, counted: bool) -> bool:
+    """Whether a weight gradient of the head over so many rows is added as one sum per element.  Only then does it round the same when
+    it is stored: a sum that the kernels cut for the sake of their last wave is the more precise one."""
+    return rows < 2048 or (counted and bool(lib.ask("ob_gemm_counted_one_sum", V, D, rows)))
+
+
 def gemm_counted(kind: int, a, b, out, counted, ce=None, scale=None, accumulate: bool = True):
     """The head's products when only the first ``counted[0]`` (int32 [1] on the device) - ``counted[1]`` rows
     of ``a`` hold anything.  kind 0: out bf16 = a b^T with the statistics ``ce``; kind 1: out fp32 += a b;

@@ -38,6 +38,7 @@ _SIGS = {
     "ob_overlap_launches": [I],
     "ob_gemm_relu_sq": [P, P, P, I, I, I, L, L, L, P, P],
     "ob_gemm_relu_sq_fits": [I, I, I],
+    "ob_gemm_counted_one_sum": [I, I, I],
     "ob_gemm_step": [P, P, P, P, I, I, I, L, L, L, L, P, P, F, P, I, P, P],
     "ob_gemm_few": [P, P, P, P, I, I, I, L, L, L, L, I, P, I, P, P],
     "ob_gemm_counted_rows": [I, P, P, P, I, I, I, L, L, L, P, I, P, P, P, P, I, P, P],

@@ -505,6 +505,26 @@ def test_weights_padded_in_a_recorded_step_are_those_of_the_step():
     _check(lib)
 
 
+@pytest.mark.parametrize("M,V,D,chunk", [(8192, 18992, 1024, 8192), (2300, 18992, 1024, 2300), (3000, 4096, 1024, 1024), (1000, 4096, 1024, 1000)])
+def test_first_gradient_of_the_head_is_no_longer_sum_than_an_added_one(M, V, D, chunk):
+    """Stored over what was there, or added to zeros: the same products, in as many slices.  Adding up to eight of them in another order moves an
+    element by three roundings of 2^-24; one sum over all rows of the first size is 9e-6 from 64 bits, eight slices 3e-6."""
+    from omegalax_b200.ops import functional as Fn, lib
+    torch.manual_seed(4)
+    h = torch.randn(M, D, device=_dev()).to(bf16).requires_grad_()
+    w = torch.nn.Parameter((torch.randn(V, D, device=_dev()) * D ** -0.5).to(bf16))
+    y, mask = torch.randint(0, V, (M,), device=_dev()), torch.ones(M, device=_dev())
+    w.main_grad = torch.empty(V, D, device=_dev())
+    grads = []
+    for old in (True, False):
+        w.main_grad.fill_(3.0 if old else 0.0)
+        w.grad_is_old = old
+        Fn.linear_cross_entropy(h, w, y, mask, 1.0 / M, chunk=chunk).backward()
+        grads.append(w.main_grad.clone())
+    _check(lib)
+    assert float((grads[0] - grads[1]).norm()) <= 3 * 2.0 ** -24 * float(grads[1].norm())
+
+
 @pytest.mark.parametrize("M,H,G", [(999, 16, 8), (5, 3, 1)])
 def test_qk_norm_sums_squares_in_the_order_of_a_warp(M, H, G):
     """Heads of 128: the same bits as lanes of two channels of either half that exchange their sums, 16 lanes apart first.  Squares of
