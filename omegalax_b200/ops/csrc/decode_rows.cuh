@@ -6,7 +6,8 @@
 // tiles with the heads as rows.  Their eight spare rows carry precision instead of padding: a probability p enters as three bf16
 // terms hi + mid + lo (24 bits, all of an fp32 mantissa), hi in row r and mid in row r + 8 of one product, lo in row r of a
 // second, so a lane splits its own values and no shuffle is involved.  Queries, keys and values are bf16 in memory and enter
-// exactly; scores, maxima, sums and outputs are fp32.  (An infinite value comes out as NaN.)
+// exactly; scores, maxima, sums and outputs are fp32.  (A term that is zero makes a NaN of an infinite value, so sums that are none while
+// their denominators are numbers look at the values again.)
 //
 // In us, before and now, alone: 32 sequences of 2048 tokens, 32 heads on 8 70.9 48.0 (268 MB: 5.6 TB/s); one of 4096 13.6 11.0; 8 of
 // 4096, 32 heads on 4 34.0 19.7; 64 of 300, 16 on 8 23.4 18.1; 64 of one token, 16 on 16 9.0 6.8; Difedra's windowed
@@ -226,6 +227,19 @@ static __global__ void __launch_bounds__(32 * kWarps, 8 / kWarps) decode_rows_ke
       const float e = sm_m[w][r] == -INFINITY ? 0.f : __expf(sm_m[w][r] - mm);
       ll += sm_l[w][r] * e;
       oo += sm_o[w][r][c] * e;
+    }
+    if (oo != oo && ll == ll) {      // infinite values of one sign among this CTA's keys
+      bool up = false, down = false, none = false;
+#pragma unroll 1
+      for (int t = sp * per * kGroup; t < min(n, (sp * per + per) * kGroup); ++t) {
+        const int key = first + t;
+        const long long row = (long long)table[key / p.page_size] * p.page_size + key % p.page_size;
+        const float v = __bfloat162float(p.v[row * p.pitch + (long long)g * p.head + c]);
+        up |= v == INFINITY;
+        down |= v == -INFINITY;
+        none |= v != v;
+      }
+      if (up != down && !none) oo = up ? INFINITY : -INFINITY;
     }
     if (p.splits == 1) {
       p.out[bh * 128 + c] = __float2bfloat16(ll > 0.f ? oo / ll : 0.f);

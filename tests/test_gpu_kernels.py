@@ -899,6 +899,29 @@ def test_decode_attention_lengths(R, splits):
         torch.testing.assert_close(out[b].float(), torch.einsum("hs,shd->hd", p, vb), rtol=2.0 ** -8, atol=2.0 ** -10)
 
 
+@pytest.mark.parametrize("R,splits", [(1, 1), (8, 1), (4, 3)])
+def test_decode_attention_of_infinite_values(R, splits):
+    """A channel with infinite values of one sign is infinite, one with both, or with a NaN, is NaN; the others are what they are without."""
+    from omegalax_b200.ops import kernels as Kn, lib
+    torch.manual_seed(36)
+    G, HD, ps, lens = 2, 128, 64, [40, 200]
+    B, blocks = len(lens), 4
+    k, v = (torch.randn(B * blocks, ps, G, HD, device=_dev()).to(bf16) for _ in range(2))
+    table = torch.randperm(B * blocks, device=_dev()).to(torch.int32).view(B, blocks)
+    q = torch.randn(B, G * R, HD, device=_dev()).to(bf16)
+    n = torch.tensor(lens, device=_dev(), dtype=torch.int32)
+    run = lambda: Kn.decode_attn(q, k, v, table, n, ps, HD ** -0.5, splits=splits)  # noqa: E731
+    plain = run()
+    for key, channel, x in ((3, 5, math.inf), (39, 7, -math.inf), (0, 9, math.inf), (17, 9, -math.inf), (20, 11, math.inf), (21, 11, math.nan)):
+        v[table[:, key // ps].long(), key % ps, 1, channel] = x
+    out = run()
+    _check(lib)
+    hit = out[:, R:]
+    assert (hit[..., 5] == math.inf).all() and (hit[..., 7] == -math.inf).all() and hit[..., 9].isnan().all() and hit[..., 11].isnan().all()
+    plain[:, R:, [5, 7, 9, 11]] = out[:, R:, [5, 7, 9, 11]]
+    assert torch.equal(out.nan_to_num(), plain.nan_to_num())
+
+
 @pytest.mark.parametrize("n", [1, 511, 513, 4099, 1 << 20])
 def test_adamw_passes_over_zero_gradients(n):
     """Blocks of 128 gradients that are all zero are neither read nor cleared: the same update to the bit, and gradients end as zeros."""
