@@ -56,10 +56,9 @@ struct GdnArgs {
   float *kd, *pr;       // backward: (k k^T) D, and P as it is
   float* dstate;        // backward: [B,H,j1-j0,U,A] gradients of the chunk-end states
   const float* d_o;     // [B,T,H,U]
-  float* dr;            // [B,T,H,U]
   float* dq;            // [B,T,Hk,A]  accumulated (zero-initialised by the caller)
   float* dk;            // [B,T,Hk,A]  accumulated
-  float* dv;            // [B,T,H,U]
+  float* dv;            // [B,T,H,U]: dr between the walk and gdn_grad_kernel, which makes beta dr of it
   float* dg;            // [B,T,H]     accumulated
   float* dbeta;         // [B,T,H]     accumulated
   int B, T, H, Hk, U;   // T is a multiple of 64
@@ -599,10 +598,7 @@ __global__ void __launch_bounds__(256, 1) gdn_dstate_kernel(GdnArgs p) {
 #pragma unroll
     for (int c = 0; c < 4; ++c)
 #pragma unroll
-      for (int d = 0; d < 4; ++d) {
-        p.dr[out + c * v_pitch + 16 * d] = dr[c][d];
-        p.dv[out + c * v_pitch + 16 * d] = be[c] * dr[c][d];
-      }
+      for (int d = 0; d < 4; ++d) p.dv[out + c * v_pitch + 16 * d] = dr[c][d];
 #pragma unroll
     for (int d = 0; d < 4; ++d)
       *reinterpret_cast<float4*>(dot + (tx + 16 * d) * LDC_ + 4 * ty) =
@@ -658,7 +654,7 @@ __global__ void __launch_bounds__(256, 1) gdn_grad_kernel(GdnArgs p) {
   const long long vat = row0 * v_pitch + (long long)h * U + u0, mat = ((long long)bh * Jn + jn) * (GC * GC);
   copy_rows64(n_s, p.n + vat, v_pitch, tid);
   copy_rows64(do_s, p.d_o + vat, v_pitch, tid);
-  copy_rows64(dr_s, p.dr + vat, v_pitch, tid);
+  copy_rows64(dr_s, p.dv + vat, v_pitch, tid);
   copies_commit();
   copy_rows128(k_s, p.k + (row0 * p.Hk + hk) * GA, (long long)p.Hk * GA, tid);
   copy_rows128(St, p.states + (((long long)bh * J + j) * U + u0) * GA, GA, tid);
@@ -741,7 +737,11 @@ __global__ void __launch_bounds__(256, 1) gdn_grad_kernel(GdnArgs p) {
       const int i = 4 * ty + c;
       float s = 0.f;
 #pragma unroll
-      for (int d = 0; d < 4; ++d) s = fmaf(dr_s[i * LDC_ + tx + 16 * d], vv[c][d] - a_s[i] * w[c][d], s);
+      for (int d = 0; d < 4; ++d) {
+        const float dr = dr_s[i * LDC_ + tx + 16 * d];
+        s = fmaf(dr, vv[c][d] - a_s[i] * w[c][d], s);
+        p.dv[vat + i * v_pitch + tx + 16 * d] = beta_s[i] * dr;
+      }
       s = half_warp_sum(s);
       if (tx == 0) atomicAdd(dbeta_s + i, s);
     }
@@ -871,16 +871,16 @@ int ob_gdn_fwd(const float* q, const float* k, const float* v, const float* g, c
 }
 
 // The same ranges from the last chunk to the first.  dq, dk, dg, dbeta are accumulated into: the caller zero-fills them.  Work buffers: inv, pm,
-// kd, pr [B,H,j1-j0,64,64]; dstate [B,H,j1-j0,U,128]; dr [B,T,H,U]; carry as above.
+// kd, pr [B,H,j1-j0,64,64]; dstate [B,H,j1-j0,U,128]; carry as above.
 int ob_gdn_bwd(const float* q, const float* k, const float* v, const float* g, const float* beta, const float* n_out,
                const float* states, const float* d_o, const float* d_sfinal, float* dq, float* dk, float* dv, float* dg, float* dbeta,
-               float* ds0, float* inv, float* pm, float* kd, float* pr, float* dstate, float* dr, float* carry, int B, int T, int H,
+               float* ds0, float* inv, float* pm, float* kd, float* pr, float* dstate, float* carry, int B, int T, int H,
                int Hk, int A, int U, int j0, int j1, cudaStream_t stream) {
   if (int e = check_shape(B, T, H, Hk, A, U, j0, j1)) return e;
   GdnArgs p{};
   p.q = q; p.k = k; p.v = v; p.g = g; p.beta = beta; p.s0 = d_sfinal; p.s1 = ds0; p.carry = carry;
   p.n = const_cast<float*>(n_out); p.states = const_cast<float*>(states); p.d_o = d_o;
-  p.inv = inv; p.pm = pm; p.kd = kd; p.pr = pr; p.dstate = dstate; p.dr = dr;
+  p.inv = inv; p.pm = pm; p.kd = kd; p.pr = pr; p.dstate = dstate;
   p.dq = dq; p.dk = dk; p.dv = dv; p.dg = dg; p.dbeta = dbeta;
   p.B = B; p.T = T; p.H = H; p.Hk = Hk; p.U = U;
   p.j0 = j0; p.j1 = j1; p.first = j1 == T / GC; p.last = j0 == 0;

@@ -678,6 +678,19 @@ def _gdn_ranges(B: int, H: int, T: int, floats: int):
     return n, [(j, min(J, j + n)) for j in range(0, J, n)]
 
 
+def _gdn_work(B: int, H: int, T: int, floats: int, new):
+    """Ranges of chunks and ``new(chunks of a range)``, their work buffers: half as many chunks where the device has no room for more."""
+    n, ranges = _gdn_ranges(B, H, T, floats)
+    while True:
+        try:
+            return ranges, new(n)
+        except torch.cuda.OutOfMemoryError:
+            if n == 1:
+                raise
+            n = -(-n // 2)
+            ranges = [(j, min(T // 64, j + n)) for j in range(0, T // 64, n)]
+
+
 def gdn_fwd(q, k, v, g, beta, s0=None, save=True, want_final=False):
     """Chunked gated delta rule, fp32.  q,k [B,T,Hk,128]; v [B,T,H,U]; g,beta [B,T,H]; T % 64 == 0."""
     B, T, Hk, A = q.shape
@@ -687,9 +700,7 @@ def gdn_fwd(q, k, v, g, beta, s0=None, save=True, want_final=False):
     n_out = torch.empty_like(v) if save else None
     states = new(B, H, T // 64, U, A) if save else None
     s_final = new(B, H, A, U) if want_final else None
-    n, ranges = _gdn_ranges(B, H, T, 2 * 64 * 64)
-    work = new(2, B, H, n, 64, 64)
-    carry = new(B, H, U, A) if len(ranges) > 1 else None
+    ranges, (work, carry) = _gdn_work(B, H, T, 2 * 64 * 64, lambda n: (new(2, B, H, n, 64, 64), new(B, H, U, A) if n < T // 64 else None))
     for j0, j1 in ranges:
         _call("ob_gdn_fwd", q.data_ptr(), k.data_ptr(), v.data_ptr(), g.data_ptr(), beta.data_ptr(), lib.ptr(s0), o.data_ptr(),
               lib.ptr(n_out), lib.ptr(states), lib.ptr(s_final), work[0].data_ptr(), work[1].data_ptr(), lib.ptr(carry), B, T, H, Hk,
@@ -702,16 +713,15 @@ def gdn_bwd(q, k, v, g, beta, n_out, states, d_o, d_sfinal=None, want_ds0=False)
     H, U = v.shape[2], v.shape[3]
     new = lambda *shape: torch.empty(*shape, dtype=torch.float32, device=v.device)  # noqa: E731
     dq, dk = torch.zeros_like(q), torch.zeros_like(k)
-    dv, dr = torch.empty_like(v), torch.empty_like(v)
+    dv = torch.empty_like(v)
     dg, dbeta = torch.zeros_like(g), torch.zeros_like(beta)
     ds0 = new(B, H, A, U) if want_ds0 else None
-    n, ranges = _gdn_ranges(B, H, T, 4 * 64 * 64 + U * A)
-    work, dstate = new(4, B, H, n, 64, 64), new(B, H, n, U, A)
-    carry = new(B, H, U, A) if len(ranges) > 1 else None
+    ranges, (work, dstate, carry) = _gdn_work(B, H, T, 4 * 64 * 64 + U * A, lambda n: (
+        new(4, B, H, n, 64, 64), new(B, H, n, U, A), new(B, H, U, A) if n < T // 64 else None))
     for j0, j1 in reversed(ranges):
         _call("ob_gdn_bwd", q.data_ptr(), k.data_ptr(), v.data_ptr(), g.data_ptr(), beta.data_ptr(), n_out.data_ptr(), states.data_ptr(),
               d_o.data_ptr(), lib.ptr(d_sfinal), dq.data_ptr(), dk.data_ptr(), dv.data_ptr(), dg.data_ptr(), dbeta.data_ptr(),
-              lib.ptr(ds0), *(w.data_ptr() for w in work), dstate.data_ptr(), dr.data_ptr(), lib.ptr(carry), B, T, H, Hk, A, U, j0, j1,
+              lib.ptr(ds0), *(w.data_ptr() for w in work), dstate.data_ptr(), lib.ptr(carry), B, T, H, Hk, A, U, j0, j1,
               lib.stream_ptr())
     return dq, dk, dv, dg, dbeta, ds0
 

@@ -112,7 +112,7 @@ _SIGS = {
     "ob_gdn_rows_in_bwd": [P] * 15 + [I] * 6 + [F, F, P],
     "ob_gdn_rows_cast": [P, P, I, I, I, I, I, P],
     "ob_gdn_fwd": [P] * 13 + [I] * 8 + [P],
-    "ob_gdn_bwd": [P] * 22 + [I] * 8 + [P],
+    "ob_gdn_bwd": [P] * 21 + [I] * 8 + [P],
     "ob_conv1d_silu_fwd": [P, P, P, I, I, I, I, P],
     "ob_conv1d_silu_bwd": [P, P, P, P, P, I, I, I, I, P],
     "ob_rmsnorm_fwd": [P, P, P, P, L, I, F, I, P],

@@ -1301,6 +1301,46 @@ def test_gated_delta_rule_in_ranges_of_chunks(monkeypatch, B, H, Hk, U, J, n):
         assert torch.equal(a, b) if i in (0, 1, 2, 3, 6, 9) else _rel_err(a, b) < 1e-5, i
 
 
+def test_gated_delta_rule_takes_the_memory_that_is_there(monkeypatch):
+    """Where the device has no room for the work buffers of all chunks, fewer chunks go at a time, and the backward pass holds no more than them
+    beside its results: the same bits, sums by atomics to 1e-5.  Without room for a single chunk the error is the allocator's."""
+    from omegalax_b200.ops import kernels as Kn, lib
+    torch.manual_seed(46)
+    B, H, Hk, U, J = 1, 4, 2, 64, 16
+    T = 64 * J
+    unit = lambda *s: torch.nn.functional.normalize(torch.randn(*s, device=_dev()), dim=-1)  # noqa: E731
+    q, k, v = unit(B, T, Hk, 128) * 128 ** -0.5, unit(B, T, Hk, 128), torch.randn(B, T, H, U, device=_dev())
+    g, beta, do = -torch.rand(B, T, H, device=_dev()), torch.rand(B, T, H, device=_dev()), torch.randn(B, T, H, U, device=_dev())
+    empty, runs, room = torch.empty, [], [1 << 40]
+
+    def bounded(*shape, **kw):
+        if math.prod(shape) > room[0]:
+            raise torch.cuda.OutOfMemoryError("no room")
+        return empty(*shape, **kw)
+
+    monkeypatch.setattr(torch, "empty", bounded)
+    for elements in (1 << 40, 4 * 4096 * 4 * H, 4 * 4096 * H):      # 16, 4 and 1 chunks of the backward pass
+        room[0] = 1 << 40
+        o, rows, states, _ = Kn.gdn_fwd(q, k, v, g, beta)
+        torch.cuda.synchronize()
+        before = torch.cuda.memory_allocated()
+        room[0] = elements
+        torch.cuda.reset_peak_memory_stats()
+        grads = Kn.gdn_bwd(q, k, v, g, beta, rows, states, do)[:5]
+        torch.cuda.synchronize()
+        results = sum(t.numel() for t in grads) * 4
+        chunks = min(J, elements // (4 * 4096 * H))
+        assert torch.cuda.max_memory_allocated() - before - results <= (chunks * (4 * 4096 + 128 * U) * H + H * U * 128) * 4 + (1 << 16)
+        runs.append((o, rows, states) + grads)
+    _check(lib)
+    for other in runs[1:]:
+        for i, (a, b) in enumerate(zip(runs[0], other)):      # o, n, states, dq, dk, dv, dg, dbeta
+            assert torch.equal(a, b) if i in (0, 1, 2, 5) else _rel_err(a, b) < 1e-5, i
+    room[0] = 1000
+    with pytest.raises(torch.cuda.OutOfMemoryError):
+        Kn.gdn_bwd(q, k, v, g, beta, rows, states, do)
+
+
 def test_gated_delta_rule_strong_decay_against_fp64_recurrence():
     """Decay rates as large as a freshly initialised model produces (|g| up to ~20 per token).
     Ground truth is the token-by-token recurrence in float64; the kernel must be about as close
