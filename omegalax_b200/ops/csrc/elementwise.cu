@@ -629,6 +629,7 @@ template <typename T>
 __global__ void __launch_bounds__(256) column_sum_kernel(const T* __restrict__ x, T* __restrict__ out, long long M, int N, float scale) {
   __shared__ float red[32][66];
   __shared__ float part[64];
+  grid_begin();
   const int ctas = gridDim.x, rank = blockIdx.x, tx = threadIdx.x & 7, ty = threadIdx.x >> 3;
   const int c = blockIdx.y * 64 + tx * 8;
   float acc[8] = {};

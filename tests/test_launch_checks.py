@@ -159,3 +159,23 @@ def test_the_compiler_of_the_launch_module_may_have_arguments(monkeypatch, tmp_p
     monkeypatch.setattr(build, "BUILD", tmp_path / "build")
     lib.build_launch_module()
     assert (tmp_path / "_launch.so").exists() and build.launch_stamp().read_text() == lib._launch_table()[1]
+
+
+def test_kernels_that_may_overlap_wait_for_the_one_before():
+    """Every kernel whose launch takes the overlap of a recorded step: one without the wait reads what is not there yet, and the ones behind it
+    no longer know that all before them have ended."""
+    import re
+
+    from omegalax_b200.ops import build
+
+    launched, bodies = set(), {}
+    for path in sorted(build.CSRC.glob("*.cu")) + sorted(build.CSRC.glob("*.cuh")):
+        text = path.read_text()
+        calls = re.findall(r"(?:OB_LAUNCH|[ =:)]launch)\(\(*(\w+)", text)
+        launched |= {c for c in calls if c.endswith("_kernel")}
+        if "kern" in calls:
+            launched |= set(re.findall(r"auto kern = (\w+)", text))
+        for m in re.finditer(r"__global__ void[^;{]*?(\w+_kernel)\(", text):
+            bodies[m[1]] = text[m.end():text.index("\n}\n", m.end())]
+    assert len(launched) > 25 and {"column_sum_kernel", "gemm_few_kernel", "decode_rows_kernel", "experts_few_kernel", "paged_decode_kernel"} <= launched
+    assert [k for k in sorted(launched) if not re.search(r"grid_(begin|wait)\(\)", bodies[k])] == []
