@@ -279,7 +279,7 @@ __global__ void __launch_bounds__(256) gdn_prep_kernel(GdnArgs p) {
   float *k_s = gsm, *q_s = gsm + kTileA;      // then the L of four heads in their place
   __shared__ float gam[4][GC], ex[4][2][GC], beta[4][GC];
   const int tid = threadIdx.x, ty = tid >> 4, tx = tid & 15;
-  const int j = p.j0 + blockIdx.x, hk = blockIdx.y, b = blockIdx.z, rep = p.H / p.Hk, Jn = p.j1 - p.j0;
+  const int rep = p.H / p.Hk, Jn = p.j1 - p.j0, jn = blockIdx.x % Jn, j = p.j0 + jn, hk = blockIdx.x / Jn % p.Hk, b = blockIdx.x / Jn / p.Hk;
   const long long row0 = (long long)b * p.T + (long long)j * GC;
   copy_rows128(k_s, p.k + (row0 * p.Hk + hk) * GA, (long long)p.Hk * GA, tid);
   copy_rows128(q_s, p.q + (row0 * p.Hk + hk) * GA, (long long)p.Hk * GA, tid);
@@ -301,7 +301,7 @@ __global__ void __launch_bounds__(256) gdn_prep_kernel(GdnArgs p) {
     __syncthreads();
     for (int w = 0; w < nh; ++w) {
       float* L = gsm + w * kTileC;
-      const long long at = (((long long)b * p.H + hk * rep + h0 + w) * Jn + blockIdx.x) * (GC * GC);
+      const long long at = (((long long)b * p.H + hk * rep + h0 + w) * Jn + jn) * (GC * GC);
 #pragma unroll
       for (int c = 0; c < 4; ++c) {
         const int i = 4 * ty + c;
@@ -337,7 +337,7 @@ __global__ void __launch_bounds__(256) gdn_prep_kernel(GdnArgs p) {
         }
         x[i] = s;
       }
-      float* out = p.inv + (((long long)b * p.H + hk * rep + h0 + w) * Jn + blockIdx.x) * (GC * GC);
+      float* out = p.inv + (((long long)b * p.H + hk * rep + h0 + w) * Jn + jn) * (GC * GC);
       if (kBwd) {
 #pragma unroll
         for (int i = 0; i < GC; i += 4) *reinterpret_cast<float4*>(out + col * GC + i) = make_float4(x[i], x[i + 1], x[i + 2], x[i + 3]);
@@ -839,7 +839,7 @@ int check_shape(int B, int T, int H, int Hk, int A, int U, int j0, int j1) {
   if (U % 64 || U <= 0) return 6102;
   if (T % GC || T <= 0) return 6103;
   if (Hk <= 0 || H % Hk) return 6104;
-  if (B <= 0 || B > 65535 || Hk > 65535) return 6105;
+  if (B <= 0) return 6105;
   if (j0 < 0 || j1 > T / GC || j0 >= j1) return 6106;
   if ((long long)B * H * (U / BU) * (j1 - j0) > 0x7fffffff) return 6105;
   return 0;
@@ -863,7 +863,7 @@ int ob_gdn_fwd(const float* q, const float* k, const float* v, const float* g, c
   if (!carry && !(p.first && p.last)) return 6106;
   OB_ENSURE_DYN_SMEM(gdn_prep_kernel<false>, kPrepSmem);
   OB_ENSURE_DYN_SMEM(gdn_fwd_kernel, kWalkSmem);
-  gdn_prep_kernel<false><<<dim3(j1 - j0, Hk, B), 256, kPrepSmem, stream>>>(p);
+  gdn_prep_kernel<false><<<B * Hk * (j1 - j0), 256, kPrepSmem, stream>>>(p);
   OB_CHECK_LAUNCH();
   gdn_fwd_kernel<<<B * H * (U / BU), 256, kWalkSmem, stream>>>(p);
   OB_CHECK_LAUNCH();
@@ -888,7 +888,7 @@ int ob_gdn_bwd(const float* q, const float* k, const float* v, const float* g, c
   OB_ENSURE_DYN_SMEM(gdn_prep_kernel<true>, kPrepSmem);
   OB_ENSURE_DYN_SMEM(gdn_dstate_kernel, kWalkSmem);
   OB_ENSURE_DYN_SMEM(gdn_grad_kernel, kGradSmem);
-  gdn_prep_kernel<true><<<dim3(j1 - j0, Hk, B), 256, kPrepSmem, stream>>>(p);
+  gdn_prep_kernel<true><<<B * Hk * (j1 - j0), 256, kPrepSmem, stream>>>(p);
   OB_CHECK_LAUNCH();
   gdn_dstate_kernel<<<B * H * (U / BU), 256, kWalkSmem, stream>>>(p);
   OB_CHECK_LAUNCH();

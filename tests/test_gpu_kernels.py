@@ -1341,6 +1341,25 @@ def test_gated_delta_rule_takes_the_memory_that_is_there(monkeypatch):
         Kn.gdn_bwd(q, k, v, g, beta, rows, states, do)
 
 
+def test_gated_delta_rule_of_many_sequences():
+    """More sequences than a grid has rows: each is what it is among few."""
+    from omegalax_b200.ops import kernels as Kn, lib
+    torch.manual_seed(47)
+    few, B = 7, 65537
+    unit = lambda *s: torch.nn.functional.normalize(torch.randn(*s, device=_dev()), dim=-1)  # noqa: E731
+    x = [unit(few, 64, 1, 128) * 128 ** -0.5, unit(few, 64, 1, 128), torch.randn(few, 64, 1, 64, device=_dev()), -torch.rand(few, 64, 1, device=_dev()),
+         torch.rand(few, 64, 1, device=_dev()), torch.randn(few, 64, 1, 64, device=_dev())]
+    outs = []
+    for n in (few, B):
+        *given, do = (t[torch.arange(n, device=_dev()) % few] for t in x)
+        o, rows, states, _ = Kn.gdn_fwd(*given)
+        outs.append((o, rows) + Kn.gdn_bwd(*given, rows, states, do)[:5])
+    _check(lib)
+    last = torch.arange(B - few, B)
+    for i, (a, b) in enumerate(zip(*outs)):
+        assert torch.equal(a[last % few], b[last]) if i in (0, 1, 4) else _rel_err(b[last], a[last % few]) < 1e-5, i
+
+
 def test_gated_delta_rule_strong_decay_against_fp64_recurrence():
     """Decay rates as large as a freshly initialised model produces (|g| up to ~20 per token).
     Ground truth is the token-by-token recurrence in float64; the kernel must be about as close
