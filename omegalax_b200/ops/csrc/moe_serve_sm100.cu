@@ -107,11 +107,11 @@ __global__ void __launch_bounds__(256) expert_rows_any_kernel(const T* __restric
 // Pairs in the order of their experts, and units: at most `cap` consecutive pairs of one expert.
 //   order [P]  pairs by expert (in any order within one: a pair's results do not depend on its place)
 //   unit [2 * max]  first place in the order, expert << 8 | pairs - 1;  count: number of units
-// One CTA; ids outside 0 ... E - 1 belong to no unit.
+// One CTA; pairs whose id is not in 0 ... E - 1 belong to no unit and add nothing: their rows of y [P, D] become zeros.
 constexpr int kPlanExperts = 8192;      // counted in shared memory; more of them in `wide` [E]
 
 __global__ void __launch_bounds__(1024) expert_units_kernel(const int* __restrict__ idx, int P, int E, int cap, int* __restrict__ order,
-                                                            int* __restrict__ unit, int* __restrict__ count, int* wide) {
+                                                            int* __restrict__ unit, int* __restrict__ count, int* wide, float* __restrict__ y, int D) {
   extern __shared__ int near[];
   __shared__ int part[2][32];
   int* hist = wide ? wide : near;      // [E] pairs, then the next free place
@@ -161,8 +161,13 @@ __global__ void __launch_bounds__(1024) expert_units_kernel(const int* __restric
     sp += n;
   }
   __syncthreads();
-  for (int i = tid; i < P; i += 1024)
-    if ((unsigned)idx[i] < (unsigned)E) order[atomicAdd(hist + idx[i], 1)] = i;
+  for (int i = tid; i < P; i += 1024) {
+    if ((unsigned)idx[i] < (unsigned)E) {
+      order[atomicAdd(hist + idx[i], 1)] = i;
+    } else {
+      for (int d = 0; d < D; ++d) y[(long long)i * D + d] = 0.f;
+    }
+  }
 }
 
 // xs[place] = h[order[place] / k]; one warp per row, D % 8 == 0.  Places past the pairs that have an expert hold no pair.
@@ -447,7 +452,8 @@ int ob_experts_few(const void* h, const int* idx, const float* weight, const voi
   if ((((uintptr_t)h) | ((uintptr_t)gate_up) | ((uintptr_t)down) | ((uintptr_t)act) | ((uintptr_t)xs)) & 15) return 6002;
   int *count = plan, *order = plan + 1, *unit = order + P;
   const bool wide = E > kPlanExperts;
-  OB_LAUNCH(expert_units_kernel, 1, 1024, wide ? 0 : E * 4, s, idx, P, E, cap, order, unit, count, wide ? unit + 2 * (size_t)P : (int*)nullptr);
+  OB_LAUNCH(expert_units_kernel, 1, 1024, wide ? 0 : E * 4, s, idx, P, E, cap, order, unit, count, wide ? unit + 2 * (size_t)P : (int*)nullptr,
+            y, D);
   OB_CHECK_LAUNCH();
   OB_LAUNCH(expert_rows_kernel, (unsigned)((P + 7) / 8), 256, 0, s, (const bf16*)h, idx, (const int*)order, (bf16*)xs, P, E, k, D);
   OB_CHECK_LAUNCH();

@@ -275,6 +275,29 @@ def test_experts_of_few_pairs(monkeypatch, cap, E, D, F):
     close(into - cu(base), want - base.double(), bf16, k=2)
 
 
+@pytest.mark.parametrize("few", [True, False])
+def test_pairs_without_an_expert_add_nothing(few):
+    """On either path; memory that came with other values in it is not read for them."""
+    M_, k, E, D, F = 40, 2, 4, 64, 32
+    h, gu, down = rnd(1, M_, D, dtype=bf16), rnd(2, E, 2 * F, D, dtype=bf16) * D ** -0.5, rnd(3, E, D, F, dtype=bf16) * F ** -0.5
+    idx = torch.arange(M_ * k, dtype=i32).view(M_, k) % E
+    idx[3, 0], idx[9, 1], idx[39, :] = -1, E, -1
+    w = torch.rand(M_, k, generator=gen(5)) * 0.9 + 0.1
+    want = torch.zeros(M_, D, dtype=torch.float64)
+    for m in range(M_):
+        for e, a in zip(idx[m].tolist(), w[m].double()):
+            if 0 <= e < E:
+                x = a * h[m].double()
+                want[m] += (O.silu(gu[e, :F].double() @ x) * (gu[e, F:].double() @ x)) @ down[e].double().t()
+    dirty = [torch.full((M_ * k, D), float("nan"), device="cuda") for _ in range(8)]
+    del dirty
+    into = torch.zeros(M_, D, device="cuda")
+    S.experts_into(cu(h), cu(w), cu(idx), cu(gu), cu(down), "silu", into, few=few)
+    done()
+    close(into, want, bf16, k=2)
+    assert not into[39].any()
+
+
 # ------------------------------------------------------------------------------------------ whole models
 MODELS = {"even": M.EVEN, "odd": M.ODD}
 ALL = pytest.mark.parametrize("name", list(MODELS))
