@@ -478,6 +478,17 @@ __device__ __forceinline__ void head_factors(const bf16* w, const float* cosT, c
   }
 }
 
+// (a, b) turned by the angle (sign 1) or back (-1) in separate products and sums, as the plain operations on heads without a norm round
+// (vision towers: a single flipped bit of a bf16 head shows in the gradients of the whole model).
+__device__ __forceinline__ void turn_apart(float* a, float* b, const float* c, const float* sn, float sign) {
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    const float x1 = a[i], x2 = b[i], s = sign * sn[i];
+    a[i] = __fsub_rn(__fmul_rn(x1, c[i]), __fmul_rn(x2, s));
+    b[i] = __fadd_rn(__fmul_rn(x2, c[i]), __fmul_rn(x1, s));
+  }
+}
+
 template <int L, bool kOnePlus>
 __global__ void __launch_bounds__(256)
 qknorm_rope_fwd_vec_kernel(const bf16* __restrict__ qkv, const bf16* __restrict__ qw, const bf16* __restrict__ kw,
@@ -502,12 +513,16 @@ qknorm_rope_fwd_vec_kernel(const bf16* __restrict__ qkv, const bf16* __restrict_
   for (int i = 0; i < 8; i += 2) squares[i / 2] = a[i] * a[i] + a[i + 1] * a[i + 1] + b[i] * b[i] + b[i + 1] * b[i + 1];
   const float ss = head_sum<L>(squares);
   if (!live) return;
-  const float rstd = w ? rsqrtf(ss / (float)K + eps) : 1.f;
+  if (w) {
+    const float rstd = rsqrtf(ss / (float)K + eps);
 #pragma unroll
-  for (int i = 0; i < 8; ++i) {
-    const float x1 = bf16r(a[i] * rstd * wa[i]), x2 = bf16r(b[i] * rstd * wb[i]);
-    a[i] = x1 * c[i] - x2 * sn[i];
-    b[i] = x2 * c[i] + x1 * sn[i];
+    for (int i = 0; i < 8; ++i) {
+      const float x1 = bf16r(a[i] * rstd * wa[i]), x2 = bf16r(b[i] * rstd * wb[i]);
+      a[i] = x1 * c[i] - x2 * sn[i];
+      b[i] = x2 * c[i] + x1 * sn[i];
+    }
+  } else {
+    turn_apart(a, b, c, sn, 1.f);
   }
   bf16* dst = is_q ? q_out + (m * H + h) * K : k_out + (m * G + (h - H)) * K;
   *reinterpret_cast<uint4*>(dst + at.a) = pack8(a);
@@ -536,7 +551,7 @@ qknorm_rope_bwd_vec_kernel(const bf16* __restrict__ qkv, const bf16* __restrict_
     const int h = live ? (int)(item - m * HT) : 0;
     bf16* ddst = dqkv + (m * HT + h) * K;
     const bool is_q = h < QH, norm = live && (is_q ? h % q_in_stride_heads == 0 : h < QH + G);
-    float squares[4] = {}, dots[4] = {}, rstd = 1.f, a[8], b[8], n1[8], n2[8], wa[8], wb[8];
+    float squares[4] = {}, dots[4] = {}, a[8], b[8], n1[8], n2[8], wa[8], wb[8];
     const bf16* w = is_q ? qw : kw;
     if (norm) {
       const bf16* src = qkv + (m * HT + h) * K;
@@ -547,10 +562,19 @@ qknorm_rope_bwd_vec_kernel(const bf16* __restrict__ qkv, const bf16* __restrict_
       unpack8(*reinterpret_cast<const uint4*>(dsrc + at.a), da);
       unpack8(*reinterpret_cast<const uint4*>(dsrc + at.b), db);
       head_factors<kOnePlus>(w, cosT, sinT, m, rot, at, wa, wb, c, sn);
+      if (w) {
 #pragma unroll
-      for (int i = 0; i < 8; ++i) {      // un-rotate: gradient of the normalised, weighted values
-        n1[i] = da[i] * c[i] + db[i] * sn[i];
-        n2[i] = db[i] * c[i] - da[i] * sn[i];
+        for (int i = 0; i < 8; ++i) {      // un-rotate: gradient of the normalised, weighted values
+          n1[i] = da[i] * c[i] + db[i] * sn[i];
+          n2[i] = db[i] * c[i] - da[i] * sn[i];
+        }
+      } else {
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+          n1[i] = da[i];
+          n2[i] = db[i];
+        }
+        turn_apart(n1, n2, c, sn, -1.f);
       }
 #pragma unroll
       for (int i = 0; i < 8; i += 2) {
@@ -567,7 +591,7 @@ qknorm_rope_bwd_vec_kernel(const bf16* __restrict__ qkv, const bf16* __restrict_
     const float ss = head_sum<L>(squares), dot = head_sum<L>(dots);
     if (!norm) continue;
     if (w) {
-      rstd = rsqrtf(ss / (float)K + eps);
+      const float rstd = rsqrtf(ss / (float)K + eps);
 #pragma unroll
       for (int i = 0; i < 8; ++i) {
         if (is_q) {
@@ -578,12 +602,12 @@ qknorm_rope_bwd_vec_kernel(const bf16* __restrict__ qkv, const bf16* __restrict_
           gk[8 + i] = fmaf(n2[i] * b[i], rstd, gk[8 + i]);
         }
       }
-    }
-    const float cc = w ? dot * rstd * rstd * rstd / (float)K : 0.f;
+      const float cc = dot * rstd * rstd * rstd / (float)K;
 #pragma unroll
-    for (int i = 0; i < 8; ++i) {
-      n1[i] = n1[i] * wa[i] * rstd - a[i] * cc;
-      n2[i] = n2[i] * wb[i] * rstd - b[i] * cc;
+      for (int i = 0; i < 8; ++i) {
+        n1[i] = n1[i] * wa[i] * rstd - a[i] * cc;
+        n2[i] = n2[i] * wb[i] * rstd - b[i] * cc;
+      }
     }
     *reinterpret_cast<uint4*>(ddst + at.a) = pack8(n1);
     *reinterpret_cast<uint4*>(ddst + at.b) = pack8(n2);

@@ -525,6 +525,28 @@ def test_first_gradient_of_the_head_is_no_longer_sum_than_an_added_one(M, V, D, 
     assert float((grads[0] - grads[1]).norm()) <= 3 * 2.0 ** -24 * float(grads[1].norm())
 
 
+@pytest.mark.parametrize("N,H,Kd", [(784, 16, 64), (37, 3, 128), (5, 2, 256)])
+def test_vision_heads_turn_as_separate_operations_round(N, H, Kd):
+    """Heads without a norm: the bits of products, sums and casts one by one, forward and backward, also beside infinite values."""
+    from omegalax_b200.models.qwen3_5.rope import apply_vision_rope
+    from omegalax_b200.ops import functional as Fn, lib
+    torch.manual_seed(N)
+    x = torch.randn(N, 3 * H * Kd, device=_dev()).to(bf16)
+    x[1, 5] = math.inf
+    a, b = x.clone().requires_grad_(), x.clone().requires_grad_()
+    angle = torch.rand(N, Kd // 2, device=_dev()) * 40
+    outs = Fn.qk_norm_rope(a, None, None, angle.sin(), angle.cos(), H, H, Kd)[:3]
+    cos, sin = torch.cat([angle.cos()] * 2, -1), torch.cat([angle.sin()] * 2, -1)
+    q, k, v = b.view(N, 3, H, Kd).unbind(1)
+    want = apply_vision_rope(q, cos, sin), apply_vision_rope(k, cos, sin), v
+    grads = [torch.randn(N, H, Kd, device=_dev()).to(bf16) for _ in range(3)]
+    torch.autograd.backward(outs, grads)
+    torch.autograd.backward(want, grads)
+    _check(lib)
+    for got, t in zip((*outs, a.grad), (*want, b.grad)):
+        assert torch.equal(got.nan_to_num(), t.nan_to_num())
+
+
 @pytest.mark.parametrize("M,H,G", [(999, 16, 8), (5, 3, 1)])
 def test_qk_norm_sums_squares_in_the_order_of_a_warp(M, H, G):
     """Heads of 128: the same bits as lanes of two channels of either half that exchange their sums, 16 lanes apart first.  Squares of
