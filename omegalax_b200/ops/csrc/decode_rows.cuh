@@ -210,10 +210,9 @@ static __global__ void __launch_bounds__(32 * kWarps, 8 / kWarps) decode_rows_ke
       *reinterpret_cast<float2*>(&sm_o[warp][hr][i * 8 + tq * 2]) = make_float2(o[i][0] + o[i][2], o[i][1] + o[i][3]);
   }
   __syncthreads();
-  for (int i = threadIdx.x; i < R * 128; i += 32 * kWarps) {
-    const int r = i >> 7, c = i & 127;
-    const long long bh = (long long)b * p.H + g * R + r;
-    float mm = -INFINITY, ll = 0.f, oo = 0.f;
+  auto merge = [&](int r, int c, float& mm, float& ll, float& oo) {
+    mm = -INFINITY;
+    ll = oo = 0.f;
     if (p.splits == 1 && p.sink) {
       mm = __bfloat162float(p.sink[g * R + r]);
       ll = 1.f;
@@ -228,25 +227,51 @@ static __global__ void __launch_bounds__(32 * kWarps, 8 / kWarps) decode_rows_ke
       ll += sm_l[w][r] * e;
       oo += sm_o[w][r][c] * e;
     }
-    if (oo != oo && ll == ll) {      // infinite values of one sign among this CTA's keys
-      bool up = false, down = false, none = false;
-#pragma unroll 1
-      for (int t = sp * per * kGroup; t < min(n, (sp * per + per) * kGroup); ++t) {
-        const int key = first + t;
-        const long long row = (long long)table[key / p.page_size] * p.page_size + key % p.page_size;
-        const float v = __bfloat162float(p.v[row * p.pitch + (long long)g * p.head + c]);
-        up |= v == INFINITY;
-        down |= v == -INFINITY;
-        none |= v != v;
-      }
-      if (up != down && !none) oo = up ? INFINITY : -INFINITY;
-    }
+  };
+  bool none = false;
+  for (int i = threadIdx.x; i < R * 128; i += 32 * kWarps) {
+    const int r = i >> 7, c = i & 127;
+    const long long bh = (long long)b * p.H + g * R + r;
+    float mm, ll, oo;
+    merge(r, c, mm, ll, oo);
+    none |= oo != oo;
     if (p.splits == 1) {
       p.out[bh * 128 + c] = __float2bfloat16(ll > 0.f ? oo / ll : 0.f);
     } else {
       const long long at = bh * p.splits + sp;
       p.part_o[at * 128 + c] = oo;
       if (c == 0) *reinterpret_cast<float2*>(p.part_ml + at * 2) = make_float2(mm, ll);
+    }
+  }
+  // Infinite values of one sign among this CTA's keys: apart from the loop above, whose iterations overlap without it (0.6 us), and with the CTA's
+  // keys worked out anew, so that nothing is kept for it through the walk.
+  if (none) {
+    unsigned cta;
+    asm volatile("mov.u32 %0, %%ctaid.x;" : "=r"(cta) : : "memory");
+    const int split = cta / p.G % p.splits, seq = cta / p.G / p.splits, end = p.len[seq];
+    const int begin = p.window > 0 ? max(0, end - p.window) : 0;
+    const int share = ((end - begin + kGroup - 1) / kGroup + p.splits - 1) / p.splits * kGroup;
+    const int* pages = p.table + (long long)seq * p.max_blocks;
+#pragma unroll 1
+    for (int i = threadIdx.x; i < R * 128; i += 32 * kWarps) {
+      const int r = i >> 7, c = i & 127;
+      const long long bh = (long long)b * p.H + g * R + r;
+      float mm, ll, oo;
+      merge(r, c, mm, ll, oo);
+      if (oo == oo || ll != ll) continue;
+      bool up = false, down = false, nan = false;
+#pragma unroll 1
+      for (int key = begin + split * share; key < min(end, begin + split * share + share); ++key) {
+        const long long row = (long long)pages[key / p.page_size] * p.page_size + key % p.page_size;
+        const float v = __bfloat162float(p.v[row * p.pitch + (long long)g * p.head + c]);
+        up |= v == INFINITY;
+        down |= v == -INFINITY;
+        nan |= v != v;
+      }
+      if (up == down || nan) continue;
+      const float x = up ? INFINITY : -INFINITY;
+      if (p.splits == 1) p.out[bh * 128 + c] = __float2bfloat16(x);
+      else p.part_o[(bh * p.splits + sp) * 128 + c] = x;
     }
   }
 }
