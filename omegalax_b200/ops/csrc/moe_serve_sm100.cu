@@ -191,7 +191,7 @@ __global__ void __launch_bounds__(256) expert_rows_kernel(const bf16* __restrict
 // input, so its scale is applied to them).  Otherwise out[pair] = fp32 rows.
 // Bound by reading the weights (128 experts of 768, width 2048, 8 per token: 1.21 GB, 184 us).  In us, whole experts with plan and sum, a
 // CTA per 16 rows that looked for its pairs before and now, 64 tokens: 255, 209 (5.8 TB/s); against padded
-// tiles, 500 tokens: 300, 239; 1000: 311, 287; 2000: 370, 443.
+// tiles, 500 tokens: 300, 239; 1000: 311, 287; 2000: 370, 443, where calls go to the tiles (64 pairs per expert are the line).
 // Roles (192 threads): warp 0 TMA, warp 1 TMEM and MMA, warps 2 ... 5 empty the accumulators.  Every wait is bounded.
 struct ExpertArgs {
   const int *unit, *count, *order;

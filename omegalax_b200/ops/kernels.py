@@ -635,7 +635,7 @@ def kv_store(k, v, rows, k_pages, v_pages):
 
 
 def decode_splits(blocks: int, keys: int) -> int:
-    """CTAs that share a sequence's keys: as many as fit at once, two on an SM, with at least 128 keys of capacity each.  In us by
+    """CTAs that share a sequence's keys: as many as fit at once (296: two on each of 148 SMs), with at least 128 keys of capacity each.  In us by
     splits, alone: 32 sequences of 2048 on 8 key heads 1 / 2 / 4: 48 54 62; one of 4096, 8 / 16 / 32 / 48: 13.8 11.3 11.8 16.2; eight of
     4096 on 4, 4 / 8 / 16: 23.8 19.9 25.1; 64 of 1000 on 4, 1 / 2: 28.9 36.6."""
     return max(1, min(32, 296 // max(blocks, 1), keys // 128))
